@@ -1,4 +1,4 @@
-"""Build libflare_b200.so (sm_100a) from csrc/ with nvcc.  Objects are cached by content hash."""
+"""Build libflare_b200.so (sm_100a) from csrc/ with nvcc and the native host layer with g++.  Objects are cached by content hash."""
 
 from __future__ import annotations
 
@@ -13,6 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build", "obj")
 LIB = os.path.join(HERE, "libflare_b200.so")
+HOST = os.path.join(HERE, "causal_flare", "_host.so")  # native host layer of the Python package (host_ext.cpp)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -89,7 +90,33 @@ def build(verbose: bool = False, jobs: int | None = None) -> str:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_host()
     return LIB
+
+
+def _build_host() -> None:
+    """The native host layer: plain C++ against torch's headers (no CUDA code in it)."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    stamp = os.path.join(OBJ, "host_ext.sha")
+    dig = _digest("host_ext.cpp", [torch.__version__])
+    if os.path.exists(HOST) and os.path.exists(stamp) and open(stamp).read() == dig:
+        return
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-isystem{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include"))),
+           os.path.join(CSRC, "host_ext.cpp"), "-o", HOST,
+           f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for host_ext.cpp:\n{res.stdout}\n{res.stderr}")
+    with open(stamp, "w") as f:
+        f.write(dig)
 
 
 if __name__ == "__main__":

@@ -84,6 +84,21 @@ EXPORTS = (
 )
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native host layer (host_ext.cpp), bound to the loaded library: serves the plain calls of the operators."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _host as native
+        except ImportError as e:
+            raise RuntimeError(f"the native host layer is missing ({e}). Build it with `python causal-flare_b200/build.py`.") from e
+        native.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in EXPORTS})
+        _host = native
+    return _host
 
 
 def load() -> C.CDLL:

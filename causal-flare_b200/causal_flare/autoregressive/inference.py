@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import torch
 
-from .. import _ops
+from .. import _lib, _ops
 from .._common import _normalize_input_precision, _refresh_profile_totals, _timed
 from .._reference_utils import resolve_flare_causal_decode_inputs
 
@@ -98,6 +98,11 @@ def flare_autoregressive_decode_triton(Q, K, V, state=None, scale=1.0, input_pre
 
     The state tensors are updated IN PLACE when the passed state is already fp32 and contiguous
     (the returned dict then shares storage with the caller's)."""
+    if K.is_cuda and state is not None and input_precision is None and attention_mask is None and Q_dec is None and \
+            K_dec is None and not profile:
+        out = _lib.host().decode(Q, K, V, state, scale)
+        if out is not None:
+            return out
     if not Q.is_cuda:
         raise RuntimeError("flare_autoregressive_decode requires CUDA tensors. ")
     K_input = K
@@ -144,6 +149,10 @@ def flare_autoregressive_prefill_triton(Q, K, V, state=None, scale=1.0, input_pr
     """Prefill T tokens on top of an optional carry-in state.  Returns ``(Y [B,T,H,Dv] in V.dtype, state)``.
 
     A token whose ``attention_mask`` entry is 0 leaves the state untouched and yields y = 0."""
+    if K.is_cuda and input_precision is None and Q_dec is None and K_dec is None and not profile:
+        out = _lib.host().prefill(Q, K, V, state, scale, attention_mask)
+        if out is not None:
+            return out
     if not Q.is_cuda:
         raise RuntimeError("flare_autoregressive_prefill requires CUDA tensors.")
     if K.dim() != 4 or V.dim() != 4:

@@ -92,5 +92,9 @@ def flare_autoregressive_stablemax_triton(Q, K, V, scale=None, eps=None, profile
         raise NotImplementedError("flare_autoregressive_stablemax_triton does not support return_state=True")
     if write_gate or write_gate_fixed_value is not None or write_gate_tensor is not None:
         raise NotImplementedError("flare_autoregressive_stablemax_triton currently implements the non-write-gated path only.")
+    if K.is_cuda and Q_dec is None and K_dec is None and chunk_size is None and input_precision is None:
+        y = _lib.host().causal(Q, K, V, scale, _lib.STABLEMAX, float(power))
+        if y is not None:
+            return y
     Q_dec_r, K_dec_r, _, _, _ = resolve_flare_causal_decode_inputs(Q, K, Q_dec, K_dec)
     return FLAREAutoregressiveStablemaxTriton.apply(Q, K, V, Q_dec_r, K_dec_r, scale, chunk_size, power, input_precision)

@@ -104,6 +104,10 @@ def flare_autoregressive_triton(Q, K, V, scale=None, chunk_size=None, input_prec
     ``chunk_size`` and ``input_precision`` are validated and otherwise unused: tiling is fixed by the
     kernels.  With ``profile=True`` returns ``(Y, timings)``; the backward section of ``timings`` is
     filled in place when the output is differentiated."""
+    if K.is_cuda and chunk_size is None and input_precision is None and not profile and Q_dec is None and K_dec is None:
+        y = _lib.host().causal(Q, K, V, scale, _lib.SOFTMAX, 2.0)
+        if y is not None:
+            return y
     return AutoRegressiveFLARE.apply(Q, K, V, scale, chunk_size, input_precision, profile, Q_dec, K_dec)
 
 

@@ -10,7 +10,7 @@ from __future__ import annotations
 
 from torch import autograd
 
-from .. import _ops
+from .. import _lib, _ops
 from .._common import _normalize_input_precision, _refresh_profile_totals, _resolve_attn_scale, _timed
 from .._reference_utils import resolve_flare_causal_decode_inputs, validate_flare_qkv_layouts
 from .reference import _validate_block_causal_config
@@ -80,4 +80,9 @@ def flare_semi_autoregressive_trition(Q, K, V, *, block_size, chunk_size, scale=
                                       profile: bool = False, Q_dec=None, K_dec=None):
     """Block-causal FLARE.  ``block_size`` (multiple of 16, divides N) and ``chunk_size`` (16/32/64/128, divides
     block_size) are both required; ``chunk_size`` does not change the result."""
+    if K.is_cuda and input_precision is None and not profile and Q_dec is None and K_dec is None and \
+            isinstance(block_size, int) and isinstance(chunk_size, int):
+        out = _lib.host().block_causal(Q, K, V, scale, block_size, chunk_size)
+        if out is not None:
+            return out[0], {"LSE_dec": out[1], "LSE_enc": out[2]}
     return SemiAutoRegressiveFLARE.apply(Q, K, V, scale, block_size, chunk_size, input_precision, profile, Q_dec, K_dec)
