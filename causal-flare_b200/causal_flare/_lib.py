@@ -56,6 +56,7 @@ class BwdArgs(C.Structure):
         ("phase", C.c_int32),
         ("y", C.c_void_p), ("y_stride_b", C.c_int64), ("y_stride_n", C.c_int64), ("y_stride_h", C.c_int64),
         ("lse_dec", C.c_void_p),
+        ("dq_dtype", C.c_int32),
     ]
 
 

@@ -80,6 +80,7 @@ namespace {
 // --------------------------------------------------------------------------------------------------
 template <int MM_MAX, int DD>
 __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) bwd_replay_kernel(const BwdParams p) {
+  pdl_begin();
   if (p.gate != nullptr && *p.gate == 0) return;
   extern __shared__ __align__(16) float smem_raw[];
   const int lane_id = blockIdx.x, dt = blockIdx.y;
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) bwd_replay_ke
 // --------------------------------------------------------------------------------------------------
 template <int MM_MAX, int DD>
 __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) bwd_reverse_kernel(const BwdParams p) {
+  pdl_begin();
   if (p.gate != nullptr && *p.gate == 0) return;
   extern __shared__ __align__(16) float smem_raw[];
   const int lane_id = blockIdx.x, dt = blockIdx.y;
@@ -655,6 +657,7 @@ constexpr int RC = 128;   // output columns per CTA (grid.z tiles wider rows)
 // Register-tiled fp32 product: 256 threads, thread (ty, tx) owns rows ty*4 .. +3 and columns tx*8 .. +7 of the
 // RT x RC output tile; per latent 6 shared-memory loads feed 32 FMAs.
 __global__ void __launch_bounds__(NT) bwd_rows_kernel(const RowsParams p) {
+  pdl_begin();
   if (p.gate != nullptr && *p.gate == 0) return;
   __shared__ __align__(16) float ds_s[RT][RM + 4];
   __shared__ __align__(16) float lat_s[RM][RC];
@@ -743,6 +746,7 @@ constexpr int LDK = 128;  // score columns per CTA
 constexpr int LT = 32;    // token rows per shared-memory stage
 
 __global__ void __launch_bounds__(NT) bwd_lat_kernel(const LatParams p) {
+  pdl_begin();
   if (p.gate != nullptr && *p.gate == 0) return;
   __shared__ __align__(16) float ds_s[LT][LM + 4];
   __shared__ __align__(16) float rw_s[LT][LDK + 4];
@@ -815,13 +819,14 @@ __global__ void __launch_bounds__(NT) bwd_lat_kernel(const LatParams p) {
 }
 
 // (5) out[i] = sum_split partial[split][i], fixed order
-__global__ void bwd_sum_splits_kernel(float* out, const float* partial, int64_t n, int splits, const int* gate) {
+__global__ void bwd_sum_splits_kernel(void* out, int out_dtype, const float* partial, int64_t n, int splits, const int* gate) {
+  pdl_begin();
   if (gate != nullptr && *gate == 0) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = 0.f;
   for (int s = 0; s < splits; ++s) acc += partial[(int64_t)s * n + i];
-  out[i] = acc;
+  store1(out, out_dtype, i, acc);
 }
 
 size_t replay_smem(int M, int Dk, int dd) {
@@ -933,16 +938,17 @@ template <int MM_MAX, int DD>
 static int launch_bwd_one(const BwdParams& p, dim3 grid, size_t smem1, size_t smem2, cudaStream_t stream, int stage) {
   if (stage == 0) {
     auto k1 = bwd_replay_kernel<MM_MAX, DD>;
-    FLARE_CUDA_CHECK(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+    static int granted[64] = {};
+    FLARE_CUDA_CHECK(allow_smem(k1, smem1, granted));
     LaunchTimer timer("bwd_replay_kernel", stream);
-    k1<<<grid, NT, smem1, stream>>>(p);
+    FLARE_CUDA_CHECK(launch_pdl(k1, grid, dim3(NT), smem1, stream, p));
   } else {
     auto k2 = bwd_reverse_kernel<MM_MAX, DD>;
-    FLARE_CUDA_CHECK(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+    static int granted[64] = {};
+    FLARE_CUDA_CHECK(allow_smem(k2, smem2, granted));
     LaunchTimer timer("bwd_reverse_kernel", stream);
-    k2<<<grid, NT, smem2, stream>>>(p);
+    FLARE_CUDA_CHECK(launch_pdl(k2, grid, dim3(NT), smem2, stream, p));
   }
-  FLARE_CUDA_CHECK(cudaGetLastError());
   return FLARE_OK;
 }
 
@@ -969,6 +975,7 @@ __global__ void __launch_bounds__(NT) bwd_seg_carry_kernel(const float* __restri
                                                            int64_t dy_stride_n, int64_t dy_stride_h, float* seg_b,
                                                            float* seg_c, float* seg_gam, int nseg, int seg_len, int N,
                                                            int H, int M, int Dv, const int* gate) {
+  pdl_begin();
   if (gate != nullptr && *gate == 0) return;
   __shared__ __align__(16) float x_s[LT][LM + 4];
   __shared__ __align__(16) float dy_s[LT][LDK + 4];
@@ -1067,6 +1074,7 @@ __global__ void __launch_bounds__(256) bwd_seg_scan_kernel(float* seg_b, float* 
                                                            const float* carry_rho, int write_slots, float* span_b0,
                                                            float* span_c0, float* span_gam, float* span_rho_first,
                                                            const int* gate) {
+  pdl_begin();
   if (gate != nullptr && *gate == 0) return;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t per_lane = (int64_t)M * (Dv + 1);  // Dv columns of b, then c
@@ -1173,11 +1181,11 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
   const int64_t nscan = lanes * f.M * (f.Dv + 1);
   auto scan = [&](bool write_slots, bool with_carry, bool summary) -> int {
     LaunchTimer timer("bwd_seg_scan_kernel", stream);
-    bwd_seg_scan_kernel<<<(unsigned)((nscan + 255) / 256), 256, 0, stream>>>(
-        p.seg_b, p.seg_c, p.seg_gam, pl.nseg, pl.seg_len, lanes, f.N, f.M, f.Dv, p.E, p.RHO, f.block_size,
-        with_carry ? a.carry_b : nullptr, with_carry ? a.carry_c : nullptr, with_carry ? a.carry_rho : nullptr,
-        write_slots ? 1 : 0, summary ? a.span_b0 : nullptr, a.span_c0, a.span_gam, a.span_rho_first, gate);
-    FLARE_CUDA_CHECK(cudaGetLastError());
+    FLARE_CUDA_CHECK(launch_pdl(bwd_seg_scan_kernel, dim3((unsigned)((nscan + 255) / 256)), dim3(256), 0, stream, p.seg_b,
+                                p.seg_c, p.seg_gam, pl.nseg, pl.seg_len, lanes, f.N, f.M, f.Dv, p.E, p.RHO, f.block_size,
+                                with_carry ? a.carry_b : nullptr, with_carry ? a.carry_c : nullptr,
+                                with_carry ? a.carry_rho : nullptr, write_slots ? 1 : 0, summary ? a.span_b0 : nullptr,
+                                a.span_c0, a.span_gam, a.span_rho_first, gate));
     return FLARE_OK;
   };
   int rcw = FLARE_OK;
@@ -1195,10 +1203,9 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
       const int mt = (f.M + LM - 1) / LM;
       dim3 g((unsigned)(lanes * mt), pl.nseg, (f.Dv + LDK - 1) / LDK);
       LaunchTimer timer("bwd_seg_carry_kernel", stream);
-      bwd_seg_carry_kernel<<<g, NT, 0, stream>>>(p.X, p.P, pl.DT, pl.plane, a.dy, f.dtype, a.dy_stride_b, a.dy_stride_n,
-                                                 a.dy_stride_h, p.seg_b, p.seg_c, p.seg_gam, pl.nseg, pl.seg_len, f.N,
-                                                 f.H, f.M, f.Dv, gate);
-      FLARE_CUDA_CHECK(cudaGetLastError());
+      FLARE_CUDA_CHECK(launch_pdl(bwd_seg_carry_kernel, g, dim3(NT), 0, stream, p.X, p.P, pl.DT, pl.plane, a.dy, f.dtype,
+                                  a.dy_stride_b, a.dy_stride_n, a.dy_stride_h, p.seg_b, p.seg_c, p.seg_gam, pl.nseg,
+                                  pl.seg_len, f.N, f.H, f.M, f.Dv, gate));
       if (a.span_b0 != nullptr) {
         rcw = scan(false, false, true);  // summary of the span for a zero carry-in from the right
         if (rcw != FLARE_OK) return rcw;
@@ -1219,8 +1226,7 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
     r.gate = gate;
     dim3 g(f.B * f.H, (f.N + RT - 1) / RT, (f.Dk + RC - 1) / RC);
     LaunchTimer timer("bwd_rows_kernel", stream);
-    bwd_rows_kernel<<<g, NT, 0, stream>>>(r);
-    FLARE_CUDA_CHECK(cudaGetLastError());
+    FLARE_CUDA_CHECK(launch_pdl(bwd_rows_kernel, g, dim3(NT), 0, stream, r));
     return FLARE_OK;
   };
   {
@@ -1252,19 +1258,19 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
   // ---- dQ (+ dK_dec): split partial sums, then a fixed-order reduction -------------------------------
   const int mt = (f.M + LM - 1) / LM, dkc = (f.Dk + LDK - 1) / LDK;
   const int64_t lat_n = (int64_t)f.H * f.M * f.Dk;
-  auto lat_launch = [&](LatParams& l, float* partial, float* out) -> int {
+  auto lat_launch = [&](LatParams& l, float* partial, void* out, int out_dtype) -> int {
     l.plane = pl.plane; l.B = f.B; l.N = f.N; l.H = f.H; l.M = f.M; l.Dk = f.Dk; l.dtype = f.dtype; l.scale = f.scale;
     l.gate = gate;
     l.rows_per_split = pl.rows_per_split; l.splits = pl.splits; l.partial = partial;
     dim3 g(f.H * mt, pl.splits, dkc);
     {
       LaunchTimer timer("bwd_lat_kernel", stream);
-      bwd_lat_kernel<<<g, NT, 0, stream>>>(l);
+      FLARE_CUDA_CHECK(launch_pdl(bwd_lat_kernel, g, dim3(NT), 0, stream, l));
     }
-    FLARE_CUDA_CHECK(cudaGetLastError());
     LaunchTimer timer("bwd_sum_splits_kernel", stream);
-    bwd_sum_splits_kernel<<<(unsigned)((lat_n + 255) / 256), 256, 0, stream>>>(out, partial, lat_n, pl.splits, gate);
-    FLARE_CUDA_CHECK(cudaGetLastError());
+    FLARE_CUDA_CHECK(launch_pdl(bwd_sum_splits_kernel, dim3((unsigned)((lat_n + 255) / 256)), dim3(256), 0, stream, out,
+                                out_dtype, partial,
+                                lat_n, pl.splits, gate));
     return FLARE_OK;
   };
   {
@@ -1278,7 +1284,7 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
       l.rows_stride_b[1] = f.qd_stride_b; l.rows_stride_n[1] = f.qd_stride_n; l.rows_stride_h[1] = f.qd_stride_h;
       l.nsrc = 2;
     }
-    int rc = lat_launch(l, reinterpret_cast<float*>(ws + pl.off_part_q), a.dq);
+    int rc = lat_launch(l, reinterpret_cast<float*>(ws + pl.off_part_q), a.dq, a.dq_dtype);
     if (rc != FLARE_OK) return rc;
   }
   if (f.k_dec != nullptr) {
@@ -1290,7 +1296,7 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
     l.rows_stride_n[0] = f.q_dec ? f.qd_stride_n : f.k_stride_n;
     l.rows_stride_h[0] = f.q_dec ? f.qd_stride_h : f.k_stride_h;
     l.nsrc = 1;
-    int rc = lat_launch(l, reinterpret_cast<float*>(ws + pl.off_part_kd), a.dk_dec);
+    int rc = lat_launch(l, reinterpret_cast<float*>(ws + pl.off_part_kd), a.dk_dec, FLARE_F32);
     if (rc != FLARE_OK) return rc;
   }
   return FLARE_OK;

@@ -155,6 +155,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   using L = BL<DVB>;
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int DV = DVB * 64;
+  pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   Misc* misc = reinterpret_cast<Misc*>(smem + L::OFF_MISC);
@@ -235,6 +236,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 #pragma unroll
         for (int vb = 0; vb < DVB; ++vb) tma_load_4d(smem + L::OFF_DY + vb * 16384, &tm_dy, &misc->dy_full, vb * 64, h, t0, b);
       }
+      pdl_trigger();
     }
   } else if (warp == W_MMA) {
     // ======================================= MMA issuer =======================================
@@ -821,10 +823,10 @@ template <int DKB, int DVB, int MODE>
 int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy, const CUtensorMap& tu,
                 const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = bwd_tc_kernel<DKB, DVB, MODE>;
-  FLARE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BL<DVB>::SMEM_BYTES));
+  static int granted[64] = {};
+  FLARE_CUDA_CHECK(allow_smem(kern, BL<DVB>::SMEM_BYTES, granted));
   LaunchTimer timer("bwd_tc_kernel", stream);
-  kern<<<grid, NT_MAIN, BL<DVB>::SMEM_BYTES, stream>>>(tk, tv, tdy, tu, p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_MAIN), BL<DVB>::SMEM_BYTES, stream, tk, tv, tdy, tu, p));
   return FLARE_OK;
 }
 
@@ -858,7 +860,16 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
                                                                   const __nv_bfloat16* __restrict__ y, int64_t y_sb,
                                                                   int64_t y_sn, int64_t y_sh, const float* __restrict__ lse,
                                                                   int B, int N, int H, int Dv, int npad, float* tok_l2,
-                                                                  float* tok_delta) {
+                                                                  float* tok_delta, const int* fwd_gate,
+                                                                  int fwd_gate_words, int* gate) {
+  pdl_begin();
+  if (blockIdx.x == 0) {
+    // this call's gate word starts as "did any CTA of the forward find its tokens outside the numeric domain"
+    int raised = 0;
+    for (int i = threadIdx.x; i < fwd_gate_words; i += 256) raised |= fwd_gate[i];
+    raised = __syncthreads_or(raised);
+    if (threadIdx.x == 0) *gate = raised ? 1 : 0;
+  }
   // Dv / 8 threads per (b, n, h) row (8 or 16, a divisor of the warp size), one 16-byte load of dY and of y each
   const int tpr = Dv >> 3;
   const int64_t row = (int64_t)blockIdx.x * (256 / tpr) + threadIdx.x / tpr;  // (b, n, h), h fastest
@@ -888,6 +899,7 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
 // sum of the latent groups' dV partials (bf16) in fp32
 __global__ void __launch_bounds__(256) bwd_tc_sum_groups_kernel(const __nv_bfloat16* __restrict__ part, int groups, int64_t n8,
                                                                  __nv_bfloat16* out) {
+  pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n8) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -901,7 +913,9 @@ __global__ void __launch_bounds__(256) bwd_tc_sum_groups_kernel(const __nv_bfloa
 }
 
 // dq[i] = sum over the (batch, split) partials in fixed order
-__global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* __restrict__ part, int count, int64_t n4, float* out) {
+__global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* __restrict__ part, int count, int64_t n4, void* out,
+                                                             int out_dtype) {
+  pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n4) return;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -909,7 +923,7 @@ __global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* __restr
     const float4 v = __ldcs(reinterpret_cast<const float4*>(part + (int64_t)s * n4 * 4) + idx);
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
-  reinterpret_cast<float4*>(out)[idx] = acc;
+  store4(out, out_dtype, idx * 4, acc.x, acc.y, acc.z, acc.w);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -942,6 +956,7 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
                     const __grid_constant__ CUtensorMap tm_q, const GradTcParams p) {
   using L = GL<DKB>;
   constexpr int DK = DKB * 64;
+  pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   const int G = p.groups;
@@ -1004,6 +1019,7 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
                         lane_id);
         }
       }
+      pdl_trigger();
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -1114,10 +1130,10 @@ int launch_grads(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMa
                  cudaStream_t stream) {
   auto kern = bwd_tc_grads_kernel<DKB>;
   const int smem = GL<DKB>::smem_bytes(p.groups);
-  FLARE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  static int granted[64] = {};
+  FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
   LaunchTimer timer("bwd_tc_grads_kernel", stream);
-  kern<<<grid, NT_GRAD, smem, stream>>>(tds, tk, tq, p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_GRAD), smem, stream, tds, tk, tq, p));
   return FLARE_OK;
 }
 
@@ -1128,7 +1144,7 @@ bool have_saved(const flare_bwd_args_t& a);  // defined below, with the keep-buf
 
 struct TcBwdPlan {
   int nch, npad, groups, nsplit, chunks_per_split;
-  size_t gate_bytes;  // per-call gate words come first
+  size_t gate_words, gate_bytes;  // the call's gate word and those of the forward's replay come first
   size_t exact_bytes;  // path AUTO: scratch of the exact pass standing by (shares the space behind the gate words)
   size_t fwd_ws;  // then the forward's own scratch
   size_t off_y, off_lse, off_l2, off_delta, off_cu, off_cc, off_cd, off_ds, off_dqp, off_dvp, total;
@@ -1158,7 +1174,8 @@ TcBwdPlan plan_tc(const flare_bwd_args_t& a) {
   probe.keep = nullptr; probe.keep_bytes = 0;
   const bool saved = have_saved(a);
   pl.fwd_ws = saved ? 0 : align_up(flare_forward_workspace_bytes(&probe), 256);
-  pl.gate_bytes = align_up((size_t)(1 + lanes) * sizeof(int), 256);
+  pl.gate_words = saved ? 1 : forward_gate_words(&probe);
+  pl.gate_bytes = align_up(pl.gate_words * sizeof(int), 256);
   size_t off = pl.gate_bytes + pl.fwd_ws;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -1213,7 +1230,8 @@ KeepLayout keep_layout(const flare_fwd_args_t& f) {
     off += align_up(bytes, 256);
     return o;
   };
-  k.off_gate = take((1 + lanes) * sizeof(int));
+  k.gate_words = forward_gate_words(&f);
+  k.off_gate = take(k.gate_words * sizeof(int));
   k.off_u = take(lanes * k.nch * f.M * f.Dv * 2);
   k.off_c = take(lanes * k.nch * f.M * 4);
   k.off_d = take(lanes * k.nch * f.M * 4);
@@ -1252,6 +1270,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
   const int64_t lanes = (int64_t)f.B * f.H;
   int* gate = reinterpret_cast<int*>(ws);
   const bool saved = have_saved(a);
+  const int* fwd_gate;
+  int fwd_gate_words;
   const void* y = nullptr;
   int64_t y_sb, y_sn, y_sh;
   const float* lse = nullptr;
@@ -1260,7 +1280,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     // (1') the training forward kept everything: its output, its log-sum-exp, the chunk states, its gate words
     const KeepLayout kl = keep_layout(f);
     char* kb = reinterpret_cast<char*>(f.keep);
-    FLARE_CUDA_CHECK(cudaMemcpyAsync(gate, kb + kl.off_gate, (size_t)(1 + lanes) * sizeof(int), cudaMemcpyDeviceToDevice, stream));
+    fwd_gate = reinterpret_cast<const int*>(kb + kl.off_gate) + 1;
+    fwd_gate_words = (int)kl.gate_words - 1;
     keep.u = kb + kl.off_u;
     keep.c = reinterpret_cast<float*>(kb + kl.off_c);
     keep.d = reinterpret_cast<float*>(kb + kl.off_d);
@@ -1268,7 +1289,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     lse = a.lse_dec;
   } else {
     // (1) forward on the tensor path: y, the decode log-sum-exp and the per-chunk prefix states
-    FLARE_CUDA_CHECK(cudaMemsetAsync(gate, 0, pl.gate_bytes, stream));
+    fwd_gate = gate + 1;
+    fwd_gate_words = (int)pl.gate_words - 1;
     keep.u = ws + pl.off_cu;
     keep.c = reinterpret_cast<float*>(ws + pl.off_cc);
     keep.d = reinterpret_cast<float*>(ws + pl.off_cd);
@@ -1294,11 +1316,10 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     const int64_t rows = (int64_t)f.B * pl.npad * f.H;
     const int rows_per_block = 256 / (f.Dv / 8);
     LaunchTimer timer("bwd_tc_token_stats_kernel", stream);
-    bwd_tc_token_stats_kernel<<<(unsigned)((rows + rows_per_block - 1) / rows_per_block), 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(a.dy), a.dy_stride_b, a.dy_stride_n, a.dy_stride_h,
-        reinterpret_cast<const __nv_bfloat16*>(y), y_sb, y_sn, y_sh, lse, f.B, f.N,
-        f.H, f.Dv, pl.npad, tok_l2, tok_delta);
-    FLARE_CUDA_CHECK(cudaGetLastError());
+    FLARE_CUDA_CHECK(launch_pdl(bwd_tc_token_stats_kernel, dim3((unsigned)((rows + rows_per_block - 1) / rows_per_block)),
+                                dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(a.dy), a.dy_stride_b, a.dy_stride_n,
+                                a.dy_stride_h, reinterpret_cast<const __nv_bfloat16*>(y), y_sb, y_sn, y_sh, lse, f.B, f.N, f.H,
+                                f.Dv, pl.npad, tok_l2, tok_delta, fwd_gate, fwd_gate_words, gate));
     count_launches(1);
   }
   int* err = nullptr;
@@ -1355,9 +1376,9 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     if (pl.groups > 1) {
       const int64_t n8 = (int64_t)f.B * f.N * f.H * f.Dv / 8;
       LaunchTimer timer("bwd_tc_sum_groups_kernel", stream);
-      bwd_tc_sum_groups_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(
-          reinterpret_cast<const __nv_bfloat16*>(ws + pl.off_dvp), pl.groups, n8, reinterpret_cast<__nv_bfloat16*>(a.dv));
-      FLARE_CUDA_CHECK(cudaGetLastError());
+      FLARE_CUDA_CHECK(launch_pdl(bwd_tc_sum_groups_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), 0, stream,
+                                  reinterpret_cast<const __nv_bfloat16*>(ws + pl.off_dvp), pl.groups, n8,
+                                  reinterpret_cast<__nv_bfloat16*>(a.dv)));
       count_launches(1);
     }
   }
@@ -1374,8 +1395,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     if (rc != FLARE_OK) return rc;
     const int64_t n4 = (int64_t)f.H * f.M * f.Dk / 4;
     LaunchTimer timer("bwd_tc_sum_dq_kernel", stream);
-    bwd_tc_sum_dq_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(g.dq_part, f.B * pl.nsplit, n4, a.dq);
-    FLARE_CUDA_CHECK(cudaGetLastError());
+    FLARE_CUDA_CHECK(launch_pdl(bwd_tc_sum_dq_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, g.dq_part,
+                                f.B * pl.nsplit, n4, a.dq, a.dq_dtype));
     count_launches(2);
   }
   // (5) path AUTO: the exact pass stands by.  Each of its kernels looks at the gate word and returns at once unless the

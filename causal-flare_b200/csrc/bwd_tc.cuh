@@ -15,6 +15,7 @@ struct ChunkStates {
 // Layout of flare_fwd_args_t::keep for a problem (all offsets in bytes; total == 0: the problem keeps nothing)
 struct KeepLayout {
   size_t off_gate, off_u, off_c, off_d, total;
+  size_t gate_words;
   int nch;
 };
 KeepLayout keep_layout(const flare_fwd_args_t& f);
@@ -26,8 +27,10 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream);
 
 // Forward on the tensor path that also writes y, the decode log-sum-exp and the per-chunk prefix states
 // (defined with the forward dispatch).
-// `gate` (may be null): per-call gate words, 1 + lanes ints, zeroed by the caller (see TcParams::gate).
+// `gate` (may be null): forward_gate_words() ints, written by the kernels from the second on (see TcParams::gate).
 int forward_keep_states(const flare_fwd_args_t* a, const ChunkStates& keep, int* gate, cudaStream_t stream);
+// gate words of a forward on the tensor path: one leading word and the CTAs' words
+size_t forward_gate_words(const flare_fwd_args_t* a);
 // diagnostic buffer set with flare_set_trace_buffer (null in normal use)
 long long* trace_buffer();
 // kernels launched so far by the current forward / backward call of this thread (measurement hook)

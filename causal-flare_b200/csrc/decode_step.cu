@@ -55,6 +55,7 @@ template <int PRE, int UNR, int MINB>
 __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParams p) {
   extern __shared__ __align__(16) float smem[];
   const int lane_id = blockIdx.x;
+  pdl_begin();
   const int b = lane_id / p.H, h = lane_id % p.H;
   const int M = p.M, Dk = p.Dk, Dv = p.Dv;
   const int tid = threadIdx.x;
@@ -192,10 +193,10 @@ bool decode_step_supported(int M, int Dk, int Dv) {
 template <int PRE, int UNR, int MINB>
 static int launch_variant(const DecodeParams& p, size_t smem, cudaStream_t stream) {
   auto kern = decode_step_kernel<PRE, UNR, MINB>;
-  if (smem > 48 * 1024) FLARE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static int granted[64] = {};
+  if (smem > 48 * 1024) FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
   LaunchTimer timer("decode_step_kernel", stream);
-  kern<<<p.B * p.H, NT, smem, stream>>>(p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(kern, dim3(p.B * p.H), dim3(NT), smem, stream, p));
   return FLARE_OK;
 }
 

@@ -137,13 +137,15 @@ struct FwdPlan {
   size_t state_floats;  // floats per state: 2M + M*Dv
   size_t ws_bytes;
   size_t part_off, part_bytes;  // tensor path with more than 128 latents: partial read-outs behind the segment states
-  // Path AUTO on the tensor kernels: per-call gate words (1 + lanes ints) that the kernels raise for tokens outside
-  // their numeric domain; the exact kernels then run for the flagged lanes only (0 bytes: no guard)
+  // Tensor kernels: gate words, gate_stride per lane behind one leading word: one for every CTA of the call's passes, set
+  // by CTAs that met tokens outside their numeric domain.  Path AUTO has them in the workspace (gate_bytes, else 0) and
+  // runs the exact kernels for the flagged lanes.
+  int gate_stride;
   size_t gate_off, gate_bytes;
 };
 
 FwdPlan plan_forward(const flare_fwd_args_t* a) {
-  FwdPlan pl{false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0};
   if (a->B == 0 || a->N == 0) return pl;
   const int64_t lanes = (int64_t)a->B * a->H;
   pl.state_floats = (size_t)2 * a->M + (size_t)a->M * a->Dv;
@@ -170,9 +172,11 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
     pl.part_off = pl.ws_bytes;
     pl.part_bytes = a->y != nullptr ? align_up(prefill_tc_partial_bytes(a), 256) : 0;
     pl.ws_bytes += pl.part_bytes;
+    pl.gate_stride = pl.nseg * prefill_tc_grid_z(a, pl.nseg);
+    if (pl.nseg > 1) pl.gate_stride += (pl.nseg - 1) * prefill_tc_grid_z(a, pl.nseg - 1);
     if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
       pl.gate_off = pl.ws_bytes;
-      pl.gate_bytes = align_up((size_t)(1 + lanes) * sizeof(int), 256);
+      pl.gate_bytes = align_up((size_t)(1 + lanes * pl.gate_stride) * sizeof(int), 256);
       pl.ws_bytes += pl.gate_bytes;
     }
     return pl;
@@ -233,6 +237,9 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
   }
   t.trace = g_trace;
   t.gate = g_gate;
+  t.gate_stride = pl.gate_stride;
+  // (the state pass over all segments but the last comes first)
+  t.gate_off = nseg_grid == pl.nseg && pl.nseg > 1 ? (pl.nseg - 1) * prefill_tc_grid_z(a, pl.nseg - 1) : 0;
   if (t.y != nullptr && g_keep.u != nullptr) {
     t.dump_u = g_keep.u; t.dump_c = g_keep.c; t.dump_d = g_keep.d; t.dump_nch = g_keep.nch;
   }
@@ -244,7 +251,7 @@ int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaSt
 // The exact kernels standing by behind a tensor-core forward: one CTA per (lane, value tile) walks the whole sequence,
 // but only for the lanes whose gate word the tensor kernels raised (inputs outside their numeric domain, e.g. score
 // spreads of several hundred nats).  For in-domain calls this launch ends at once.
-int launch_guard_walk(const flare_fwd_args_t* a, const int* lane_gates, cudaStream_t stream) {
+int launch_guard_walk(const flare_fwd_args_t* a, const int* lane_gates, int gate_stride, cudaStream_t stream) {
   WalkParams w;
   fill_walk(w, a);
   w.seg_len = a->N;
@@ -257,7 +264,7 @@ int launch_guard_walk(const flare_fwd_args_t* a, const int* lane_gates, cudaStre
   w.write_y = a->y != nullptr;
   w.lse_dec = a->lse_dec; w.lse_enc = a->lse_enc;
   w.gate = lane_gates;
-  w.gate_stride = 1;
+  w.gate_stride = w.gate_count = gate_stride;
   return launch_walk_exact(w, 1, stream);
 }
 
@@ -274,9 +281,7 @@ struct FinishCast {
 int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, FinishCast* fin = nullptr) {
   const FwdPlan pl = plan_forward(a);
   if (g_keep.u != nullptr) return forward_tensor_or_exact(a, pl, stream);  // the backward's own replay of the forward
-  const int64_t lanes = (int64_t)a->B * a->H;
   int* gate = nullptr;
-  size_t gate_bytes = 0;
   if (a->keep != nullptr) {
     // training: the chunk states and the gate words go to the caller's keep buffer
     const KeepLayout kl = keep_layout(*a);
@@ -285,20 +290,12 @@ int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, FinishCast* fin 
       return FLARE_ERR_BAD_CONFIG;
     char* kb = reinterpret_cast<char*>(a->keep);
     gate = reinterpret_cast<int*>(kb + kl.off_gate);
-    gate_bytes = (size_t)(1 + lanes) * sizeof(int);
     g_keep = ChunkStates{kb + kl.off_u, reinterpret_cast<float*>(kb + kl.off_c), reinterpret_cast<float*>(kb + kl.off_d), kl.nch};
   } else if (pl.gate_bytes > 0) {
     if (a->workspace == nullptr || a->workspace_bytes < pl.ws_bytes || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
     gate = reinterpret_cast<int*>(reinterpret_cast<char*>(a->workspace) + pl.gate_off);
-    gate_bytes = pl.gate_bytes;
   }
   if (gate == nullptr) return forward_tensor_or_exact(a, pl, stream);
-  const cudaError_t e = cudaMemsetAsync(gate, 0, gate_bytes, stream);
-  if (e != cudaSuccess) {
-    g_keep = ChunkStates{nullptr, nullptr, nullptr, 0};
-    set_cuda_error(e, "cudaMemsetAsync (gate words)");
-    return FLARE_ERR_CUDA;
-  }
   g_gate = gate;
   int rc = forward_tensor_or_exact(a, pl, stream);
   g_gate = nullptr;
@@ -314,7 +311,7 @@ int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, FinishCast* fin 
       }
       walk_args = fin->orig;
     }
-    rc = launch_guard_walk(walk_args, gate + 1, stream);
+    rc = launch_guard_walk(walk_args, gate + 1, pl.gate_stride, stream);
     g_last_launches += 1;
   }
   return rc;
@@ -470,6 +467,10 @@ int forward_keep_states(const flare_fwd_args_t* a, const ChunkStates& keep, int*
   return rc2;
 }
 
+size_t forward_gate_words(const flare_fwd_args_t* a) {
+  return 1 + (size_t)a->B * a->H * plan_forward(a).gate_stride;
+}
+
 int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, float* seg_m, float* seg_d, float* seg_u,
                           const flare_state_t* init, cudaStream_t stream, const int* gate) {
   flare_fwd_args_t a = *f;
@@ -480,7 +481,7 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
   memset(&a.state_in, 0, sizeof(a.state_in));
   memset(&a.state_out, 0, sizeof(a.state_out));
   a.state_out.m = seg_m; a.state_out.d = seg_d; a.state_out.u = seg_u;  // marks "a state is wanted" for the checks
-  FwdPlan pl{false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0};
   pl.use_tc = a.path != FLARE_PATH_EXACT && (seg_len % 128) == 0 && prefill_tc_supported(&a);
   const int64_t lanes = (int64_t)a.B * a.H;
   WalkParams w;
@@ -490,7 +491,7 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
   w.y = nullptr; w.write_y = 0;
   w.out_m = seg_m; w.out_d = seg_d; w.out_u = seg_u;
   w.out_lane_stride = nseg; w.out_seg_stride = 1; w.out_mode = 1;
-  w.gate = gate; w.gate_stride = 0;  // (a gated pass always runs on the exact kernels: its caller forces that path)
+  w.gate = gate; w.gate_stride = 0; w.gate_count = 1;  // (a gated pass always runs on the exact kernels: its caller forces that path)
   if (nseg > 1) {
     const int rc = launch_walk(&a, pl, w, nseg - 1, stream);  // local states of all segments but the last
     if (rc != FLARE_OK) return rc;
@@ -564,6 +565,7 @@ static int check_backward(const flare_bwd_args_t* args) {
   if (rc != FLARE_OK) return rc;
   if (args->fwd.B == 0 || args->fwd.N == 0) return FLARE_OK;
   if (!args->dq || !args->dk || !args->dv || !args->dy) return FLARE_ERR_BAD_POINTER;
+  if (args->dq_dtype != FLARE_F32 && args->dq_dtype != args->fwd.dtype) return FLARE_ERR_BAD_DTYPE;
   if ((args->fwd.q_dec != nullptr) != (args->dq_dec != nullptr)) return FLARE_ERR_BAD_POINTER;
   if ((args->fwd.k_dec != nullptr) != (args->dk_dec != nullptr)) return FLARE_ERR_BAD_POINTER;
   return FLARE_OK;

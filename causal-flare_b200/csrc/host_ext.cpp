@@ -246,9 +246,8 @@ struct FlareNode : public torch::autograd::Function<FlareNode> {
     fill(a.fwd, p);
     a.dy = dy.data_ptr();
     a.dy_stride_b = dy.stride(0); a.dy_stride_n = dy.stride(1); a.dy_stride_h = dy.stride(2);
-    const Tensor dq = at::empty(q0.sizes(), opts.dtype(at::kFloat));
-    const Tensor dk = at::empty(k0.sizes(), opts), dv = at::empty(v0.sizes(), opts);
-    a.dq = dq.data_ptr<float>(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
+    const Tensor dq = at::empty(q0.sizes(), opts), dk = at::empty(k0.sizes(), opts), dv = at::empty(v0.sizes(), opts);
+    a.dq = dq.data_ptr(); a.dq_dtype = a.fwd.dtype; a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
     if (saved.size() > 3) {
       const Tensor &y = saved[3], &lse = saved[4], &keep = saved[5];
       a.y = y.data_ptr();
@@ -264,7 +263,7 @@ struct FlareNode : public torch::autograd::Function<FlareNode> {
       a.fwd.workspace_bytes = need;
     }
     check(api.backward(&a, c10::cuda::getCurrentCUDAStream(k0.device().index()).stream()), "flare_backward");
-    out[0] = dq.scalar_type() == q0.scalar_type() ? dq : dq.to(q0.scalar_type());
+    out[0] = dq;
     out[1] = dk;
     out[2] = dv;
     return out;

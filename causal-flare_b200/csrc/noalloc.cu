@@ -39,7 +39,7 @@ int flare_forward_noalloc(const flare_fwd_args_t* args, flare_stream_t stream) {
     need = flare_forward_workspace_bytes(&a);
   }
   if (need > FLARE_NOALLOC_SCRATCH_BYTES) return FLARE_ERR_TOO_LARGE;
-  // What must start at zero is cleared by flare_forward itself, on the stream (the gate words of the default path);
+  // Nothing has to start at zero (the gate words of the default path are written by every CTA of the tensor kernels);
   // the segment pass writes every state slot before the scan and the output pass read it.  The rest of the previous
   // call's contents is simply overwritten.
   a.workspace = scratch;

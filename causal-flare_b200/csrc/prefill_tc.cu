@@ -114,6 +114,7 @@ struct Misc {
                                 // the partner has read the rows this CTA sent
   uint32_t tmem_base;
   volatile int abort_flag;
+  volatile int out_of_domain;  // some token of this CTA left the numeric domain
   float wmax[2][4];
   float kap[4];  // decode frame of chunk i in slot i % 4, for the token group (log-sum-exp, weight mass of a latent group)
   float xmax[2][2][128], xsum[2][2][128];  // [chunk parity][half][latent]
@@ -186,6 +187,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 OFF_B16 = L::OFF_B16, OFF_Q = L::OFF_Q, OFF_MISC = L::OFF_MISC, VB = L::VB, D_BYTES = L::D_BYTES;
   constexpr bool Q_SMEM = L::Q_SMEM;
   constexpr uint32_t TM_S = L::TM_S, TM_W = L::TM_W, TM_U = L::TM_U, TM_Y = L::TM_Y, TM_DEN = L::TM_DEN, TM_Q = L::TM_Q;
+  pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   Misc* misc = reinterpret_cast<Misc*>(smem + OFF_MISC);
@@ -228,6 +230,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_init(&misc->xfree[i], 32);
     }
     misc->abort_flag = 0;
+    misc->out_of_domain = 0;
     fence_barrier_init();
   }
   // zero the denominator operand tile once (rows 1..15 stay zero for the whole kernel)
@@ -613,10 +616,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // previous chunk): the denominators of this row leave the range in which the read-out weights are safe, see
         // the token group's check; an overflow (or a NaN) lands here as well.  Outside the numeric domain of this path.
         atomicOr(p.err, 2);
-        if (p.gate != nullptr) {
-          p.gate[0] = 1;
-          p.gate[1 + lane_id] = 1;
-        }
+        misc->out_of_domain = 1;
       }
       warp_arrive(&misc->psum[q], lane);
       // E has one buffer: the products that read the previous chunk's E and R (issued together, the state update last)
@@ -999,10 +999,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const bool den_ok = den >= 9.1e-13f && den < INFINITY;
       if (tt < nvalid && !den_ok) {
         atomicOr(p.err, 2);
-        if (p.gate != nullptr) {
-          p.gate[0] = 1;
-          p.gate[1 + lane_id] = 1;
-        }
+        misc->out_of_domain = 1;
       }
       const float inv = (SPLIT && !den_ok) ? 0.f : rcp_approx(den);  // (a true division compiles to a call here)
       if (SPLIT && !xmerge && p.part_y != nullptr && tt < nvalid && value_col0<ZS, SPLIT>() == 0)
@@ -1076,10 +1073,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // every group's weights underflowed: outside the numeric domain of this path
             if (rank == 0 && tt < nvalid) {
               atomicOr(p.err, 2);
-              if (p.gate != nullptr) {
-                p.gate[0] = 1;
-                p.gate[1 + lane_id] = 1;
-              }
+              misc->out_of_domain = 1;
             }
           } else {
             const float wa = ex2_approx(lw_own - mx), wb = ex2_approx(lw_p - mx);
@@ -1197,6 +1191,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (tid == 0 && p.gate != nullptr)
+    p.gate[1 + (int64_t)lane_id * p.gate_stride + p.gate_off + (int)(blockIdx.y * gridDim.z + blockIdx.z)] = misc->out_of_domain;
   // the partner may still write to this CTA's shared memory or arrive on its barriers until it is done as well
   if (xmerge) cluster_sync_all();
   if (warp == 12) tmem_dealloc(tmem, TM_COLS);
@@ -1210,7 +1206,8 @@ template <bool PADDED, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool W
 int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = prefill_tc_kernel<PADDED, DKB, DVB, SPLIT, MODE, KEEP, WIDE>;
-  FLARE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<DKB, WIDE>::SMEM_BYTES));
+  static int granted[64] = {};
+  FLARE_CUDA_CHECK(allow_smem(kern, Lay<DKB, WIDE>::SMEM_BYTES, granted));
   LaunchTimer timer(p.y == nullptr ? "prefill_tc_kernel (state only)" : (WIDE ? "prefill_tc_kernel (wide)" : "prefill_tc_kernel"),
                     stream);
   if (WIDE && SPLIT && p.cluster_merge) {
@@ -1220,18 +1217,19 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = Lay<DKB, WIDE>::SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 2;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 2;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     FLARE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, ty, p));
   } else {
-    kern<<<grid, NTHREADS, Lay<DKB, WIDE>::SMEM_BYTES, stream>>>(tq, tk, tv, ty, p);
+    FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NTHREADS), Lay<DKB, WIDE>::SMEM_BYTES, stream, tq, tk, tv, ty, p));
   }
-  FLARE_CUDA_CHECK(cudaGetLastError());
   return FLARE_OK;
 }
 
@@ -1327,7 +1325,9 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __re
                                                                int groups, int64_t rows /* B*N*H */, int N, int H, int dv,
                                                                __nv_bfloat16* y, int64_t y_stride_b, int64_t y_stride_n,
                                                                int64_t y_stride_h, float* lse_dec /* [B, H, N] or null */,
-                                                               const int32_t* lens /* [B] or null */, int* gate) {
+                                                               const int32_t* lens /* [B] or null */, int* gate,
+                                                               int gate_stride, int gate_off) {
+  pdl_begin();
   const int cols8 = dv >> 3;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * cols8) return;
@@ -1344,10 +1344,8 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __re
   if (mx == -INFINITY) {
     if (c8 == 0) {  // every group's weights underflowed: outside the numeric domain
       atomicOr(&g_tc_error, 2);
-      if (gate != nullptr) {
-        gate[0] = 1;
-        gate[1 + (row / ((int64_t)H * N)) * H + (row % H)] = 1;
-      }
+      // (the lane's words were written by the CTAs before this kernel: raise the first of them)
+      if (gate != nullptr) gate[1 + ((row / ((int64_t)H * N)) * H + (row % H)) * gate_stride + gate_off] = 1;
     }
   } else {
 #pragma unroll
@@ -1382,6 +1380,19 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __re
 
 int prefill_tc_latent_groups(const flare_fwd_args_t* a) { return (a->M + M - 1) / M; }
 
+// (128, 128) heads: two CTAs per (lane, group), each repeating the score / E / R work for 64 value columns, while
+// they all fit the SMs at once; beyond that the wide instance, one CTA for all 128 columns.  (Not for a padded
+// latent bank.)  FLARE_B200_WIDE=0 / 1 forces the choice.
+bool prefill_tc_wide(const flare_fwd_args_t* a, int nseg_grid) {
+  if (a->Dk != 128 || a->Dv != 128 || (a->M % M) != 0) return false;
+  if (const char* env = getenv("FLARE_B200_WIDE")) return env[0] == '1';
+  return (int64_t)a->B * a->H * nseg_grid * prefill_tc_latent_groups(a) * 2 > sm_count();
+}
+
+int prefill_tc_grid_z(const flare_fwd_args_t* a, int nseg_grid) {
+  return prefill_tc_latent_groups(a) * (prefill_tc_wide(a, nseg_grid) ? 1 : a->Dv / D);
+}
+
 int prefill_tc_ctas_per_lane(const flare_fwd_args_t* a) { return a->Dv / D * prefill_tc_latent_groups(a); }
 
 // fp16 partial read-outs [groups][B][N][H][Dv], then fp32 weight masses [groups][B][N][H]
@@ -1399,9 +1410,8 @@ size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a) {
 int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_grid, cudaStream_t stream) {
   TcParams p = p_in;
   {
-    void* err = nullptr;
-    FLARE_CUDA_CHECK(cudaGetSymbolAddress(&err, g_tc_error));  // of the current device
-    p.err = reinterpret_cast<int*>(err);
+    const int rc = tc_error_word(&p.err);
+    if (rc != FLARE_OK) return rc;
   }
   p.block = a->block_size;
   p.power = a->power;
@@ -1437,11 +1447,7 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   const int groups = prefill_tc_latent_groups(a);
   const bool padded = (a->M % M) != 0;
   const int mode = a->variant == FLARE_STABLEMAX ? 2 : (a->block_size > 1 ? 1 : 0);
-  // (128, 128) heads: two CTAs per (lane, group), each repeating the score / E / R work for 64 value columns, while
-  // they all fit the SMs at once; beyond that the wide instance, one CTA for all 128 columns.  (Not for a padded
-  // latent bank.)  FLARE_B200_WIDE=0 / 1 forces the choice.
-  bool wide = a->Dk == 128 && a->Dv == 128 && !padded && (int64_t)a->B * a->H * nseg_grid * groups * 2 > sm_count();
-  if (const char* env = getenv("FLARE_B200_WIDE")) wide = a->Dk == 128 && a->Dv == 128 && !padded && env[0] == '1';
+  const bool wide = prefill_tc_wide(a, nseg_grid);
   // Read-out rows leave through tiled bulk stores of 32 tokens x 32 columns (64-byte swizzle): into y, or with several
   // latent groups into the dense fp16 partials.  Per-row lengths (rows beyond a length stay untouched) and output
   // strides the tiled copy cannot express fall back to per-thread stores.
@@ -1472,7 +1478,7 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   }
   if (const char* env = getenv("FLARE_B200_ROW_STORES"))  // diagnostic: per-thread row stores instead
     if (env[0] == '1' && !p.cluster_merge) p.y_tma = 0;
-  const dim3 grid(a->B * a->H, nseg_grid, wide ? groups : a->Dv / D * groups);
+  const dim3 grid(a->B * a->H, nseg_grid, prefill_tc_grid_z(a, nseg_grid));
   int rc;
   const int combo = a->Dk == 128 ? 1 : (a->Dv == 128 ? 2 : 0);  // (64, 64), (128, 128), (64, 128)
   if (wide)
@@ -1491,17 +1497,25 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);
   LaunchTimer timer("tc_merge_groups_kernel", stream);
-  tc_merge_groups_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
-      reinterpret_cast<const __half*>(p.part_y), p.part_lw, groups, rows, a->N, a->H, a->Dv, reinterpret_cast<__nv_bfloat16*>(p.y), p.y_stride_b,
-      p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens, p.gate);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(tc_merge_groups_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream,
+                              reinterpret_cast<const __half*>(p.part_y), p.part_lw, groups, rows, a->N, a->H, a->Dv,
+                              reinterpret_cast<__nv_bfloat16*>(p.y), p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
+                              p.gate, p.gate_stride, p.gate_off));
   return FLARE_OK;
 }
 
 int tc_error_word(int** device_address) {
+  static int* known[64] = {};  // per device ordinal: the address does not change while the library is loaded
+  int dev = 0;
+  FLARE_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && known[dev] != nullptr) {
+    *device_address = known[dev];
+    return FLARE_OK;
+  }
   void* err = nullptr;
-  FLARE_CUDA_CHECK(cudaGetSymbolAddress(&err, g_tc_error));  // of the current device
+  FLARE_CUDA_CHECK(cudaGetSymbolAddress(&err, g_tc_error));
   *device_address = reinterpret_cast<int*>(err);
+  if (dev >= 0 && dev < 64) known[dev] = *device_address;
   return FLARE_OK;
 }
 

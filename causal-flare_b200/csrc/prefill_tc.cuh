@@ -43,9 +43,11 @@ struct TcParams {
   void* dump_u;
   float *dump_c, *dump_d;
   int dump_nch;
-  // Optional per-call gate words (in the caller's workspace, zeroed before the launch): gate[0] is raised when any
-  // token of the call left the numeric domain of these kernels, gate[1 + lane] for the (batch, head) lane it is in.
+  // Optional gate words (in the caller's workspace): CTA (lane, segment, z) writes gate[1 + lane * gate_stride + gate_off +
+  // segment * grid.z + z] when it ends, 1 if a token it handled left the numeric domain of these kernels, else 0 (so
+  // nothing has to be cleared before the launch).
   int* gate;
+  int gate_stride, gate_off;
   int* err;                  // device error word (bit 0: a wait gave up, bit 1: numeric domain exceeded)
   long long* trace;  // optional diagnostic cycle stamps of CTA (0, 0), see TC_TRACE; null in normal use
 };
@@ -57,6 +59,10 @@ int prefill_tc_ctas_per_lane(const flare_fwd_args_t* a);
 // array inside it
 size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a);
 size_t prefill_tc_partial_lw_offset(const flare_fwd_args_t* a);
+// True when a launch of nseg_grid segments takes the wide (128, 128) instance (one CTA for all 128 value columns).
+bool prefill_tc_wide(const flare_fwd_args_t* a, int nseg_grid);
+// grid.z of a launch of nseg_grid segments
+int prefill_tc_grid_z(const flare_fwd_args_t* a, int nseg_grid);
 // launches segments 0 .. nseg_grid-1
 int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, cudaStream_t stream);
 // device address (current device) of the error word shared by all tensor-core kernels

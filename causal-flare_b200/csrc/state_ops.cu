@@ -25,6 +25,7 @@ __device__ __forceinline__ void merge_factors(float ma, float mb, float& mn, flo
 }
 
 __global__ void __launch_bounds__(NT) fold_kernel(const FoldParams p) {
+  pdl_begin();
   if (p.gate != nullptr && *p.gate == 0) return;
   const int64_t lane_id = blockIdx.x;
   const int m = blockIdx.y * LAT_PER_CTA + (threadIdx.x >> 5);
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(NT) fold_kernel(const FoldParams p) {
 
 template <bool TO_F16>
 __global__ void __launch_bounds__(256) cast_rows_kernel(const CastParams p) {
+  pdl_begin();
   const int c8n = p.d >> 3;
   const int64_t total = p.n0 * p.n1 * p.n2 * c8n;
   const uint16_t* in = reinterpret_cast<const uint16_t*>(p.in);
@@ -132,11 +134,8 @@ int launch_cast_rows(const CastParams& p, cudaStream_t stream) {
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   LaunchTimer timer(p.to_f16 ? "cast_rows_kernel<bf16 to fp16>" : "cast_rows_kernel<fp16 to bf16>", stream);
-  if (p.to_f16)
-    cast_rows_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else
-    cast_rows_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(p.to_f16 ? cast_rows_kernel<true> : cast_rows_kernel<false>, dim3((unsigned)blocks), dim3(256), 0,
+                              stream, p));
   return FLARE_OK;
 }
 
@@ -144,8 +143,7 @@ int launch_fold(const FoldParams& p, cudaStream_t stream) {
   if (p.lanes <= 0 || p.count <= 0) return FLARE_OK;
   dim3 grid((unsigned)p.lanes, (p.M + LAT_PER_CTA - 1) / LAT_PER_CTA);
   LaunchTimer timer("fold_kernel", stream);
-  fold_kernel<<<grid, NT, 0, stream>>>(p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(fold_kernel, grid, dim3(NT), 0, stream, p));
   return FLARE_OK;
 }
 

@@ -22,7 +22,12 @@ template <int MM_MAX, int DD>
 __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) walk_exact_kernel(const WalkParams p) {
   extern __shared__ __align__(16) float smem_raw[];
   const int lane_id = blockIdx.x;  // (b, h) lane
-  if (p.gate != nullptr && p.gate[(int64_t)lane_id * p.gate_stride] == 0) return;
+  pdl_begin();
+  if (p.gate != nullptr) {
+    int raised = 0;
+    for (int i = 0; i < p.gate_count; ++i) raised |= p.gate[(int64_t)lane_id * p.gate_stride + i];
+    if (raised == 0) return;
+  }
   const int seg = blockIdx.y;
   const int b = lane_id / p.H, h = lane_id % p.H;
   const int dvt = 32 * DD;
@@ -268,10 +273,10 @@ static size_t walk_exact_smem_bytes(int M, int Dk, int dd) {
 template <int MM_MAX, int DD>
 static int launch_one(const WalkParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
   auto kern = walk_exact_kernel<MM_MAX, DD>;
-  FLARE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static int granted[64] = {};
+  FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
   LaunchTimer timer(p.gate != nullptr ? "walk_exact_kernel (standby)" : "walk_exact_kernel", stream);
-  kern<<<grid, NT, smem, stream>>>(p);
-  FLARE_CUDA_CHECK(cudaGetLastError());
+  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT), smem, stream, p));
   return FLARE_OK;
 }
 

@@ -29,11 +29,12 @@ struct WalkParams {
   int write_y;
   float scale, power;
   int dtype, variant, block_size;
-  // Optional gate: a CTA does nothing unless gate[lane * gate_stride] != 0 (gate_stride 0: one word for the whole
-  // call, 1: one word per (batch, head) lane).  Used when these kernels stand by behind the tensor-core path and
-  // only run for calls (lanes) whose inputs left that path's numeric domain.  Null: always run.
+  // Optional gate: a CTA does nothing unless one of the words gate[lane * gate_stride + 0 .. gate_count - 1] is set
+  // (gate_stride 0, one word: a gate for the whole call; otherwise the words of the (batch, head) lane).  Used when these
+  // kernels stand by behind the tensor-core path and only run for calls (lanes) whose inputs left that path's numeric
+  // domain.  Null: always run.
   const int* gate;
-  int gate_stride;
+  int gate_stride, gate_count;
 };
 
 // grid.y = nseg_grid segments are launched (segments 0 .. nseg_grid-1)

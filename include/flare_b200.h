@@ -139,7 +139,7 @@ typedef struct flare_bwd_args {
   flare_fwd_args_t fwd; /* y, mask, lengths, state_out, lse_* are ignored; state_in only in span mode (below) */
   const void* dy;       /* [B, N, H, Dv], input dtype */
   int64_t dy_stride_b, dy_stride_n, dy_stride_h;
-  float* dq;            /* [H, M, Dk] fp32 */
+  void* dq;             /* [H, M, Dk], fp32 unless dq_dtype says otherwise */
   void* dk;             /* [B, N, H, Dk] contiguous */
   void* dv;             /* [B, N, H, Dv] contiguous */
   void* dq_dec;         /* [B, N, H, Dk] contiguous or NULL */
@@ -167,6 +167,7 @@ typedef struct flare_bwd_args {
   const void* y;
   int64_t y_stride_b, y_stride_n, y_stride_h;
   const float* lse_dec;
+  int32_t dq_dtype; /* flare_dtype of dq: FLARE_F32 (0), or the input dtype (rounded once, from the fp32 sum) */
 } flare_bwd_args_t;
 
 size_t flare_backward_workspace_bytes(const flare_bwd_args_t* args);
