@@ -131,7 +131,7 @@ int check_forward(const flare_fwd_args_t* a) {
 }
 
 struct FwdPlan {
-  bool use_tc;
+  bool use_tc, wide;
   int nseg;
   int seg_len;
   size_t state_floats;  // floats per state: 2M + M*Dv
@@ -145,25 +145,15 @@ struct FwdPlan {
 };
 
 FwdPlan plan_forward(const flare_fwd_args_t* a) {
-  FwdPlan pl{false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0};
   if (a->B == 0 || a->N == 0) return pl;
   const int64_t lanes = (int64_t)a->B * a->H;
   pl.state_floats = (size_t)2 * a->M + (size_t)a->M * a->Dv;
   if (a->path != FLARE_PATH_EXACT && prefill_tc_supported(a)) {
-    // tensor-core path: one CTA per SM walks a (lane, segment); split the sequence only when lanes are scarce
+    // tensor-core path: one CTA per SM walks a (lane, segment)
     pl.use_tc = true;
     int nseg = 1;
-    const int sms = sm_count();
-    const int64_t ctas = lanes * prefill_tc_ctas_per_lane(a);
-    if (ctas * 2 <= sms) {
-      // as many segments as still fit the SMs in ONE wave (a second, partly filled wave costs more than it gains:
-      // 64 lanes in 3 segments = 192 CTAs measured 0.140 ms for the read-out pass against 0.185 ms unsegmented,
-      // plus 0.06 ms for the state-only pass and the fold)
-      nseg = (int)(sms / ctas);
-      const int max_seg = a->N / 256;
-      if (nseg > max_seg) nseg = max_seg;
-      if (nseg < 1) nseg = 1;
-    }
+    prefill_tc_plan(a, &nseg, &pl.wide);
     int seg_len = (a->N + nseg - 1) / nseg;
     seg_len = (seg_len + 127) / 128 * 128;
     pl.nseg = (a->N + seg_len - 1) / seg_len;
@@ -172,8 +162,7 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
     pl.part_off = pl.ws_bytes;
     pl.part_bytes = a->y != nullptr ? align_up(prefill_tc_partial_bytes(a), 256) : 0;
     pl.ws_bytes += pl.part_bytes;
-    pl.gate_stride = pl.nseg * prefill_tc_grid_z(a, pl.nseg);
-    if (pl.nseg > 1) pl.gate_stride += (pl.nseg - 1) * prefill_tc_grid_z(a, pl.nseg - 1);
+    pl.gate_stride = (2 * pl.nseg - 1) * prefill_tc_grid_z(a, pl.wide);  // state pass over all segments but the last
     if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
       pl.gate_off = pl.ws_bytes;
       pl.gate_bytes = align_up((size_t)(1 + lanes * pl.gate_stride) * sizeof(int), 256);
@@ -239,11 +228,11 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
   t.gate = g_gate;
   t.gate_stride = pl.gate_stride;
   // (the state pass over all segments but the last comes first)
-  t.gate_off = nseg_grid == pl.nseg && pl.nseg > 1 ? (pl.nseg - 1) * prefill_tc_grid_z(a, pl.nseg - 1) : 0;
+  t.gate_off = nseg_grid == pl.nseg && pl.nseg > 1 ? (pl.nseg - 1) * prefill_tc_grid_z(a, pl.wide) : 0;
   if (t.y != nullptr && g_keep.u != nullptr) {
     t.dump_u = g_keep.u; t.dump_c = g_keep.c; t.dump_d = g_keep.d; t.dump_nch = g_keep.nch;
   }
-  return launch_prefill_tc(a, t, nseg_grid, stream);
+  return launch_prefill_tc(a, t, nseg_grid, pl.wide, stream);
 }
 
 int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaStream_t stream);
@@ -481,9 +470,16 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
   memset(&a.state_in, 0, sizeof(a.state_in));
   memset(&a.state_out, 0, sizeof(a.state_out));
   a.state_out.m = seg_m; a.state_out.d = seg_d; a.state_out.u = seg_u;  // marks "a state is wanted" for the checks
-  FwdPlan pl{false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0};
   pl.use_tc = a.path != FLARE_PATH_EXACT && (seg_len % 128) == 0 && prefill_tc_supported(&a);
   const int64_t lanes = (int64_t)a.B * a.H;
+  if (pl.use_tc) {
+    // the wide instance where the two-slice grid would not fit the SMs in one wave
+    int n = 1;
+    flare_fwd_args_t one = a;
+    one.B = (int32_t)(a.B * nseg);
+    prefill_tc_plan(&one, &n, &pl.wide);
+  }
   WalkParams w;
   fill_walk(w, &a);
   w.seg_len = seg_len;

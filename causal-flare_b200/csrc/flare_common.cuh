@@ -44,9 +44,10 @@ struct LaunchTimer {
 // before it have completed and their writes are visible before it touches anything, so nothing is read or written earlier
 // than in a plain launch; only the launch latencies overlap.  The short kernels let the next kernel of the stream be set up
 // as soon as they start (pdl_begin), the tensor-core backward when a CTA has fetched its last tile, the tensor-core forward
-// when it ends (no trigger): with CTAs of the next kernel waiting on the GPU it ran 2 % slower (forward B=8 N=8192 H=16
-// M=128 D=64: 188.7 us triggered at the start, 185.2 us at its last tile, 183.5 us at its end; stablemax training step
-// B=2 N=1000 H=8: 203.6, 205.9 and 191.5 us; 216 us without programmatic launches).
+// and the walk that stands by behind it when they end (no trigger).  CTAs of the next kernel that wait on the GPU slow the
+// forward down (B=8 N=8192 H=16 M=128 D=64: 188.7 us triggered at the start, 185.2 us at its last tile, 183.5 us at its end),
+// and a forward whose CTAs are placed while the walk of the call before still drains runs slower from its first chunk to its
+// last (block-causal B=2 N=65536 H=32 M=256 D=128 back to back: 2244 us against 2132 us).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {

@@ -115,9 +115,15 @@ struct Misc {
   uint32_t tmem_base;
   volatile int abort_flag;
   volatile int out_of_domain;  // some token of this CTA left the numeric domain
-  float wmax[2][4];
+  float wmax[4][4];  // (the packed instance uses four slots, the others two: see there)
   float kap[4];  // decode frame of chunk i in slot i % 4, for the token group (log-sum-exp, weight mass of a latent group)
-  float xmax[2][2][128], xsum[2][2][128];  // [chunk parity][half][latent]
+  // exchange of the token parts' row maxima and sums of E: [chunk parity][part][latent]
+  union {
+    struct {
+      float xmax[2][2][128], xsum[2][2][128];
+    };
+    float x4[2][2][4][64];  // packed instance: (maxima, sums)
+  };
 };
 
 
@@ -153,13 +159,20 @@ __device__ __forceinline__ int latent0() {
 // The kernel instances are compiled in separate translation units (FLARE_TC_UNIT = 0..5: head widths (64, 64) / (128, 128) / (64, 128), without /
 // with the latent-group split) to keep build times short; the unit without FLARE_TC_UNIT holds the host side.
 template <int UNIT>
-int launch_prefill_tc_unit(bool padded, int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+int launch_prefill_tc_unit(int lat, int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                            const CUtensorMap& ty, const TcParams& p, dim3 grid, cudaStream_t stream);
 
 #ifdef FLARE_TC_UNIT
 
 
-// PADDED: fewer than 128 latents (rows padded); the full-width instance carries none of the padding predicates
+// LAT: 0 = groups of 128 latents, 1 = the (last) group is padded, 2 = at most 64 latents (PACK).  The full-width instance
+//        carries none of the padding predicates.
+// PACK: at most 64 latents would leave half of the 128 tensor-memory lanes, and with them half of the latent warps, without
+//        work.  The latent bank is laid down twice (rows 0..63 and 64..127), so the score product gives every latent's
+//        scores on two lanes, and a thread takes 32 tokens of the chunk instead of 64: four warps per 32 latents, the two
+//        of the lower lanes the even quarters of the chunk, the two of the upper lanes the odd ones.  E is stored on both
+//        rows, so both lanes carry the state; each lane maintains half of its columns (the others are never read).
+//        Products over the latents take four 16-latent steps instead of eight.
 // SPLIT: more than 128 latents, partial read-outs
 // BLOCK: block-causal (semi-autoregressive) read-out with blocks of 16, 32, 64 or 128 tokens: a token reads the state
 //        at the end of its block, so the denominator of a block's tokens is the one at the block's end and the mask
@@ -175,12 +188,19 @@ int launch_prefill_tc_unit(bool padded, int mode, const CUtensorMap& tq, const C
 //       SMs in one wave.  Differences: U and Y are 128 columns wide; W and Y0 = R^T U_bf16 come out of ONE product of
 //       width 256 ([E | U_bf16] as one B operand, [W | Y] adjacent in tensor memory), so R is read once for both; W
 //       shares the columns of S; E and R are single-buffered.
-template <bool PADDED, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y, const TcParams p) {
   using L = Lay<DKB, WIDE>;
+  constexpr bool PADDED = LAT != 0, PACK = LAT == 2;
   static_assert(!WIDE || (DVB == 2 && !PADDED), "wide instance");
+  static_assert(!PACK || !SPLIT, "one group of at most 64 latents");
+  constexpr int NP = PACK ? 4 : 2;       // token parts of a chunk = latent warps per 32 latents
+  constexpr int TOK = C / NP;            // tokens per latent thread
+  constexpr int ROWS = PACK ? 64 : 128;  // latent rows of the operand buffers that the products over the latents read
+  constexpr int KSM = ROWS / 16;         // their 16-latent steps
+  constexpr int WS = PACK ? 4 : 2;       // slots of the frame maximum's exchange
   constexpr int ZS = WIDE ? 1 : DVB;  // value slices on grid.z
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_E = L::OFF_E, OFF_R = L::OFF_R, OFF_U = L::OFF_U,
@@ -217,8 +237,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_init(&misc->kap_done, 4);
     mbar_init(&misc->p1_done, 8);
     for (int i = 0; i < 4; ++i) {
-      mbar_init(&misc->pmax[i], 2);
-      mbar_init(&misc->psum[i], 2);
+      mbar_init(&misc->pmax[i], NP);
+      mbar_init(&misc->psum[i], NP);
     }
     mbar_init(&misc->u_done, 1);
     mbar_init(&misc->w_ready, 1);
@@ -260,6 +280,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (Q_SMEM) {
         mbar_arrive_expect_tx(&misc->q_full, 16384);
         tma_load_3d(smem + OFF_Q, &tm_q, &misc->q_full, 0, latent0<ZS, SPLIT>(), h);  // rows beyond M read as zero
+        if (PACK) tma_load_3d(smem + OFF_Q + 8192, &tm_q, &misc->q_full, 0, 0, h);    // (boxes of 64 rows)
       }
       const int vc0 = value_col0<ZS, SPLIT>();
       for (int i = 0; ok && i < nchunks; ++i) {
@@ -370,7 +391,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // lie 16384 bytes apart: the E t-blocks, then the two value blocks of the bf16 state, or its one value
             // block and the block whose column 0 is d
 #pragma unroll
-            for (int j = 0; j < 8; ++j) mma_ss(tmem + TM_W, drm + (j * 2048 >> 4), dem + (j * 2048 >> 4), ID_WY, j > 0);
+            for (int j = 0; j < KSM; ++j) mma_ss(tmem + TM_W, drm + (j * 2048 >> 4), dem + (j * 2048 >> 4), ID_WY, j > 0);
             tc_commit(&misc->w_ready);
             TC_TRACE(2, i, 5);
             if constexpr (WIDE) {
@@ -398,7 +419,29 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // row sum of E through shared memory.
     const int hf = warp >> 2, q = warp & 3;
     const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
-    const int m = q * 32 + lane;
+    const int lm = q * 32 + lane;                       // TMEM lane
+    const int m = PACK ? (lm & 63) : lm;                // latent of the group
+    const int tp = PACK ? hf * 2 + (q >> 1) : hf;       // token part of this thread
+    const int pq = PACK ? (q & 1) : q;                  // exchange group: the NP warps of the same 32 latents
+    // exchange arrays [chunk parity][part][latent]
+    auto xs = [&](int par_, int part) -> float& {
+      if constexpr (PACK) return misc->x4[1][par_][part][m];
+      else return misc->xsum[par_][part][m];
+    };
+    auto xm = [&](int par_, int part) -> float& {
+      if constexpr (PACK) return misc->x4[0][par_][part][m];
+      else return misc->xmax[par_][part][m];
+    };
+    auto xsum_all = [&](int par_) -> float {
+      float t = xs(par_, 0) + xs(par_, 1);
+      if constexpr (PACK) t += xs(par_, 2) + xs(par_, 3);
+      return t;
+    };
+    auto xmax_all = [&](int par_) -> float {
+      float t = fmaxf(xm(par_, 0), xm(par_, 1));
+      if constexpr (PACK) t = fmaxf(t, fmaxf(xm(par_, 2), xm(par_, 3)));
+      return t;
+    };
     const float sc2 = p.scale * kLog2e;
     const int64_t st_idx = (int64_t)lane_id * p.in_lane_stride + (int64_t)seg * p.in_seg_stride;
     // Fewer than 128 latents: the missing rows are padding (zero rows of Q).  A padding latent gets the frame +inf,
@@ -433,34 +476,46 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       tc_fence_before_sync();
       warp_arrive(&misc->q_full, lane);
     }
-    // columns of the numerator each half-group thread looks after: 32 of the CTA's 64, or (wide) 64 of its 128
-    constexpr int UW = WIDE ? 64 : 32;
+    // columns of the numerator each thread looks after: 32 of the CTA's 64, (wide) 64 of its 128, (packed) 16 of 64
+    constexpr int UW = WIDE ? 64 : (PACK ? 16 : 32);
+    const int ucol = PACK ? (q >> 1) * 32 + hf * 16 : hf * UW;
+    if constexpr (PACK) {
+      // carry-in numerator -> tensor memory (the columns of the row's other copy are whatever is there: never read)
+      uint32_t r[16];
 #pragma unroll
-    for (int c0 = 0; c0 < UW; c0 += 32) {
-      // carry-in numerator -> tensor memory
-      uint32_t r[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        r[i] = (p.in_u && live) ? __float_as_uint(p.in_u[(st_idx * p.M + latent0<ZS, SPLIT>() + m) * DV +
-                                                         value_col0<ZS, SPLIT>() + hf * UW + c0 + i])
-                                : 0u;
-      tmem_st32(tl + TM_U + hf * UW + c0, r);
+      for (int i = 0; i < 16; ++i)
+        r[i] = (p.in_u && live) ? __float_as_uint(p.in_u[(st_idx * p.M + m) * DV + value_col0<ZS, SPLIT>() + ucol + i]) : 0u;
+      tmem_st16(tl + TM_U + ucol, r);
       tmem_wait_st();
+    } else {
+#pragma unroll
+      for (int c0 = 0; c0 < UW; c0 += 32) {
+        // carry-in numerator -> tensor memory
+        uint32_t r[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          r[i] = (p.in_u && live) ? __float_as_uint(p.in_u[(st_idx * p.M + latent0<ZS, SPLIT>() + m) * DV +
+                                                           value_col0<ZS, SPLIT>() + ucol + c0 + i])
+                                  : 0u;
+        tmem_st32(tl + TM_U + ucol + c0, r);
+        tmem_wait_st();
+      }
     }
 
     for (int i = 0; ok && i < nchunks; ++i) {
       const uint32_t par = i & 1;
       const int nvalid = min(C, seg_end - (seg_begin + i * C));
-      const int tok0 = hf * 64;
-      uint8_t* e_row = smem + OFF_E + hf * 16384;  // t-block hf of the operand buffers
-      uint8_t* r_row = smem + OFF_R + hf * 16384;
+      const int tok0 = tp * TOK;
+      uint8_t* e_row = smem + OFF_E + (tok0 >> 6) * 16384;  // this thread's t-block of the operand buffers
+      uint8_t* r_row = smem + OFF_R + (tok0 >> 6) * 16384;
+      const int ch0 = PACK ? (tp & 1) * 4 : 0;              // and its first 8-token piece there
       if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
       tc_fence_after_sync();
       if (tid == 0) TC_TRACE(0, i, 0);
-      // the 64 scores of this thread stay in registers for the whole chunk
+      // the 64 (packed: 32) scores of this thread stay in registers for the whole chunk
       uint32_t ra[32], rb[32];
       tmem_ld32(tl + TM_S + tok0, ra);
-      tmem_ld32(tl + TM_S + tok0 + 32, rb);
+      if constexpr (!PACK) tmem_ld32(tl + TM_S + tok0 + 32, rb);
       // Frame of this chunk.  Chunk 0 exchanges the two halves' maxima synchronously (the carried frame may be
       // empty).  Later chunks use the running max through the PREVIOUS chunk, known without waiting (this bookkeeping
       // runs while the scores are on their way out of tensor memory); E may then exceed 1 by the growth of the max
@@ -469,13 +524,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       float c_new = c2;
       if (i > 0) {
         // bookkeeping of chunk i - 1: both halves' sums and maxima are published once its psum phase completed
-        if (!(ok = wait_or_abort(&misc->psum[q], (i - 1) & 1, misc))) break;
-        dsum = d_prev + (misc->xsum[par ^ 1][0][m] + misc->xsum[par ^ 1][1][m]);
-        c_new = fmaxf(c2, fmaxf(misc->xmax[par ^ 1][0][m], misc->xmax[par ^ 1][1][m]));
+        if (!(ok = wait_or_abort(&misc->psum[pq], (i - 1) & 1, misc))) break;
+        dsum = d_prev + xsum_all(par ^ 1);
+        c_new = fmaxf(c2, xmax_all(par ^ 1));
       }
       tmem_wait_ld();
       tmem_fence_regs(ra);
-      tmem_fence_regs(rb);
+      if constexpr (!PACK) tmem_fence_regs(rb);
       tc_fence_before_sync();
       warp_arrive(&misc->s_free, lane);  // the S columns may take the next chunk's scores
       if (i == 0) {
@@ -484,12 +539,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
         for (int k = 0; k < 32; ++k) {
           if (tok0 + k < nvalid) cm0 = fmaxf(cm0, __uint_as_float(ra[k]) * sc2);
-          if (tok0 + 32 + k < nvalid) cm2 = fmaxf(cm2, __uint_as_float(rb[k]) * sc2);
+          if (!PACK && tok0 + 32 + k < nvalid) cm2 = fmaxf(cm2, __uint_as_float(rb[k]) * sc2);
         }
-        misc->xmax[0][hf][m] = live ? fmaxf(cm0, cm2) : -INFINITY;
-        warp_arrive(&misc->pmax[q], lane);
-        if (!(ok = wait_or_abort(&misc->pmax[q], 0, misc))) break;
-        c_new = fmaxf(c2, fmaxf(misc->xmax[0][0][m], misc->xmax[0][1][m]));
+        xm(0, tp) = live ? fmaxf(cm0, cm2) : -INFINITY;
+        warp_arrive(&misc->pmax[pq], lane);
+        if (!(ok = wait_or_abort(&misc->pmax[pq], 0, misc))) break;
+        c_new = fmaxf(c2, xmax_all(0));
       }
       float alpha = STABLE ? 1.0f : ex2_approx(c2 - c_new);  // 0 when the old state is empty
       // kappa: common frame of the decode weights = max over latents of the running max.  Chunk 0 synchronises;
@@ -505,13 +560,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // the state update it waits for follows the product that waits for all of them - and has 3 000 cycles of passes
         // of its own in between, while a reader needs a few hundred from the end of this chunk to its read.  Four
         // slots indexed by chunk % 4 measured 4 % slower: one more live value in a register-capped loop.)
-        if (lane == 0) misc->wmax[par][q] = wm;
+        // (The packed instance has registers to spare and passes half as long: four slots there.)
+        if (lane == 0) misc->wmax[i & (WS - 1)][q] = wm;
       }
       if (i == 0) {
         if (hf == 0 && lane == 0) mbar_arrive(&misc->kap_done);
         if (!(ok = wait_or_abort(&misc->kap_done, 0, misc))) break;
       }
-      const float* wsrc = misc->wmax[i == 0 ? 0 : ((i - 1) & 1)];
+      const float* wsrc = misc->wmax[i == 0 ? 0 : ((i - 1) & (WS - 1))];
       const float kappa = fmaxf(fmaxf(wsrc[0], wsrc[1]), fmaxf(wsrc[2], wsrc[3]));
       // ordered before the token group's read by the barrier chain
       if ((SPLIT || BLOCK || p.lse_dec != nullptr) && tid == 0) misc->kap[i & 3] = kappa;
@@ -536,10 +592,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (!(ok = wait_or_abort(&misc->u_done, (i - 1) & 1, misc))) break;
         tc_fence_after_sync();
       }
+      auto store_e = [&](int ch, const uint4& v) {  // 8 tokens of the E operand's row (packed: both copies of it)
+        *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, ch0 + ch)) = v;
+        if constexpr (PACK) *reinterpret_cast<uint4*>(e_row + 8192 + swz_chunk_off(m, ch0 + ch)) = v;
+      };
       if constexpr (STABLE) {
         // encoder weights sigma(s): packed and stored 8 tokens at a time; the raw scores stay in ra / rb for phase b
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
+        for (int ch = 0; ch < TOK / 8; ++ch) {
           float sg[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -548,8 +608,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             sg[j] = (tok0 + ch * 8 + j < nvalid) ? sigma_fast(raw * p.scale, p.power) : 0.f;
             tot0 += sg[j];
           }
-          *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, ch)) =
-              make_uint4(pack_bf16(sg[0], sg[1]), pack_bf16(sg[2], sg[3]), pack_bf16(sg[4], sg[5]), pack_bf16(sg[6], sg[7]));
+          store_e(ch, make_uint4(pack_bf16(sg[0], sg[1]), pack_bf16(sg[2], sg[3]), pack_bf16(sg[4], sg[5]), pack_bf16(sg[6], sg[7])));
         }
       } else if (nvalid == C) {
         // two tokens per FMA / add instruction (packed fp32 pairs): the passes are bound by instruction issue
@@ -557,18 +616,22 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         uint64_t sa[2] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)}, sb[2] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)};
 #pragma unroll
         for (int k = 0; k < 32; k += 2) {
-          float xa0, xa1, xb0, xb1;
+          float xa0, xa1;
           f2_unpack(f2_fma(f2_pack(__uint_as_float(ra[k]), __uint_as_float(ra[k + 1])), sc2p, cnp), xa0, xa1);
-          f2_unpack(f2_fma(f2_pack(__uint_as_float(rb[k]), __uint_as_float(rb[k + 1])), sc2p, cnp), xb0, xb1);
           cma = fmax3(cma, xa0, xa1);
-          cmb = fmax3(cmb, xb0, xb1);
-          const float ea0 = ex2_approx(xa0), ea1 = ex2_approx(xa1), eb0 = ex2_approx(xb0), eb1 = ex2_approx(xb1);
+          const float ea0 = ex2_approx(xa0), ea1 = ex2_approx(xa1);
           ra[k] = __float_as_uint(ea0);
           ra[k + 1] = __float_as_uint(ea1);
-          rb[k] = __float_as_uint(eb0);
-          rb[k + 1] = __float_as_uint(eb1);
           sa[BLOCK ? (k >> 4) : 0] = f2_add(sa[BLOCK ? (k >> 4) : 0], f2_pack(ea0, ea1));
-          sb[BLOCK ? (k >> 4) : 0] = f2_add(sb[BLOCK ? (k >> 4) : 0], f2_pack(eb0, eb1));
+          if constexpr (!PACK) {
+            float xb0, xb1;
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(rb[k]), __uint_as_float(rb[k + 1])), sc2p, cnp), xb0, xb1);
+            cmb = fmax3(cmb, xb0, xb1);
+            const float eb0 = ex2_approx(xb0), eb1 = ex2_approx(xb1);
+            rb[k] = __float_as_uint(eb0);
+            rb[k + 1] = __float_as_uint(eb1);
+            sb[BLOCK ? (k >> 4) : 0] = f2_add(sb[BLOCK ? (k >> 4) : 0], f2_pack(eb0, eb1));
+          }
         }
         float lo, hi;
         if (BLOCK) {
@@ -576,31 +639,35 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           for (int g = 0; g < 2; ++g) {
             f2_unpack(sa[g], lo, hi);
             g16[g] = lo + hi;
-            f2_unpack(sb[g], lo, hi);
-            g16[2 + g] = lo + hi;
+            if constexpr (!PACK) {
+              f2_unpack(sb[g], lo, hi);
+              g16[2 + g] = lo + hi;
+            }
           }
         } else {
           f2_unpack(sa[0], lo, hi);
           tot0 = lo + hi;
-          f2_unpack(sb[0], lo, hi);
-          tot1 = lo + hi;
+          if constexpr (!PACK) {
+            f2_unpack(sb[0], lo, hi);
+            tot1 = lo + hi;
+          }
         }
       } else {
 #pragma unroll
         for (int k = 0; k < 32; ++k) {
-          const float x0 = __uint_as_float(ra[k]) * sc2 - c_new, x1 = __uint_as_float(rb[k]) * sc2 - c_new;
+          const float x0 = __uint_as_float(ra[k]) * sc2 - c_new;
           if (tok0 + k < nvalid) cma = fmaxf(cma, x0);
-          if (tok0 + 32 + k < nvalid) cmb = fmaxf(cmb, x1);
           const float e0 = (tok0 + k < nvalid) ? ex2_approx(x0) : 0.f;
-          const float e1 = (tok0 + 32 + k < nvalid) ? ex2_approx(x1) : 0.f;
           ra[k] = __float_as_uint(e0);
-          rb[k] = __float_as_uint(e1);
-          if (BLOCK) {
-            g16[k >> 4] += e0;
-            g16[2 + (k >> 4)] += e1;
-          } else {
-            tot0 += e0;
-            tot1 += e1;
+          if (BLOCK) g16[k >> 4] += e0;
+          else tot0 += e0;
+          if constexpr (!PACK) {
+            const float x1 = __uint_as_float(rb[k]) * sc2 - c_new;
+            if (tok0 + 32 + k < nvalid) cmb = fmaxf(cmb, x1);
+            const float e1 = (tok0 + 32 + k < nvalid) ? ex2_approx(x1) : 0.f;
+            rb[k] = __float_as_uint(e1);
+            if (BLOCK) g16[2 + (k >> 4)] += e1;
+            else tot1 += e1;
           }
         }
       }
@@ -608,9 +675,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tot0 = g16[0] + g16[1];
         tot1 = g16[2] + g16[3];
       }
-      misc->xsum[par][hf][m] = tot0 + tot1;
-      // (chunk 0 published its maximum before the pass; an empty half stays at -inf)
-      if (i > 0) misc->xmax[par][hf][m] = live ? fmaxf(cma, cmb) + c_new : -INFINITY;
+      xs(par, tp) = tot0 + tot1;
+      // (chunk 0 published its maximum before the pass; an empty part stays at -inf)
+      if (i > 0) xm(par, tp) = live ? fmaxf(cma, cmb) + c_new : -INFINITY;
       if (!(tot0 + tot1 < 1.15e18f)) {
         // the running max grew by more than 60 powers of two inside one chunk (the frame is the max through the
         // previous chunk): the denominators of this row leave the range in which the read-out weights are safe, see
@@ -618,7 +685,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         atomicOr(p.err, 2);
         misc->out_of_domain = 1;
       }
-      warp_arrive(&misc->psum[q], lane);
+      warp_arrive(&misc->psum[pq], lane);
       // E has one buffer: the products that read the previous chunk's E and R (issued together, the state update last)
       // must have run.  (Storing inside the pass would need this wait before it, where it is not yet satisfied.)
       if (!STABLE && i > 0) {
@@ -628,25 +695,29 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if constexpr (!STABLE)
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
-        *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, ch)) =
-            make_uint4(pack_bf16(__uint_as_float(ra[ch * 8 + 0]), __uint_as_float(ra[ch * 8 + 1])),
-                       pack_bf16(__uint_as_float(ra[ch * 8 + 2]), __uint_as_float(ra[ch * 8 + 3])),
-                       pack_bf16(__uint_as_float(ra[ch * 8 + 4]), __uint_as_float(ra[ch * 8 + 5])),
-                       pack_bf16(__uint_as_float(ra[ch * 8 + 6]), __uint_as_float(ra[ch * 8 + 7])));
-        *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, 4 + ch)) =
-            make_uint4(pack_bf16(__uint_as_float(rb[ch * 8 + 0]), __uint_as_float(rb[ch * 8 + 1])),
-                       pack_bf16(__uint_as_float(rb[ch * 8 + 2]), __uint_as_float(rb[ch * 8 + 3])),
-                       pack_bf16(__uint_as_float(rb[ch * 8 + 4]), __uint_as_float(rb[ch * 8 + 5])),
-                       pack_bf16(__uint_as_float(rb[ch * 8 + 6]), __uint_as_float(rb[ch * 8 + 7])));
+        store_e(ch, make_uint4(pack_bf16(__uint_as_float(ra[ch * 8 + 0]), __uint_as_float(ra[ch * 8 + 1])),
+                               pack_bf16(__uint_as_float(ra[ch * 8 + 2]), __uint_as_float(ra[ch * 8 + 3])),
+                               pack_bf16(__uint_as_float(ra[ch * 8 + 4]), __uint_as_float(ra[ch * 8 + 5])),
+                               pack_bf16(__uint_as_float(ra[ch * 8 + 6]), __uint_as_float(ra[ch * 8 + 7]))));
+        if constexpr (!PACK)
+          store_e(4 + ch, make_uint4(pack_bf16(__uint_as_float(rb[ch * 8 + 0]), __uint_as_float(rb[ch * 8 + 1])),
+                                     pack_bf16(__uint_as_float(rb[ch * 8 + 2]), __uint_as_float(rb[ch * 8 + 3])),
+                                     pack_bf16(__uint_as_float(rb[ch * 8 + 4]), __uint_as_float(rb[ch * 8 + 5])),
+                                     pack_bf16(__uint_as_float(rb[ch * 8 + 6]), __uint_as_float(rb[ch * 8 + 7]))));
       }
       d_prev = d_carry;
-      // the upper half continues the lower half's running denominator; the lower half needs nothing from its partner
-      // (except for blocks of 128 tokens, whose end lies in the upper half)
+      // a later part continues the earlier parts' running denominator; the first one needs nothing from its partners
+      // (except for blocks that end in a later part)
       float run = d_carry;
-      if (!state_only && (hf || (BLOCK && p.block == 128))) {
-        if (!(ok = wait_or_abort(&misc->psum[q], par, misc))) break;
-        run += misc->xsum[par][0][m];
-        if (BLOCK && p.block == 128 && hf == 0) run = d_carry;  // lower half: only the wait was needed
+      if (!state_only && (tp || (BLOCK && p.block > TOK))) {
+        if (!(ok = wait_or_abort(&misc->psum[pq], par, misc))) break;
+        if constexpr (PACK) {
+#pragma unroll
+          for (int t = 0; t < NP - 1; ++t) run += t < tp ? xs(par, t) : 0.f;
+        } else {
+          run += xs(par, 0);
+          if (BLOCK && p.block > TOK && hf == 0) run = d_carry;  // lower half: only the wait was needed
+        }
       }
       if (tid == 0) TC_TRACE(0, i, 2);
       if (state_only) {
@@ -654,7 +725,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       } else if constexpr (STABLE) {
         // phase b, stablemax: D = running sum of sigma (recomputed), decode numerator exp2(s - c) a_m, R = numerator / D
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
+        for (int blk = 0; blk < TOK / 32; ++blk) {
           uint32_t rp[16];
 #pragma unroll
           for (int k = 0; k < 32; k += 2) {
@@ -668,7 +739,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch)
-            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, blk * 4 + ch)) =
+            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + blk * 4 + ch)) =
                 make_uint4(rp[ch * 4], rp[ch * 4 + 1], rp[ch * 4 + 2], rp[ch * 4 + 3]);
         }
       } else if constexpr (!BLOCK) {
@@ -677,7 +748,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // depending on the box, and carrying the denominator pre-divided by a_m (one FMA + reciprocal + multiply per
         // element) measured 1.5 % slower than this form.
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
+        for (int blk = 0; blk < TOK / 32; ++blk) {
           uint32_t rp[16];
 #pragma unroll
           for (int k = 0; k < 32; k += 2) {
@@ -693,15 +764,30 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch)
-            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, blk * 4 + ch)) =
+            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + blk * 4 + ch)) =
                 make_uint4(rp[ch * 4], rp[ch * 4 + 1], rp[ch * 4 + 2], rp[ch * 4 + 3]);
         }
       } else {
         // phase b, block-causal: the denominator of a token is the one at the end of its block.  dend[g] is that
         // value for the g-th group of 16 tokens of this half (`run` = denominator before this half).
         const int bs = p.block;
-        float dend[4];
-        {
+        constexpr int NG = TOK / 16;
+        float dend[NG];
+        if constexpr (PACK) {
+          const float p0 = run + g16[0], p1 = p0 + g16[1];
+          if (bs == 16) {
+            dend[0] = p0; dend[1] = p1;
+          } else if (bs == 32) {
+            dend[0] = dend[1] = p1;
+          } else {
+            // the block ends in a later part (or this one): add the parts up to its last one
+            const int last = bs == 64 ? (tp | 1) : NP - 1;
+            float t = p1;
+#pragma unroll
+            for (int u = 1; u < NP; ++u) t += (u > tp && u <= last) ? xs(par, u) : 0.f;
+            dend[0] = dend[1] = t;
+          }
+        } else {
           const float p0 = run + g16[0], p1 = p0 + g16[1], p2 = p1 + g16[2], p3 = p2 + g16[3];
           if (bs == 16) {
             dend[0] = p0; dend[1] = p1; dend[2] = p2; dend[3] = p3;
@@ -711,7 +797,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             dend[0] = dend[1] = dend[2] = dend[3] = p3;
           } else {
             // one block per chunk: both halves use the chunk's end
-            const float whole = d_carry + (misc->xsum[par][0][m] + misc->xsum[par][1][m]);
+            const float whole = d_carry + xsum_all(par);
             dend[0] = dend[1] = dend[2] = dend[3] = whole;
           }
         }
@@ -720,17 +806,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           const int t_half = seg_begin + i * C + tok0;  // first token of this half in the sequence
           float* dst = p.lse_enc + ((int64_t)lane_id * (p.N / bs)) * p.M + latent0<ZS, SPLIT>() + m;
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
+          for (int g = 0; g < NG; ++g) {
             const int t_end = t_half + g * 16 + 15;            // last token of the group
             const bool ends = ((t_end + 1) % bs) == 0;         // a block ends with this group
             if (ends && tok0 + g * 16 < nvalid) dst[(int64_t)(t_end / bs) * p.M] = (c_new + __log2f(dend[g])) * kLn2;
           }
         }
-        float inv[4];
+        float inv[NG];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) inv[g] = a_m * rcp_approx(dend[g]);
+        for (int g = 0; g < NG; ++g) inv[g] = a_m * rcp_approx(dend[g]);
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
+        for (int blk = 0; blk < TOK / 32; ++blk) {
           uint32_t rp[16];
 #pragma unroll
           for (int k = 0; k < 32; k += 2) {
@@ -742,7 +828,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch)
-            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, blk * 4 + ch)) =
+            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + blk * 4 + ch)) =
                 make_uint4(rp[ch * 4], rp[ch * 4 + 1], rp[ch * 4 + 2], rp[ch * 4 + 3]);
         }
       }
@@ -750,7 +836,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // state part: needs the numerator update of the previous chunk to have landed (waited for before the E rows
       // were written)
       if (tid == 0) TC_TRACE(0, i, 4);
-      if (hf == 0 && !state_only) {
+      if (tp == 0 && !state_only) {
         // d of the carried state: column 0 of row m of the MN-major block (merged product with one value block), or
         // element m of row 0 of the small K-major tile
         if (!WIDE)
@@ -792,10 +878,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               }
               if constexpr (KEEP) {
                 // training: the state before this chunk in the exact running-max frame through it (see below)
-                if (c0 == 0 && !(ok = wait_or_abort(&misc->psum[q], par, misc))) break;
+                if (c0 == 0 && !(ok = wait_or_abort(&misc->psum[pq], par, misc))) break;
                 float fin = 1.0f, c_true = c2;
                 if (!STABLE) {
-                  c_true = fmaxf(c2, fmaxf(misc->xmax[par][0][m], misc->xmax[par][1][m]));
+                  c_true = fmaxf(c2, xmax_all(par));
                   fin = ex2_approx(c2 - c_true);
                 }
                 const int64_t o = ((int64_t)lane_id * p.dump_nch + (seg_begin / C + i)) * p.M + latent0<ZS, SPLIT>() + m;
@@ -821,46 +907,50 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       } else
       if (!state_only || need) {
-        uint32_t r[32];
-        tmem_ld32(tl + TM_U + hf * 32, r);
+        constexpr int NU = PACK ? 16 : 32;  // columns of this thread
+        uint32_t r[NU];
+        if constexpr (PACK) tmem_ld16(tl + TM_U + ucol, r);
+        else tmem_ld32(tl + TM_U + ucol, r);
         tmem_wait_ld();
-        tmem_fence_regs(r);
+        if constexpr (PACK) tmem_fence_regs16(r);
+        else tmem_fence_regs(r);
         if (need) {
 #pragma unroll
-          for (int k = 0; k < 32; k += 2) {
+          for (int k = 0; k < NU; k += 2) {
             float u0, u1;
             f2_unpack(f2_mul(f2_pack(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), f2_pack(alpha, alpha)), u0, u1);
             r[k] = __float_as_uint(u0);
             r[k + 1] = __float_as_uint(u1);
           }
-          tmem_st32(tl + TM_U + hf * 32, r);
+          if constexpr (PACK) tmem_st16(tl + TM_U + ucol, r);
+          else tmem_st32(tl + TM_U + ucol, r);
         }
         if (!state_only) {
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
+          for (int ch = 0; ch < NU / 8; ++ch) {
             uint4 v;
             v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1]));
             v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3]));
             v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5]));
             v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7]));
-            *reinterpret_cast<uint4*>(smem + OFF_U + swz_chunk_off(m, hf * 4 + ch)) = v;
+            *reinterpret_cast<uint4*>(smem + OFF_U + swz_chunk_off(m, (ucol >> 3) + ch)) = v;
           }
           if constexpr (KEEP) {
             // Training: the state before this chunk is kept for the backward pass, in the EXACT running-max frame
             // through this chunk (= the frame the next chunk will use), so that the backward's encoder weights of
-            // the chunk never exceed 1.  Both halves' maxima of this chunk are published once its psum phase completed.
-            if (!(ok = wait_or_abort(&misc->psum[q], par, misc))) break;
+            // the chunk never exceed 1.  All parts' maxima of this chunk are published once its psum phase completed.
+            if (!(ok = wait_or_abort(&misc->psum[pq], par, misc))) break;
             float fin = 1.0f, c_true = c2;
             if (!STABLE) {
-              c_true = fmaxf(c2, fmaxf(misc->xmax[par][0][m], misc->xmax[par][1][m]));
+              c_true = fmaxf(c2, xmax_all(par));
               fin = ex2_approx(c2 - c_true);
             }
             if (live) {
               const int64_t o = ((int64_t)lane_id * p.dump_nch + (seg_begin / C + i)) * p.M + latent0<ZS, SPLIT>() + m;
               uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dump_u) + o * DV +
-                                                    value_col0<ZS, SPLIT>() + hf * 32);
+                                                    value_col0<ZS, SPLIT>() + ucol);
 #pragma unroll
-              for (int ch = 0; ch < 4; ++ch) {
+              for (int ch = 0; ch < NU / 8; ++ch) {
                 uint4 v;
                 v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]) * fin, __uint_as_float(r[ch * 8 + 1]) * fin);
                 v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]) * fin, __uint_as_float(r[ch * 8 + 3]) * fin);
@@ -868,7 +958,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]) * fin, __uint_as_float(r[ch * 8 + 7]) * fin);
                 dst[ch] = v;
               }
-              if (hf == 0 && value_col0<ZS, SPLIT>() == 0) {
+              if (tp == 0 && value_col0<ZS, SPLIT>() == 0) {
                 p.dump_c[o] = c_true;          // log2 units (unused for the stablemax encoder)
                 p.dump_d[o] = d_carry * fin;   // denominator before the chunk in that frame
               }
@@ -887,11 +977,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       float fin = 1.0f;  // factor from the last chunk's frame to the exact running-max frame
       if (nchunks > 0) {
         const int lp = (nchunks - 1) & 1;
-        ok = wait_or_abort(&misc->u_done, lp, misc) && wait_or_abort(&misc->psum[q], lp, misc);
+        ok = wait_or_abort(&misc->u_done, lp, misc) && wait_or_abort(&misc->psum[pq], lp, misc);
         if (ok) {
-          dsum = d_prev + (misc->xsum[lp][0][m] + misc->xsum[lp][1][m]);
+          dsum = d_prev + xsum_all(lp);
           if (!STABLE) {
-            const float c_true = fmaxf(c2, fmaxf(misc->xmax[lp][0][m], misc->xmax[lp][1][m]));
+            const float c_true = fmaxf(c2, xmax_all(lp));
             fin = ex2_approx(c2 - c_true);
             c2 = c_true;
           }
@@ -901,20 +991,23 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (ok) {
         const int64_t so = (int64_t)lane_id * p.out_lane_stride + (int64_t)seg * p.out_seg_stride;
         const int mg = latent0<ZS, SPLIT>() + m;  // latent index in the whole bank
-        if (hf == 0 && live && value_col0<ZS, SPLIT>() == 0) {
+        if (tp == 0 && live && value_col0<ZS, SPLIT>() == 0) {
           p.out_m[so * p.M + mg] = STABLE ? 0.f : c2 * kLn2;
           p.out_d[so * p.M + mg] = dsum * fin;
         }
+        constexpr int NU = PACK ? 16 : 32;
 #pragma unroll
-        for (int c0 = 0; c0 < UW; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(tl + TM_U + hf * UW + c0, r);
+        for (int c0 = 0; c0 < UW; c0 += NU) {
+          uint32_t r[NU];
+          if constexpr (PACK) tmem_ld16(tl + TM_U + ucol + c0, r);
+          else tmem_ld32(tl + TM_U + ucol + c0, r);
           tmem_wait_ld();
-          tmem_fence_regs(r);
+          if constexpr (PACK) tmem_fence_regs16(r);
+          else tmem_fence_regs(r);
           float4* dst = reinterpret_cast<float4*>(p.out_u + (so * p.M + (live ? mg : 0)) * DV +
-                                                  value_col0<ZS, SPLIT>() + hf * UW + c0);
+                                                  value_col0<ZS, SPLIT>() + ucol + c0);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
+          for (int k = 0; k < NU / 4; ++k)
             if (live) dst[k] = make_float4(__uint_as_float(r[4 * k]) * fin, __uint_as_float(r[4 * k + 1]) * fin,
                                  __uint_as_float(r[4 * k + 2]) * fin, __uint_as_float(r[4 * k + 3]) * fin);
         }
@@ -1202,10 +1295,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 namespace {
 
-template <bool PADDED, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE = false>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE = false>
 int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
-  auto kern = prefill_tc_kernel<PADDED, DKB, DVB, SPLIT, MODE, KEEP, WIDE>;
+  auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE>;
   static int granted[64] = {};
   FLARE_CUDA_CHECK(allow_smem(kern, Lay<DKB, WIDE>::SMEM_BYTES, granted));
   LaunchTimer timer(p.y == nullptr ? "prefill_tc_kernel (state only)" : (WIDE ? "prefill_tc_kernel (wide)" : "prefill_tc_kernel"),
@@ -1233,45 +1326,48 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   return FLARE_OK;
 }
 
-template <bool PADDED, int DKB, int DVB, bool SPLIT, int MODE>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE>
 int launch_instance(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                     const TcParams& p, dim3 grid, cudaStream_t stream) {
-  return p.dump_u != nullptr ? launch_keep<PADDED, DKB, DVB, SPLIT, MODE, true>(tq, tk, tv, ty, p, grid, stream)
-                             : launch_keep<PADDED, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
+  return p.dump_u != nullptr ? launch_keep<LAT, DKB, DVB, SPLIT, MODE, true>(tq, tk, tv, ty, p, grid, stream)
+                             : launch_keep<LAT, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
 }
 
 }  // namespace
 
 template <>
-int launch_prefill_tc_unit<FLARE_TC_UNIT>(bool padded, int mode, const CUtensorMap& tq, const CUtensorMap& tk,
+int launch_prefill_tc_unit<FLARE_TC_UNIT>(int lat, int mode, const CUtensorMap& tq, const CUtensorMap& tk,
                                           const CUtensorMap& tv, const CUtensorMap& ty, const TcParams& p, dim3 grid,
                                           cudaStream_t stream) {
   // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128); units 3..5: the same with the latent-group split;
   // units 6, 7: the wide (128, 128) instance (one CTA for both value blocks) without / with the latent-group split
 #if FLARE_TC_UNIT >= 6
   constexpr bool WSPLIT = FLARE_TC_UNIT == 7;
-  (void)padded;
+  (void)lat;
   if (p.dump_u != nullptr) {  // training forward that keeps its per-chunk states
-    if (mode == 1) return launch_keep<false, 2, 2, WSPLIT, 1, true, true>(tq, tk, tv, ty, p, grid, stream);
-    if (mode == 2) return launch_keep<false, 2, 2, WSPLIT, 2, true, true>(tq, tk, tv, ty, p, grid, stream);
-    return launch_keep<false, 2, 2, WSPLIT, 0, true, true>(tq, tk, tv, ty, p, grid, stream);
+    if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, true, true>(tq, tk, tv, ty, p, grid, stream);
+    if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, true, true>(tq, tk, tv, ty, p, grid, stream);
+    return launch_keep<0, 2, 2, WSPLIT, 0, true, true>(tq, tk, tv, ty, p, grid, stream);
   }
-  if (mode == 1) return launch_keep<false, 2, 2, WSPLIT, 1, false, true>(tq, tk, tv, ty, p, grid, stream);
-  if (mode == 2) return launch_keep<false, 2, 2, WSPLIT, 2, false, true>(tq, tk, tv, ty, p, grid, stream);
-  return launch_keep<false, 2, 2, WSPLIT, 0, false, true>(tq, tk, tv, ty, p, grid, stream);
+  if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, false, true>(tq, tk, tv, ty, p, grid, stream);
+  if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, false, true>(tq, tk, tv, ty, p, grid, stream);
+  return launch_keep<0, 2, 2, WSPLIT, 0, false, true>(tq, tk, tv, ty, p, grid, stream);
 #else
   constexpr int COMBO = FLARE_TC_UNIT % 3;
   constexpr int DKB = COMBO == 1 ? 2 : 1;
   constexpr int DVB = COMBO == 0 ? 1 : 2;
   constexpr bool SPLIT = FLARE_TC_UNIT >= 3;
-  if (mode == 1)
-    return padded ? launch_instance<true, DKB, DVB, SPLIT, 1>(tq, tk, tv, ty, p, grid, stream)
-                  : launch_instance<false, DKB, DVB, SPLIT, 1>(tq, tk, tv, ty, p, grid, stream);
-  if (mode == 2)
-    return padded ? launch_instance<true, DKB, DVB, SPLIT, 2>(tq, tk, tv, ty, p, grid, stream)
-                  : launch_instance<false, DKB, DVB, SPLIT, 2>(tq, tk, tv, ty, p, grid, stream);
-  return padded ? launch_instance<true, DKB, DVB, SPLIT, 0>(tq, tk, tv, ty, p, grid, stream)
-                : launch_instance<false, DKB, DVB, SPLIT, 0>(tq, tk, tv, ty, p, grid, stream);
+  // one instance family per kind of latent bank; the packed one exists for a single group only
+#define FLARE_TC_MODES(LAT)                                                                                \
+  return mode == 1 ? launch_instance<LAT, DKB, DVB, SPLIT, 1>(tq, tk, tv, ty, p, grid, stream)             \
+         : mode == 2 ? launch_instance<LAT, DKB, DVB, SPLIT, 2>(tq, tk, tv, ty, p, grid, stream)           \
+                     : launch_instance<LAT, DKB, DVB, SPLIT, 0>(tq, tk, tv, ty, p, grid, stream)
+  if (lat == 0) FLARE_TC_MODES(0);
+  if constexpr (!SPLIT) {
+    if (lat == 2) FLARE_TC_MODES(2);
+  }
+  FLARE_TC_MODES(1);
+#undef FLARE_TC_MODES
 #endif
 }
 
@@ -1279,14 +1375,14 @@ int launch_prefill_tc_unit<FLARE_TC_UNIT>(bool padded, int mode, const CUtensorM
 
 __device__ int g_tc_error = 0;
 
-template <> int launch_prefill_tc_unit<0>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<1>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<2>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<3>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<4>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<5>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<6>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<7>(bool, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<0>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<1>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<2>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<3>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<4>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<5>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<6>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+template <> int launch_prefill_tc_unit<7>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
 
 // -------------------------------------------------------------------------------------------------
 // host side
@@ -1380,20 +1476,44 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __re
 
 int prefill_tc_latent_groups(const flare_fwd_args_t* a) { return (a->M + M - 1) / M; }
 
-// (128, 128) heads: two CTAs per (lane, group), each repeating the score / E / R work for 64 value columns, while
-// they all fit the SMs at once; beyond that the wide instance, one CTA for all 128 columns.  (Not for a padded
-// latent bank.)  FLARE_B200_WIDE=0 / 1 forces the choice.
-bool prefill_tc_wide(const flare_fwd_args_t* a, int nseg_grid) {
-  if (a->Dk != 128 || a->Dv != 128 || (a->M % M) != 0) return false;
-  if (const char* env = getenv("FLARE_B200_WIDE")) return env[0] == '1';
-  return (int64_t)a->B * a->H * nseg_grid * prefill_tc_latent_groups(a) * 2 > sm_count();
-}
+int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide) { return prefill_tc_latent_groups(a) * (wide ? 1 : a->Dv / D); }
 
-int prefill_tc_grid_z(const flare_fwd_args_t* a, int nseg_grid) {
-  return prefill_tc_latent_groups(a) * (prefill_tc_wide(a, nseg_grid) ? 1 : a->Dv / D);
+// Which instance of the (128, 128) head shape runs - two CTAs per (lane, latent group), each repeating the score / E / R
+// work for 64 value columns, or the wide one, one CTA for all 128 columns (not for a padded latent bank) - and into how
+// many sequence segments a lane is cut: whatever an estimate of the call's time makes shortest.  Segments cost a state-only
+// pass over all but the last and a scan of the segment states, and are taken only as far as all CTAs run in ONE wave (64
+// lanes in 3 segments = 192 CTAs measured 0.140 ms for the read-out pass alone against 0.185 ms unsegmented).
+// The constants are fits to runs on B200 in us per chunk of 128 tokens and pass: two-slice or 64-column instance 2.55
+// (M = 64, 128 at D = 64; M = 128 at D = 128) and 1.4 for its state-only pass, wide 3.2 and 1.3; launch and fill 8, with
+// segments 22 and 3 per MB of segment states.  Measured against the choices of the rule before it (half a wave of CTAs is
+// the most that is cut, at 256 tokens or more per segment; wide only beyond one wave): B=1 H=16 M=128 D=128 N=32768
+// 306 -> 190 us (4 segments of two slices -> 9 wide), B=1 H=32 N=8192 166 -> 124 us, B=1 H=16 M=64 D=64 N=777
+// 32 -> 26 us (3 segments -> 1).
+void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg_out, bool* wide_out) {
+  const int nch = (a->N + C - 1) / C;
+  const int64_t lanes = (int64_t)a->B * a->H;
+  const int sms = sm_count();
+  const bool can_wide = a->Dk == 128 && a->Dv == 128 && (a->M % M) == 0;
+  bool try_wide[2] = {true, can_wide};
+  if (const char* env = getenv("FLARE_B200_WIDE")) {  // 0 / 1 forces the instance
+    try_wide[0] = env[0] != '1' || !can_wide;
+    try_wide[1] = env[0] == '1' && can_wide;
+  }
+  double best = 1e30;
+  for (int w = 0; w < 2; ++w) {
+    if (!try_wide[w]) continue;
+    const double pass = w ? 3.2 : 2.55, state_pass = w ? 1.3 : 1.4;
+    const int64_t ctas = lanes * prefill_tc_grid_z(a, w != 0);
+    const double waves = (double)((ctas + sms - 1) / sms);
+    double t = 8.0 + waves * nch * pass;
+    if (t < best) best = t, *nseg_out = 1, *wide_out = w != 0;
+    if (ctas * 2 > sms) continue;
+    const int most = (int)(sms / ctas) < nch ? (int)(sms / ctas) : nch;
+    const int len = (nch + most - 1) / most, n = (nch + len - 1) / len;  // chunks per segment, segments that many make
+    t = 22.0 + 3e-6 * (double)lanes * n * a->M * a->Dv * 4 + len * (pass + state_pass);
+    if (1.1 * t < best) best = t, *nseg_out = n, *wide_out = w != 0;  // (worth two more launches)
+  }
 }
-
-int prefill_tc_ctas_per_lane(const flare_fwd_args_t* a) { return a->Dv / D * prefill_tc_latent_groups(a); }
 
 // fp16 partial read-outs [groups][B][N][H][Dv], then fp32 weight masses [groups][B][N][H]
 size_t prefill_tc_partial_lw_offset(const flare_fwd_args_t* a) {
@@ -1407,7 +1527,7 @@ size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a) {
   return prefill_tc_partial_lw_offset(a) + (size_t)groups * a->B * a->N * a->H * sizeof(float);
 }
 
-int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_grid, cudaStream_t stream) {
+int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_grid, bool wide, cudaStream_t stream) {
   TcParams p = p_in;
   {
     const int rc = tc_error_word(&p.err);
@@ -1427,7 +1547,7 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
     // latent bank (used by the Dk = 64 instances only; any valid map otherwise)
     const uint64_t dims[3] = {(uint64_t)a->Dk, (uint64_t)a->M, (uint64_t)a->H};
     const int64_t str[2] = {a->q_stride_m, a->q_stride_h};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, a->M <= 64 ? 64u : 128u, 1};
     if (!make_map(&tq, a->q, 3, dims, str, box)) {
       set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (latent bank)");
       return FLARE_ERR_CUDA;
@@ -1445,9 +1565,9 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
     }
   }
   const int groups = prefill_tc_latent_groups(a);
-  const bool padded = (a->M % M) != 0;
+  // packed below 65 latents (see PACK)
+  const int lat = a->M <= 64 ? 2 : ((a->M % M) != 0 ? 1 : 0);
   const int mode = a->variant == FLARE_STABLEMAX ? 2 : (a->block_size > 1 ? 1 : 0);
-  const bool wide = prefill_tc_wide(a, nseg_grid);
   // Read-out rows leave through tiled bulk stores of 32 tokens x 32 columns (64-byte swizzle): into y, or with several
   // latent groups into the dense fp16 partials.  Per-row lengths (rows beyond a length stay untouched) and output
   // strides the tiled copy cannot express fall back to per-thread stores.
@@ -1478,21 +1598,21 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   }
   if (const char* env = getenv("FLARE_B200_ROW_STORES"))  // diagnostic: per-thread row stores instead
     if (env[0] == '1' && !p.cluster_merge) p.y_tma = 0;
-  const dim3 grid(a->B * a->H, nseg_grid, prefill_tc_grid_z(a, nseg_grid));
+  const dim3 grid(a->B * a->H, nseg_grid, prefill_tc_grid_z(a, wide));
   int rc;
   const int combo = a->Dk == 128 ? 1 : (a->Dv == 128 ? 2 : 0);  // (64, 64), (128, 128), (64, 128)
   if (wide)
-    rc = groups > 1 ? launch_prefill_tc_unit<7>(padded, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<6>(padded, mode, tq, tk, tv, ty, p, grid, stream);
+    rc = groups > 1 ? launch_prefill_tc_unit<7>(lat, mode, tq, tk, tv, ty, p, grid, stream)
+                    : launch_prefill_tc_unit<6>(lat, mode, tq, tk, tv, ty, p, grid, stream);
   else if (combo == 0)
-    rc = groups > 1 ? launch_prefill_tc_unit<3>(padded, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<0>(padded, mode, tq, tk, tv, ty, p, grid, stream);
+    rc = groups > 1 ? launch_prefill_tc_unit<3>(lat, mode, tq, tk, tv, ty, p, grid, stream)
+                    : launch_prefill_tc_unit<0>(lat, mode, tq, tk, tv, ty, p, grid, stream);
   else if (combo == 1)
-    rc = groups > 1 ? launch_prefill_tc_unit<4>(padded, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<1>(padded, mode, tq, tk, tv, ty, p, grid, stream);
+    rc = groups > 1 ? launch_prefill_tc_unit<4>(lat, mode, tq, tk, tv, ty, p, grid, stream)
+                    : launch_prefill_tc_unit<1>(lat, mode, tq, tk, tv, ty, p, grid, stream);
   else
-    rc = groups > 1 ? launch_prefill_tc_unit<5>(padded, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<2>(padded, mode, tq, tk, tv, ty, p, grid, stream);
+    rc = groups > 1 ? launch_prefill_tc_unit<5>(lat, mode, tq, tk, tv, ty, p, grid, stream)
+                    : launch_prefill_tc_unit<2>(lat, mode, tq, tk, tv, ty, p, grid, stream);
   if (rc != FLARE_OK || groups == 1 || p.y == nullptr || p.cluster_merge) return rc;
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);

@@ -53,18 +53,16 @@ struct TcParams {
 };
 
 bool prefill_tc_supported(const flare_fwd_args_t* a);
-// CTAs the kernel launches per (lane, segment)
-int prefill_tc_ctas_per_lane(const flare_fwd_args_t* a);
 // scratch for the partial read-outs of the latent groups (0 for M <= 128), and the byte offset of the weight-mass
 // array inside it
 size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a);
 size_t prefill_tc_partial_lw_offset(const flare_fwd_args_t* a);
-// True when a launch of nseg_grid segments takes the wide (128, 128) instance (one CTA for all 128 value columns).
-bool prefill_tc_wide(const flare_fwd_args_t* a, int nseg_grid);
-// grid.z of a launch of nseg_grid segments
-int prefill_tc_grid_z(const flare_fwd_args_t* a, int nseg_grid);
+// segments per lane, and whether the wide (128, 128) instance runs (one CTA for all 128 value columns)
+void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg, bool* wide);
+// grid.z of a launch
+int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide);
 // launches segments 0 .. nseg_grid-1
-int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, cudaStream_t stream);
+int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, bool wide, cudaStream_t stream);
 // device address (current device) of the error word shared by all tensor-core kernels
 int tc_error_word(int** device_address);
 // reads (and optionally clears) the device-side error flag of the tensor-core kernels; synchronises

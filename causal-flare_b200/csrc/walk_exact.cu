@@ -22,7 +22,7 @@ template <int MM_MAX, int DD>
 __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) walk_exact_kernel(const WalkParams p) {
   extern __shared__ __align__(16) float smem_raw[];
   const int lane_id = blockIdx.x;  // (b, h) lane
-  pdl_begin();
+  pdl_wait();
   if (p.gate != nullptr) {
     int raised = 0;
     for (int i = 0; i < p.gate_count; ++i) raised |= p.gate[(int64_t)lane_id * p.gate_stride + i];
