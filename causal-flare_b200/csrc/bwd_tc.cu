@@ -45,6 +45,8 @@ using tc::sigma_fast;
 using tc::swz_chunk_off;
 using tc::warp_arrive;
 
+constexpr int kMaxBwdSegments = 16;
+
 struct BwdTcParams {
   const void* q;  // bf16 latent bank [H, M, Dk]
   int64_t q_stride_h, q_stride_m;
@@ -58,6 +60,12 @@ struct BwdTcParams {
   void* ds;      // bf16 [lanes][npad][2][M]: dS of every token as a hi row and a lo row over the latents (dS = hi + lo)
   void* dv;      // bf16 [B, N, H, Dv] contiguous, or (more than one latent group) bf16 [groups][B][N][H][Dv]
   int groups;
+  // Sequence segments (grid.z = the segments from seg_first on, segment s = chunks seg_begin[s] .. seg_begin[s + 1] - 1).
+  int nseg, seg_first;
+  int lead;       // the CTA of a segment first walks all later chunks for their carries alone (no exchange)
+  int emit_only;  // carries of the segment alone, written to xg / xc in the frame of the chunk before the segment
+  float *xg, *xc;  // [lanes][nseg][M][Dv], [lanes][nseg][M]; null: no exchange
+  int seg_begin[kMaxBwdSegments + 1];
   int* gate;  // per-call gate word (may be null): raised when a carry turns non-finite (inputs outside the numeric domain)
   int* err;
   long long* trace;  // optional diagnostic cycle stamps of CTA (0, 0), see BT_TRACE; null in normal use
@@ -128,7 +136,7 @@ __device__ __forceinline__ bool wait_partner(uint64_t* bar, uint32_t parity, Mis
 // optional cycle trace of CTA (0, 0): [role < 4][chunk step < 8][slot < 8] clock64 stamps (diagnostic hook)
 #define BT_TRACE(role, step, slot)                                                             \
   do {                                                                                         \
-    if (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && (step) < 8)                \
+    if (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (step) < 8) \
       p.trace[((role) * 8 + (step)) * 8 + (slot)] = clock64();                                 \
   } while (0)
 
@@ -163,6 +171,14 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   const int lane_id = blockIdx.x, group = blockIdx.y;
   const int b = lane_id / p.H, h = lane_id % p.H;
   const int nch = p.nch;
+  // This CTA walks the chunks first - 1 .. begin.  Those from full_end on only move the carries (G, Cc): no X, no dV,
+  // no dS.  All barriers run through the same phases in both kinds of chunk.
+  const int seg = p.seg_first + blockIdx.z;
+  const int begin = p.seg_begin[seg], end = p.seg_begin[seg + 1];
+  const int full_end = p.emit_only ? begin : end;
+  const int first = p.lead ? nch : end;
+  const int steps = first - begin;
+  const bool carry_in = p.xg != nullptr && !p.emit_only && seg + 1 < p.nseg;  // carries of the later segments, exchanged
   if ((int)(smem - smem_dyn) + L::OFF_MISC + (int)sizeof(Misc) > L::SMEM_BYTES) {
     // the dynamic shared memory window starts less aligned than this layout can absorb: report, do nothing
     if (tid == 0) atomicOr(p.err, 1);
@@ -214,8 +230,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       prefetch_tensormap(&tm_v);
       prefetch_tensormap(&tm_dy);
       prefetch_tensormap(&tm_u);
-      for (int j = 0; ok && j < nch; ++j) {
-        const int i = nch - 1 - j, t0 = i * C;
+      for (int j = 0; ok && j < steps; ++j) {
+        const int i = first - 1 - j, t0 = i * C;
         const uint32_t pp = (j - 1) & 1;
         // K, V: free once the previous chunk's P / X products (which read the masked A and V) have run
         if (j > 0 && !(ok = wait_or_abort(&misc->px_ready, pp, misc))) break;
@@ -266,8 +282,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 
       ok = wait_or_abort(&misc->q_ready, 0, misc);  // the latent bank is in tensor memory
       tc_fence_after_sync();
-      for (int j = 0; ok && j < nch; ++j) {
+      for (int j = 0; ok && j < steps; ++j) {
         const uint32_t par = j & 1, pp = (j - 1) & 1;
+        const bool full = first - 1 - j < full_end;
+        const uint32_t fpar = (j - (first - full_end)) & 1;  // parity among the full chunks
+        const uint32_t have = (j > 0 || carry_in) ? 1u : 0u;  // G holds something
         // scores S^T = Q K^T -> T1 (the previous chunk's X has been read)
         if (!(ok = wait_or_abort(&misc->k_full, par, misc))) break;
         if (j > 0 && !(ok = wait_or_abort(&misc->x_done, pp, misc))) break;
@@ -296,31 +315,35 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         for (int s = 0; s < 4 * DVB; ++s) mma_ss(tmem + T0, kmaj_step(d_u_k, s), kmaj_step(d_dy_k, s), ID_SS, s > 0);
 #pragma unroll
         for (int s = 0; s < 8; ++s) mma_ss(tmem + T0, kmaj_step(d_e_k, s), mnmaj_step(d_am_mn, s), ID_PE, 1);
-        if (j > 0) {
+        if (full) {
+          if (have) {
 #pragma unroll
-          for (int s = 0; s < 4 * DVB; ++s) mma_ss(tmem + T1, kmaj_step(d_g_k, s), kmaj_step(d_v_k, s), ID_SS, s > 0);
+            for (int s = 0; s < 4 * DVB; ++s) mma_ss(tmem + T1, kmaj_step(d_g_k, s), kmaj_step(d_v_k, s), ID_SS, s > 0);
+          }
+#pragma unroll
+          for (int s = 0; s < 8; ++s) mma_ss(tmem + T1, kmaj_step(d_r_k, s), kmaj_step(d_am_k, s), ID_SS, s > 0 ? 1u : have);
         }
-#pragma unroll
-        for (int s = 0; s < 8; ++s) mma_ss(tmem + T1, kmaj_step(d_r_k, s), kmaj_step(d_am_k, s), ID_SS, (j > 0 || s > 0) ? 1u : 0u);
         tc_commit(&misc->px_ready);
 #pragma unroll
         for (int s = 0; s < 8; ++s)
-          mma_ss(tmem + TG, kmaj_step(d_r_k, s), mnmaj_step(d_dy_mn, s), ID_G, (j > 0 || s > 0) ? 1u : 0u);
+          mma_ss(tmem + TG, kmaj_step(d_r_k, s), mnmaj_step(d_dy_mn, s), ID_G, s > 0 ? 1u : have);
         tc_commit(&misc->g_ready);
-        // W^T = E^T R -> T0 (P has been read)
+        if (!full) tc_commit(&misc->dv_ready);  // (no dV: E, R and dY have been read)
+        // W^T = E^T R -> T0 (P has been read; the wt_ready / wm_done phases count the full chunks only)
         if (!(ok = wait_or_abort(&misc->p_free, par, misc))) break;
         tc_fence_after_sync();
         BT_TRACE(2, j, 3);
+        if (!full) continue;
         for (int s = 0; s < ksm; ++s) mma_ss(tmem + T0, mnmaj_step(d_e_mn, s), mnmaj_step(d_r_mn, s), ID_WT, s > 0);
         tc_commit(&misc->wt_ready);
         // dV = E^T G + (masked W^T) dY -> T0
-        if (!(ok = wait_or_abort(&misc->wm_done, par, misc))) break;
+        if (!(ok = wait_or_abort(&misc->wm_done, fpar, misc))) break;
         tc_fence_after_sync();
         BT_TRACE(2, j, 4);
-        if (j > 0)
+        if (have)
           for (int s = 0; s < ksm; ++s) mma_ss(tmem + T0, mnmaj_step(d_e_mn, s), mnmaj_step(d_g_mn, s), ID_DV1, s > 0);
 #pragma unroll
-        for (int s = 0; s < 8; ++s) mma_ts(tmem + T0, tmem + T2 + s * 8, mnmaj_step(d_dy_mn, s), ID_DV2, (j > 0 || s > 0) ? 1u : 0u);
+        for (int s = 0; s < 8; ++s) mma_ts(tmem + T0, tmem + T2 + s * 8, mnmaj_step(d_dy_mn, s), ID_DV2, s > 0 ? 1u : have);
         tc_commit(&misc->dv_ready);
       }
     }
@@ -353,7 +376,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         tmem_wait_st();
       }
       tc_fence_before_sync();
-      warp_arrive(&misc->q_ready, lane);
+      if (!carry_in) warp_arrive(&misc->q_ready, lane);
     }
     float cc_carry = 0.f;  // Cc: sum over later chunks of R p, in the current chunk's frame
     const int64_t stat0 = (int64_t)lane_id * nch * p.M + mg;
@@ -365,6 +388,46 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const int gcol = tq * GCOLS;
     uint8_t* const g_dst = smem + L::OFF_GC + (gcol >> 6) * 16384;
     const int gch0 = (gcol & 63) >> 3;
+    if (carry_in) {
+      // Carries of the later segments, summed from the last one on: every segment's are in the frame of the chunk before
+      // it, and the frames only grow with the chunk, so the factors between them never exceed 1.
+      float g[GCOLS];
+#pragma unroll
+      for (int k = 0; k < GCOLS; ++k) g[k] = 0.f;
+      if (live) {
+        float c_from = 0.f;
+        for (int s = p.nseg - 1; s > seg; --s) {
+          const int64_t xo = ((int64_t)lane_id * p.nseg + s) * p.M + mg;
+          const float c_to = STABLE ? 0.f : __ldg(p.chunk_c + stat0 + (int64_t)(p.seg_begin[s] - 1) * p.M);
+          const float f = s == p.nseg - 1 ? 0.f : (STABLE ? 1.f : ex2_approx(c_to - c_from));
+          c_from = c_to;
+          cc_carry = fmaf(cc_carry, f, p.xc[xo]);
+          const float4* src = reinterpret_cast<const float4*>(p.xg + xo * DV + gcol);
+#pragma unroll
+          for (int k = 0; k < GCOLS / 4; ++k) {
+            const float4 x = src[k];
+            g[4 * k] = fmaf(g[4 * k], f, x.x);
+            g[4 * k + 1] = fmaf(g[4 * k + 1], f, x.y);
+            g[4 * k + 2] = fmaf(g[4 * k + 2], f, x.z);
+            g[4 * k + 3] = fmaf(g[4 * k + 3], f, x.w);
+          }
+        }
+      }
+      uint32_t r[GCOLS];
+#pragma unroll
+      for (int k = 0; k < GCOLS; ++k) r[k] = __float_as_uint(g[k]);
+      if constexpr (DVB == 2) tmem_st32(tl + TG + gcol, r);
+      else tmem_st16(tl + TG + gcol, r);
+#pragma unroll
+      for (int ch = 0; ch < GCOLS / 8; ++ch)
+        *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) =
+            make_uint4(pack_bf16(g[ch * 8 + 0], g[ch * 8 + 1]), pack_bf16(g[ch * 8 + 2], g[ch * 8 + 3]),
+                       pack_bf16(g[ch * 8 + 4], g[ch * 8 + 5]), pack_bf16(g[ch * 8 + 6], g[ch * 8 + 7]));
+      tmem_wait_st();
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      warp_arrive(&misc->q_ready, lane);
+    }
 
     if (!__any_sync(0xffffffffu, live)) {
       // A warp whose 32 latents all lie beyond M (M <= 96, or the ragged last group): its operand rows are zero for
@@ -378,7 +441,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       for (int ch = 0; ch < GCOLS / 8; ++ch)
         *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) = make_uint4(0, 0, 0, 0);
       fence_proxy_async_smem();
-      for (int j = 0; ok && j < nch; ++j) {
+      for (int j = 0; ok && j < steps; ++j) {
         const uint32_t par = j & 1, pp = (j - 1) & 1;
         if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
         if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
@@ -386,24 +449,32 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         if (!(ok = wait_or_abort(&misc->px_ready, par, misc))) break;
         warp_arrive(&misc->p_free, lane);
         warp_arrive(&misc->x_done, lane);
-        if (j + 1 < nch) {
+        if (j + 1 < steps) {
           if (!(ok = wait_or_abort(&misc->dv_ready, par, misc))) break;
           warp_arrive(&misc->gc_done, lane);
         }
       }
     } else {
+      auto emit_g = [&](const uint32_t(&r)[GCOLS]) {  // this thread's columns of the segment's G, for the segments before
+        if (!live) return;
+        float4* dst = reinterpret_cast<float4*>(p.xg + (((int64_t)lane_id * p.nseg + seg) * p.M + mg) * DV + gcol);
+#pragma unroll
+        for (int k = 0; k < GCOLS / 4; ++k)
+          dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]),
+                               __uint_as_float(r[4 * k + 3]));
+      };
       // Per-chunk statistics of this thread's latent and per-token statistics of this warp's 32 tokens (lane l keeps
       // token tok0 + l; the loops broadcast them with shuffles), all fetched one chunk ahead so that the global-memory
       // latency never sits between two phases.
       const float* const l2_row = p.tok_l2 + (int64_t)lane_id * p.npad + tok0 + lane;
       const float* const dl_row = p.tok_delta + (int64_t)lane_id * p.npad + tok0 + lane;
-      float c_cur = (live && !STABLE) ? __ldg(p.chunk_c + stat0 + (int64_t)(nch - 1) * p.M) : 0.f;
-      float d_cur = live ? __ldg(p.chunk_d + stat0 + (int64_t)(nch - 1) * p.M) : 1.f;
-      float c_nxt = (live && !STABLE && nch > 1) ? __ldg(p.chunk_c + stat0 + (int64_t)(nch - 2) * p.M) : c_cur;
-      float l2_cur = __ldg(l2_row + (int64_t)(nch - 1) * C), dl_cur = __ldg(dl_row + (int64_t)(nch - 1) * C);
+      float c_cur = (live && !STABLE) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 1) * p.M) : 0.f;
+      float d_cur = live ? __ldg(p.chunk_d + stat0 + (int64_t)(first - 1) * p.M) : 1.f;
+      float c_nxt = (live && !STABLE && first > 1) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 2) * p.M) : c_cur;
+      float l2_cur = __ldg(l2_row + (int64_t)(first - 1) * C), dl_cur = __ldg(dl_row + (int64_t)(first - 1) * C);
 
-      for (int j = 0; ok && j < nch; ++j) {
-        const int i = nch - 1 - j, t0 = i * C;
+      for (int j = 0; ok && j < steps; ++j) {
+        const int i = first - 1 - j, t0 = i * C;
         const uint32_t par = j & 1, pp = (j - 1) & 1;
         const int nvalid = min(C, p.N - t0);
         const int lim = live ? nvalid - tok0 : 0;  // tokens of this thread's quarter that exist (may be <= 0)
@@ -564,7 +635,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         }
 
         // ---- phase 2b (descending): encoder part, dS rows to global memory as a hi + lo pair
-        {
+        if (i < full_end) {
           float ccg[2];  // block-causal: Cc + sum of R p from the start of the group's block on
           float cc = cc_carry + rp_later;
           if constexpr (BLOCK) {
@@ -637,7 +708,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           atomicOr(p.err, 2);
           if (p.gate != nullptr) p.gate[0] = 1;
         }
-        if (i > 0) {
+        if (p.emit_only && i == begin && tq == 0 && live)
+          p.xc[((int64_t)lane_id * p.nseg + seg) * p.M + mg] = cc_carry;
+        if (i > begin || p.emit_only) {
           // G has taken this chunk's R dY: rescale this warp's value columns in tensor memory and pack them as bf16.
           // The shared-memory copy is still read by this chunk's dV product, so the packed rows wait in registers
           // until that product has run.
@@ -656,6 +729,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
               for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * phi);
               tmem_st32(tl + TG + gcol, r);
             }
+            if (i == begin) emit_g(r);
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch)
               gv[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
@@ -672,6 +746,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
               for (int k = 0; k < 16; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * phi);
               tmem_st16(tl + TG + gcol, r);
             }
+            if (i == begin) emit_g(r);
 #pragma unroll
             for (int ch = 0; ch < 2; ++ch)
               gv[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
@@ -682,6 +757,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           if (need) tmem_wait_st();
           if (tid == 0) BT_TRACE(3, j, 6);
           if (!(ok = wait_or_abort(&misc->dv_ready, par, misc))) break;
+          if (i == begin) break;
           if (tid == 0) BT_TRACE(0, j, 6);
 #pragma unroll
           for (int ch = 0; ch < GCOLS / 8; ++ch) *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) = gv[ch];
@@ -710,9 +786,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       dv_base = reinterpret_cast<__nv_bfloat16*>(p.dv) + group_off + ((int64_t)b * p.N * p.H + h) * DV;
       dv_stride_n = (int64_t)p.H * DV;
     }
-    for (int j = 0; ok && j < nch; ++j) {
-      const int i = nch - 1 - j, t0 = i * C;
-      const uint32_t par = j & 1;
+    for (int j = 0; ok && j < steps; ++j) {
+      const int i = first - 1 - j, t0 = i * C;
+      const uint32_t par = j & 1, fpar = (j - (first - full_end)) & 1;
       const int nvalid = min(C, p.N - t0);
       // masked A (bf16) into the K tile's buffer
       if (!(ok = wait_or_abort(&misc->a_ready, par, misc))) break;
@@ -749,8 +825,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       tc_fence_before_sync();
       warp_arrive(&misc->am_done, lane);
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 1);
+      if (i >= full_end) {  // carries only: T0 holds nothing of this group's
+        warp_arrive(&misc->dv_free, lane);
+        continue;
+      }
       // masked E^T R (bf16) into tensor memory
-      if (!(ok = wait_or_abort(&misc->wt_ready, par, misc))) break;
+      if (!(ok = wait_or_abort(&misc->wt_ready, fpar, misc))) break;
       tc_fence_after_sync();
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 2);
 #pragma unroll 1
@@ -1142,11 +1222,77 @@ int launch_grads(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMa
 // -------------------------------------------------------------------------------------------------
 bool have_saved(const flare_bwd_args_t& a);  // defined below, with the keep-buffer layout
 
+// Sequence segments of the reverse sweep, one CTA each per (lane, latent group).  A carry-only chunk (scores, E, R, A, P
+// and G, but no X, dV, dS) takes kCarryCost of a full one.
+//  * lead: the CTA of a segment first walks every later chunk carry-only.  Later segments are longer so that all CTAs take
+//    equally long; no second launch, no exchange, bit-identical results.  Good for two or three CTAs per lane.
+//  * exchange: equal segments; a first launch takes the carries of every segment but the first, the second starts from
+//    their sum.  Good when many SMs are idle.
+// Every alternative is estimated in chunks of the longest SM (CTAs per SM x chunks per CTA) and the least one is taken;
+// kExchangeCost stands for the second launch and the carries' way through L2.
+struct SegmentPlan {
+  int n;
+  bool lead;
+  int begin[kMaxBwdSegments + 1];
+};
+// B200: B=4 N=4096 H=16 M=64 D=128 (64 lanes, 2 lead segments) 583 -> 504 us a training step, stablemax B=2 N=1000 H=8
+// M=64 D=64 (16 lanes, 8 segments with an exchange) 170 -> 112 us.
+constexpr double kCarryCost = 0.55, kExchangeCost = 0.6;
+
+SegmentPlan plan_segments(int64_t ctas, int nch) {
+  SegmentPlan pl;
+  pl.n = 1;
+  pl.lead = false;
+  pl.begin[0] = 0;
+  pl.begin[1] = nch;
+  const int64_t sms = sm_count();
+  auto waves = [&](int64_t n) { return (double)((n + sms - 1) / sms); };
+  double best = waves(ctas) * nch * 0.97;  // (a split has to gain more than the estimate's error)
+  for (int s = 2; s <= kMaxBwdSegments && s <= nch; ++s) {
+    if (ctas * s <= sms) {
+      double q = 1.0;
+      for (int k = 0; k < s; ++k) q *= 1.0 - kCarryCost;
+      const double t = nch * kCarryCost / (1.0 - q);
+      SegmentPlan c;
+      c.n = s;
+      c.lead = true;
+      c.begin[s] = nch;
+      double worst = 0.0;
+      bool fits = true;
+      for (int k = s - 1; k >= 0; --k) {
+        const int later = nch - c.begin[k + 1];
+        int len = k == 0 ? c.begin[1] : (int)(t - kCarryCost * later + 0.5);
+        if (len < 1) len = 1;
+        if (len > c.begin[k + 1] - k) fits = false;
+        c.begin[k] = c.begin[k + 1] - len;
+        const double cost = len + kCarryCost * later;
+        if (cost > worst) worst = cost;
+      }
+      if (fits && worst < best) {
+        best = worst;
+        pl = c;
+      }
+    }
+    const int len = (nch + s - 1) / s;
+    if ((nch + len - 1) / len != s) continue;  // the same as a smaller number of segments
+    const double cost = len * (waves(ctas * s) + kCarryCost * waves(ctas * (s - 1))) + kExchangeCost;
+    if (cost < best) {
+      best = cost;
+      pl.n = s;
+      pl.lead = false;
+      for (int k = 0; k <= s; ++k) pl.begin[k] = k * len < nch ? k * len : nch;
+    }
+  }
+  return pl;
+}
+
 struct TcBwdPlan {
   int nch, npad, groups, nsplit, chunks_per_split;
   size_t gate_words, gate_bytes;  // the call's gate word and those of the forward's replay come first
   size_t exact_bytes;  // path AUTO: scratch of the exact pass standing by (shares the space behind the gate words)
   size_t fwd_ws;  // then the forward's own scratch
+  SegmentPlan seg;
+  size_t off_xg, off_xc;  // carries that the segments exchange
   size_t off_y, off_lse, off_l2, off_delta, off_cu, off_cc, off_cd, off_ds, off_dqp, off_dvp, total;
 };
 
@@ -1158,6 +1304,7 @@ TcBwdPlan plan_tc(const flare_bwd_args_t& a) {
   pl.npad = pl.nch * C;
   pl.groups = (f.M + 127) / 128;
   const int64_t lanes = (int64_t)f.B * f.H;
+  pl.seg = plan_segments(lanes * pl.groups, pl.nch);
   int nsplit = (int)(sm_count() / (lanes > 0 ? lanes : 1));
   if (nsplit < 1) nsplit = 1;
   if (nsplit > pl.nch) nsplit = pl.nch;
@@ -1192,6 +1339,9 @@ TcBwdPlan plan_tc(const flare_bwd_args_t& a) {
   pl.off_ds = take((size_t)2 * lanes * f.M * pl.npad * 2);  // a hi and a lo row per token
   pl.off_dqp = take((size_t)f.B * pl.nsplit * f.H * f.M * f.Dk * 4);
   pl.off_dvp = pl.groups > 1 ? take((size_t)pl.groups * f.B * f.N * f.H * f.Dv * 2) : 0;
+  const size_t xrows = pl.seg.n > 1 && !pl.seg.lead ? (size_t)lanes * pl.seg.n * f.M : 0;
+  pl.off_xg = xrows ? take(xrows * f.Dv * 4) : 0;
+  pl.off_xc = xrows ? take(xrows * 4) : 0;
   pl.total = off;
   if (f.path == FLARE_PATH_AUTO) {
     flare_bwd_args_t ex = a;
@@ -1366,13 +1516,27 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     p.gate = gate;
     p.trace = trace_buffer();
     const int mode = f.variant == FLARE_STABLEMAX ? 2 : (f.block_size > 1 ? 1 : 0);
-    const dim3 grid((unsigned)lanes, pl.groups, 1);
-    int rc;
-    if (f.Dk == 128) rc = launch_bwd_tc_unit<1>(mode, tk, tv, tdy, tu, p, grid, stream);
-    else if (f.Dv == 128) rc = launch_bwd_tc_unit<2>(mode, tk, tv, tdy, tu, p, grid, stream);
-    else rc = launch_bwd_tc_unit<0>(mode, tk, tv, tdy, tu, p, grid, stream);
+    p.nseg = pl.seg.n;
+    memcpy(p.seg_begin, pl.seg.begin, sizeof(p.seg_begin));
+    p.lead = pl.seg.lead ? 1 : 0;
+    auto sweep = [&](int seg_first, int emit_only) -> int {
+      p.seg_first = seg_first;
+      p.emit_only = emit_only;
+      const dim3 grid((unsigned)lanes, pl.groups, pl.seg.n - seg_first);
+      count_launches(1);
+      if (f.Dk == 128) return launch_bwd_tc_unit<1>(mode, tk, tv, tdy, tu, p, grid, stream);
+      if (f.Dv == 128) return launch_bwd_tc_unit<2>(mode, tk, tv, tdy, tu, p, grid, stream);
+      return launch_bwd_tc_unit<0>(mode, tk, tv, tdy, tu, p, grid, stream);
+    };
+    int rc = FLARE_OK;
+    if (pl.seg.n > 1 && !pl.seg.lead) {
+      p.xg = reinterpret_cast<float*>(ws + pl.off_xg);
+      p.xc = reinterpret_cast<float*>(ws + pl.off_xc);
+      rc = sweep(1, 1);
+      if (rc != FLARE_OK) return rc;
+    }
+    rc = sweep(0, 0);
     if (rc != FLARE_OK) return rc;
-    count_launches(1);
     if (pl.groups > 1) {
       const int64_t n8 = (int64_t)f.B * f.N * f.H * f.Dv / 8;
       LaunchTimer timer("bwd_tc_sum_groups_kernel", stream);

@@ -213,3 +213,21 @@ def test_decode_shape_all_512_steps_against_oracle():
     z = st["u"] / st["d"][..., None]
     z_ref = (st_ref["u"] / st_ref["d"][..., None]).float()
     assert orc.rel_l2(z.cpu(), z_ref) <= 5e-3 and orc.max_abs(z.cpu(), z_ref) <= 2e-2
+
+
+# Segments of the reverse sweep: 64 to 74 lanes are cut in two and 40 in three, each CTA walking the later chunks for their
+# carries first; few lanes are cut into many that exchange their carries; latents in groups of 128, at most 64 latents packed.
+@pytest.mark.parametrize("B,N,H,M,Dk,Dv,variant,bs", [
+    (4, 700, 16, 64, 64, 64, "softmax", 1), (4, 640, 10, 128, 64, 128, "softmax", 1), (2, 900, 32, 48, 128, 128, "stablemax", 1),
+    (1, 2100, 2, 64, 128, 128, "softmax", 1), (1, 2048, 2, 192, 64, 64, "softmax", 32), (1, 1500, 3, 32, 64, 64, "stablemax", 1),
+    (1, 1024, 2, 64, 64, 128, "softmax", 128), (1, 1024, 2, 16, 64, 64, "softmax", 16),
+])
+def test_segments_of_the_sweep(B, N, H, M, Dk, Dv, variant, bs):
+    q, k, v, dy = orc.make_inputs(B, N, H, M, Dk, Dv, seed0=6, dtype=torch.bfloat16, with_dy=True)
+    kw = dict(variant="stablemax", power=2.0) if variant == "stablemax" else dict(block_size=bs)
+    ref = orc.ar_backward_closed_form(q, k, v, dy, **kw)
+    got = grads(q, k, v, dy, variant=variant, block_size=bs)
+    check_gate(got, ref, f"segments {(B, N, H, M, Dk, Dv, variant, bs)}", rel_l2=SWEEP)
+    again = grads(q, k, v, dy, variant=variant, block_size=bs)
+    assert all(torch.equal(got[key], again[key]) for key in got), "not run-to-run deterministic"
+    assert _ops.device_status() == 0
