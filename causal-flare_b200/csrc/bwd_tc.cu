@@ -15,8 +15,8 @@
 //   dS   = R (P - D delta_t)  +  E slope (X - Cc - sum_{t' >= t} R p)          slope = 1 | sigma'/sigma
 //   dV   = E^T G + (E^T R . vis) dY
 //   G   += R dY,  Cc += sum_t R p,  then both are rescaled by exp2(c_{i-1} - c_i) for the next chunk.
-// dS is written per token as a hi and a lo bf16 row over the latents ([lane][t][2][m], dS = hi + lo, every warp store
-// one contiguous segment); a second tensor-core kernel forms dK = scale dS^T Q per chunk and
+// dS is written per latent as a hi and a lo bf16 row over the tokens ([lane][2][m][t], dS = hi + lo: a latent thread's
+// eight tokens are one 16-byte store each); a second tensor-core kernel forms dK = scale dS^T Q per chunk and
 // dQ = scale sum_t dS K per (lane, split) (fp32 partials, summed in fixed order: no atomics, deterministic).
 //
 // Main kernel, one CTA per (lane, group of 128 latents), 14 warps: 0-7 latent group (thread = latent = TMEM lane,
@@ -57,7 +57,7 @@ struct BwdTcParams {
   float scale, power;
   const float *chunk_c, *chunk_d;  // [lanes][nch][M]
   const float *tok_l2, *tok_delta;  // [lanes][npad]
-  void* ds;      // bf16 [lanes][npad][2][M]: dS of every token as a hi row and a lo row over the latents (dS = hi + lo)
+  void* ds;      // bf16 [lanes][2][M][npad]: dS of every latent as a hi row and a lo row over the tokens (dS = hi + lo)
   void* dv;      // bf16 [B, N, H, Dv] contiguous, or (more than one latent group) bf16 [groups][B][N][H][Dv]
   int groups;
   // Sequence segments (grid.z = the segments from seg_first on, segment s = chunks seg_begin[s] .. seg_begin[s + 1] - 1).
@@ -90,7 +90,6 @@ namespace {
 
 constexpr int C = 128;
 constexpr int LW = 4;                           // latent warps per lane quarter
-constexpr int TOK = C / LW;                     // tokens per latent thread
 constexpr int NT_MAIN = (4 * LW + 4 + 2) * 32;  // latent warps, token warps, MMA issuer, TMA producer
 constexpr int W_TOKEN = 4 * LW, W_MMA = 4 * LW + 4, W_TMA = 4 * LW + 5;  // first token warp, issuer, producer
 constexpr float kLog2e = 1.4426950408889634f;
@@ -120,7 +119,7 @@ struct Misc {
   uint64_t psum[4], prp[4];
   uint32_t tmem_base;
   volatile int abort_flag;
-  float xch[LW][128];  // exchange between the token quarters of a latent row: sums of E, then sums of R p
+  float xch[LW * 128];  // exchange between the token parts of a latent row, [part][latent]: sums of E, then sums of R p
 };
 static_assert(sizeof(Misc) <= 2560, "Misc must leave room for the alignment slack");
 
@@ -156,13 +155,24 @@ __device__ __forceinline__ float slope_from_sigma(float e, float p) {
 #ifdef FLARE_BT_UNIT
 
 // MODE 0: softmax encoder, token-causal; 1: block-causal read-out; 2: stablemax encoder, token-causal
-template <int DKB, int DVB, int MODE>
+// PACK: at most 64 latents would leave half of the 128 tensor-memory lanes, and with them the latent warps of two of the
+//       four schedulers, without work in a kernel that is bound by the instructions of the latent passes.  As in the
+//       forward the bank is laid down twice (rows 0..63 and 64..127): every latent's scores, P and X appear on two lanes, a
+//       thread takes 16 tokens of the chunk instead of 32 and the two lanes share the columns of G (each maintains its own
+//       ones, the others of its lane are never read).  Products over the latents read rows 0..63 only.
+//       B200: training step B=4 N=4096 H=16 M=64 D=128 504 -> 412 us.
+template <int DKB, int DVB, int MODE, bool PACK>
 __global__ void __launch_bounds__(NT_MAIN, 1)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
               const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_u, const BwdTcParams p) {
   using L = BL<DVB>;
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int DV = DVB * 64;
+  constexpr int NP = PACK ? 2 * LW : LW;  // token parts of a chunk = latent warps per 32 latents
+  constexpr int TOK = C / NP;             // tokens per latent thread
+  constexpr int NG = TOK / 16;            // groups of 16 tokens among them
+  constexpr int NCH = TOK / 8;            // 16-byte pieces of its operand rows
+  constexpr int XL = PACK ? 64 : 128;     // latents of an exchange row
   pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -205,8 +215,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_init(&misc->dv_free, 4);
     mbar_init(&misc->gc_done, 4 * LW);
     for (int i = 0; i < 4; ++i) {
-      mbar_init(&misc->psum[i], LW);
-      mbar_init(&misc->prp[i], LW);
+      mbar_init(&misc->psum[i], NP);
+      mbar_init(&misc->prp[i], NP);
     }
     misc->abort_flag = 0;
     fence_barrier_init();
@@ -244,8 +254,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         // U_i: read by the previous chunk's P product (which has run: px_ready above)
         mbar_arrive_expect_tx(&misc->u_full, DVB * 16384);
 #pragma unroll
-        for (int vb = 0; vb < DVB; ++vb)
+        for (int vb = 0; vb < DVB; ++vb) {
           tma_load_4d(smem + L::OFF_UR + vb * 16384, &tm_u, &misc->u_full, vb * 64, group * 128, i, lane_id);
+          if constexpr (PACK)  // (boxes of 64 rows)
+            tma_load_4d(smem + L::OFF_UR + vb * 16384 + 8192, &tm_u, &misc->u_full, vb * 64, 0, i, lane_id);
+        }
         // dY: read by the previous chunk's dV and G products
         if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
         mbar_arrive_expect_tx(&misc->dy_full, DVB * 16384);
@@ -348,18 +361,26 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       }
     }
   } else if (warp < 4 * LW) {
-    // ======== latent group: thread = (latent = TMEM lane, quarter of the chunk's tokens); 4 warps per lane quarter ========
+    // ======== latent group: thread = (latent = TMEM lane, part of the chunk's tokens); 4 warps per lane quarter ========
     const int tq = warp >> 2, q = warp & 3;
     const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
-    const int m = q * 32 + lane;
+    const int m = PACK ? (q & 1) * 32 + lane : q * 32 + lane;  // latent of the group
+    const int tp = PACK ? tq * 2 + (q >> 1) : tq;              // token part
+    const int pq = PACK ? (q & 1) : q;                         // exchange group: the NP warps of the same 32 latents
+    auto xch = [&](int part) -> float& { return misc->xch[part * XL + m]; };
+    // one 16-byte piece of an operand row (packed: of both copies)
+    auto put = [&](uint8_t* rows, int ch, const uint4& v) {
+      *reinterpret_cast<uint4*>(rows + swz_chunk_off(m, ch)) = v;
+      if constexpr (PACK) *reinterpret_cast<uint4*>(rows + 8192 + swz_chunk_off(m, ch)) = v;
+    };
     const int mg = group * 128 + m;
     const bool live = mg < p.M;
     const float sc2 = p.scale * kLog2e;
-    const int tok0 = tq * TOK;
-    // this thread's 32 tokens are 16-byte chunks ch0 .. ch0 + 3 of row m in t-block tq / 2 of the [2][128][64] buffers
-    const int ch0 = (tq & 1) * 4;
-    uint8_t* const e_row = smem + L::OFF_E + (tq >> 1) * 16384;
-    uint8_t* const r_row = smem + L::OFF_R + (tq >> 1) * 16384;
+    const int tok0 = tp * TOK;
+    // this thread's tokens are the 16-byte pieces from ch0 on of row m in t-block tok0 / 64 of the [2][128][64] buffers
+    const int ch0 = (tok0 & 63) >> 3;
+    uint8_t* const e_row = smem + L::OFF_E + (tok0 >> 6) * 16384;
+    uint8_t* const r_row = smem + L::OFF_R + (tok0 >> 6) * 16384;
     {
       // latent bank row -> tensor memory as packed bf16 (element k in column k / 2); each warp of the quarter writes
       // 32 elements of the row (Dk = 64: the first two warps)
@@ -380,12 +401,13 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
     float cc_carry = 0.f;  // Cc: sum over later chunks of R p, in the current chunk's frame
     const int64_t stat0 = (int64_t)lane_id * nch * p.M + mg;
-    // dS rows of this lane: element (token t, part, latent) at (t * 2 + part) * M + latent; a warp's 32 latents are
-    // contiguous, so every store instruction of a warp writes one 64-byte segment
-    __nv_bfloat16* const ds_col = reinterpret_cast<__nv_bfloat16*>(p.ds) + (int64_t)lane_id * p.npad * 2 * p.M + (live ? mg : 0);
-    // value columns of G this warp rescales and repacks: a quarter of them
-    constexpr int GCOLS = DVB * 16;
-    const int gcol = tq * GCOLS;
+    // dS rows of this latent: element (part, latent, token t) of the lane at (part * M + latent) * npad + t.  Token-wise rows
+    // over the latents took a 2-byte store per element and plane, 64 instead of 8 stores per thread and chunk.
+    __nv_bfloat16* const ds_row = reinterpret_cast<__nv_bfloat16*>(p.ds) +
+                                  ((int64_t)lane_id * 2 * p.M + (live ? mg : 0)) * p.npad + tok0;
+    // value columns of G this warp rescales and repacks
+    constexpr int GCOLS = DV / NP;
+    const int gcol = tp * GCOLS;
     uint8_t* const g_dst = smem + L::OFF_GC + (gcol >> 6) * 16384;
     const int gch0 = (gcol & 63) >> 3;
     if (carry_in) {
@@ -416,13 +438,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       uint32_t r[GCOLS];
 #pragma unroll
       for (int k = 0; k < GCOLS; ++k) r[k] = __float_as_uint(g[k]);
-      if constexpr (DVB == 2) tmem_st32(tl + TG + gcol, r);
-      else tmem_st16(tl + TG + gcol, r);
+      tmem_write(tl + TG + gcol, r);
 #pragma unroll
       for (int ch = 0; ch < GCOLS / 8; ++ch)
-        *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) =
+        put(g_dst, gch0 + ch,
             make_uint4(pack_bf16(g[ch * 8 + 0], g[ch * 8 + 1]), pack_bf16(g[ch * 8 + 2], g[ch * 8 + 3]),
-                       pack_bf16(g[ch * 8 + 4], g[ch * 8 + 5]), pack_bf16(g[ch * 8 + 6], g[ch * 8 + 7]));
+                       pack_bf16(g[ch * 8 + 4], g[ch * 8 + 5]), pack_bf16(g[ch * 8 + 6], g[ch * 8 + 7])));
       tmem_wait_st();
       fence_proxy_async_smem();
       tc_fence_before_sync();
@@ -433,13 +454,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       // A warp whose 32 latents all lie beyond M (M <= 96, or the ragged last group): its operand rows are zero for
       // the whole kernel and it only keeps the barrier phases in step with the working warps.
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, ch0 + ch)) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + ch)) = make_uint4(0, 0, 0, 0);
+      for (int ch = 0; ch < NCH; ++ch) {
+        put(e_row, ch0 + ch, make_uint4(0, 0, 0, 0));
+        put(r_row, ch0 + ch, make_uint4(0, 0, 0, 0));
       }
 #pragma unroll
-      for (int ch = 0; ch < GCOLS / 8; ++ch)
-        *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) = make_uint4(0, 0, 0, 0);
+      for (int ch = 0; ch < GCOLS / 8; ++ch) put(g_dst, gch0 + ch, make_uint4(0, 0, 0, 0));
       fence_proxy_async_smem();
       for (int j = 0; ok && j < steps; ++j) {
         const uint32_t par = j & 1, pp = (j - 1) & 1;
@@ -463,11 +483,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]),
                                __uint_as_float(r[4 * k + 3]));
       };
-      // Per-chunk statistics of this thread's latent and per-token statistics of this warp's 32 tokens (lane l keeps
-      // token tok0 + l; the loops broadcast them with shuffles), all fetched one chunk ahead so that the global-memory
+      // Per-chunk statistics of this thread's latent and per-token statistics of this warp's tokens (lane l keeps
+      // token tok0 + l % TOK; the loops broadcast them with shuffles), all fetched one chunk ahead so that the global-memory
       // latency never sits between two phases.
-      const float* const l2_row = p.tok_l2 + (int64_t)lane_id * p.npad + tok0 + lane;
-      const float* const dl_row = p.tok_delta + (int64_t)lane_id * p.npad + tok0 + lane;
+      const float* const l2_row = p.tok_l2 + (int64_t)lane_id * p.npad + tok0 + (lane & (TOK - 1));
+      const float* const dl_row = p.tok_delta + (int64_t)lane_id * p.npad + tok0 + (lane & (TOK - 1));
       float c_cur = (live && !STABLE) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 1) * p.M) : 0.f;
       float d_cur = live ? __ldg(p.chunk_d + stat0 + (int64_t)(first - 1) * p.M) : 1.f;
       float c_nxt = (live && !STABLE && first > 1) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 2) * p.M) : c_cur;
@@ -477,7 +497,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         const int i = first - 1 - j, t0 = i * C;
         const uint32_t par = j & 1, pp = (j - 1) & 1;
         const int nvalid = min(C, p.N - t0);
-        const int lim = live ? nvalid - tok0 : 0;  // tokens of this thread's quarter that exist (may be <= 0)
+        const int lim = live ? nvalid - tok0 : 0;  // tokens of this thread's part that exist (may be <= 0)
         const bool fast = __all_sync(0xffffffffu, lim >= TOK);
         const float c_i = c_cur, d_i = d_cur;
         const float c_prev = i > 0 ? c_nxt : c_i;
@@ -493,15 +513,13 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
         tc_fence_after_sync();
         if (tid == 0) BT_TRACE(0, j, 0);
-        uint32_t rs[32];  // the 32 raw scores of this thread
-        tmem_ld32(tl + T1 + tok0, rs);
-        tmem_wait_ld();
-        tmem_fence_regs(rs);
+        uint32_t rs[TOK];  // the raw scores of this thread
+        tmem_read(tl + T1 + tok0, rs);
         if (tid == 0) BT_TRACE(3, j, 1);
         // ---- phase 1a: E rows (bf16) and their sums
-        float g16[2] = {0.f, 0.f};  // sums of the rounded E per 16 tokens
+        float g16[NG] = {};  // sums of the rounded E per 16 tokens
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
+        for (int ch = 0; ch < NCH; ++ch) {
           float e[8];
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
@@ -515,39 +533,44 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           v.x = pack_bf16(e[0], e[1]); v.y = pack_bf16(e[2], e[3]); v.z = pack_bf16(e[4], e[5]); v.w = pack_bf16(e[6], e[7]);
           g16[ch >> 1] += (bf16_lo(v.x) + bf16_hi(v.x)) + (bf16_lo(v.y) + bf16_hi(v.y)) + (bf16_lo(v.z) + bf16_hi(v.z)) +
                           (bf16_lo(v.w) + bf16_hi(v.w));
-          *reinterpret_cast<uint4*>(e_row + swz_chunk_off(m, ch0 + ch)) = v;
+          put(e_row, ch0 + ch, v);
         }
-        misc->xch[tq][m] = g16[0] + g16[1];
-        warp_arrive(&misc->psum[q], lane);
+        xch(tp) = NG == 2 ? g16[0] + g16[NG - 1] : g16[0];
+        warp_arrive(&misc->psum[pq], lane);
         if (tid == 0) BT_TRACE(3, j, 2);
-        if (!(ok = wait_partner(&misc->psum[q], par, misc))) break;
+        if (!(ok = wait_partner(&misc->psum[pq], par, misc))) break;
         if (tid == 0) BT_TRACE(3, j, 3);
         // denominator before this thread's first token
         float base_run = d_i;
 #pragma unroll
-        for (int t = 0; t < LW - 1; ++t) base_run += t < tq ? misc->xch[t][m] : 0.f;
-        float dend[2], invg[2];  // block-causal: denominator at the end of the block of each 16-token group
+        for (int t = 0; t < NP - 1; ++t) base_run += t < tp ? xch(t) : 0.f;
+        float dend[NG], invg[NG];  // block-causal: denominator at the end of the block of each 16-token group
         if constexpr (BLOCK) {
           const int bs = p.block;
-          const float p0 = base_run + g16[0], p1 = p0 + g16[1];
-          if (bs == 16) { dend[0] = p0; dend[1] = p1; }
-          else if (bs == 32) { dend[0] = dend[1] = p1; }
-          else {
-            // blocks of 64 or 128 tokens end in a later quarter: add the quarters up to the block's last one
-            const int last = bs == 64 ? (tq | 1) : LW - 1;
-            float tot = p1;
+          if (bs <= TOK) {  // the blocks end inside this part
+            const float p0 = base_run + g16[0];
+            dend[0] = p0;
+            if constexpr (NG == 2) {
+              dend[1] = p0 + g16[1];
+              if (bs == 32) dend[0] = dend[1];
+            }
+          } else {
+            // the block ends in a later part (or with this one): add the parts up to its last one
+            const int last = tp | (bs / TOK - 1);
+            float tot = base_run + xch(tp);
 #pragma unroll
-            for (int t = 1; t < LW; ++t) tot += (t > tq && t <= last) ? misc->xch[t][m] : 0.f;
-            dend[0] = dend[1] = tot;
+            for (int t = 1; t < NP; ++t) tot += (t > tp && t <= last) ? xch(t) : 0.f;
+#pragma unroll
+            for (int g = 0; g < NG; ++g) dend[g] = tot;
           }
-          invg[0] = rcp_approx(dend[0]);
-          invg[1] = rcp_approx(dend[1]);
+#pragma unroll
+          for (int g = 0; g < NG; ++g) invg[g] = rcp_approx(dend[g]);
         }
         // ---- phase 1b: R = g / D rows (bf16)
         {
           float run = base_run;
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
+          for (int ch = 0; ch < NCH; ++ch) {
             const uint4 ev = *reinterpret_cast<const uint4*>(e_row + swz_chunk_off(m, ch0 + ch));
             float r[8];
 #pragma unroll
@@ -566,8 +589,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
               if (!fast) x = k < lim ? x : 0.f;
               r[jj] = x;
             }
-            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + ch)) =
-                make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7]));
+            put(r_row, ch0 + ch,
+                make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7])));
           }
         }
         fence_proxy_async_smem();
@@ -579,18 +602,16 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         if (!(ok = wait_or_abort(&misc->px_ready, par, misc))) break;
         tc_fence_after_sync();
         if (tid == 0) BT_TRACE(0, j, 2);
-        uint32_t pd[32];   // P accumulators of the 32 tokens, replaced in place by the decode-side dS (fp32)
-        uint32_t rpk[16];  // R p, packed bf16 pairs
-        float rg16[2] = {0.f, 0.f};  // sums of the rounded R p per 16 tokens
-        tmem_ld32(tl + T0 + tok0, pd);
-        tmem_wait_ld();
-        tmem_fence_regs(pd);
+        uint32_t pd[TOK];       // P accumulators of the tokens, replaced in place by the decode-side dS (fp32)
+        uint32_t rpk[TOK / 2];  // R p, packed bf16 pairs
+        float rg16[NG] = {};    // sums of the rounded R p per 16 tokens
+        tmem_read(tl + T0 + tok0, pd);
         tc_fence_before_sync();
         warp_arrive(&misc->p_free, lane);  // T0 may take E^T R
         {
           float run = base_run;
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
+          for (int ch = 0; ch < NCH; ++ch) {
             const uint4 ev = *reinterpret_cast<const uint4*>(e_row + swz_chunk_off(m, ch0 + ch));
             const uint4 rv = *reinterpret_cast<const uint4*>(r_row + swz_chunk_off(m, ch0 + ch));
             float rp[8];
@@ -621,44 +642,46 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           }
         }
         if (tid == 0) BT_TRACE(0, j, 3);
-        const float rp_mine = rg16[0] + rg16[1];
-        misc->xch[tq][m] = rp_mine;
-        warp_arrive(&misc->prp[q], lane);
-        if (!(ok = wait_partner(&misc->prp[q], par, misc))) break;
+        const float rp_mine = NG == 2 ? rg16[0] + rg16[NG - 1] : rg16[0];
+        xch(tp) = rp_mine;
+        warp_arrive(&misc->prp[pq], lane);
+        if (!(ok = wait_partner(&misc->prp[pq], par, misc))) break;
         if (tid == 0) BT_TRACE(3, j, 4);
-        float rp_later = 0.f, rp_all = 0.f;  // R p of the quarters after this one, and of the whole chunk
+        float rp_later = 0.f, rp_all = 0.f;  // R p of the parts after this one, and of the whole chunk
 #pragma unroll
-        for (int t = 0; t < LW; ++t) {
-          const float x = misc->xch[t][m];
+        for (int t = 0; t < NP; ++t) {
+          const float x = xch(t);
           rp_all += x;
-          rp_later += t > tq ? x : 0.f;
+          rp_later += t > tp ? x : 0.f;
         }
 
         // ---- phase 2b (descending): encoder part, dS rows to global memory as a hi + lo pair
         if (i < full_end) {
-          float ccg[2];  // block-causal: Cc + sum of R p from the start of the group's block on
+          float ccg[NG];  // block-causal: Cc + sum of R p from the start of the group's block on
           float cc = cc_carry + rp_later;
           if constexpr (BLOCK) {
             const int bs = p.block;
-            if (bs == 16) { ccg[1] = cc + rg16[1]; ccg[0] = ccg[1] + rg16[0]; }
-            else if (bs == 32) { ccg[0] = ccg[1] = cc + rp_mine; }
-            else {
-              // the block starts in an earlier (or this) quarter: add the quarters from its first one on
-              const int first = bs == 64 ? (tq & ~1) : 0;
+            if (bs <= TOK) {
+              ccg[NG - 1] = cc + rg16[NG - 1];
+              if constexpr (NG == 2) {
+                ccg[0] = ccg[1] + rg16[0];
+                if (bs == 32) ccg[1] = ccg[0];
+              }
+            } else {
+              // the block starts in an earlier (or this) part: add the parts from its first one on
+              const int from = tp & ~(bs / TOK - 1);
               float tot = cc + rp_mine;
 #pragma unroll
-              for (int t = 0; t < LW - 1; ++t) tot += (t >= first && t < tq) ? misc->xch[t][m] : 0.f;
-              ccg[0] = ccg[1] = tot;
+              for (int t = 0; t < NP - 1; ++t) tot += (t >= from && t < tp) ? xch(t) : 0.f;
+#pragma unroll
+              for (int g = 0; g < NG; ++g) ccg[g] = tot;
             }
           }
-          __nv_bfloat16* const dst = ds_col + (int64_t)(t0 + tok0) * 2 * p.M;
-          const int64_t tstride = 2 * (int64_t)p.M;
+          __nv_bfloat16* const dst = ds_row + t0;
 #pragma unroll
-          for (int blk = 1; blk >= 0; --blk) {
+          for (int blk = NG - 1; blk >= 0; --blk) {
             uint32_t xr[16];
-            tmem_ld16(tl + T1 + tok0 + blk * 16, xr);
-            tmem_wait_ld();
-            tmem_fence_regs16(xr);
+            tmem_read(tl + T1 + tok0 + blk * 16, xr);
 #pragma unroll
             for (int c2 = 1; c2 >= 0; --c2) {
               const int ch = blk * 2 + c2;
@@ -682,15 +705,15 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                 ds[jj] = __uint_as_float(pd[k]) + ((STABLE && eb == 0.f) ? 0.f : enc);
               }
               // dS = hi + lo, two bf16 values: the dK / dQ products then see it with 16 mantissa bits
-              if (live) {
+              uint32_t hi[4], lo[4];
 #pragma unroll
-                for (int jj = 0; jj < 8; ++jj) {
-                  const __nv_bfloat16 hi = __float2bfloat16_rn(ds[jj]);
-                  const __nv_bfloat16 lo = __float2bfloat16_rn(ds[jj] - __bfloat162float(hi));
-                  __nv_bfloat16* d = dst + (int64_t)(ch * 8 + jj) * tstride;
-                  d[0] = hi;
-                  d[p.M] = lo;
-                }
+              for (int jj = 0; jj < 8; jj += 2) {
+                hi[jj >> 1] = pack_bf16(ds[jj], ds[jj + 1]);
+                lo[jj >> 1] = pack_bf16(ds[jj] - bf16_lo(hi[jj >> 1]), ds[jj + 1] - bf16_hi(hi[jj >> 1]));
+              }
+              if (live) {
+                *reinterpret_cast<uint4*>(dst + ch * 8) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(dst + (int64_t)p.M * p.npad + ch * 8) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
               }
             }
           }
@@ -708,7 +731,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           atomicOr(p.err, 2);
           if (p.gate != nullptr) p.gate[0] = 1;
         }
-        if (p.emit_only && i == begin && tq == 0 && live)
+        if (p.emit_only && i == begin && tp == 0 && live)
           p.xc[((int64_t)lane_id * p.nseg + seg) * p.M + mg] = cc_carry;
         if (i > begin || p.emit_only) {
           // G has taken this chunk's R dY: rescale this warp's value columns in tensor memory and pack them as bf16.
@@ -719,48 +742,27 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           if (tid == 0) BT_TRACE(0, j, 5);
           const bool need = __any_sync(0xffffffffu, phi != 1.0f);
           uint4 gv[GCOLS / 8];
-          if constexpr (DVB == 2) {
-            uint32_t r[32];
-            tmem_ld32(tl + TG + gcol, r);
-            tmem_wait_ld();
-            tmem_fence_regs(r);
-            if (need) {
+          uint32_t r[GCOLS];
+          tmem_read(tl + TG + gcol, r);
+          if (need) {
 #pragma unroll
-              for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * phi);
-              tmem_st32(tl + TG + gcol, r);
-            }
-            if (i == begin) emit_g(r);
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch)
-              gv[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7])));
-          } else {
-            uint32_t r[16];
-            tmem_ld16(tl + TG + gcol, r);
-            tmem_wait_ld();
-            tmem_fence_regs16(r);
-            if (need) {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * phi);
-              tmem_st16(tl + TG + gcol, r);
-            }
-            if (i == begin) emit_g(r);
-#pragma unroll
-            for (int ch = 0; ch < 2; ++ch)
-              gv[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5])),
-                                  pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7])));
+            for (int k = 0; k < GCOLS; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * phi);
+            tmem_write(tl + TG + gcol, r);
           }
+          if (i == begin) emit_g(r);
+#pragma unroll
+          for (int ch = 0; ch < GCOLS / 8; ++ch)
+            gv[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
+                                pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3])),
+                                pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5])),
+                                pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7])));
           if (need) tmem_wait_st();
           if (tid == 0) BT_TRACE(3, j, 6);
           if (!(ok = wait_or_abort(&misc->dv_ready, par, misc))) break;
           if (i == begin) break;
           if (tid == 0) BT_TRACE(0, j, 6);
 #pragma unroll
-          for (int ch = 0; ch < GCOLS / 8; ++ch) *reinterpret_cast<uint4*>(g_dst + swz_chunk_off(m, gch0 + ch)) = gv[ch];
+          for (int ch = 0; ch < GCOLS / 8; ++ch) put(g_dst, gch0 + ch, gv[ch]);
           fence_proxy_async_smem();
           tc_fence_before_sync();
           warp_arrive(&misc->gc_done, lane);
@@ -899,10 +901,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 
 namespace {
 
-template <int DKB, int DVB, int MODE>
+template <int DKB, int DVB, int MODE, bool PACK>
 int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy, const CUtensorMap& tu,
                 const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
-  auto kern = bwd_tc_kernel<DKB, DVB, MODE>;
+  auto kern = bwd_tc_kernel<DKB, DVB, MODE, PACK>;
   static int granted[64] = {};
   FLARE_CUDA_CHECK(allow_smem(kern, BL<DVB>::SMEM_BYTES, granted));
   LaunchTimer timer("bwd_tc_kernel", stream);
@@ -915,12 +917,14 @@ int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap&
 template <>
 int launch_bwd_tc_unit<FLARE_BT_UNIT>(int mode, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy,
                                       const CUtensorMap& tu, const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
-  // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128)
-  constexpr int DKB = FLARE_BT_UNIT == 1 ? 2 : 1;
-  constexpr int DVB = FLARE_BT_UNIT == 0 ? 1 : 2;
-  if (mode == 1) return launch_main<DKB, DVB, 1>(tk, tv, tdy, tu, p, grid, stream);
-  if (mode == 2) return launch_main<DKB, DVB, 2>(tk, tv, tdy, tu, p, grid, stream);
-  return launch_main<DKB, DVB, 0>(tk, tv, tdy, tu, p, grid, stream);
+  // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128); units 3..5: the same, packed
+  constexpr int W = FLARE_BT_UNIT % 3;
+  constexpr int DKB = W == 1 ? 2 : 1;
+  constexpr int DVB = W == 0 ? 1 : 2;
+  constexpr bool PACK = FLARE_BT_UNIT >= 3;
+  if (mode == 1) return launch_main<DKB, DVB, 1, PACK>(tk, tv, tdy, tu, p, grid, stream);
+  if (mode == 2) return launch_main<DKB, DVB, 2, PACK>(tk, tv, tdy, tu, p, grid, stream);
+  return launch_main<DKB, DVB, 0, PACK>(tk, tv, tdy, tu, p, grid, stream);
 }
 
 #else  // host side, the dK / dQ kernel and the small helper kernels
@@ -928,6 +932,9 @@ int launch_bwd_tc_unit<FLARE_BT_UNIT>(int mode, const CUtensorMap& tk, const CUt
 template <> int launch_bwd_tc_unit<0>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
 template <> int launch_bwd_tc_unit<1>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
 template <> int launch_bwd_tc_unit<2>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
+template <> int launch_bwd_tc_unit<3>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
+template <> int launch_bwd_tc_unit<4>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
+template <> int launch_bwd_tc_unit<5>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
 
 namespace {
 
@@ -1015,7 +1022,7 @@ constexpr int GRAD_MAXG = 4;
 
 template <int DKB>
 struct GL {
-  static constexpr int OFF_DS = 0;                         // 2 stages x [2 m-blocks][128 t][64 m]
+  static constexpr int OFF_DS = 0;                         // 2 stages x [2 t-blocks][128 m][64 t]
   static constexpr int OFF_K = 65536;                      // 2 stages x [DKB][128 t][64]
   static constexpr int OFF_Q = OFF_K + 2 * DKB * 16384;    // groups x [DKB][128 m][64]
   static constexpr int off_misc(int groups) { return OFF_Q + groups * DKB * 16384; }
@@ -1094,8 +1101,8 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
           const int s = it & 1;
           if (it >= 2 && !(ok = wait(&misc->ds_empty[s], ((it - 2) >> 1) & 1))) break;
           mbar_arrive_expect_tx(&misc->ds_full[s], 32768);
-          for (int mb = 0; mb < 2; ++mb)
-            tma_load_4d(smem + L::OFF_DS + s * 32768 + mb * 16384, &tm_ds, &misc->ds_full[s], g * 128 + mb * 64, part, t0,
+          for (int tb = 0; tb < 2; ++tb)  // (rows beyond M read as zero)
+            tma_load_4d(smem + L::OFF_DS + s * 32768 + tb * 16384, &tm_ds, &misc->ds_full[s], t0 + tb * 64, g * 128, part,
                         lane_id);
         }
       }
@@ -1103,8 +1110,8 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t ID_DK = make_idesc_bf16(128, DK, 0, 1);  // dS (K-major: rows = tokens, latents contiguous) x Q (MN-major)
-      constexpr uint32_t ID_DQ = make_idesc_bf16(128, DK, 1, 1);  // dS (MN-major) x K tile (MN-major)
+      constexpr uint32_t ID_DK = make_idesc_bf16(128, DK, 1, 1);  // dS (MN-major: tokens contiguous) x Q (MN-major)
+      constexpr uint32_t ID_DQ = make_idesc_bf16(128, DK, 0, 1);  // dS (K-major: rows = latents) x K tile (MN-major)
       ok = wait(&misc->q_full, 0);
       int it = 0;
       for (int cc = 0; ok && cc < ncs; ++cc) {
@@ -1124,10 +1131,10 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
           const int rows = min(128, p.M - g * 128);
           const int ksm = (rows + 15) >> 4;
           for (int st = 0; st < ksm; ++st)  // contraction over the latents of the group
-            mma_ss(tmem + L::TM_DK + kb * DK, kmaj_step(d_ds_k, st), mnmaj_step(d_q_mn, st), ID_DK, (gp > 0 || st > 0) ? 1u : 0u);
+            mma_ss(tmem + L::TM_DK + kb * DK, mnmaj_step(d_ds_mn, st), mnmaj_step(d_q_mn, st), ID_DK, (gp > 0 || st > 0) ? 1u : 0u);
 #pragma unroll
           for (int st = 0; st < 8; ++st)  // contraction over the tokens of the chunk
-            mma_ss(tmem + L::TM_DQ + g * DK, mnmaj_step(d_ds_mn, st), mnmaj_step(d_k_mn, st), ID_DQ,
+            mma_ss(tmem + L::TM_DQ + g * DK, kmaj_step(d_ds_k, st), mnmaj_step(d_k_mn, st), ID_DQ,
                    (cc > 0 || (gp & 1) || st > 0) ? 1u : 0u);
           tc_commit(&misc->ds_empty[s]);
         }
@@ -1336,7 +1343,7 @@ TcBwdPlan plan_tc(const flare_bwd_args_t& a) {
   pl.off_cu = saved ? 0 : take((size_t)lanes * pl.nch * f.M * f.Dv * 2);
   pl.off_cc = saved ? 0 : take((size_t)lanes * pl.nch * f.M * 4);
   pl.off_cd = saved ? 0 : take((size_t)lanes * pl.nch * f.M * 4);
-  pl.off_ds = take((size_t)2 * lanes * f.M * pl.npad * 2);  // a hi and a lo row per token
+  pl.off_ds = take((size_t)2 * lanes * f.M * pl.npad * 2);  // a hi and a lo row per latent
   pl.off_dqp = take((size_t)f.B * pl.nsplit * f.H * f.M * f.Dk * 4);
   pl.off_dvp = pl.groups > 1 ? take((size_t)pl.groups * f.B * f.N * f.H * f.Dv * 2) : 0;
   const size_t xrows = pl.seg.n > 1 && !pl.seg.lead ? (size_t)lanes * pl.seg.n * f.M : 0;
@@ -1478,6 +1485,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     if (rc != FLARE_OK) return rc;
   }
   // (3) reverse chunk sweep: dV and the dS plane
+  const bool pack = f.M <= 64;
   CUtensorMap tk, tv, tdy, tu, tds, tq;
   {
     const uint64_t dimk[4] = {(uint64_t)f.Dk, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B};
@@ -1488,10 +1496,10 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     const int64_t strd[3] = {a.dy_stride_h, a.dy_stride_n, a.dy_stride_b};
     const uint64_t dimu[4] = {(uint64_t)f.Dv, (uint64_t)f.M, (uint64_t)pl.nch, (uint64_t)lanes};
     const int64_t stru[3] = {f.Dv, (int64_t)f.M * f.Dv, (int64_t)pl.nch * f.M * f.Dv};
-    const uint32_t boxu[4] = {64, 128, 1, 1};
-    const uint64_t dims[4] = {(uint64_t)f.M, 2, (uint64_t)pl.npad, (uint64_t)lanes};
-    const int64_t strs[3] = {f.M, 2 * (int64_t)f.M, 2 * (int64_t)f.M * pl.npad};
-    const uint32_t boxs[4] = {64, 1, 128, 1};
+    const uint32_t boxu[4] = {64, pack ? 64u : 128u, 1, 1};
+    const uint64_t dims[4] = {(uint64_t)pl.npad, (uint64_t)f.M, 2, (uint64_t)lanes};
+    const int64_t strs[3] = {pl.npad, (int64_t)f.M * pl.npad, 2 * (int64_t)f.M * pl.npad};
+    const uint32_t boxs[4] = {64, 128, 1, 1};
     const uint64_t dimq[3] = {(uint64_t)f.Dk, (uint64_t)f.M, (uint64_t)f.H};
     const int64_t strq[2] = {f.q_stride_m, f.q_stride_h};
     const uint32_t boxq[3] = {64, 128, 1};
@@ -1524,9 +1532,10 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
       p.emit_only = emit_only;
       const dim3 grid((unsigned)lanes, pl.groups, pl.seg.n - seg_first);
       count_launches(1);
-      if (f.Dk == 128) return launch_bwd_tc_unit<1>(mode, tk, tv, tdy, tu, p, grid, stream);
-      if (f.Dv == 128) return launch_bwd_tc_unit<2>(mode, tk, tv, tdy, tu, p, grid, stream);
-      return launch_bwd_tc_unit<0>(mode, tk, tv, tdy, tu, p, grid, stream);
+      const auto launch = f.Dk == 128   ? (pack ? launch_bwd_tc_unit<4> : launch_bwd_tc_unit<1>)
+                          : f.Dv == 128 ? (pack ? launch_bwd_tc_unit<5> : launch_bwd_tc_unit<2>)
+                                        : (pack ? launch_bwd_tc_unit<3> : launch_bwd_tc_unit<0>);
+      return launch(mode, tk, tv, tdy, tu, p, grid, stream);
     };
     int rc = FLARE_OK;
     if (pl.seg.n > 1 && !pl.seg.lead) {

@@ -271,6 +271,43 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_fence_regs8(uint32_t (&r)[8]) {
+  asm volatile(""
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
+// N = 8, 16 or 32 columns: load and wait, store
+template <int N>
+__device__ __forceinline__ void tmem_read(uint32_t taddr, uint32_t (&r)[N]) {
+  static_assert(N == 8 || N == 16 || N == 32, "columns");
+  if constexpr (N == 8) tmem_ld8(taddr, r);
+  else if constexpr (N == 16) tmem_ld16(taddr, r);
+  else tmem_ld32(taddr, r);
+  tmem_wait_ld();
+  if constexpr (N == 8) tmem_fence_regs8(r);
+  else if constexpr (N == 16) tmem_fence_regs16(r);
+  else tmem_fence_regs(r);
+}
+template <int N>
+__device__ __forceinline__ void tmem_write(uint32_t taddr, const uint32_t (&r)[N]) {
+  static_assert(N == 8 || N == 16 || N == 32, "columns");
+  if constexpr (N == 8) tmem_st8(taddr, r);
+  else if constexpr (N == 16) tmem_st16(taddr, r);
+  else tmem_st32(taddr, r);
+}
+
 // Read-only global load that the compiler may not move: issued exactly where it is written, so a value needed one
 // loop iteration later is in flight during the whole iteration (a plain load gets sunk to its first use).
 __device__ __forceinline__ float ldg_pinned(const float* p) {
