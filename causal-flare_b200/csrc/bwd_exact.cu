@@ -16,10 +16,13 @@
 // (2) reverse: reverse walk carrying (b, c), emits dV and the dS planes; (3) rows: dK / dQ_dec = dS Lat;
 // (4) latents: per-split partial dQ / dK_dec = dS^T Rows; (5) fixed-order sum of the partials
 // (deterministic: no atomics anywhere).
+// Heads up to 32 wide take narrow_exact.cu instead: its replay also forms the segment carries, its reverse walk also dK
+// and dQ, so (3), (4) and the dS planes fall away.
 #include "bwd_exact.cuh"
 
 #include <string.h>
 
+#include "narrow_exact.cuh"
 #include "walk_device.cuh"
 #include "walk_exact.cuh"
 
@@ -840,6 +843,7 @@ size_t reverse_smem(int M, int dd, bool stablemax) {
 }
 
 struct BwdPlan {
+  bool narrow;
   int dd, DT, splits, rows_per_split;
   int nseg, seg_len;  // sequence segments of the replay / reverse walks (token-causal read-out only)
   int64_t plane;
@@ -855,6 +859,40 @@ bool span_mode(const flare_bwd_args_t& a) {
 BwdPlan plan_backward(const flare_bwd_args_t& a) {
   const flare_fwd_args_t& f = a.fwd;
   BwdPlan pl;
+  memset(&pl, 0, sizeof(pl));
+  pl.narrow = !span_mode(a) && narrow_shape(f.M, f.Dk, f.Dv, f.block_size, f.q_dec != nullptr || f.k_dec != nullptr);
+  if (pl.narrow) {
+    // as many segments as keep about twelve warps per SM in flight (the replay's registers allow no more), of 64 tokens at least
+    const int64_t lanes = (int64_t)f.B * f.H;
+    int64_t nseg = 12LL * sm_count() / (lanes * narrow_warps(f.M));
+    if (nseg > f.N / 64) nseg = f.N / 64;
+    if (nseg < 1) nseg = 1;
+    pl.seg_len = (int)(((f.N + nseg - 1) / nseg + 15) / 16 * 16);
+    pl.nseg = (f.N + pl.seg_len - 1) / pl.seg_len;
+    pl.plane = lanes * f.N * f.M;
+    size_t off = 0;
+    auto take = [&](size_t floats) {
+      const size_t o = off;
+      off += align_up(floats * 4, 256);
+      return o;
+    };
+    pl.off_E = take((size_t)pl.plane);
+    pl.off_G = take((size_t)pl.plane);
+    pl.off_W2 = f.variant == FLARE_STABLEMAX ? take((size_t)pl.plane) : pl.off_E;
+    pl.off_P = take((size_t)pl.plane);
+    pl.off_part_q = take((size_t)f.B * pl.nseg * f.H * f.M * f.Dk);
+    if (pl.nseg > 1) {
+      const size_t ls = (size_t)lanes * pl.nseg;
+      pl.off_seg_m = take(ls * f.M);
+      pl.off_seg_d = take(ls * f.M);
+      pl.off_seg_u = take(ls * f.M * f.Dv);
+      pl.off_seg_b = take(ls * f.M * f.Dv);
+      pl.off_seg_c = take(ls * f.M);
+      pl.off_seg_gam = take(ls * f.M);
+    }
+    pl.total = off;
+    return pl;
+  }
   pl.dd = walk_exact_dd(f.M, f.Dv);
   pl.DT = (f.Dv + 32 * pl.dd - 1) / (32 * pl.dd);
   // The walks are sequential in the tokens; with few (lane, value tile) CTAs the sequence is cut into segments that
@@ -1116,6 +1154,49 @@ size_t bwd_exact_workspace_bytes(const flare_bwd_args_t& a) {
   return plan_backward(a).total;
 }
 
+static int bwd_narrow(const flare_bwd_args_t& a, const BwdPlan& pl, cudaStream_t stream, const int* gate) {
+  const flare_fwd_args_t& f = a.fwd;
+  if (gate != nullptr) return FLARE_ERR_UNSUPPORTED;  // (never: the tensor kernels, which it gates, take no narrow heads)
+  char* ws = reinterpret_cast<char*>(f.workspace);
+  auto at = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
+  NarrowBwdParams p;
+  memset(&p, 0, sizeof(p));
+  p.q = f.q; p.k = f.k; p.v = f.v; p.dy = a.dy;
+  p.B = f.B; p.N = f.N; p.H = f.H; p.M = f.M; p.Dk = f.Dk; p.Dv = f.Dv;
+  p.q_stride_h = f.q_stride_h; p.q_stride_m = f.q_stride_m;
+  p.k_stride_b = f.k_stride_b; p.k_stride_n = f.k_stride_n; p.k_stride_h = f.k_stride_h;
+  p.v_stride_b = f.v_stride_b; p.v_stride_n = f.v_stride_n; p.v_stride_h = f.v_stride_h;
+  p.dy_stride_b = a.dy_stride_b; p.dy_stride_n = a.dy_stride_n; p.dy_stride_h = a.dy_stride_h;
+  p.scale = f.scale; p.power = f.power; p.dtype = f.dtype; p.variant = f.variant;
+  p.E = at(pl.off_E); p.G = at(pl.off_G); p.W2 = at(pl.off_W2); p.P = at(pl.off_P);
+  p.seg_len = pl.seg_len; p.nseg = pl.nseg;
+  p.dk = a.dk; p.dv = a.dv; p.dq_part = at(pl.off_part_q);
+  int rc;
+  if (pl.nseg > 1) {
+    p.in_m = at(pl.off_seg_m); p.in_d = at(pl.off_seg_d); p.in_u = at(pl.off_seg_u);
+    p.seg_b = at(pl.off_seg_b); p.seg_c = at(pl.off_seg_c); p.seg_gam = at(pl.off_seg_gam);
+    rc = segment_prefix_states(&f, pl.nseg, pl.seg_len, at(pl.off_seg_m), at(pl.off_seg_d), at(pl.off_seg_u), nullptr, stream,
+                               nullptr);
+    if (rc != FLARE_OK) return rc;
+  }
+  rc = launch_narrow_replay(p, stream);
+  if (rc != FLARE_OK) return rc;
+  if (pl.nseg > 1) {
+    const int64_t lanes = (int64_t)f.B * f.H, nscan = lanes * f.M * (f.Dv + 1);
+    LaunchTimer timer("bwd_seg_scan_kernel", stream);
+    FLARE_CUDA_CHECK(launch_pdl(bwd_seg_scan_kernel, dim3((unsigned)((nscan + 255) / 256)), dim3(256), 0, stream, p.seg_b, p.seg_c,
+                                p.seg_gam, pl.nseg, pl.seg_len, lanes, f.N, f.M, f.Dv, p.E, nullptr, 1, nullptr, nullptr, nullptr,
+                                1, nullptr, nullptr, nullptr, nullptr, nullptr));
+  }
+  rc = launch_narrow_reverse(p, stream);
+  if (rc != FLARE_OK) return rc;
+  const int64_t lat_n = (int64_t)f.H * f.M * f.Dk;
+  LaunchTimer timer("bwd_sum_splits_kernel", stream);
+  FLARE_CUDA_CHECK(launch_pdl(bwd_sum_splits_kernel, dim3((unsigned)((lat_n + 255) / 256)), dim3(256), 0, stream, a.dq, a.dq_dtype,
+                              p.dq_part, lat_n, f.B * pl.nseg, nullptr));
+  return FLARE_OK;
+}
+
 int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
   const flare_fwd_args_t& f = a.fwd;
   if (f.B == 0 || f.N == 0) return FLARE_OK;
@@ -1123,6 +1204,7 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
   const BwdPlan pl = plan_backward(a);
   if (f.workspace == nullptr || f.workspace_bytes < pl.total || (reinterpret_cast<uintptr_t>(f.workspace) & 15u))
     return FLARE_ERR_WORKSPACE;
+  if (pl.narrow) return bwd_narrow(a, pl, stream, gate);
   char* ws = reinterpret_cast<char*>(f.workspace);
   const bool stablemax = f.variant == FLARE_STABLEMAX;
   const bool shared_w = f.q_dec == nullptr && f.k_dec == nullptr;

@@ -7,6 +7,7 @@
 #include "bwd_tc.cuh"
 #include "decode_step.cuh"
 #include "flare_common.cuh"
+#include "narrow_exact.cuh"
 #include "prefill_tc.cuh"
 #include "state_ops.cuh"
 #include "walk_exact.cuh"
@@ -168,6 +169,18 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
       pl.gate_bytes = align_up((size_t)(1 + lanes * pl.gate_stride) * sizeof(int), 256);
       pl.ws_bytes += pl.gate_bytes;
     }
+    return pl;
+  }
+  if (narrow_shape(a->M, a->Dk, a->Dv, a->block_size, a->q_dec != nullptr || a->k_dec != nullptr)) {
+    // Narrow heads: a CTA has M / 32 warps and about twelve warps per SM run at once.  A cut pays for the state pass and the
+    // scan that come before the read-out (0.6 of its time, two launches) from three segments on; 32 tokens at least.
+    const int64_t warps = lanes * narrow_warps(a->M);
+    int64_t nseg = 12LL * sm_count() / warps;
+    if (nseg > a->N / 32) nseg = a->N / 32;
+    if (nseg < 3) nseg = 1;
+    pl.seg_len = (int)(((a->N + nseg - 1) / nseg + 15) / 16 * 16);
+    pl.nseg = (a->N + pl.seg_len - 1) / pl.seg_len;
+    pl.ws_bytes = pl.nseg > 1 ? align_up((size_t)lanes * pl.nseg * pl.state_floats * 4, 256) : 0;
     return pl;
   }
   const int dd = walk_exact_dd(a->M, a->Dv);

@@ -12,6 +12,8 @@
 // value columns l, l+32, ... of the tile; state and per-token output partials live in registers,
 // (6) cross-warp reduction of the output partials through shared memory.
 #include "walk_exact.cuh"
+
+#include "narrow_exact.cuh"
 #include "walk_device.cuh"
 
 namespace flare {
@@ -303,6 +305,8 @@ int walk_exact_dd(int M, int Dv) {
 int launch_walk_exact(const WalkParams& p, int nseg_grid, cudaStream_t stream) {
   if (p.M % 16 != 0 || p.M > 512) return FLARE_ERR_UNSUPPORTED;
   if (nseg_grid <= 0 || p.B * p.H <= 0) return FLARE_OK;
+  if (p.gate == nullptr && narrow_shape(p.M, p.Dk, p.Dv, p.block_size, p.qd != nullptr || p.kd != nullptr))
+    return launch_walk_narrow(p, nseg_grid, stream);
   const int mm = p.M / NW;
   const int dd = walk_exact_dd(p.M, p.Dv);
   const int dvt = 32 * dd;
