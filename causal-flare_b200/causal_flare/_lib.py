@@ -128,6 +128,11 @@ def load() -> C.CDLL:
     lib.flare_state_merge.restype = C.c_int
     lib.flare_state_merge.argtypes = [C.POINTER(State), C.POINTER(State), C.POINTER(State), C.c_int64, C.c_int32,
                                       C.c_int32, C.c_int32, C.c_void_p]
+    i64x3 = C.POINTER(C.c_int64)
+    lib.flare_mask_pack.restype = C.c_int
+    lib.flare_mask_pack.argtypes = [C.c_void_p, C.c_void_p, i64x3, C.c_void_p, i64x3] + [C.c_int32] * 5 + [C.c_void_p] * 5
+    lib.flare_mask_unpack.restype = C.c_int
+    lib.flare_mask_unpack.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, i64x3] + [C.c_int32] * 4 + [C.c_void_p]
     lib.flare_status_string.restype = C.c_char_p
     lib.flare_status_string.argtypes = [C.c_int]
     lib.flare_last_cuda_error.restype = C.c_char_p

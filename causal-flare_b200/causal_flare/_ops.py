@@ -115,24 +115,26 @@ def _masked_on_tensor_path(q, k, v, qd, kd, y, st_out, scale, variant, power, bl
 
 
 def _forward_compacted(q, k, v, y, mask, *, scale, variant, power, state_in, st_out, path):
-    """Masked forward on the tensor path: gather the valid tokens of every batch row to the front (stable order), run
-    the kernel with per-row lengths, scatter the outputs back; masked positions get y = 0 and leave the state as is."""
+    """Masked forward on the tensor path: pack the valid tokens of every batch row to the front (original order), run the
+    kernel with per-row lengths, unpack the outputs; masked positions get y = 0 and leave the state as is."""
     B, N, H, Dk = k.shape
     Dv = v.shape[-1]
-    valid = mask != 0
-    order = torch.argsort((~valid).to(torch.uint8), dim=1, stable=True)  # valid positions first, original order kept
-    lens = valid.sum(dim=1).to(torch.int32)
-    idx = order[:, :, None, None]
-    kc = torch.gather(k, 1, idx.expand(B, N, H, Dk))
-    vc = torch.gather(v, 1, idx.expand(B, N, H, Dv))
-    yc = torch.empty((B, N, H, Dv), device=k.device, dtype=k.dtype) if y is not None else None
+    lib, dev = _lib.load(), k.device
+    slot = torch.empty((B * (N + 1),), device=dev, dtype=torch.int32)  # slots, then the rows' lengths
+    lens = slot[B * N:]
+    kc = torch.empty((B, N, H, Dk), device=dev, dtype=k.dtype)
+    vc = torch.empty((B, N, H, Dv), device=dev, dtype=k.dtype)
+    yc = torch.empty((B, N, H, Dv), device=dev, dtype=k.dtype) if y is not None else None
+    strides = lambda t: (C.c_int64 * 3)(*t.stride()[:3])  # noqa: E731
+    _lib.check(lib.flare_mask_pack(mask.data_ptr(), k.data_ptr(), strides(k), v.data_ptr(), strides(v), B, N, H, Dk, Dv,
+                                   slot.data_ptr(), lens.data_ptr(), kc.data_ptr(), vc.data_ptr(), _lib.stream_handle(dev)),
+               "flare_mask_pack")
     args = _lib.make_fwd_args(q, kc, vc, None, None, yc, scale=scale, variant=variant, power=power, state_in=state_in,
                               state_out=st_out, path=path, lengths=lens)
-    _lib.run_forward(args, k.device)
+    _lib.run_forward(args, dev)
     if y is not None:
-        pad = torch.arange(N, device=k.device)[None, :] >= lens[:, None]
-        yc.masked_fill_(pad[:, :, None, None], 0)  # rows beyond a row's length were not written by the kernel
-        y.scatter_(1, idx.expand(B, N, H, Dv), yc)
+        _lib.check(lib.flare_mask_unpack(slot.data_ptr(), yc.data_ptr(), y.data_ptr(), strides(y), B, N, H, Dv,
+                                         _lib.stream_handle(dev)), "flare_mask_unpack")
 
 
 def backward(Q, K, V, dY, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, power=2.0, block_size=1,

@@ -736,6 +736,48 @@ int flare_state_merge(const flare_state_t* a, const flare_state_t* b, const flar
   return launch_fold(f, stream);
 }
 
+static bool rows_ok(const void* t, const int64_t st[3]) {
+  return t != nullptr && aligned16(t) && mult8(st[0]) && mult8(st[1]) && mult8(st[2]);
+}
+
+int flare_mask_pack(const int32_t* mask, const void* k, const int64_t k_strides_bnh[3], const void* v,
+                    const int64_t v_strides_bnh[3], int32_t B, int32_t N, int32_t H, int32_t Dk, int32_t Dv, int32_t* slot,
+                    int32_t* lengths, void* k_out, void* v_out, flare_stream_t stream) {
+  if (B < 0 || N < 0 || H <= 0 || Dk <= 0 || Dv <= 0 || (Dk % 8) || (Dv % 8)) return FLARE_ERR_BAD_SHAPE;
+  if (B == 0 || N == 0) return FLARE_OK;
+  if (!mask || !slot || !lengths || !k_strides_bnh || !v_strides_bnh || !rows_ok(k, k_strides_bnh) || !rows_ok(v, v_strides_bnh) ||
+      !k_out || !v_out || !aligned16(k_out) || !aligned16(v_out))
+    return FLARE_ERR_BAD_POINTER;
+  const int rc = launch_mask_slots(mask, B, N, slot, lengths, stream);
+  if (rc != FLARE_OK) return rc;
+  MoveRowsParams p;
+  memset(&p, 0, sizeof(p));
+  const void* in[2] = {k, v};
+  void* out[2] = {k_out, v_out};
+  const int64_t* st[2] = {k_strides_bnh, v_strides_bnh};
+  for (int w = 0; w < 2; ++w) {
+    p.in[w] = in[w]; p.out[w] = out[w]; p.d[w] = w ? Dv : Dk;
+    p.is_b[w] = st[w][0]; p.is_n[w] = st[w][1]; p.is_h[w] = st[w][2];
+    p.os_h[w] = p.d[w]; p.os_n[w] = (int64_t)H * p.d[w]; p.os_b[w] = (int64_t)N * H * p.d[w];
+  }
+  p.B = B; p.N = N; p.H = H; p.slot = slot; p.lens = lengths;
+  return launch_move_rows(p, 2, stream);
+}
+
+int flare_mask_unpack(const int32_t* slot, const void* y_in, void* y, const int64_t y_strides_bnh[3], int32_t B, int32_t N,
+                      int32_t H, int32_t Dv, flare_stream_t stream) {
+  if (B < 0 || N < 0 || H <= 0 || Dv <= 0 || (Dv % 8)) return FLARE_ERR_BAD_SHAPE;
+  if (B == 0 || N == 0) return FLARE_OK;
+  if (!slot || !y_in || !aligned16(y_in) || !y_strides_bnh || !rows_ok(y, y_strides_bnh)) return FLARE_ERR_BAD_POINTER;
+  MoveRowsParams p;
+  memset(&p, 0, sizeof(p));
+  p.in[0] = y_in; p.out[0] = y; p.d[0] = Dv;
+  p.is_h[0] = Dv; p.is_n[0] = (int64_t)H * Dv; p.is_b[0] = (int64_t)N * H * Dv;
+  p.os_b[0] = y_strides_bnh[0]; p.os_n[0] = y_strides_bnh[1]; p.os_h[0] = y_strides_bnh[2];
+  p.B = B; p.N = N; p.H = H; p.slot = slot; p.unpack = 1;
+  return launch_move_rows(p, 1, stream);
+}
+
 const char* flare_status_string(int status) {
   switch (status) {
     case FLARE_OK: return "ok";

@@ -208,6 +208,21 @@ int flare_decode_step(const flare_decode_args_t* args, flare_stream_t stream);
 int flare_state_merge(const flare_state_t* a, const flare_state_t* b, const flare_state_t* out,
                       int64_t lanes, int32_t M, int32_t Dv, int32_t count, flare_stream_t stream);
 
+/*
+ * Masked calls on the tensor-core kernels, which take per-row lengths instead of masks: pack the valid tokens of every batch
+ * row to its front, run flare_forward on the copies with `lengths`, unpack.  All tensors hold 2-byte elements (bf16 / fp16),
+ * rows of D contiguous elements (D a multiple of 8), 16-byte aligned, strides multiples of 8 elements.
+ * pack:   slot[B][N] (rank among the valid tokens, -1 for a masked one) and lengths[B] from mask[B][N] (0: masked), and
+ *         k_out, v_out (contiguous [B, N, H, D]); rows from lengths[b] on are zero up to the end of their 128-token chunk and
+ *         unspecified behind it.
+ * unpack: y[b, n] = y_in[b, slot[n]] (contiguous [B, N, H, Dv]), 0 for masked tokens.
+ */
+int flare_mask_pack(const int32_t* mask, const void* k, const int64_t k_strides_bnh[3], const void* v,
+                    const int64_t v_strides_bnh[3], int32_t B, int32_t N, int32_t H, int32_t Dk, int32_t Dv, int32_t* slot,
+                    int32_t* lengths, void* k_out, void* v_out, flare_stream_t stream);
+int flare_mask_unpack(const int32_t* slot, const void* y_in, void* y, const int64_t y_strides_bnh[3], int32_t B, int32_t N,
+                      int32_t H, int32_t Dv, flare_stream_t stream);
+
 const char* flare_status_string(int status);
 const char* flare_last_cuda_error(void);
 int flare_abi_version(void);
