@@ -45,6 +45,8 @@ static thread_local long long* g_trace = nullptr;
 static thread_local ChunkStates g_keep = {nullptr, nullptr, nullptr, 0};
 // gate words of the tensor-core forward in flight on this thread (null: none), see FwdPlan::gate_bytes
 static thread_local int* g_gate = nullptr;
+// y of the forward in flight on this thread is fp16 although its inputs are bf16 (copies), see forward_cast
+static thread_local bool g_y_f16 = false;
 
 void count_launches(int n) { g_last_launches += n; }
 
@@ -238,6 +240,7 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
     t.part_lw = reinterpret_cast<float*>(reinterpret_cast<char*>(t.part_y) + prefill_tc_partial_lw_offset(a));
   }
   t.trace = g_trace;
+  t.y_f16 = g_y_f16 ? 1 : 0;
   t.gate = g_gate;
   t.gate_stride = pl.gate_stride;
   // (the state pass over all segments but the last comes first)
@@ -270,17 +273,10 @@ int launch_guard_walk(const flare_fwd_args_t* a, const int* lane_gates, int gate
   return launch_walk_exact(w, 1, stream);
 }
 
-// What an fp16 call that runs on bf16 copies (forward_cast below) still has to do once the tensor kernels are enqueued:
-// y back to fp16, and then the standby walk of the flagged lanes on the caller's own fp16 tensors, so that the lanes
-// whose score spreads left the tensor kernels' domain - where the rounding of q and k to bf16 would move the scores
-// most - are computed from the unrounded inputs.
-struct FinishCast {
-  const flare_fwd_args_t* orig;
-  const CastParams* y_back;  // null: no y wanted
-  bool y_done;
-};
-
-int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, FinishCast* fin = nullptr) {
+// `orig`: the fp16 call behind one that runs on bf16 copies (forward_cast below).  The standby walk of the flagged lanes takes
+// the caller's own fp16 tensors, so that the lanes whose score spreads left the tensor kernels' domain - where the rounding
+// of q and k to bf16 would move the scores most - are computed from the unrounded inputs.
+int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, const flare_fwd_args_t* orig = nullptr) {
   const FwdPlan pl = plan_forward(a);
   if (g_keep.u != nullptr) return forward_tensor_or_exact(a, pl, stream);  // the backward's own replay of the forward
   int* gate = nullptr;
@@ -304,16 +300,7 @@ int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, FinishCast* fin 
   g_keep = ChunkStates{nullptr, nullptr, nullptr, 0};
   if (rc != FLARE_OK) return rc;
   if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
-    const flare_fwd_args_t* walk_args = a;
-    if (fin != nullptr) {
-      if (fin->y_back != nullptr) {
-        rc = launch_cast_rows(*fin->y_back, stream);
-        if (rc != FLARE_OK) return rc;
-        fin->y_done = true;
-      }
-      walk_args = fin->orig;
-    }
-    rc = launch_guard_walk(walk_args, gate + 1, pl.gate_stride, stream);
+    rc = launch_guard_walk(orig != nullptr ? orig : a, gate + 1, pl.gate_stride, stream);
     g_last_launches += 1;
   }
   return rc;
@@ -376,19 +363,19 @@ int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaSt
 
 // fp16 inputs on the tensor-core kernels.  The kernels multiply bf16 operands (the tensor-core products of E, R, W
 // and the running state are bf16 whatever the inputs are), so an fp16 call is served by rounding q, k, v to bf16
-// copies in the workspace, running the bf16 forward on those, and writing y back as fp16: three streaming passes
-// around a kernel that is 40 to 60 times faster than the exact walk the call would otherwise take.  Lanes that the
+// copies in the workspace and running the bf16 forward on those, which writes y as fp16: one streaming pass over q, k and v
+// before a kernel that is 40 to 60 times faster than the exact walk the call would otherwise take.  Lanes that the
 // kernels flag as outside their numeric domain are recomputed by the exact kernels from the fp16 tensors themselves.
 // States and log-sum-exps are fp32 on both sides and go straight to the caller's buffers.  Not for the training
 // forward (no state is kept for a backward) and not with separate decode weights or a mask, which the tensor kernels
 // do not take.
 struct CastPlan {
   bool on;
-  size_t off_q, off_k, off_v, off_y, total;
+  size_t off_q, off_k, off_v, total;
 };
 
 CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
-  CastPlan cp{false, 0, 0, 0, 0, 0};
+  CastPlan cp{false, 0, 0, 0, 0};
   if (a->dtype != FLARE_F16 || a->path == FLARE_PATH_EXACT || a->keep != nullptr || a->q_dec != nullptr ||
       a->k_dec != nullptr || a->mask != nullptr || a->B == 0 || a->N == 0)
     return cp;
@@ -400,15 +387,14 @@ CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
   b->q_stride_m = a->Dk; b->q_stride_h = (int64_t)a->M * a->Dk;
   b->k_stride_h = a->Dk; b->k_stride_n = (int64_t)a->H * a->Dk; b->k_stride_b = (int64_t)a->N * b->k_stride_n;
   b->v_stride_h = a->Dv; b->v_stride_n = (int64_t)a->H * a->Dv; b->v_stride_b = (int64_t)a->N * b->v_stride_n;
-  b->y_stride_h = a->Dv; b->y_stride_n = (int64_t)a->H * a->Dv; b->y_stride_b = (int64_t)a->N * b->y_stride_n;
   if (!prefill_tc_supported(b)) return cp;
   const size_t rows = (size_t)a->B * a->N * a->H;
   cp.on = true;
   cp.off_q = 0;
   cp.off_k = align_up((size_t)a->H * a->M * a->Dk * 2, 256);
   cp.off_v = cp.off_k + align_up(rows * a->Dk * 2, 256);
-  cp.off_y = cp.off_v + align_up(rows * a->Dv * 2, 256);
-  cp.total = cp.off_y + (a->y != nullptr ? align_up(rows * a->Dv * 2, 256) : 0);
+  // (the size that callers plan with has room for a y in bf16, which nothing uses)
+  cp.total = cp.off_v + align_up(rows * a->Dv * 2, 256) * (a->y != nullptr ? 2 : 1);
   return cp;
 }
 
@@ -417,41 +403,25 @@ int forward_cast(const flare_fwd_args_t* a, flare_fwd_args_t& b, const CastPlan&
   if (a->workspace == nullptr || a->workspace_bytes < cp.total + inner || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
   char* ws = reinterpret_cast<char*>(a->workspace);
   b.q = ws + cp.off_q; b.k = ws + cp.off_k; b.v = ws + cp.off_v;
-  b.y = a->y != nullptr ? ws + cp.off_y : nullptr;
   b.workspace = inner > 0 ? ws + cp.total : nullptr;
   b.workspace_bytes = inner > 0 ? a->workspace_bytes - cp.total : 0;
-  CastParams c;
-  memset(&c, 0, sizeof(c));
-  c.in = a->q; c.out = const_cast<void*>(b.q); c.n0 = 1; c.n1 = a->H; c.n2 = a->M; c.d = a->Dk;
-  c.is1 = a->q_stride_h; c.is2 = a->q_stride_m; c.os1 = b.q_stride_h; c.os2 = b.q_stride_m;
-  int rc = launch_cast_rows(c, stream);
+  CastParams c[3];
+  memset(c, 0, sizeof(c));
+  c[0].in = a->q; c[0].out = const_cast<void*>(b.q); c[0].n0 = 1; c[0].n1 = a->H; c[0].n2 = a->M; c[0].d = a->Dk;
+  c[0].is1 = a->q_stride_h; c[0].is2 = a->q_stride_m; c[0].os1 = b.q_stride_h; c[0].os2 = b.q_stride_m;
+  c[1].in = a->k; c[1].out = const_cast<void*>(b.k); c[1].n0 = a->B; c[1].n1 = a->N; c[1].n2 = a->H; c[1].d = a->Dk;
+  c[1].is0 = a->k_stride_b; c[1].is1 = a->k_stride_n; c[1].is2 = a->k_stride_h;
+  c[1].os0 = b.k_stride_b; c[1].os1 = b.k_stride_n; c[1].os2 = b.k_stride_h;
+  c[2].in = a->v; c[2].out = const_cast<void*>(b.v); c[2].n0 = a->B; c[2].n1 = a->N; c[2].n2 = a->H; c[2].d = a->Dv;
+  c[2].is0 = a->v_stride_b; c[2].is1 = a->v_stride_n; c[2].is2 = a->v_stride_h;
+  c[2].os0 = b.v_stride_b; c[2].os1 = b.v_stride_n; c[2].os2 = b.v_stride_h;
+  int rc = launch_cast_rows(c, 3, false, stream);
   if (rc != FLARE_OK) return rc;
-  c.in = a->k; c.out = const_cast<void*>(b.k); c.n0 = a->B; c.n1 = a->N; c.n2 = a->H; c.d = a->Dk;
-  c.is0 = a->k_stride_b; c.is1 = a->k_stride_n; c.is2 = a->k_stride_h;
-  c.os0 = b.k_stride_b; c.os1 = b.k_stride_n; c.os2 = b.k_stride_h;
-  rc = launch_cast_rows(c, stream);
+  g_y_f16 = true;
+  rc = forward_run(&b, stream, a);  // gate words in b's workspace
+  g_y_f16 = false;
   if (rc != FLARE_OK) return rc;
-  c.in = a->v; c.out = const_cast<void*>(b.v); c.d = a->Dv;
-  c.is0 = a->v_stride_b; c.is1 = a->v_stride_n; c.is2 = a->v_stride_h;
-  c.os0 = b.v_stride_b; c.os1 = b.v_stride_n; c.os2 = b.v_stride_h;
-  rc = launch_cast_rows(c, stream);
-  if (rc != FLARE_OK) return rc;
-  CastParams yb = c;
-  yb.in = b.y; yb.out = a->y; yb.to_f16 = 1;
-  yb.is0 = b.y_stride_b; yb.is1 = b.y_stride_n; yb.is2 = b.y_stride_h;
-  yb.os0 = a->y_stride_b; yb.os1 = a->y_stride_n; yb.os2 = a->y_stride_h;
-  FinishCast fin{a, a->y != nullptr ? &yb : nullptr, false};
-  rc = forward_run(&b, stream, &fin);  // gate words in b's workspace; the standby walk reads the caller's fp16 tensors
-  if (rc != FLARE_OK) return rc;
-  int casts = 3;
-  if (a->y != nullptr) {
-    if (!fin.y_done) {  // no standby on this path (forced tensor path, per-row lengths)
-      rc = launch_cast_rows(yb, stream);
-      if (rc != FLARE_OK) return rc;
-    }
-    ++casts;
-  }
-  g_last_launches += casts;
+  g_last_launches += 1;
   return FLARE_OK;
 }
 
@@ -636,39 +606,34 @@ int backward_cast(const flare_bwd_args_t* a, flare_bwd_args_t& b, const BwdCastP
   b.dy = ws + cp.off_dy; b.dk = ws + cp.off_dk; b.dv = ws + cp.off_dv;
   g.workspace = ws + cp.total;
   g.workspace_bytes = f.workspace_bytes - cp.total;
-  CastParams c;
-  memset(&c, 0, sizeof(c));
-  c.in = f.q; c.out = const_cast<void*>(g.q); c.n0 = 1; c.n1 = f.H; c.n2 = f.M; c.d = f.Dk;
-  c.is1 = f.q_stride_h; c.is2 = f.q_stride_m; c.os1 = g.q_stride_h; c.os2 = g.q_stride_m;
-  int rc = launch_cast_rows(c, stream);
-  if (rc != FLARE_OK) return rc;
-  c.in = f.k; c.out = const_cast<void*>(g.k); c.n0 = f.B; c.n1 = f.N; c.n2 = f.H; c.d = f.Dk;
-  c.is0 = f.k_stride_b; c.is1 = f.k_stride_n; c.is2 = f.k_stride_h;
-  c.os0 = g.k_stride_b; c.os1 = g.k_stride_n; c.os2 = g.k_stride_h;
-  rc = launch_cast_rows(c, stream);
-  if (rc != FLARE_OK) return rc;
-  c.in = f.v; c.out = const_cast<void*>(g.v); c.d = f.Dv;
-  c.is0 = f.v_stride_b; c.is1 = f.v_stride_n; c.is2 = f.v_stride_h;
-  c.os0 = g.v_stride_b; c.os1 = g.v_stride_n; c.os2 = g.v_stride_h;
-  rc = launch_cast_rows(c, stream);
-  if (rc != FLARE_OK) return rc;
-  c.in = a->dy; c.out = const_cast<void*>(b.dy);
-  c.is0 = a->dy_stride_b; c.is1 = a->dy_stride_n; c.is2 = a->dy_stride_h;
-  c.os0 = b.dy_stride_b; c.os1 = b.dy_stride_n; c.os2 = b.dy_stride_h;
-  rc = launch_cast_rows(c, stream);
+  CastParams c[4];
+  memset(c, 0, sizeof(c));
+  c[0].in = f.q; c[0].out = const_cast<void*>(g.q); c[0].n0 = 1; c[0].n1 = f.H; c[0].n2 = f.M; c[0].d = f.Dk;
+  c[0].is1 = f.q_stride_h; c[0].is2 = f.q_stride_m; c[0].os1 = g.q_stride_h; c[0].os2 = g.q_stride_m;
+  const void* in[3] = {f.k, f.v, a->dy};
+  const void* out[3] = {g.k, g.v, b.dy};
+  const int64_t is[3][3] = {{f.k_stride_b, f.k_stride_n, f.k_stride_h}, {f.v_stride_b, f.v_stride_n, f.v_stride_h},
+                            {a->dy_stride_b, a->dy_stride_n, a->dy_stride_h}};
+  const int64_t os[3][3] = {{g.k_stride_b, g.k_stride_n, g.k_stride_h}, {g.v_stride_b, g.v_stride_n, g.v_stride_h},
+                            {b.dy_stride_b, b.dy_stride_n, b.dy_stride_h}};
+  for (int i = 0; i < 3; ++i) {
+    CastParams& t = c[1 + i];
+    t.in = in[i]; t.out = const_cast<void*>(out[i]); t.n0 = f.B; t.n1 = f.N; t.n2 = f.H; t.d = i == 0 ? f.Dk : f.Dv;
+    t.is0 = is[i][0]; t.is1 = is[i][1]; t.is2 = is[i][2];
+    t.os0 = os[i][0]; t.os1 = os[i][1]; t.os2 = os[i][2];
+  }
+  int rc = launch_cast_rows(c, 4, false, stream);
   if (rc != FLARE_OK) return rc;
   rc = bwd_tc(b, stream);
   if (rc != FLARE_OK) return rc;
-  c.to_f16 = 1;
-  c.in = b.dv; c.out = a->dv;
-  c.is0 = c.os0 = b.dy_stride_b; c.is1 = c.os1 = b.dy_stride_n; c.is2 = c.os2 = b.dy_stride_h;
-  rc = launch_cast_rows(c, stream);
+  // dK and dV, contiguous on both sides, laid out like the copies of k and v
+  c[0] = c[1];
+  c[0].in = b.dk; c[0].out = a->dk; c[0].is0 = c[0].os0; c[0].is1 = c[0].os1; c[0].is2 = c[0].os2;
+  c[1] = c[2];
+  c[1].in = b.dv; c[1].out = a->dv; c[1].is0 = c[1].os0; c[1].is1 = c[1].os1; c[1].is2 = c[1].os2;
+  rc = launch_cast_rows(c, 2, true, stream);
   if (rc != FLARE_OK) return rc;
-  c.in = b.dk; c.out = a->dk; c.d = f.Dk;
-  c.is0 = c.os0 = g.k_stride_b; c.is1 = c.os1 = g.k_stride_n; c.is2 = c.os2 = g.k_stride_h;
-  rc = launch_cast_rows(c, stream);
-  if (rc != FLARE_OK) return rc;
-  g_last_launches += 6;
+  g_last_launches += 2;
   return FLARE_OK;
 }
 }  // namespace

@@ -44,6 +44,7 @@
 #include <string.h>
 
 #include "sm100_ptx.cuh"
+#include "state_ops.cuh"
 #include "tc_device.cuh"
 
 // polling rounds of every wait of the prefill kernel before it suspends (see tc::wait_or_abort)
@@ -141,6 +142,17 @@ using tc::sigma_fast;
 // bounded wait that also gives up as soon as another role of the CTA has given up
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, Misc* misc) {
   return tc::wait_or_abort(bar, parity, &misc->abort_flag, FLARE_TC_FWD_POLLS);
+}
+
+// eight values as fp16 or bf16 pairs (uniform per launch)
+__device__ __forceinline__ void pack_out(const float (&y)[8], bool f16, uint32_t (&o)[4]) {
+  if (f16) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = pack_f16(y[2 * j], y[2 * j + 1]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = pack_bf16(y[2 * j], y[2 * j + 1]);
+  }
 }
 
 // grid.z = latent group * DKB + value slice.  First value column of this CTA's slice (a compile-time zero when there
@@ -1187,14 +1199,15 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               const uint4 x = xp[half * 4 + ch];
               const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
               uint32_t o[4];
+              float y[8];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[j]));
-                float y0, y1;  // own raw values * ca + partner's normalised values * cb, two columns per instruction
+                // own raw values * ca + partner's normalised values * cb, two columns per instruction
                 f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
-                                 f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y0, y1);
-                o[j] = pack_bf16(y0, y1);
+                                 f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
               }
+              pack_out(y, false, o);
               *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
                   make_uint4(o[0], o[1], o[2], o[3]);
             }
@@ -1228,18 +1241,18 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int half = 0; half < 2; ++half) {
           const uint32_t(&r)[32] = half ? rb : ra;
           const int col = value_col0<ZS, SPLIT>() + vb * 64 + half * 32;
-          // 32 columns of this thread's row as 16-bit values: bf16 of y, or fp16 of a latent group's partial
+          // 32 columns of this thread's row as 16-bit values: y in its type, or fp16 of a latent group's partial
           uint4 v[4];
           const uint64_t inv2 = f2_pack(inv, inv);
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) {
             uint32_t o[4];
+            float y[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float y0, y1;  // two columns per multiply
-              f2_unpack(f2_mul(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])), inv2), y0, y1);
-              o[j] = SPLIT ? pack_f16(y0, y1) : pack_bf16(y0, y1);
-            }
+            for (int j = 0; j < 4; ++j)  // two columns per multiply
+              f2_unpack(f2_mul(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])), inv2), y[2 * j],
+                        y[2 * j + 1]);
+            pack_out(y, SPLIT || (!WIDE && p.y_f16 != 0), o);
             v[ch] = make_uint4(o[0], o[1], o[2], o[3]);
           }
           if (p.y_tma) {
@@ -1419,7 +1432,7 @@ bool prefill_tc_supported(const flare_fwd_args_t* a) {
 // One thread per (token, head, 8 value columns).
 __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __restrict__ part_y, const float* __restrict__ part_lw,
                                                                int groups, int64_t rows /* B*N*H */, int N, int H, int dv,
-                                                               __nv_bfloat16* y, int64_t y_stride_b, int64_t y_stride_n,
+                                                               uint16_t* y, int y_f16, int64_t y_stride_b, int64_t y_stride_n,
                                                                int64_t y_stride_h, float* lse_dec /* [B, H, N] or null */,
                                                                const int32_t* lens /* [B] or null */, int* gate,
                                                                int gate_stride, int gate_off) {
@@ -1465,12 +1478,12 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __re
   const int n = (int)(bn % N);
   const int64_t b = bn / N;
   if (lse_dec != nullptr && c8 == 0) lse_dec[(b * H + h) * N + n] = (mx + log2f(wsum)) * kLn2;
-  uint4 v;
-  v.x = pack_bf16(acc[0] * inv, acc[1] * inv);
-  v.y = pack_bf16(acc[2] * inv, acc[3] * inv);
-  v.z = pack_bf16(acc[4] * inv, acc[5] * inv);
-  v.w = pack_bf16(acc[6] * inv, acc[7] * inv);
-  *reinterpret_cast<uint4*>(y + b * y_stride_b + (int64_t)n * y_stride_n + (int64_t)h * y_stride_h + c8 * 8) = v;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] *= inv;
+  uint32_t o[4];
+  pack_out(acc, y_f16 != 0, o);
+  *reinterpret_cast<uint4*>(y + b * y_stride_b + (int64_t)n * y_stride_n + (int64_t)h * y_stride_h + c8 * 8) =
+      make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 
@@ -1613,13 +1626,22 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   else
     rc = groups > 1 ? launch_prefill_tc_unit<5>(lat, mode, tq, tk, tv, ty, p, grid, stream)
                     : launch_prefill_tc_unit<2>(lat, mode, tq, tk, tv, ty, p, grid, stream);
+  if (rc == FLARE_OK && p.y_f16 && wide && p.y != nullptr && (groups == 1 || p.cluster_merge)) {
+    // the wide instance writes bf16 whatever the call's type (the choice between two packings in its epilogue cost it 8 %):
+    // converted in place
+    CastParams c;
+    memset(&c, 0, sizeof(c));
+    c.in = p.y; c.out = p.y; c.n0 = a->B; c.n1 = a->N; c.n2 = a->H; c.d = a->Dv;
+    c.is0 = c.os0 = p.y_stride_b; c.is1 = c.os1 = p.y_stride_n; c.is2 = c.os2 = p.y_stride_h;
+    rc = launch_cast_rows(&c, 1, true, stream);
+  }
   if (rc != FLARE_OK || groups == 1 || p.y == nullptr || p.cluster_merge) return rc;
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);
   LaunchTimer timer("tc_merge_groups_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(tc_merge_groups_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream,
                               reinterpret_cast<const __half*>(p.part_y), p.part_lw, groups, rows, a->N, a->H, a->Dv,
-                              reinterpret_cast<__nv_bfloat16*>(p.y), p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
+                              reinterpret_cast<uint16_t*>(p.y), p.y_f16, p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
                               p.gate, p.gate_stride, p.gate_off));
   return FLARE_OK;
 }

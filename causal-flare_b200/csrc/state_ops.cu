@@ -5,6 +5,8 @@
 // m = max(m_a, m_b); a side whose max is -inf contributes with factor 0 (factor 1 if both are -inf).
 #include "state_ops.cuh"
 
+#include <string.h>
+
 namespace flare {
 
 namespace {
@@ -92,21 +94,34 @@ __global__ void __launch_bounds__(NT) fold_kernel(const FoldParams p) {
   }
 }
 
+struct CastList {
+  CastParams t[4];
+};
+
+// blockIdx.y = tensor.  Bound by memory; a tensor that is one dense run needs no index arithmetic (three 64-bit divisions for
+// every 16-byte piece otherwise).
 template <bool TO_F16>
-__global__ void __launch_bounds__(256) cast_rows_kernel(const CastParams p) {
+__global__ void __launch_bounds__(256) cast_rows_kernel(const __grid_constant__ CastList list) {
   pdl_begin();
-  const int c8n = p.d >> 3;
+  const CastParams& p = list.t[blockIdx.y];
+  const int64_t c8n = p.d >> 3;
   const int64_t total = p.n0 * p.n1 * p.n2 * c8n;
+  const bool dense = c8n == total;
   const uint16_t* in = reinterpret_cast<const uint16_t*>(p.in);
   uint16_t* out = reinterpret_cast<uint16_t*>(p.out);
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c8 = (int)(idx % c8n);
-    int64_t r = idx / c8n;
-    const int64_t i2 = r % p.n2;
-    r /= p.n2;
-    const int64_t i1 = r % p.n1;
-    const int64_t i0 = r / p.n1;
-    uint4 x = *reinterpret_cast<const uint4*>(in + i0 * p.is0 + i1 * p.is1 + i2 * p.is2 + c8 * 8);
+    int64_t io = idx * 8, oo = idx * 8;
+    if (!dense) {
+      const int64_t c8 = idx % c8n;
+      int64_t r = idx / c8n;
+      const int64_t i2 = r % p.n2;
+      r /= p.n2;
+      const int64_t i1 = r % p.n1;
+      const int64_t i0 = r / p.n1;
+      io = i0 * p.is0 + i1 * p.is1 + i2 * p.is2 + c8 * 8;
+      oo = i0 * p.os0 + i1 * p.os1 + i2 * p.os2 + c8 * 8;
+    }
+    const uint4 x = *reinterpret_cast<const uint4*>(in + io);
     uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -120,7 +135,7 @@ __global__ void __launch_bounds__(256) cast_rows_kernel(const CastParams p) {
         w[j] = *reinterpret_cast<const uint32_t*>(&h);
       }
     }
-    *reinterpret_cast<uint4*>(out + i0 * p.os0 + i1 * p.os1 + i2 * p.os2 + c8 * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(out + oo) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -195,16 +210,31 @@ int launch_move_rows(const MoveRowsParams& p, int tensors, cudaStream_t stream) 
   return FLARE_OK;
 }
 
-int launch_cast_rows(const CastParams& p, cudaStream_t stream) {
-  const int64_t total = p.n0 * p.n1 * p.n2 * (p.d >> 3);
-  if (total <= 0) return FLARE_OK;
-  if (p.d % 8) return FLARE_ERR_BAD_SHAPE;
-  int64_t blocks = (total + 255) / 256;
+int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t stream) {
+  CastList list;
+  memset(&list, 0, sizeof(list));
+  int64_t most = 0;
+  for (int i = 0; i < count; ++i) {
+    CastParams c = p[i];
+    if (c.d % 8) return FLARE_ERR_BAD_SHAPE;
+    // rows that lie behind one another on both sides become one longer row
+    for (int level = 0; level < 3 && (c.n2 == 1 || (c.is2 == c.d && c.os2 == c.d)); ++level) {
+      c.d *= c.n2;
+      c.n2 = c.n1; c.is2 = c.is1; c.os2 = c.os1;
+      c.n1 = c.n0; c.is1 = c.is0; c.os1 = c.os0;
+      c.n0 = 1;
+    }
+    const int64_t total = c.n0 * c.n1 * c.n2 * (c.d >> 3);
+    if (total > most) most = total;
+    list.t[i] = c;
+  }
+  if (most <= 0) return FLARE_OK;
+  int64_t blocks = (most + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  LaunchTimer timer(p.to_f16 ? "cast_rows_kernel<bf16 to fp16>" : "cast_rows_kernel<fp16 to bf16>", stream);
-  FLARE_CUDA_CHECK(launch_pdl(p.to_f16 ? cast_rows_kernel<true> : cast_rows_kernel<false>, dim3((unsigned)blocks), dim3(256), 0,
-                              stream, p));
+  LaunchTimer timer(to_f16 ? "cast_rows_kernel<bf16 to fp16>" : "cast_rows_kernel<fp16 to bf16>", stream);
+  FLARE_CUDA_CHECK(launch_pdl(to_f16 ? cast_rows_kernel<true> : cast_rows_kernel<false>, dim3((unsigned)blocks, count), dim3(256),
+                              0, stream, list));
   return FLARE_OK;
 }
 

@@ -28,14 +28,13 @@ int launch_fold(const FoldParams& p, cudaStream_t stream);
 struct CastParams {
   const void* in;
   void* out;
-  int64_t n0, n1, n2;
-  int d;
+  int64_t n0, n1, n2, d;
   int64_t is0, is1, is2;
   int64_t os0, os1, os2;
-  int to_f16;  // 1: bf16 -> fp16, 0: fp16 -> bf16
 };
 
-int launch_cast_rows(const CastParams& p, cudaStream_t stream);
+// up to four tensors in one launch, all in one direction
+int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t stream);
 
 // Compaction of masked rows (2-byte elements, head widths that are multiples of 8, 16-byte aligned rows).
 // slot[b][n] = number of valid tokens before token n of row b, or -1 for a masked token; lens[b] = valid tokens of the row.
