@@ -97,8 +97,18 @@ bool same_kind(const Tensor& t, const Tensor& like) {
   return t.is_cuda() && t.device() == like.device() && t.scalar_type() == like.scalar_type();
 }
 
+// Storage that the kernels may read, and nothing that a call past the Python autograd functions would lose: no wrapper of a
+// function transform or of a Python tensor class (no storage of its own), no forward-mode tangent (the Python functions
+// refuse one; it would be dropped here).
+bool ordinary(const Tensor& t) {
+  constexpr c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                         c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize});
+  return t.defined() && !t.key_set().has_any(wrapped) && !t._fw_grad(/*level=*/0).defined();
+}
+
 // Q [H, M, Dk], K [B, N, H, Dk], V [B, N, H, Dv] of one 16/32-bit float type on one GPU, not empty, sizes the kernels take
 bool plain_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
+  if (!ordinary(q) || !ordinary(k) || !ordinary(v)) return false;
   if (q.dim() != 3 || k.dim() != 4 || v.dim() != 4 || !k.is_cuda()) return false;
   if (!same_kind(q, k) || !same_kind(v, k) || dtype_code(k.scalar_type()) < 0) return false;
   if (k.layout() != at::kStrided || v.layout() != at::kStrided || q.layout() != at::kStrided) return false;

@@ -1,0 +1,32 @@
+"""GPU: calls that the native host layer must leave to the Python layer (what it would lose, refuse or word differently)."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+import causal_flare as cf
+from causal_flare.autoregressive import flare_autoregressive_stablemax_triton
+from oracle import flare_oracle as orc
+from util import to_dev
+
+pytestmark = pytest.mark.gpu
+
+OPS = {
+    "softmax": lambda q, k, v: cf.flare_autoregressive_triton(q, k, v),
+    "stablemax": lambda q, k, v: flare_autoregressive_stablemax_triton(q, k, v),
+    "block": lambda q, k, v: cf.flare_semi_autoregressive_trition(q, k, v, block_size=32, chunk_size=32)[0],
+}
+
+
+def inputs(dtype=torch.bfloat16):
+    return to_dev(*orc.make_inputs(1, 64, 2, 32, 64, seed0=21, dtype=dtype))
+
+
+@pytest.mark.parametrize("requires_grad", [False, True])
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("op", sorted(OPS))
+def test_a_forward_mode_tangent_is_refused_not_dropped(op, which, requires_grad):
+    args = [t.requires_grad_(requires_grad) for t in inputs()]
+    with fwAD.dual_level():
+        args[which] = fwAD.make_dual(args[which], torch.ones_like(args[which]))
+        with pytest.raises((NotImplementedError, RuntimeError), match="jvp|forward mode"):
+            OPS[op](*args)
