@@ -15,6 +15,7 @@
 #include <string.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <cmath>
@@ -108,6 +109,8 @@ bool ordinary(const Tensor& t) {
 
 // Q [H, M, Dk], K [B, N, H, Dk], V [B, N, H, Dv] of one 16/32-bit float type on one GPU, not empty, sizes the kernels take
 bool plain_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
+  // (torch.jit.trace records the Python autograd functions as calls; of this layer it would record the empty output tensor)
+  if (torch::jit::tracer::isTracing()) return false;
   if (!ordinary(q) || !ordinary(k) || !ordinary(v)) return false;
   if (q.dim() != 3 || k.dim() != 4 || v.dim() != 4 || !k.is_cuda()) return false;
   if (!same_kind(q, k) || !same_kind(v, k) || dtype_code(k.scalar_type()) < 0) return false;
