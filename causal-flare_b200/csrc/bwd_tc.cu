@@ -951,9 +951,11 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
                                                                   int fwd_gate_words, int* gate) {
   pdl_begin();
   if (blockIdx.x == 0) {
-    // this call's gate word starts as "did any CTA of the forward find its tokens outside the numeric domain"
+    // this call's gate word starts as "did any CTA of the forward find its tokens outside the numeric domain" (the forward's
+    // leading word says how many words per lane it wrote; after a replay it is the word written here)
+    const int words = min(B * H * fwd_gate[0], fwd_gate_words - 1);
     int raised = 0;
-    for (int i = threadIdx.x; i < fwd_gate_words; i += 256) raised |= fwd_gate[i];
+    for (int i = threadIdx.x; i < words; i += 256) raised |= fwd_gate[1 + i];
     raised = __syncthreads_or(raised);
     if (threadIdx.x == 0) *gate = raised ? 1 : 0;
   }
@@ -1437,8 +1439,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     // (1') the training forward kept everything: its output, its log-sum-exp, the chunk states, its gate words
     const KeepLayout kl = keep_layout(f);
     char* kb = reinterpret_cast<char*>(f.keep);
-    fwd_gate = reinterpret_cast<const int*>(kb + kl.off_gate) + 1;
-    fwd_gate_words = (int)kl.gate_words - 1;
+    fwd_gate = reinterpret_cast<const int*>(kb + kl.off_gate);
+    fwd_gate_words = (int)kl.gate_words;
     keep.u = kb + kl.off_u;
     keep.c = reinterpret_cast<float*>(kb + kl.off_c);
     keep.d = reinterpret_cast<float*>(kb + kl.off_d);
@@ -1446,8 +1448,8 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     lse = a.lse_dec;
   } else {
     // (1) forward on the tensor path: y, the decode log-sum-exp and the per-chunk prefix states
-    fwd_gate = gate + 1;
-    fwd_gate_words = (int)pl.gate_words - 1;
+    fwd_gate = gate;
+    fwd_gate_words = (int)pl.gate_words;
     keep.u = ws + pl.off_cu;
     keep.c = reinterpret_cast<float*>(ws + pl.off_cc);
     keep.d = reinterpret_cast<float*>(ws + pl.off_cd);

@@ -12,7 +12,8 @@ struct ChunkStates {
   int nch;
 };
 
-// Layout of flare_fwd_args_t::keep for a problem (all offsets in bytes; total == 0: the problem keeps nothing)
+// Layout of flare_fwd_args_t::keep for a problem (all offsets in bytes; total == 0: the problem keeps nothing).  It depends on
+// the sizes alone: the forward that fills it and the backward that reads it may run under different instance choices.
 struct KeepLayout {
   size_t off_gate, off_u, off_c, off_d, total;
   size_t gate_words;
@@ -27,9 +28,9 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream);
 
 // Forward on the tensor path that also writes y, the decode log-sum-exp and the per-chunk prefix states
 // (defined with the forward dispatch).
-// `gate` (may be null): forward_gate_words() ints, written by the kernels from the second on (see TcParams::gate).
+// `gate` (may be null): forward_gate_words() ints, of which the kernels write 1 + lanes * gate[0] (see TcParams::gate).
 int forward_keep_states(const flare_fwd_args_t* a, const ChunkStates& keep, int* gate, cudaStream_t stream);
-// gate words of a forward on the tensor path: one leading word and the CTAs' words
+// room for the gate words of any forward of these sizes on the tensor path: one leading word and the CTAs' words
 size_t forward_gate_words(const flare_fwd_args_t* a);
 // diagnostic buffer set with flare_set_trace_buffer (null in normal use)
 long long* trace_buffer();

@@ -140,7 +140,7 @@ struct FwdPlan {
   size_t state_floats;  // floats per state: 2M + M*Dv
   size_t ws_bytes;
   size_t part_off, part_bytes;  // tensor path with more than 128 latents: partial read-outs behind the segment states
-  // Tensor kernels: gate words, gate_stride per lane behind one leading word: one for every CTA of the call's passes, set
+  // Tensor kernels: gate words, gate_stride per lane behind one leading word (gate_stride itself): one for every CTA of the call's passes, set
   // by CTAs that met tokens outside their numeric domain.  Path AUTO has them in the workspace (gate_bytes, else 0) and
   // runs the exact kernels for the flagged lanes.
   int gate_stride;
@@ -165,7 +165,7 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
     pl.part_off = pl.ws_bytes;
     pl.part_bytes = a->y != nullptr ? align_up(prefill_tc_partial_bytes(a), 256) : 0;
     pl.ws_bytes += pl.part_bytes;
-    pl.gate_stride = (2 * pl.nseg - 1) * prefill_tc_grid_z(a, pl.wide);  // state pass over all segments but the last
+    pl.gate_stride = prefill_tc_gate_stride(a, pl.nseg, pl.wide);
     if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
       pl.gate_off = pl.ws_bytes;
       pl.gate_bytes = align_up((size_t)(1 + lanes * pl.gate_stride) * sizeof(int), 256);
@@ -440,7 +440,7 @@ int forward_keep_states(const flare_fwd_args_t* a, const ChunkStates& keep, int*
 }
 
 size_t forward_gate_words(const flare_fwd_args_t* a) {
-  return 1 + (size_t)a->B * a->H * plan_forward(a).gate_stride;
+  return 1 + (size_t)a->B * a->H * prefill_tc_max_gate_stride(a);
 }
 
 int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, float* seg_m, float* seg_d, float* seg_u,

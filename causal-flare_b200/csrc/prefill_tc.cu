@@ -1297,8 +1297,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && p.gate != nullptr)
+  if (tid == 0 && p.gate != nullptr) {
     p.gate[1 + (int64_t)lane_id * p.gate_stride + p.gate_off + (int)(blockIdx.y * gridDim.z + blockIdx.z)] = misc->out_of_domain;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) p.gate[0] = p.gate_stride;  // (both passes write the same)
+  }
   // the partner may still write to this CTA's shared memory or arrive on its barriers until it is done as well
   if (xmerge) cluster_sync_all();
   if (warp == 12) tmem_dealloc(tmem, TM_COLS);
@@ -1502,30 +1504,55 @@ int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide) { return prefill_tc_
 // the most that is cut, at 256 tokens or more per segment; wide only beyond one wave): B=1 H=16 M=128 D=128 N=32768
 // 306 -> 190 us (4 segments of two slices -> 9 wide), B=1 H=32 N=8192 166 -> 124 us, B=1 H=16 M=64 D=64 N=777
 // 32 -> 26 us (3 segments -> 1).
-void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg_out, bool* wide_out) {
+static bool can_wide(const flare_fwd_args_t* a) { return a->Dk == 128 && a->Dv == 128 && (a->M % M) == 0; }
+
+// estimated time of the call on one instance, and the segments that give it
+static double plan_instance(const flare_fwd_args_t* a, bool wide, int* nseg_out) {
   const int nch = (a->N + C - 1) / C;
   const int64_t lanes = (int64_t)a->B * a->H;
   const int sms = sm_count();
-  const bool can_wide = a->Dk == 128 && a->Dv == 128 && (a->M % M) == 0;
-  bool try_wide[2] = {true, can_wide};
+  const double pass = wide ? 3.2 : 2.55, state_pass = wide ? 1.3 : 1.4;
+  const int64_t ctas = lanes * prefill_tc_grid_z(a, wide);
+  const double waves = (double)((ctas + sms - 1) / sms);
+  double best = 8.0 + waves * nch * pass;
+  *nseg_out = 1;
+  if (ctas * 2 > sms) return best;
+  const int most = (int)(sms / ctas) < nch ? (int)(sms / ctas) : nch;
+  const int len = (nch + most - 1) / most, n = (nch + len - 1) / len;  // chunks per segment, segments that many make
+  const double t = 22.0 + 3e-6 * (double)lanes * n * a->M * a->Dv * 4 + len * (pass + state_pass);
+  if (1.1 * t < best) best = t, *nseg_out = n;  // (worth two more launches)
+  return best;
+}
+
+void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg_out, bool* wide_out) {
+  bool try_wide[2] = {true, can_wide(a)};
   if (const char* env = getenv("FLARE_B200_WIDE")) {  // 0 / 1 forces the instance
-    try_wide[0] = env[0] != '1' || !can_wide;
-    try_wide[1] = env[0] == '1' && can_wide;
+    try_wide[0] = env[0] != '1' || !try_wide[1];
+    try_wide[1] = env[0] == '1' && try_wide[1];
   }
   double best = 1e30;
   for (int w = 0; w < 2; ++w) {
     if (!try_wide[w]) continue;
-    const double pass = w ? 3.2 : 2.55, state_pass = w ? 1.3 : 1.4;
-    const int64_t ctas = lanes * prefill_tc_grid_z(a, w != 0);
-    const double waves = (double)((ctas + sms - 1) / sms);
-    double t = 8.0 + waves * nch * pass;
-    if (t < best) best = t, *nseg_out = 1, *wide_out = w != 0;
-    if (ctas * 2 > sms) continue;
-    const int most = (int)(sms / ctas) < nch ? (int)(sms / ctas) : nch;
-    const int len = (nch + most - 1) / most, n = (nch + len - 1) / len;  // chunks per segment, segments that many make
-    t = 22.0 + 3e-6 * (double)lanes * n * a->M * a->Dv * 4 + len * (pass + state_pass);
-    if (1.1 * t < best) best = t, *nseg_out = n, *wide_out = w != 0;  // (worth two more launches)
+    int n = 1;
+    const double t = plan_instance(a, w != 0, &n);
+    // (segments are worth it only if they also beat the other instance by a tenth)
+    if ((n > 1 ? 1.1 * t : t) < best) best = t, *nseg_out = n, *wide_out = w != 0;
   }
+}
+
+int prefill_tc_gate_stride(const flare_fwd_args_t* a, int nseg, bool wide) {
+  return (2 * nseg - 1) * prefill_tc_grid_z(a, wide);  // state pass over all segments but the last, read-out over all
+}
+
+int prefill_tc_max_gate_stride(const flare_fwd_args_t* a) {
+  int most = 0;
+  for (int w = 0; w < (can_wide(a) ? 2 : 1); ++w) {
+    int n = 1;
+    plan_instance(a, w != 0, &n);
+    const int stride = prefill_tc_gate_stride(a, n, w != 0);
+    if (stride > most) most = stride;
+  }
+  return most;
 }
 
 // fp16 partial read-outs [groups][B][N][H][Dv], then fp32 weight masses [groups][B][N][H]

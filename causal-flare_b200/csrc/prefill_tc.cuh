@@ -46,7 +46,7 @@ struct TcParams {
   int dump_nch;
   // Optional gate words (in the caller's workspace): CTA (lane, segment, z) writes gate[1 + lane * gate_stride + gate_off +
   // segment * grid.z + z] when it ends, 1 if a token it handled left the numeric domain of these kernels, else 0 (so
-  // nothing has to be cleared before the launch).
+  // nothing has to be cleared before the launch).  gate[0] = gate_stride, for a backward that reads the words later.
   int* gate;
   int gate_stride, gate_off;
   int* err;                  // device error word (bit 0: a wait gave up, bit 1: numeric domain exceeded)
@@ -62,6 +62,10 @@ size_t prefill_tc_partial_lw_offset(const flare_fwd_args_t* a);
 void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg, bool* wide);
 // grid.z of a launch
 int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide);
+// gate words per lane of a call on that instance with that many segments, and the most that any plan of these sizes needs,
+// whatever instance the environment asks for (what a backward sizes by, see keep_layout)
+int prefill_tc_gate_stride(const flare_fwd_args_t* a, int nseg, bool wide);
+int prefill_tc_max_gate_stride(const flare_fwd_args_t* a);
 // launches segments 0 .. nseg_grid-1
 int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, bool wide, cudaStream_t stream);
 // device address (current device) of the error word shared by all tensor-core kernels

@@ -155,3 +155,19 @@ def test_cpu_tensors_are_refused():
         cf.flare_recurrent_triton(q, k, v)
     with pytest.raises(RuntimeError, match="CUDA"):
         cf.flare_semi_autoregressive_trition(q, torch.randn(1, 16, 2, 16), torch.randn(1, 16, 2, 16), block_size=16, chunk_size=16)
+
+
+@pytest.mark.parametrize("B, N, H, M", [(1, 4096, 1, 128), (1, 32768, 16, 128), (1, 2000, 2, 256), (1, 32768, 8, 256)])
+def test_kept_buffer_does_not_depend_on_the_instance_choice(monkeypatch, B, N, H, M):
+    # a forward fills the buffer and a backward, possibly under another FLARE_B200_WIDE, looks the parts up by this layout
+    lib = _lib.load()
+    a = _fake_args(B=B, N=N, H=H, M=M, Dk=128, Dv=128)
+    monkeypatch.delenv("FLARE_B200_WIDE", raising=False)
+    sizes = [lib.flare_forward_keep_bytes(C.byref(a))]
+    plans = [lib.flare_forward_workspace_bytes(C.byref(a))]
+    for wide in ("0", "1"):
+        monkeypatch.setenv("FLARE_B200_WIDE", wide)
+        sizes.append(lib.flare_forward_keep_bytes(C.byref(a)))
+        plans.append(lib.flare_forward_workspace_bytes(C.byref(a)))
+    assert len(set(sizes)) == 1, sizes
+    assert len(set(plans)) > 1  # (the plans themselves do differ)

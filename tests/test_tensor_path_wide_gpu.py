@@ -5,6 +5,7 @@ two-slice instance (FLARE_B200_WIDE=0) on the same inputs."""
 import pytest
 import torch
 
+import causal_flare as cf
 from causal_flare import _lib, _ops
 from oracle import flare_oracle as orc
 from util import assert_bf16_gate, assert_close, to_dev
@@ -143,3 +144,29 @@ def test_wide_training_forward_keeps_the_same_states_as_the_two_slice_instance(w
     ref = orc.ar_backward_closed_form(q, k, v, dy, scale=sc, block_size=bs)
     for name, got in zip(("dQ", "dK", "dV"), out["1"][1]):
         assert orc.rel_l2(got.float().cpu(), ref[name]) <= 6.5e-3, name
+
+
+@pytest.mark.parametrize("sharp", [False, True])
+@pytest.mark.parametrize("Ml, N", [(128, 4096), (256, 2000)])
+def test_backward_reads_what_a_forward_under_another_instance_choice_kept(monkeypatch, Ml, N, sharp):
+    # shapes whose two instances take different numbers of segments, hence gate words; sharp: flagged by the forward, so
+    # that the backward has to find its gate words
+    q, k, v, dy = to_dev(*orc.make_inputs(1, N, 1, Ml, D, seed0=16, dtype=torch.bfloat16, with_dy=True))
+    if sharp:
+        q = q * 40.0
+    got = {}
+    for fwd, bwd in (("0", "0"), ("0", "1"), ("1", "1"), ("1", "0")):
+        monkeypatch.setenv("FLARE_B200_WIDE", fwd)
+        leaves = [t.detach().requires_grad_() for t in (q, k, v)]
+        y = cf.flare_autoregressive_triton(*leaves)
+        monkeypatch.setenv("FLARE_B200_WIDE", bwd)
+        got[fwd + bwd] = torch.autograd.grad(y, leaves, dy)
+    for fwd in "01":
+        for a, b in zip(got[fwd + "0"], got[fwd + "1"]):
+            assert torch.equal(a, b)
+    if sharp:
+        ref = _ops.backward(q, k, v, dy, scale=D ** -0.5, path=_lib.PATH_EXACT)
+        for key in got:
+            for a, b in zip(got[key], ref[:3]):
+                assert torch.equal(a, b.to(a.dtype))  # the exact kernels on both sides
+    _ops.device_status()  # clear the informational flag for the tests that follow
