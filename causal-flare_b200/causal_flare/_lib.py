@@ -74,10 +74,12 @@ class DecodeArgs(C.Structure):
     ]
 
 
+ABI_VERSION = 3  # FLARE_ABI_VERSION of include/flare_b200.h
+
 EXPORTS = (
     "flare_forward_workspace_bytes", "flare_forward", "flare_forward_keep_bytes", "flare_backward_workspace_bytes",
     "flare_backward",
-    "flare_decode_step", "flare_state_merge", "flare_status_string", "flare_last_cuda_error",
+    "flare_decode_step", "flare_state_merge", "flare_mask_pack", "flare_mask_unpack", "flare_status_string", "flare_last_cuda_error",
     "flare_abi_version", "flare_abi_sizeof", "flare_set_kernel_events", "flare_last_launch_count",
     "flare_forward_uses_tensor_path", "flare_backward_uses_tensor_path", "flare_device_status", "flare_set_trace_buffer",
     "flare_forward_noalloc", "flare_noalloc_scratch_capacity",
@@ -156,6 +158,8 @@ def load() -> C.CDLL:
     lib.flare_set_trace_buffer.restype = None
     lib.flare_set_trace_buffer.argtypes = [C.c_void_p]
     lib.flare_device_status.argtypes = [C.c_int]
+    if lib.flare_abi_version() != ABI_VERSION:
+        raise RuntimeError(f"ABI mismatch: library version {lib.flare_abi_version()}, binding version {ABI_VERSION}")
     lib.flare_abi_sizeof.restype = C.c_size_t
     lib.flare_abi_sizeof.argtypes = [C.c_int]
     for which, struct in enumerate((FwdArgs, BwdArgs, DecodeArgs, State)):

@@ -552,7 +552,7 @@ static int check_backward(const flare_bwd_args_t* args) {
 
 // fp16 gradients on the tensor-core backward, the same way as the fp16 forward: bf16 copies of q, k, v and dY in the
 // workspace, the bf16 backward (with its own replay of the forward, gate and exact standby) on those, dK and dV
-// written back as fp16; dQ is fp32 on both sides.
+// written back as fp16; dQ goes to the caller's buffer in the caller's type on both sides.
 namespace {
 struct BwdCastPlan {
   bool on;
@@ -760,7 +760,7 @@ const char* flare_status_string(int status) {
 
 const char* flare_last_cuda_error(void) { return g_cuda_error; }
 
-int flare_abi_version(void) { return 2; }
+int flare_abi_version(void) { return FLARE_ABI_VERSION; }
 
 void flare_profile_enable(int on) {
   if (on) profile_clear();

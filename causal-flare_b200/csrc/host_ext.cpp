@@ -46,6 +46,9 @@ void take(F& f, const py::dict& table, const char* name) {
 }
 
 void bind(const py::dict& table) {
+  decltype(&flare_abi_version) version = nullptr;
+  take(version, table, "flare_abi_version");
+  if (version() != FLARE_ABI_VERSION) throw std::runtime_error("the native host layer was built for another version of the library");
   take(api.forward_workspace_bytes, table, "flare_forward_workspace_bytes");
   take(api.forward_keep_bytes, table, "flare_forward_keep_bytes");
   take(api.forward, table, "flare_forward");

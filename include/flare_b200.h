@@ -131,7 +131,7 @@ size_t flare_noalloc_scratch_capacity(void);
  * tensor-core one (bwd_tc.cu: a forward that keeps per-chunk states, then a reverse chunk sweep on tcgen05 and a
  * tensor-core dK / dQ product) for the shapes flare_backward_uses_tensor_path accepts, and the exact fp32 one
  * (bwd_exact.cu) for everything else; fwd.path = FLARE_PATH_EXACT forces the latter.
- * dq / dk_dec are fp32 [H, M, Dk] (summed over the batch); dk, dv, dq_dec have the input dtype and the
+ * dq / dk_dec are [H, M, Dk] (summed over the batch in fp32; dk_dec is fp32, dq as dq_dtype says); dk, dv, dq_dec have the input dtype and the
  * input's shape, densely packed.  With weight sharing (q_dec/k_dec NULL) the decode-side gradients are
  * folded into dk / dq and dq_dec / dk_dec must be NULL.
  */
@@ -225,6 +225,10 @@ int flare_mask_unpack(const int32_t* slot, const void* y_in, void* y, const int6
 
 const char* flare_status_string(int status);
 const char* flare_last_cuda_error(void);
+/* Version of the structs and functions above.  It grows with every change that a caller compiled against an older header
+ * would not survive; such a caller must not call a library whose flare_abi_version() differs from its FLARE_ABI_VERSION.
+ * 3: flare_bwd_args_t ends with dq_dtype, flare_mask_pack / flare_mask_unpack. */
+#define FLARE_ABI_VERSION 3
 int flare_abi_version(void);
 
 /* Measurement hooks (no counterpart in the reference; used by the benchmark).

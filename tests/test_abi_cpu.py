@@ -36,6 +36,18 @@ def test_library_exports_every_declared_symbol():
     assert lib.flare_abi_version() >= 1
 
 
+def test_version_of_the_structs(monkeypatch):
+    # flare_bwd_args_t grew: a binding of before the change must be able to tell
+    lib = _lib.load()
+    assert lib.flare_abi_version() == _lib.ABI_VERSION == 3
+    header = open(os.path.join(ROOT, "include", "flare_b200.h")).read()
+    assert f"#define FLARE_ABI_VERSION {_lib.ABI_VERSION}\n" in header
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "ABI_VERSION", 2)
+    with pytest.raises(RuntimeError, match="ABI mismatch"):
+        _lib.load()
+
+
 def test_struct_layouts_match():
     lib = _lib.load()
     for which, struct in enumerate((_lib.FwdArgs, _lib.BwdArgs, _lib.DecodeArgs, _lib.State)):
