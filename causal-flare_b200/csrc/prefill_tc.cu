@@ -44,7 +44,6 @@
 #include <string.h>
 
 #include "sm100_ptx.cuh"
-#include "state_ops.cuh"
 #include "tc_device.cuh"
 
 // polling rounds of every wait of the prefill kernel before it suspends (see tc::wait_or_abort)
@@ -200,13 +199,16 @@ int launch_prefill_tc_unit(int lat, int mode, const CUtensorMap& tq, const CUten
 //       SMs in one wave.  Differences: U and Y are 128 columns wide; W and Y0 = R^T U_bf16 come out of ONE product of
 //       width 256 ([E | U_bf16] as one B operand, [W | Y] adjacent in tensor memory), so R is read once for both; W
 //       shares the columns of S; E and R are single-buffered.
-template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE>
+// Y16: the wide instance writes y as fp16 (the others look at p.y_f16; here that choice, in registers of the epilogue, cost
+//       the bf16 calls 5 to 8 %)
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, bool Y16>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y, const TcParams p) {
   using L = Lay<DKB, WIDE>;
   constexpr bool PADDED = LAT != 0, PACK = LAT == 2;
   static_assert(!WIDE || (DVB == 2 && !PADDED), "wide instance");
+  static_assert(!Y16 || (WIDE && !KEEP), "fp16 read-out of the wide instance");
   static_assert(!PACK || !SPLIT, "one group of at most 64 latents");
   constexpr int NP = PACK ? 4 : 2;       // token parts of a chunk = latent warps per 32 latents
   constexpr int TOK = C / NP;            // tokens per latent thread
@@ -1207,7 +1209,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
                                  f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
               }
-              pack_out(y, false, o);
+              pack_out(y, Y16, o);
               *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
                   make_uint4(o[0], o[1], o[2], o[3]);
             }
@@ -1252,7 +1254,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             for (int j = 0; j < 4; ++j)  // two columns per multiply
               f2_unpack(f2_mul(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])), inv2), y[2 * j],
                         y[2 * j + 1]);
-            pack_out(y, SPLIT || (!WIDE && p.y_f16 != 0), o);
+            pack_out(y, SPLIT || (WIDE ? Y16 : p.y_f16 != 0), o);
             v[ch] = make_uint4(o[0], o[1], o[2], o[3]);
           }
           if (p.y_tma) {
@@ -1310,10 +1312,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 namespace {
 
-template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE = false>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE = false, bool Y16 = false>
 int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
-  auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE>;
+  auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE, Y16>;
   static int granted[64] = {};
   FLARE_CUDA_CHECK(allow_smem(kern, Lay<DKB, WIDE>::SMEM_BYTES, granted));
   LaunchTimer timer(p.y == nullptr ? "prefill_tc_kernel (state only)" : (WIDE ? "prefill_tc_kernel (wide)" : "prefill_tc_kernel"),
@@ -1363,6 +1365,11 @@ int launch_prefill_tc_unit<FLARE_TC_UNIT>(int lat, int mode, const CUtensorMap& 
     if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, true, true>(tq, tk, tv, ty, p, grid, stream);
     if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, true, true>(tq, tk, tv, ty, p, grid, stream);
     return launch_keep<0, 2, 2, WSPLIT, 0, true, true>(tq, tk, tv, ty, p, grid, stream);
+  }
+  if (p.y_f16 && p.y != nullptr && (!WSPLIT || p.cluster_merge)) {  // (partials in global memory become y in the merge kernel)
+    if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, false, true, true>(tq, tk, tv, ty, p, grid, stream);
+    if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, false, true, true>(tq, tk, tv, ty, p, grid, stream);
+    return launch_keep<0, 2, 2, WSPLIT, 0, false, true, true>(tq, tk, tv, ty, p, grid, stream);
   }
   if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, false, true>(tq, tk, tv, ty, p, grid, stream);
   if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, false, true>(tq, tk, tv, ty, p, grid, stream);
@@ -1653,15 +1660,6 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   else
     rc = groups > 1 ? launch_prefill_tc_unit<5>(lat, mode, tq, tk, tv, ty, p, grid, stream)
                     : launch_prefill_tc_unit<2>(lat, mode, tq, tk, tv, ty, p, grid, stream);
-  if (rc == FLARE_OK && p.y_f16 && wide && p.y != nullptr && (groups == 1 || p.cluster_merge)) {
-    // the wide instance writes bf16 whatever the call's type (the choice between two packings in its epilogue cost it 8 %):
-    // converted in place
-    CastParams c;
-    memset(&c, 0, sizeof(c));
-    c.in = p.y; c.out = p.y; c.n0 = a->B; c.n1 = a->N; c.n2 = a->H; c.d = a->Dv;
-    c.is0 = c.os0 = p.y_stride_b; c.is1 = c.os1 = p.y_stride_n; c.is2 = c.os2 = p.y_stride_h;
-    rc = launch_cast_rows(&c, 1, true, stream);
-  }
   if (rc != FLARE_OK || groups == 1 || p.y == nullptr || p.cluster_merge) return rc;
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);

@@ -28,6 +28,7 @@ struct TcParams {
   // per-row lengths are given); otherwise every thread stores its own row
   int y_tma;
   int y_f16;  // y is fp16 (a call on bf16 copies of fp16 inputs): rounded once, from the fp32 accumulators
+             // (the wide instance: by its template parameter Y16)
   // Two latent groups on the wide instance: the two CTAs of a lane form a thread-block cluster and merge their
   // partial read-outs on chip (each finalises one 64-column value block); no partials in global memory, no merge
   // kernel.  Set by the launch.

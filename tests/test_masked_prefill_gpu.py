@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import causal_flare as cf
+from causal_flare import _lib, _ops
 from oracle import flare_oracle as orc
 from util import assert_bf16_gate, to_dev
 
@@ -37,13 +38,50 @@ def test_packed_rows(N, M, Dk, Dv, dtype):
         assert_bf16_gate((st["u"] / st["d"][..., None])[b:b + 1], ref_st["u"] / ref_st["d"][..., None], f"state {b}")
 
 
-@pytest.mark.parametrize("shape", [(1, 300, 2, 64, 64, 64), (2, 700, 2, 192, 64, 128), (1, 384, 2, 256, 128, 128), (2, 130, 3, 48, 128, 128)])
-def test_fp16_read_out_is_rounded_once(shape):
-    # y leaves the kernels as fp16: against the same call on the bf16 copies only the last rounding differs, at most half a
-    # bf16 ulp (2^-8 relative) and half an fp16 ulp (2^-11 relative, 2^-25 absolute)
+WIDE = [None, "1", "1 merge kernel"]  # instance of (128, 128) heads: the planner's choice, the wide one, its groups in global memory
+
+
+def choose(monkeypatch, wide):
+    if wide:
+        monkeypatch.setenv("FLARE_B200_WIDE", "1")
+        monkeypatch.setenv("FLARE_B200_CLUSTER", "0" if "merge" in wide else "1")
+
+
+@pytest.mark.parametrize("bhnd", [False, True])
+@pytest.mark.parametrize("wide", WIDE)
+@pytest.mark.parametrize("shape", [(1, 300, 2, 64, 64, 64), (2, 700, 2, 192, 64, 128), (1, 384, 2, 128, 128, 128), (1, 384, 2, 256, 128, 128),
+                                   (1, 200, 1, 384, 128, 128), (2, 130, 3, 48, 128, 128)])
+def test_fp16_read_out_is_rounded_once(monkeypatch, shape, wide, bhnd):
+    # y leaves the kernels as fp16.  Against the same call on the bf16 copies only the last rounding differs, at most half a
+    # bf16 ulp (2^-8 relative) and half an fp16 ulp (2^-11 relative, 2^-25 absolute); rounded to bf16 on the way, every
+    # entry would be a bf16 value, of which there are one in eight.
     B, N, H, M, Dk, Dv = shape
+    choose(monkeypatch, wide)
     q, k, v = to_dev(*orc.make_inputs(B, N, H, M, Dk, Dv, seed0=4, dtype=torch.bfloat16))
     q, k, v = (t.half().bfloat16() for t in (q, k, v))  # values that both formats hold
-    a = cf.flare_autoregressive_triton(q.half(), k.half(), v.half()).double()
-    b = cf.flare_autoregressive_triton(q, k, v).double()
-    assert ((a - b).abs() <= b.abs() * (2.0 ** -8 + 2.0 ** -11) + 2.0 ** -24).all()
+    a = _ops.forward(q.half(), k.half(), v.half(), scale=Dk ** -0.5, out_bhnd=bhnd)[0]
+    b = _ops.forward(q, k, v, scale=Dk ** -0.5, out_bhnd=bhnd)[0].double()
+    assert a.dtype == torch.float16
+    bf16_values = (a.bfloat16().double() == a.double()).double().mean()
+    assert bf16_values < 0.3, f"{bf16_values:.2f} of the entries are bf16 values"
+    assert ((a.double() - b).abs() <= b.abs() * (2.0 ** -8 + 2.0 ** -11) + 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("wide", WIDE)
+@pytest.mark.parametrize("M, Dk", [(128, 128), (256, 128), (64, 64)])
+def test_rows_beyond_a_length_are_left_alone(monkeypatch, M, Dk, wide, dtype):
+    B, N, H = 3, 300, 2
+    choose(monkeypatch, wide)
+    q, k, v = orc.make_inputs(B, N, H, M, Dk, seed0=9, dtype=dtype)
+    lens = [300, 129, 0]
+    qc, kc, vc = to_dev(q, k, v)
+    y = torch.full_like(vc, 1.2345)
+    before = y.clone()
+    lengths = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    args = _lib.make_fwd_args(qc, kc, vc, None, None, y, scale=Dk ** -0.5, lengths=lengths)
+    _lib.run_forward(args, qc.device)
+    for b, n in enumerate(lens):
+        assert torch.equal(y[b, n:], before[b, n:]), f"row {b}"
+        if n:
+            assert_bf16_gate(y[b:b + 1, :n], orc.ar_forward(q, k[b:b + 1, :n], v[b:b + 1, :n], scale=Dk ** -0.5), f"row {b}")
