@@ -976,14 +976,12 @@ template <int MM_MAX, int DD>
 static int launch_bwd_one(const BwdParams& p, dim3 grid, size_t smem1, size_t smem2, cudaStream_t stream, int stage) {
   if (stage == 0) {
     auto k1 = bwd_replay_kernel<MM_MAX, DD>;
-    static int granted[64] = {};
-    FLARE_CUDA_CHECK(allow_smem(k1, smem1, granted));
+    FLARE_CUDA_CHECK(allow_smem(k1));
     LaunchTimer timer("bwd_replay_kernel", stream);
     FLARE_CUDA_CHECK(launch_pdl(k1, grid, dim3(NT), smem1, stream, p));
   } else {
     auto k2 = bwd_reverse_kernel<MM_MAX, DD>;
-    static int granted[64] = {};
-    FLARE_CUDA_CHECK(allow_smem(k2, smem2, granted));
+    FLARE_CUDA_CHECK(allow_smem(k2));
     LaunchTimer timer("bwd_reverse_kernel", stream);
     FLARE_CUDA_CHECK(launch_pdl(k2, grid, dim3(NT), smem2, stream, p));
   }

@@ -905,8 +905,7 @@ template <int DKB, int DVB, int MODE, bool PACK>
 int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy, const CUtensorMap& tu,
                 const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = bwd_tc_kernel<DKB, DVB, MODE, PACK>;
-  static int granted[64] = {};
-  FLARE_CUDA_CHECK(allow_smem(kern, BL<DVB>::SMEM_BYTES, granted));
+  FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("bwd_tc_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_MAIN), BL<DVB>::SMEM_BYTES, stream, tk, tv, tdy, tu, p));
   return FLARE_OK;
@@ -1219,8 +1218,7 @@ int launch_grads(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMa
                  cudaStream_t stream) {
   auto kern = bwd_tc_grads_kernel<DKB>;
   const int smem = GL<DKB>::smem_bytes(p.groups);
-  static int granted[64] = {};
-  FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
+  FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("bwd_tc_grads_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_GRAD), smem, stream, tds, tk, tq, p));
   return FLARE_OK;

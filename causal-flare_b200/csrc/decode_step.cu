@@ -193,8 +193,7 @@ bool decode_step_supported(int M, int Dk, int Dv) {
 template <int PRE, int UNR, int MINB>
 static int launch_variant(const DecodeParams& p, size_t smem, cudaStream_t stream) {
   auto kern = decode_step_kernel<PRE, UNR, MINB>;
-  static int granted[64] = {};
-  if (smem > 48 * 1024) FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
+  if (smem > 48 * 1024) FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("decode_step_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(kern, dim3(p.B * p.H), dim3(NT), smem, stream, p));
   return FLARE_OK;

@@ -70,18 +70,15 @@ inline cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
 }
 
-// Raises a kernel's dynamic shared memory limit to `bytes`, once per device and value (`granted`: a static of the launch
-// site, one entry per device ordinal; racing first calls ask for the same thing).
+constexpr int kMaxDynamicSmem = 227 * 1024;  // what a block may have beyond the system's own kilobyte
+
+// Allows a kernel (one without static shared memory) all the dynamic shared memory there is.  Always the same limit, whatever
+// the launch at hand needs: a kernel's limit is shared by all host threads, and one that lowered it for its own launch would
+// fail another's.  Asked for on every launch: the limit belongs to the context, which the host may have torn down and rebuilt
+// since the last call.
 template <typename Kern>
-inline cudaError_t allow_smem(Kern kern, size_t bytes, int (&granted)[64]) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const bool known = dev >= 0 && dev < 64;
-  if (known && granted[dev] >= (int)bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && known) granted[dev] = (int)bytes;
-  return e;
+inline cudaError_t allow_smem(Kern kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

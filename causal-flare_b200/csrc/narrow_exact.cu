@@ -578,11 +578,10 @@ __global__ void __launch_bounds__(128, 4) narrow_reverse_kernel(const NarrowBwdP
           make_float4(dq[i][0] * p.scale, dq[i][1] * p.scale, dq[i][2] * p.scale, dq[i][3] * p.scale);
 }
 
-template <int WHICH, typename Kern, typename P>
+template <typename Kern, typename P>
 int launch(Kern kern, const char* name, const P& p, int nseg_grid, int floats, cudaStream_t stream) {
-  static int granted[2][64] = {};  // (one per kernel: WHICH tells those of one signature apart)
   LaunchTimer timer(name, stream);
-  FLARE_CUDA_CHECK(allow_smem(kern, floats * sizeof(float), granted[p.variant == FLARE_STABLEMAX]));
+  FLARE_CUDA_CHECK(allow_smem(kern));
   FLARE_CUDA_CHECK(launch_pdl(kern, dim3(p.B * p.H, nseg_grid), dim3(narrow_warps(p.M) * 32), floats * sizeof(float), stream, p));
   return FLARE_OK;
 }
@@ -592,22 +591,22 @@ int launch(Kern kern, const char* name, const P& p, int nseg_grid, int floats, c
 int launch_walk_narrow(const WalkParams& p, int nseg_grid, cudaStream_t stream) {
   const int nw = narrow_warps(p.M), ms = nw * 32;
   const int floats = 2 * BT * W + 3 * BT * ms + nw * BT * W + 2 * nw * BT + BT;
-  return launch<0>(p.variant == FLARE_STABLEMAX ? walk_narrow_kernel<true> : walk_narrow_kernel<false>,
-                   "walk_exact_kernel (narrow heads)", p, nseg_grid, floats, stream);
+  return launch(p.variant == FLARE_STABLEMAX ? walk_narrow_kernel<true> : walk_narrow_kernel<false>,
+                "walk_exact_kernel (narrow heads)", p, nseg_grid, floats, stream);
 }
 
 int launch_narrow_replay(const NarrowBwdParams& p, cudaStream_t stream) {
   const int nw = narrow_warps(p.M), ms = nw * 32;
   const int floats = 3 * BT * W + 4 * BT * ms + 2 * nw * BT;
-  return launch<1>(p.variant == FLARE_STABLEMAX ? narrow_replay_kernel<true> : narrow_replay_kernel<false>,
-                   "bwd_replay_kernel (narrow heads)", p, p.nseg, floats, stream);
+  return launch(p.variant == FLARE_STABLEMAX ? narrow_replay_kernel<true> : narrow_replay_kernel<false>,
+                "bwd_replay_kernel (narrow heads)", p, p.nseg, floats, stream);
 }
 
 int launch_narrow_reverse(const NarrowBwdParams& p, cudaStream_t stream) {
   const int nw = narrow_warps(p.M), ms = nw * 32;
   const int floats = 3 * BT * W + 4 * BT * ms + ms * W + nw * BT * W + nw * BT;
-  return launch<2>(p.variant == FLARE_STABLEMAX ? narrow_reverse_kernel<true> : narrow_reverse_kernel<false>,
-                   "bwd_reverse_kernel (narrow heads)", p, p.nseg, floats, stream);
+  return launch(p.variant == FLARE_STABLEMAX ? narrow_reverse_kernel<true> : narrow_reverse_kernel<false>,
+                "bwd_reverse_kernel (narrow heads)", p, p.nseg, floats, stream);
 }
 
 }  // namespace flare

@@ -1316,8 +1316,7 @@ template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE 
 int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE, Y16>;
-  static int granted[64] = {};
-  FLARE_CUDA_CHECK(allow_smem(kern, Lay<DKB, WIDE>::SMEM_BYTES, granted));
+  FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer(p.y == nullptr ? "prefill_tc_kernel (state only)" : (WIDE ? "prefill_tc_kernel (wide)" : "prefill_tc_kernel"),
                     stream);
   if (WIDE && SPLIT && p.cluster_merge) {
@@ -1672,17 +1671,9 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
 }
 
 int tc_error_word(int** device_address) {
-  static int* known[64] = {};  // per device ordinal: the address does not change while the library is loaded
-  int dev = 0;
-  FLARE_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && known[dev] != nullptr) {
-    *device_address = known[dev];
-    return FLARE_OK;
-  }
   void* err = nullptr;
-  FLARE_CUDA_CHECK(cudaGetSymbolAddress(&err, g_tc_error));
+  FLARE_CUDA_CHECK(cudaGetSymbolAddress(&err, g_tc_error));  // of the current device and context: not remembered
   *device_address = reinterpret_cast<int*>(err);
-  if (dev >= 0 && dev < 64) known[dev] = *device_address;
   return FLARE_OK;
 }
 

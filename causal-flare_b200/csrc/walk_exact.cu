@@ -275,8 +275,7 @@ static size_t walk_exact_smem_bytes(int M, int Dk, int dd) {
 template <int MM_MAX, int DD>
 static int launch_one(const WalkParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
   auto kern = walk_exact_kernel<MM_MAX, DD>;
-  static int granted[64] = {};
-  FLARE_CUDA_CHECK(allow_smem(kern, smem, granted));
+  FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer(p.gate != nullptr ? "walk_exact_kernel (standby)" : "walk_exact_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT), smem, stream, p));
   return FLARE_OK;
