@@ -42,8 +42,10 @@ def fake(tmp_path_factory):
     d = tmp_path_factory.mktemp("fake_runtime")
     (d / "t.cu").write_text(SOURCE)
     (d / "stubs.c").write_text(STUBS)
-    res = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC", "-shared", "-cudart",
-                          "none", "-I", CSRC, str(d / "t.cu"), str(d / "stubs.c"), "-o", str(d / "t.so")], capture_output=True, text=True)
+    cmd = [nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC", "-shared", "-cudart", "none",
+           "-Xlinker", "-Bsymbolic",  # (a CUDA runtime that the test process has loaded must not take the stand-in's place)
+           "-I", CSRC, str(d / "t.cu"), str(d / "stubs.c"), "-o", str(d / "t.so")]
+    res = subprocess.run(cmd, capture_output=True, text=True)
     assert res.returncode == 0, res.stderr
     return C.CDLL(str(d / "t.so"), mode=os.RTLD_LAZY)
 
