@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(NT) bwd_rows_kernel(const RowsParams p) {
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t0 + t < N && m0 + c < M) {
           for (int part = 0; part < p.parts[src]; ++part) {
-            const float4 x = __ldcs(reinterpret_cast<const float4*>(p.ds[src] + (int64_t)part * p.plane +
+            const float4 x = load_streaming(reinterpret_cast<const float4*>(p.ds[src] + (int64_t)part * p.plane +
                                                                     ((int64_t)lane_id * N + t0 + t) * M + m0 + c));
             a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
           }
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(NT) bwd_lat_kernel(const LatParams p) {
           const int64_t bb = r / N, tt = r - bb * N;
           const float* src_p = p.ds[src] + ((bb * p.H + h) * N + tt) * M + m0 + c;
           for (int part = 0; part < p.parts[src]; ++part) {
-            const float4 x = __ldcs(reinterpret_cast<const float4*>(src_p + (int64_t)part * p.plane));
+            const float4 x = load_streaming(reinterpret_cast<const float4*>(src_p + (int64_t)part * p.plane));
             a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
           }
         }
@@ -1006,7 +1006,7 @@ int launch_bwd_mm<FLARE_WALK_MM>(const BwdParams& p, int dd, dim3 grid, size_t s
 // Carries of a segment for a zero carry-in, as products over its tokens (no sequential walk):
 //   b0[m, :] = sum_t X[t, m] dY_t,   c0[m] = sum_t X[t, m] p[t, m].
 // Register-tiled like the latent-gradient kernel: 64 latents x 128 value columns per CTA; grid.y = segment.
-__global__ void __launch_bounds__(NT) bwd_seg_carry_kernel(const float* __restrict__ X, const float* __restrict__ P,
+__global__ void __launch_bounds__(NT) bwd_seg_carry_kernel(const float* X, const float* P,
                                                            int p_parts, int64_t plane, const void* dy, int dtype, int64_t dy_stride_b,
                                                            int64_t dy_stride_n, int64_t dy_stride_h, float* seg_b,
                                                            float* seg_c, float* seg_gam, int nseg, int seg_len, int N,
@@ -1035,12 +1035,12 @@ __global__ void __launch_bounds__(NT) bwd_seg_carry_kernel(const float* __restri
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
       if (t0 + t < tend && m0 + c < M) {
         const int64_t o = (row_base + t0 + t) * M + m0 + c;
-        x = __ldcs(reinterpret_cast<const float4*>(X + o));
+        x = load_streaming(reinterpret_cast<const float4*>(X + o));
         if (dv0 == 0) {
           // c0 partial of this thread's four latents for this token (threads of other rows add theirs below)
           float4 pp = make_float4(0.f, 0.f, 0.f, 0.f);
           for (int part = 0; part < p_parts; ++part) {
-            const float4 y = __ldcs(reinterpret_cast<const float4*>(P + (int64_t)part * plane + o));
+            const float4 y = load_streaming(reinterpret_cast<const float4*>(P + (int64_t)part * plane + o));
             pp.x += y.x; pp.y += y.y; pp.z += y.z; pp.w += y.w;
           }
           // stash x * p behind the x values of the same row: columns LM/4 apart are not used, so keep it in registers
@@ -1105,7 +1105,7 @@ __global__ void __launch_bounds__(NT) bwd_seg_carry_kernel(const float* __restri
 // when those are given.
 __global__ void __launch_bounds__(256) bwd_seg_scan_kernel(float* seg_b, float* seg_c, const float* seg_gam, int nseg,
                                                            int seg_len, int64_t lanes, int N, int M, int Dv,
-                                                           const float* __restrict__ E, const float* __restrict__ RHO,
+                                                           const float* E, const float* RHO,
                                                            int block_size, const float* carry_b, const float* carry_c,
                                                            const float* carry_rho, int write_slots, float* span_b0,
                                                            float* span_c0, float* span_gam, float* span_rho_first,

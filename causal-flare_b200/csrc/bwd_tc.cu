@@ -390,7 +390,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         uint32_t r[16];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint4 x = live ? __ldg(src + i) : make_uint4(0, 0, 0, 0);
+          const uint4 x = live ? src[i] : make_uint4(0, 0, 0, 0);
           r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
         }
         tmem_st16(tl + TQ + tq * 16, r);
@@ -420,7 +420,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         float c_from = 0.f;
         for (int s = p.nseg - 1; s > seg; --s) {
           const int64_t xo = ((int64_t)lane_id * p.nseg + s) * p.M + mg;
-          const float c_to = STABLE ? 0.f : __ldg(p.chunk_c + stat0 + (int64_t)(p.seg_begin[s] - 1) * p.M);
+          const float c_to = STABLE ? 0.f : p.chunk_c[stat0 + (int64_t)(p.seg_begin[s] - 1) * p.M];
           const float f = s == p.nseg - 1 ? 0.f : (STABLE ? 1.f : ex2_approx(c_to - c_from));
           c_from = c_to;
           cc_carry = fmaf(cc_carry, f, p.xc[xo]);
@@ -488,10 +488,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       // latency never sits between two phases.
       const float* const l2_row = p.tok_l2 + (int64_t)lane_id * p.npad + tok0 + (lane & (TOK - 1));
       const float* const dl_row = p.tok_delta + (int64_t)lane_id * p.npad + tok0 + (lane & (TOK - 1));
-      float c_cur = (live && !STABLE) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 1) * p.M) : 0.f;
-      float d_cur = live ? __ldg(p.chunk_d + stat0 + (int64_t)(first - 1) * p.M) : 1.f;
-      float c_nxt = (live && !STABLE && first > 1) ? __ldg(p.chunk_c + stat0 + (int64_t)(first - 2) * p.M) : c_cur;
-      float l2_cur = __ldg(l2_row + (int64_t)(first - 1) * C), dl_cur = __ldg(dl_row + (int64_t)(first - 1) * C);
+      float c_cur = (live && !STABLE) ? p.chunk_c[stat0 + (int64_t)(first - 1) * p.M] : 0.f;
+      float d_cur = live ? p.chunk_d[stat0 + (int64_t)(first - 1) * p.M] : 1.f;
+      float c_nxt = (live && !STABLE && first > 1) ? p.chunk_c[stat0 + (int64_t)(first - 2) * p.M] : c_cur;
+      float l2_cur = l2_row[(int64_t)(first - 1) * C], dl_cur = dl_row[(int64_t)(first - 1) * C];
 
       for (int j = 0; ok && j < steps; ++j) {
         const int i = first - 1 - j, t0 = i * C;
@@ -504,10 +504,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         const float l2_mine = l2_cur, dl_mine = dl_cur;
         // the next chunk's (i - 1) values, used one iteration from now
         if (tid == 0) BT_TRACE(3, j, 0);
-        const float d_pre = (live && i > 0) ? ldg_pinned(p.chunk_d + stat0 + (int64_t)(i - 1) * p.M) : 1.f;
-        const float c_pre = (live && !STABLE && i > 1) ? ldg_pinned(p.chunk_c + stat0 + (int64_t)(i - 2) * p.M) : c_nxt;
-        const float l2_pre = i > 0 ? ldg_pinned(l2_row + (int64_t)(i - 1) * C) : 0.f;
-        const float dl_pre = i > 0 ? ldg_pinned(dl_row + (int64_t)(i - 1) * C) : 0.f;
+        const float d_pre = (live && i > 0) ? ld_pinned(p.chunk_d + stat0 + (int64_t)(i - 1) * p.M) : 1.f;
+        const float c_pre = (live && !STABLE && i > 1) ? ld_pinned(p.chunk_c + stat0 + (int64_t)(i - 2) * p.M) : c_nxt;
+        const float l2_pre = i > 0 ? ld_pinned(l2_row + (int64_t)(i - 1) * C) : 0.f;
+        const float dl_pre = i > 0 ? ld_pinned(dl_row + (int64_t)(i - 1) * C) : 0.f;
         // E / R buffers: the previous chunk's products have read them
         if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
         if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
@@ -941,10 +941,10 @@ namespace {
 // per-token statistics: delta_t = <dY_t, y_t> and the decode log-sum-exp in log2 units, rows padded to whole chunks
 // (delta = 0, log-sum-exp = +inf there, which makes every decode weight of a padding token exactly zero)
 // -------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bfloat16* __restrict__ dy, int64_t dy_sb,
+__global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bfloat16* dy, int64_t dy_sb,
                                                                   int64_t dy_sn, int64_t dy_sh,
-                                                                  const __nv_bfloat16* __restrict__ y, int64_t y_sb,
-                                                                  int64_t y_sn, int64_t y_sh, const float* __restrict__ lse,
+                                                                  const __nv_bfloat16* y, int64_t y_sb,
+                                                                  int64_t y_sn, int64_t y_sh, const float* lse,
                                                                   int B, int N, int H, int Dv, int npad, float* tok_l2,
                                                                   float* tok_delta, const int* fwd_gate,
                                                                   int fwd_gate_words, int* gate) {
@@ -969,8 +969,8 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
   const int b = (int)(bn / npad);
   float acc = 0.f;
   if (in_range && n < N) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(dy + b * dy_sb + (int64_t)n * dy_sn + h * dy_sh + sub * 8));
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(y + b * y_sb + (int64_t)n * y_sn + h * y_sh + sub * 8));
+    const uint4 a = *reinterpret_cast<const uint4*>(dy + b * dy_sb + (int64_t)n * dy_sn + h * dy_sh + sub * 8);
+    const uint4 c = *reinterpret_cast<const uint4*>(y + b * y_sb + (int64_t)n * y_sn + h * y_sh + sub * 8);
     acc = (bf16_lo(a.x) * bf16_lo(c.x) + bf16_hi(a.x) * bf16_hi(c.x)) + (bf16_lo(a.y) * bf16_lo(c.y) + bf16_hi(a.y) * bf16_hi(c.y)) +
           (bf16_lo(a.z) * bf16_lo(c.z) + bf16_hi(a.z) * bf16_hi(c.z)) + (bf16_lo(a.w) * bf16_lo(c.w) + bf16_hi(a.w) * bf16_hi(c.w));
   }
@@ -985,14 +985,14 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
 }
 
 // sum of the latent groups' dV partials (bf16) in fp32
-__global__ void __launch_bounds__(256) bwd_tc_sum_groups_kernel(const __nv_bfloat16* __restrict__ part, int groups, int64_t n8,
+__global__ void __launch_bounds__(256) bwd_tc_sum_groups_kernel(const __nv_bfloat16* part, int groups, int64_t n8,
                                                                  __nv_bfloat16* out) {
   pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n8) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int g = 0; g < groups; ++g) {
-    const uint4 v = __ldcs(reinterpret_cast<const uint4*>(part + (int64_t)g * n8 * 8) + idx);
+    const uint4 v = load_streaming(reinterpret_cast<const uint4*>(part + (int64_t)g * n8 * 8) + idx);
     acc[0] += bf16_lo(v.x); acc[1] += bf16_hi(v.x); acc[2] += bf16_lo(v.y); acc[3] += bf16_hi(v.y);
     acc[4] += bf16_lo(v.z); acc[5] += bf16_hi(v.z); acc[6] += bf16_lo(v.w); acc[7] += bf16_hi(v.w);
   }
@@ -1001,14 +1001,14 @@ __global__ void __launch_bounds__(256) bwd_tc_sum_groups_kernel(const __nv_bfloa
 }
 
 // dq[i] = sum over the (batch, split) partials in fixed order
-__global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* __restrict__ part, int count, int64_t n4, void* out,
+__global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* part, int count, int64_t n4, void* out,
                                                              int out_dtype) {
   pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n4) return;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int s = 0; s < count; ++s) {
-    const float4 v = __ldcs(reinterpret_cast<const float4*>(part + (int64_t)s * n4 * 4) + idx);
+    const float4 v = load_streaming(reinterpret_cast<const float4*>(part + (int64_t)s * n4 * 4) + idx);
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
   store4(out, out_dtype, idx * 4, acc.x, acc.y, acc.z, acc.w);

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
 #pragma unroll
   for (int i = 0; i < PRE; ++i) {
     const int idx = tid + i * NT;
-    pre[i] = idx < total4 ? __ldcs(u4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pre[i] = idx < total4 ? load_streaming(u4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
   // token vectors -> smem fp32
@@ -161,13 +161,13 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   for (; base + UNR * NT <= total4; base += UNR * NT) {
     float4 x[UNR];
 #pragma unroll
-    for (int i = 0; i < UNR; ++i) x[i] = __ldcs(u4 + base + tid + i * NT);
+    for (int i = 0; i < UNR; ++i) x[i] = load_streaming(u4 + base + tid + i * NT);
 #pragma unroll
     for (int i = 0; i < UNR; ++i) apply(x[i], (base + tid + i * NT) / dv4, base + tid + i * NT);
   }
   for (; base < total4; base += NT) {
     const int idx = base + tid;
-    if (idx < total4) apply(__ldcs(u4 + idx), idx / dv4, idx);
+    if (idx < total4) apply(load_streaming(u4 + idx), idx / dv4, idx);
   }
 
   // reduce y over the row groups that share a column

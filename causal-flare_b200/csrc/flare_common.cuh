@@ -54,6 +54,20 @@ __device__ __forceinline__ void pdl_begin() {
   pdl_trigger();
   pdl_wait();
 }
+// What a kernel reads may have been written by the kernel before it, which can still be running when this one starts.  So no
+// load goes through the read-only path (which assumes memory that nobody writes while the kernel runs, and whose loads the
+// compiler may move over the wait): no __restrict__ inputs, no read-only intrinsics; and the streaming loads below are pinned
+// behind the wait like it.
+__device__ __forceinline__ float4 load_streaming(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 load_streaming(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
@@ -94,11 +108,11 @@ __device__ __forceinline__ float bf16_bits_to_float(uint32_t bits16) { return __
 __device__ __forceinline__ void load8(const void* base, int dtype, int64_t off, float (&out)[8]) {
   if (dtype == FLARE_F32) {
     const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + off);
-    float4 a = __ldg(p), b = __ldg(p + 1);
+    float4 a = *p, b = *(p + 1);
     out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
     out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
   } else {
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + off));
+    const uint4 r = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + off);
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
     if (dtype == FLARE_BF16) {
 #pragma unroll

@@ -481,7 +481,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                                                         hf * (DKB * 32));
 #pragma unroll
       for (int i = 0; i < DKB * 4; ++i) {
-        const uint4 x = live ? __ldg(src + i) : make_uint4(0, 0, 0, 0);
+        const uint4 x = live ? src[i] : make_uint4(0, 0, 0, 0);
         r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
       }
       static_assert(Q_SMEM || DKB == 2, "store width");
@@ -1438,7 +1438,7 @@ bool prefill_tc_supported(const flare_fwd_args_t* a) {
 
 // Merge of the latent groups' partial read-outs: y = sum_g w_g y_g / sum_g w_g with w_g = exp2(lw_g - max lw).
 // One thread per (token, head, 8 value columns).
-__global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* __restrict__ part_y, const float* __restrict__ part_lw,
+__global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* part_y, const float* part_lw,
                                                                int groups, int64_t rows /* B*N*H */, int N, int H, int dv,
                                                                uint16_t* y, int y_f16, int64_t y_stride_b, int64_t y_stride_n,
                                                                int64_t y_stride_h, float* lse_dec /* [B, H, N] or null */,

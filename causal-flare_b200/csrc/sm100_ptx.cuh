@@ -308,11 +308,11 @@ __device__ __forceinline__ void tmem_write(uint32_t taddr, const uint32_t (&r)[N
   else tmem_st32(taddr, r);
 }
 
-// Read-only global load that the compiler may not move: issued exactly where it is written, so a value needed one
+// Global load that the compiler may not move: issued exactly where it is written, so a value needed one
 // loop iteration later is in flight during the whole iteration (a plain load gets sunk to its first use).
-__device__ __forceinline__ float ldg_pinned(const float* p) {
+__device__ __forceinline__ float ld_pinned(const float* p) {
   float x;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(p));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(p));
   return x;
 }
 

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) cast_rows_kernel(const __grid_constant__ 
 }
 
 // One CTA per batch row: ranks by ballots within a warp, then over the warps.
-__global__ void __launch_bounds__(1024) mask_slots_kernel(const int* __restrict__ mask, int N, int* slot, int* lens) {
+__global__ void __launch_bounds__(1024) mask_slots_kernel(const int* mask, int N, int* slot, int* lens) {
   pdl_begin();
   __shared__ int sums[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
