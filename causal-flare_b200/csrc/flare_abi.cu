@@ -45,6 +45,13 @@ static thread_local long long* g_trace = nullptr;
 static thread_local ChunkStates g_keep = {nullptr, nullptr, nullptr, 0};
 // gate words of the tensor-core forward in flight on this thread (null: none), see FwdPlan::gate_bytes
 static thread_local int* g_gate = nullptr;
+// workspace that a forward may plan with, see ScratchLimit
+static thread_local size_t g_scratch_limit = SIZE_MAX;
+ScratchLimit::ScratchLimit(size_t bytes) : before(g_scratch_limit) { g_scratch_limit = bytes; }
+ScratchLimit::~ScratchLimit() { g_scratch_limit = before; }
+static size_t scratch_left(size_t taken) {
+  return g_scratch_limit == SIZE_MAX ? SIZE_MAX : (g_scratch_limit > taken ? g_scratch_limit - taken : 0);
+}
 // y of the forward in flight on this thread is fp16 although its inputs are bf16 (copies), see forward_cast
 static thread_local bool g_y_f16 = false;
 
@@ -156,14 +163,14 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
     // tensor-core path: one CTA per SM walks a (lane, segment)
     pl.use_tc = true;
     int nseg = 1;
-    prefill_tc_plan(a, &nseg, &pl.wide);
+    pl.part_bytes = a->y != nullptr ? align_up(prefill_tc_partial_bytes(a), 256) : 0;
+    prefill_tc_plan(a, scratch_left(pl.part_bytes), &nseg, &pl.wide);
     int seg_len = (a->N + nseg - 1) / nseg;
     seg_len = (seg_len + 127) / 128 * 128;
     pl.nseg = (a->N + seg_len - 1) / seg_len;
     pl.seg_len = seg_len;
     pl.ws_bytes = pl.nseg > 1 ? align_up((size_t)lanes * pl.nseg * pl.state_floats * 4, 256) : 0;
     pl.part_off = pl.ws_bytes;
-    pl.part_bytes = a->y != nullptr ? align_up(prefill_tc_partial_bytes(a), 256) : 0;
     pl.ws_bytes += pl.part_bytes;
     pl.gate_stride = prefill_tc_gate_stride(a, pl.nseg, pl.wide);
     if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
@@ -399,6 +406,7 @@ CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
 }
 
 int forward_cast(const flare_fwd_args_t* a, flare_fwd_args_t& b, const CastPlan& cp, cudaStream_t stream) {
+  const ScratchLimit limit(scratch_left(cp.total));
   const size_t inner = plan_forward(&b).ws_bytes;
   if (a->workspace == nullptr || a->workspace_bytes < cp.total + inner || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
   char* ws = reinterpret_cast<char*>(a->workspace);
@@ -461,7 +469,7 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
     int n = 1;
     flare_fwd_args_t one = a;
     one.B = (int32_t)(a.B * nseg);
-    prefill_tc_plan(&one, &n, &pl.wide);
+    prefill_tc_plan(&one, SIZE_MAX, &n, &pl.wide);
   }
   WalkParams w;
   fill_walk(w, &a);
@@ -497,7 +505,10 @@ size_t flare_forward_workspace_bytes(const flare_fwd_args_t* args) {
   if (check_forward(args) != FLARE_OK) return 0;
   flare_fwd_args_t b;
   const CastPlan cp = plan_cast(args, &b);
-  if (cp.on) return cp.total + plan_forward(&b).ws_bytes;
+  if (cp.on) {
+    const ScratchLimit limit(scratch_left(cp.total));
+    return cp.total + plan_forward(&b).ws_bytes;
+  }
   return plan_forward(args).ws_bytes;
 }
 

@@ -95,6 +95,15 @@ inline cudaError_t allow_smem(Kern kern) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
 }
 
+// While one lives, the forwards that this thread plans take no more workspace for segment states than fits `bytes` (for
+// callers that cannot supply what flare_forward_workspace_bytes asks for).
+struct ScratchLimit {
+  explicit ScratchLimit(size_t bytes);
+  ~ScratchLimit();
+  ScratchLimit(const ScratchLimit&) = delete;
+  size_t before;
+};
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 inline int dtype_size(int dtype) { return dtype == FLARE_F32 ? 4 : 2; }

@@ -1513,7 +1513,7 @@ int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide) { return prefill_tc_
 static bool can_wide(const flare_fwd_args_t* a) { return a->Dk == 128 && a->Dv == 128 && (a->M % M) == 0; }
 
 // estimated time of the call on one instance, and the segments that give it
-static double plan_instance(const flare_fwd_args_t* a, bool wide, int* nseg_out) {
+static double plan_instance(const flare_fwd_args_t* a, bool wide, size_t state_bytes, int* nseg_out) {
   const int nch = (a->N + C - 1) / C;
   const int64_t lanes = (int64_t)a->B * a->H;
   const int sms = sm_count();
@@ -1523,14 +1523,17 @@ static double plan_instance(const flare_fwd_args_t* a, bool wide, int* nseg_out)
   double best = 8.0 + waves * nch * pass;
   *nseg_out = 1;
   if (ctas * 2 > sms) return best;
-  const int most = (int)(sms / ctas) < nch ? (int)(sms / ctas) : nch;
+  int most = (int)(sms / ctas) < nch ? (int)(sms / ctas) : nch;
+  const size_t room = state_bytes / ((size_t)lanes * (2 * a->M + (size_t)a->M * a->Dv) * sizeof(float));
+  if ((size_t)most > room) most = (int)room;
+  if (most < 2) return best;
   const int len = (nch + most - 1) / most, n = (nch + len - 1) / len;  // chunks per segment, segments that many make
   const double t = 22.0 + 3e-6 * (double)lanes * n * a->M * a->Dv * 4 + len * (pass + state_pass);
   if (1.1 * t < best) best = t, *nseg_out = n;  // (worth two more launches)
   return best;
 }
 
-void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg_out, bool* wide_out) {
+void prefill_tc_plan(const flare_fwd_args_t* a, size_t state_bytes, int* nseg_out, bool* wide_out) {
   bool try_wide[2] = {true, can_wide(a)};
   if (const char* env = getenv("FLARE_B200_WIDE")) {  // 0 / 1 forces the instance
     try_wide[0] = env[0] != '1' || !try_wide[1];
@@ -1540,7 +1543,7 @@ void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg_out, bool* wide_out) {
   for (int w = 0; w < 2; ++w) {
     if (!try_wide[w]) continue;
     int n = 1;
-    const double t = plan_instance(a, w != 0, &n);
+    const double t = plan_instance(a, w != 0, state_bytes, &n);
     // (segments are worth it only if they also beat the other instance by a tenth)
     if ((n > 1 ? 1.1 * t : t) < best) best = t, *nseg_out = n, *wide_out = w != 0;
   }
@@ -1554,7 +1557,7 @@ int prefill_tc_max_gate_stride(const flare_fwd_args_t* a) {
   int most = 0;
   for (int w = 0; w < (can_wide(a) ? 2 : 1); ++w) {
     int n = 1;
-    plan_instance(a, w != 0, &n);
+    plan_instance(a, w != 0, SIZE_MAX, &n);
     const int stride = prefill_tc_gate_stride(a, n, w != 0);
     if (stride > most) most = stride;
   }

@@ -59,8 +59,9 @@ bool prefill_tc_supported(const flare_fwd_args_t* a);
 // array inside it
 size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a);
 size_t prefill_tc_partial_lw_offset(const flare_fwd_args_t* a);
-// segments per lane, and whether the wide (128, 128) instance runs (one CTA for all 128 value columns)
-void prefill_tc_plan(const flare_fwd_args_t* a, int* nseg, bool* wide);
+// segments per lane, and whether the wide (128, 128) instance runs (one CTA for all 128 value columns); no more segments than
+// have their states (fp32, 2 M + M Dv each) in `state_bytes`
+void prefill_tc_plan(const flare_fwd_args_t* a, size_t state_bytes, int* nseg, bool* wide);
 // grid.z of a launch
 int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide);
 // gate words per lane of a call on that instance with that many segments, and the most that any plan of these sizes needs,

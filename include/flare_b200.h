@@ -111,8 +111,8 @@ size_t flare_forward_keep_bytes(const flare_fwd_args_t* args);
  * always allocate their workspaces with torch).  Same arguments and results as flare_forward, except that
  * args->workspace / workspace_bytes are ignored: the scratch for the segment-state scan lives in a fixed array
  * inside the library, flare_noalloc_scratch_capacity() bytes (8 MiB) per GPU, held from library load to exit.
- * Returns FLARE_ERR_TOO_LARGE, without launching anything, when the problem needs more scratch than that
- * (flare_forward_workspace_bytes tells how much).  The call performs no cudaMalloc / cudaFree and calls no
+ * A long sequence of few lanes is cut into no more segments than have their states in it.  Returns
+ * FLARE_ERR_TOO_LARGE, without launching anything, when the problem needs more scratch than that all the same.  The call performs no cudaMalloc / cudaFree and calls no
  * allocating library routine.  The first call on each device resolves the array's device address
  * (cudaGetSymbolAddress); make that first call outside any stream capture.  All calls share the one array:
  * two calls whose kernels may overlap on the GPU (different streams, or different host threads) race on it,

@@ -183,3 +183,19 @@ def test_kept_buffer_does_not_depend_on_the_instance_choice(monkeypatch, B, N, H
         plans.append(lib.flare_forward_workspace_bytes(C.byref(a)))
     assert len(set(sizes)) == 1, sizes
     assert len(set(plans)) > 1  # (the plans themselves do differ)
+
+
+@pytest.mark.parametrize("B, N, H, M, D, dtype", [
+    (1, 32768, 16, 128, 128, "BF16"), (3, 8192, 16, 128, 128, "BF16"), (1, 2000, 8, 256, 64, "BF16"), (3, 2000, 3, 192, 64, "BF16"),
+    (2, 2000, 2, 512, 64, "BF16"), (1, 2000, 2, 512, 128, "BF16"), (1, 8192, 2, 64, 64, "F16")])
+def test_what_the_entry_point_without_allocation_takes(B, N, H, M, D, dtype):
+    # 8 (too large) is decided on the host, before the device is asked for; without one the call ends with 7.  The number of
+    # segments that flare_forward would choose must not decide what is taken (all of these are: partial read-outs, copies and
+    # the states of two segments fit 8 MiB, or no segments are needed).
+    lib = _lib.load()
+    a = _fake_args(B=B, N=N, H=H, M=M, Dk=D, Dv=D, dtype=getattr(_lib, dtype))
+    if torch.cuda.is_available():
+        pytest.skip("planning only")
+    assert lib.flare_forward_noalloc(C.byref(a), None) == 7
+    too_large = _fake_args(B=1, N=65536, H=4, M=512, Dk=64, Dv=128, dtype=_lib.BF16)
+    assert lib.flare_forward_noalloc(C.byref(too_large), None) == 8

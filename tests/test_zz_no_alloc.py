@@ -65,6 +65,20 @@ def test_noalloc_matches_flare_forward_twice(dtype, shape):
     assert torch.equal(y3, y_ref)
 
 
+@pytest.mark.parametrize("shape", [(1, 8192, 16, 128, 128), (4, 2000, 2, 256, 64)])
+def test_noalloc_takes_fewer_segments_than_would_not_fit(shape):
+    # flare_forward cuts these into segments whose states fill more than the scratch
+    lib = _lib.load()
+    q, k, v = _problem(torch.bfloat16, *shape)
+    y = torch.full_like(v, float("nan"))
+    args = _lib.make_fwd_args(q, k, v, None, None, y, scale=q.shape[-1] ** -0.5)
+    assert lib.flare_forward_workspace_bytes(C.byref(args)) > lib.flare_noalloc_scratch_capacity()
+    assert lib.flare_forward_noalloc(C.byref(args), torch.cuda.current_stream().cuda_stream) == 0
+    y_ref, _ = _run("flare_forward", q, k, v, with_workspace=True)
+    # two roundings of y to bf16 and other segment boundaries (roundings of the bf16 state operand): twice the single bound
+    assert orc.rel_l2(y.float().cpu(), y_ref.float().cpu()) <= 1e-2
+
+
 def test_noalloc_rejects_problems_beyond_its_capacity():
     lib = _lib.load()
     cap = lib.flare_noalloc_scratch_capacity()
