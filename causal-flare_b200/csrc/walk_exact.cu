@@ -26,9 +26,9 @@ __global__ void __launch_bounds__(NT, (MM_MAX * DD <= 32) ? 2 : 1) walk_exact_ke
   const int lane_id = blockIdx.x;  // (b, h) lane
   pdl_wait();
   if (p.gate != nullptr) {
-    int raised = 0;
-    for (int i = 0; i < p.gate_count; ++i) raised |= p.gate[(int64_t)lane_id * p.gate_stride + i];
-    if (raised == 0) return;
+    int raised = 0;  // (a lane of a long sequence has up to 74 words)
+    for (int i = threadIdx.x; i < p.gate_count; i += NT) raised |= p.gate[(int64_t)lane_id * p.gate_stride + i];
+    if (!__syncthreads_or(raised)) return;
   }
   const int seg = blockIdx.y;
   const int b = lane_id / p.H, h = lane_id % p.H;
