@@ -2,7 +2,7 @@
 // allocation, the argument structs of the C ABI and the autograd node.
 //
 // Why: a call through Python (autograd.Function, a ctypes struct filled field by field, one torch.empty per buffer) kept
-// the host busy for 37 us per decode step, 66-118 us per forward and 240-310 us per training step (measured on a B200
+// the host busy for 27 us per decode step, 66-118 us per forward and 240-310 us per training step (measured on a B200
 // host, problems too small to keep the GPU busy), more than the kernels of every small call take.  Every entry point
 // here returns None for anything but the plain case (separate decode weights, odd dtypes, arguments that must raise);
 // the Python layer then serves the call and words the errors.
@@ -233,6 +233,7 @@ struct FlareNode : public torch::autograd::Function<FlareNode> {
                                                 int64_t path, bool want_lse) {
     Problem p{ready(q), ready(k), ready(v), scale, power, (int)variant, (int)block, (int)path};
     Forward r = run_forward(p, State{}, Tensor(), false, want_lse, true);
+    ctx->set_materialize_grads(false);  // (else zeros of the log-sum-exps' sizes are made for every backward)
     if (r.keep.defined()) ctx->save_for_backward({q, k, v, r.y, r.lse_dec, r.keep});
     else ctx->save_for_backward({q, k, v});
     ctx->saved_data["scale"] = scale;
@@ -248,10 +249,15 @@ struct FlareNode : public torch::autograd::Function<FlareNode> {
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     torch::autograd::variable_list out(9);
-    if (!grads[0].defined()) return out;
     const auto saved = ctx->get_saved_variables();
     const Tensor &q0 = saved[0], &k0 = saved[1], &v0 = saved[2];
     const c10::cuda::CUDAGuard guard(k0.device());
+    if (!grads[0].defined()) {  // an undefined gradient of y stands for zeros
+      out[0] = at::zeros(q0.sizes(), q0.options().requires_grad(false));
+      out[1] = at::zeros(k0.sizes(), k0.options().requires_grad(false));
+      out[2] = at::zeros(v0.sizes(), v0.options().requires_grad(false));
+      return out;
+    }
     const Problem p{ready(q0), ready(k0), ready(v0), ctx->saved_data["scale"].toDouble(), ctx->saved_data["power"].toDouble(),
                     (int)ctx->saved_data["variant"].toInt(), (int)ctx->saved_data["block"].toInt(),
                     (int)ctx->saved_data["path"].toInt()};

@@ -41,3 +41,32 @@ def test_a_traced_call_computes_when_it_is_replayed(op):
     poison = [torch.full_like(want, float("nan")) for _ in range(8)]  # what a fresh output buffer would show
     del poison
     assert torch.equal(traced(q2, k2, v2), want)
+
+
+def test_backward_of_the_block_causal_operator_allocates_no_gradients_of_the_log_sum_exps():
+    def allocations(op):
+        leaves = [t.requires_grad_() for t in inputs()]
+        y = OPS[op](*leaves)
+        dy = torch.ones_like(y)
+        torch.autograd.grad(y, leaves, dy, retain_graph=True)
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        torch.autograd.grad(y, leaves, dy)
+        return torch.cuda.memory_stats()["allocation.all.allocated"] - before
+
+    assert allocations("block") == allocations("softmax")  # three gradients and the workspace
+
+
+@pytest.mark.parametrize("op", sorted(OPS))
+def test_an_undefined_gradient_of_y_stands_for_zeros(op):
+    class Drop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, y):
+            return y.sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    leaves = [t.requires_grad_() for t in inputs()]
+    for t, g in zip(leaves, torch.autograd.grad(Drop.apply(OPS[op](*leaves)), leaves)):
+        assert g.shape == t.shape and g.dtype == t.dtype and not g.any()
