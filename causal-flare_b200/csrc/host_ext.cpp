@@ -124,9 +124,21 @@ bool plain_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
   return q.size(1) > 0 && q.size(1) % 16 == 0 && q.size(2) % 16 == 0 && v.size(3) > 0 && v.size(3) % 16 == 0 && k.size(3) > 0;
 }
 
-double default_scale(const py::object& scale, int64_t dk) {
-  if (!scale.is_none()) return scale.cast<double>();
-  return dk <= 8 ? 1.0 : std::pow(static_cast<double>(dk), -0.5);
+// float(scale), as the Python layer takes it (a text among others); false: it has to raise
+bool to_scale(const py::object& scale, double* out) {
+  PyObject* const f = PyNumber_Float(scale.ptr());
+  if (f == nullptr) {
+    PyErr_Clear();
+    return false;
+  }
+  *out = PyFloat_AS_DOUBLE(f);
+  Py_DECREF(f);
+  return true;
+}
+bool default_scale(const py::object& scale, int64_t dk, double* out) {
+  if (!scale.is_none()) return to_scale(scale, out);
+  *out = dk <= 8 ? 1.0 : std::pow(static_cast<double>(dk), -0.5);
+  return true;
 }
 
 struct Problem {
@@ -185,7 +197,7 @@ struct Forward {
   State out;
 };
 
-Forward run_forward(const Problem& p, const State& in, const Tensor& mask, bool want_state, bool want_lse, bool want_keep) {
+Forward run_forward(const Problem& p, const State& in, bool want_state, bool want_lse, bool want_keep) {
   const auto opts = p.k.options().requires_grad(false);
   const auto f32 = opts.dtype(at::kFloat);
   const int64_t B = p.k.size(0), N = p.k.size(1), H = p.k.size(2), M = p.q.size(1), Dv = p.v.size(3);
@@ -195,7 +207,6 @@ Forward run_forward(const Problem& p, const State& in, const Tensor& mask, bool 
   r.y = at::empty({B, N, H, Dv}, opts);
   a.y = r.y.data_ptr();
   a.y_stride_b = N * H * Dv; a.y_stride_n = H * Dv; a.y_stride_h = Dv;
-  if (mask.defined()) a.mask = mask.data_ptr<int32_t>();
   a.state_in = pointers(in);
   if (want_state) {
     r.out = State{at::empty({B, H, M}, f32), at::empty({B, H, M}, f32), at::empty({B, H, M, Dv}, f32)};
@@ -232,7 +243,7 @@ struct FlareNode : public torch::autograd::Function<FlareNode> {
                                                 const Tensor& v, double scale, double power, int64_t variant, int64_t block,
                                                 int64_t path, bool want_lse) {
     Problem p{ready(q), ready(k), ready(v), scale, power, (int)variant, (int)block, (int)path};
-    Forward r = run_forward(p, State{}, Tensor(), false, want_lse, true);
+    Forward r = run_forward(p, State{}, false, want_lse, true);
     ctx->set_materialize_grads(false);  // (else zeros of the log-sum-exps' sizes are made for every backward)
     if (r.keep.defined()) ctx->save_for_backward({q, k, v, r.y, r.lse_dec, r.keep});
     else ctx->save_for_backward({q, k, v});
@@ -301,12 +312,13 @@ bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
 py::object causal(const Tensor& q, const Tensor& k, const Tensor& v, const py::object& scale, int variant, double power) {
   const int path = path_from_env();
   if (path < 0 || !plain_qkv(q, k, v)) return py::none();
-  const double sc = default_scale(scale, k.size(3));
+  double sc;
+  if (!default_scale(scale, k.size(3), &sc)) return py::none();
   const c10::cuda::CUDAGuard guard(k.device());
   if (wants_grad(q, k, v))
     return py::cast(FlareNode::apply(q, k, v, sc, power, (int64_t)variant, (int64_t)1, (int64_t)path, false)[0]);
   const Problem p{ready(q), ready(k), ready(v), sc, power, variant, 1, path};
-  return py::cast(run_forward(p, State{}, Tensor(), false, false, false).y);
+  return py::cast(run_forward(p, State{}, false, false, false).y);
 }
 
 // block-causal operator, shared decode weights: (y, lse_dec, lse_enc), or None
@@ -315,33 +327,34 @@ py::object block_causal(const Tensor& q, const Tensor& k, const Tensor& v, const
   if (path < 0 || !plain_qkv(q, k, v)) return py::none();
   if (block < 16 || block % 16 || k.size(1) % block || (chunk != 16 && chunk != 32 && chunk != 64 && chunk != 128) || block % chunk)
     return py::none();
-  const double sc = default_scale(scale, k.size(3));
+  double sc;
+  if (!default_scale(scale, k.size(3), &sc)) return py::none();
   const c10::cuda::CUDAGuard guard(k.device());
   if (wants_grad(q, k, v)) {
     const auto r = FlareNode::apply(q, k, v, sc, 2.0, (int64_t)FLARE_SOFTMAX, block, (int64_t)path, true);
     return py::make_tuple(r[0], r[1], r[2]);
   }
   const Problem p{ready(q), ready(k), ready(v), sc, 2.0, FLARE_SOFTMAX, (int)block, path};
-  const Forward r = run_forward(p, State{}, Tensor(), false, true, false);
+  const Forward r = run_forward(p, State{}, false, true, false);
   return py::make_tuple(r.y, r.lse_dec, r.lse_enc);
 }
 
 // tokens on top of a state (None: empty), shared decode weights: (y, state), or None
-py::object prefill(const Tensor& q, const Tensor& k, const Tensor& v, const py::object& state, double scale, const py::object& mask) {
+py::object prefill(const Tensor& q, const Tensor& k, const Tensor& v, const py::object& state, const py::object& scale,
+                   const py::object& mask) {
   const int path = path_from_env();
-  if (path < 0 || !plain_qkv(q, k, v)) return py::none();
+  double sc;
+  if (path < 0 || !mask.is_none() || !plain_qkv(q, k, v) || !to_scale(scale, &sc)) return py::none();
   const c10::cuda::CUDAGuard guard(k.device());
   State in;
   if (!state.is_none() && !plain_state(state, k.size(0), k.size(2), q.size(1), v.size(3), k, &in)) return py::none();
-  Tensor m32;
-  if (!mask.is_none()) return py::none();
-  const Problem p{ready(q), ready(k), ready(v), scale, 2.0, FLARE_SOFTMAX, 1, path};
-  const Forward r = run_forward(p, in, m32, true, false, false);
+  const Problem p{ready(q), ready(k), ready(v), sc, 2.0, FLARE_SOFTMAX, 1, path};
+  const Forward r = run_forward(p, in, true, false, false);
   return py::make_tuple(r.y, state_dict(r.out));
 }
 
 // one token on top of a state, which is updated in place: (y [B, 1, H, Dv], state), or None
-py::object decode(const Tensor& q, const Tensor& k_in, const Tensor& v_in, const py::object& state, double scale) {
+py::object decode(const Tensor& q, const Tensor& k_in, const Tensor& v_in, const py::object& state, const py::object& scale) {
   // K, V: [B, H, D] or [B, 1, H, D]
   const bool k4 = k_in.dim() == 4 && k_in.size(1) == 1, v4 = v_in.dim() == 4 && v_in.size(1) == 1;
   if (!k_in.is_cuda() || q.dim() != 3 || !(k4 || k_in.dim() == 3) || !(v4 || v_in.dim() == 3)) return py::none();
@@ -350,6 +363,8 @@ py::object decode(const Tensor& q, const Tensor& k_in, const Tensor& v_in, const
   const int kh = k4 ? 2 : 1, vh = v4 ? 2 : 1;  // position of the head dimension
   const int64_t B = k_in.size(0), H = k_in.size(kh), Dk = k_in.size(kh + 1), M = q.size(1), Dv = v_in.size(vh + 1);
   if (dt < 0 || B == 0 || v_in.size(0) != B || v_in.size(vh) != H || q.size(0) != H || q.size(2) != Dk) return py::none();
+  double sc;
+  if (!to_scale(scale, &sc)) return py::none();
   if (k_in.stride(kh + 1) != 1 || v_in.stride(vh + 1) != 1 || !readable(q)) return py::none();
   const c10::cuda::CUDAGuard guard(k_in.device());
   State st;
@@ -363,7 +378,7 @@ py::object decode(const Tensor& q, const Tensor& k_in, const Tensor& v_in, const
   a.q_stride_h = q.stride(0); a.q_stride_m = q.stride(1);
   a.k_stride_b = k_in.stride(0); a.k_stride_h = k_in.stride(kh);
   a.v_stride_b = v_in.stride(0); a.v_stride_h = v_in.stride(vh);
-  a.scale = (float)scale;
+  a.scale = (float)sc;
   a.dtype = dt;
   const int rc = api.decode_step(&a, c10::cuda::getCurrentCUDAStream(k_in.device().index()).stream());
   if (rc == FLARE_ERR_UNSUPPORTED) return py::none();  // value width outside the streaming kernel: general walk

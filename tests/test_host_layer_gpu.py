@@ -1,4 +1,7 @@
 """GPU: calls that the native host layer must leave to the Python layer (what it would lose, refuse or word differently)."""
+from fractions import Fraction
+
+import numpy as np
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
@@ -70,3 +73,17 @@ def test_an_undefined_gradient_of_y_stands_for_zeros(op):
     leaves = [t.requires_grad_() for t in inputs()]
     for t, g in zip(leaves, torch.autograd.grad(Drop.apply(OPS[op](*leaves)), leaves)):
         assert g.shape == t.shape and g.dtype == t.dtype and not g.any()
+
+
+@pytest.mark.parametrize("scale", ["0.125", Fraction(1, 8), np.float32(0.125), torch.tensor(0.125), True])
+def test_scale_is_what_float_makes_of_it(scale):
+    q, k, v = inputs()
+    st = cf.flare_autoregressive_prefill_triton(q, k, v)[1]
+    calls = [lambda s: cf.flare_autoregressive_triton(q, k, v, scale=s),
+             lambda s: cf.flare_semi_autoregressive_trition(q, k, v, block_size=32, chunk_size=32, scale=s)[0],
+             lambda s: cf.flare_autoregressive_prefill_triton(q, k, v, scale=s)[0],
+             lambda s: cf.flare_autoregressive_decode_triton(q, k[:, 0], v[:, 0], {n: t.clone() for n, t in st.items()}, scale=s)[0]]
+    for call in calls:
+        assert torch.equal(call(scale), call(float(scale)))
+        with pytest.raises((TypeError, ValueError)):
+            call("wide")
