@@ -103,7 +103,7 @@ def _build_host() -> None:
     from torch.utils.cpp_extension import include_paths
 
     stamp = os.path.join(OBJ, "host_ext.sha")
-    dig = _digest("host_ext.cpp", [torch.__version__])
+    dig = _digest("host_ext.cpp", [torch.__version__, sys.version])  # (an extension module of this interpreter)
     if os.path.exists(HOST) and os.path.exists(stamp) and open(stamp).read() == dig:
         return
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
