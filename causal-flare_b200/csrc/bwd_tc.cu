@@ -19,9 +19,9 @@
 // eight tokens are one 16-byte store each); a second tensor-core kernel forms dK = scale dS^T Q per chunk and
 // dQ = scale sum_t dS K per (lane, split) (fp32 partials, summed in fixed order: no atomics, deterministic).
 //
-// Main kernel, one CTA per (lane, group of 128 latents), 14 warps: 0-7 latent group (thread = latent = TMEM lane,
-// the two warps of a lane quarter take 64 tokens each), 8-11 token group (thread = token = TMEM lane: causal masks of
-// A and E^T R, dV store), 12 MMA issuer, 13 TMA producer.  Ten MMAs per chunk; every operand that the latent / token
+// Main kernel, one CTA per (lane, group of 128 latents, sequence segment), 22 warps: 0-15 latent group (thread = latent = TMEM
+// lane, the four warps of a lane quarter take 32 tokens each; packed: see PACK), 16-19 token group (thread = token = TMEM lane:
+// causal masks of A and E^T R, dV store), 20 MMA issuer, 21 TMA producer.  Ten MMAs per chunk; every operand that the latent / token
 // threads produce (E, R, masked A, G as bf16) is written once into a 128-byte-swizzled buffer and read K-major or
 // MN-major as the product needs, so there is no transposition pass.
 #include "bwd_tc.cuh"
