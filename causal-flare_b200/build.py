@@ -18,6 +18,7 @@ HOST = os.path.join(HERE, "causal_flare", "_host.so")  # native host layer of th
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+    "--compress-mode=size",  # (line tables are most of the code's size: a sixth of the library)
     *os.environ.get("FLARE_B200_NVCC_FLAGS", "").split(),  # extra flags for experiments (e.g. -DNAME)
 ]
 
@@ -30,7 +31,7 @@ UNITS = [
     ("decode_step.cu", [], "decode_step"),
     ("state_ops.cu", [], "state_ops"),
     ("prefill_tc.cu", [], "prefill_tc_host"),
-    *[("prefill_tc.cu", [f"-DFLARE_TC_UNIT={u}"], f"prefill_tc_unit{u}") for u in range(8)],
+    *[("prefill_tc.cu", [f"-DFLARE_TC_UNIT={u}", f"-DFLARE_TC_MODE={m}"], f"prefill_tc_unit{u}_mode{m}") for u in range(8) for m in range(3)],
     ("noalloc.cu", [], "noalloc"),
     ("bwd_tc.cu", [], "bwd_tc_host"),
     *[("bwd_tc.cu", [f"-DFLARE_BT_UNIT={u}"], f"bwd_tc_unit{u}") for u in range(6)],

@@ -154,12 +154,19 @@ struct FwdPlan {
   size_t gate_off, gate_bytes;
 };
 
+// fp16 calls may run on the tensor kernels (FLARE_B200_FP16_TENSOR=0 keeps them on the exact ones, which multiply q, k, v at
+// their full fp16 precision in every product)
+bool f16_on_tensor_kernels() {
+  const char* env = getenv("FLARE_B200_FP16_TENSOR");
+  return env == nullptr || env[0] != '0';
+}
+
 FwdPlan plan_forward(const flare_fwd_args_t* a) {
   FwdPlan pl{false, false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0};
   if (a->B == 0 || a->N == 0) return pl;
   const int64_t lanes = (int64_t)a->B * a->H;
   pl.state_floats = (size_t)2 * a->M + (size_t)a->M * a->Dv;
-  if (a->path != FLARE_PATH_EXACT && prefill_tc_supported(a)) {
+  if (a->path != FLARE_PATH_EXACT && (prefill_tc_supported(a) || (prefill_tc_supported_f16(a) && f16_on_tensor_kernels()))) {
     // tensor-core path: one CTA per SM walks a (lane, segment)
     pl.use_tc = true;
     int nseg = 1;
@@ -247,7 +254,8 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
     t.part_lw = reinterpret_cast<float*>(reinterpret_cast<char*>(t.part_y) + prefill_tc_partial_lw_offset(a));
   }
   t.trace = g_trace;
-  t.y_f16 = g_y_f16 ? 1 : 0;
+  t.in_f16 = a->dtype == FLARE_F16 ? 1 : 0;
+  t.y_f16 = t.in_f16 || g_y_f16 ? 1 : 0;
   t.gate = g_gate;
   t.gate_stride = pl.gate_stride;
   // (the state pass over all segments but the last comes first)
@@ -368,14 +376,13 @@ int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaSt
   return launch_walk(a, pl, w, pl.nseg, stream);
 }
 
-// fp16 inputs on the tensor-core kernels.  The kernels multiply bf16 operands (the tensor-core products of E, R, W
-// and the running state are bf16 whatever the inputs are), so an fp16 call is served by rounding q, k, v to bf16
-// copies in the workspace and running the bf16 forward on those, which writes y as fp16: one streaming pass over q, k and v
-// before a kernel that is 40 to 60 times faster than the exact walk the call would otherwise take.  Lanes that the
-// kernels flag as outside their numeric domain are recomputed by the exact kernels from the fp16 tensors themselves.
-// States and log-sum-exps are fp32 on both sides and go straight to the caller's buffers.  Not for the training
-// forward (no state is kept for a backward) and not with separate decode weights or a mask, which the tensor kernels
-// do not take.
+// fp16 inputs on the tensor-core kernels.  The forward kernels take them as they are (prefill_tc_supported_f16).  What is left
+// for copies are the tensors whose strides a tiled copy cannot express (expanded over heads, say): q, k, v are copied to
+// dense bf16 in the workspace and the bf16 forward runs on those and writes y as fp16, which is 40 to 60 times faster than the
+// exact walk the call would otherwise take.  Lanes that the kernels flag as outside their numeric domain are recomputed
+// by the exact kernels from the fp16 tensors themselves, either way.  States and log-sum-exps are fp32 and go straight
+// to the caller's buffers.  Not for the training forward (no state is kept for a backward) and not with separate decode
+// weights or a mask, which the tensor kernels do not take.
 struct CastPlan {
   bool on;
   size_t off_q, off_k, off_v, total;
@@ -384,11 +391,8 @@ struct CastPlan {
 CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
   CastPlan cp{false, 0, 0, 0, 0};
   if (a->dtype != FLARE_F16 || a->path == FLARE_PATH_EXACT || a->keep != nullptr || a->q_dec != nullptr ||
-      a->k_dec != nullptr || a->mask != nullptr || a->B == 0 || a->N == 0)
+      a->k_dec != nullptr || a->mask != nullptr || a->B == 0 || a->N == 0 || !f16_on_tensor_kernels())
     return cp;
-  // FLARE_B200_FP16_TENSOR=0 keeps fp16 calls on the exact kernels (q, k, v at their full fp16 precision)
-  if (const char* env = getenv("FLARE_B200_FP16_TENSOR"))
-    if (env[0] == '0') return cp;
   *b = *a;
   b->dtype = FLARE_BF16;
   b->q_stride_m = a->Dk; b->q_stride_h = (int64_t)a->M * a->Dk;
@@ -400,7 +404,7 @@ CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
   cp.off_q = 0;
   cp.off_k = align_up((size_t)a->H * a->M * a->Dk * 2, 256);
   cp.off_v = cp.off_k + align_up(rows * a->Dk * 2, 256);
-  // (the size that callers plan with has room for a y in bf16, which nothing uses)
+  // (The size that callers plan with: it has room for a y in bf16, which nothing uses, and a call without copies asks for it too.)
   cp.total = cp.off_v + align_up(rows * a->Dv * 2, 256) * (a->y != nullptr ? 2 : 1);
   return cp;
 }
@@ -539,7 +543,12 @@ int flare_forward(const flare_fwd_args_t* args, flare_stream_t stream) {
   }
   flare_fwd_args_t b;
   const CastPlan cp = plan_cast(args, &b);
-  if (cp.on) return forward_cast(args, b, cp, stream);
+  if (cp.on && !prefill_tc_supported_f16(args)) return forward_cast(args, b, cp, stream);
+  if (cp.on) {  // nothing is copied, but a workspace that would not have held the copies is refused all the same
+    const ScratchLimit limit(scratch_left(cp.total));
+    if (args->workspace == nullptr || args->workspace_bytes < cp.total + plan_forward(&b).ws_bytes) return FLARE_ERR_WORKSPACE;
+    return forward_run(args, stream);  // (planned within what is left, as the size was)
+  }
   return forward_run(args, stream);
 }
 
@@ -576,8 +585,7 @@ BwdCastPlan plan_bwd_cast(const flare_bwd_args_t* a, flare_bwd_args_t* b) {
   const flare_fwd_args_t& f = a->fwd;
   if (f.dtype != FLARE_F16 || f.path == FLARE_PATH_EXACT || f.q_dec != nullptr || f.k_dec != nullptr || f.B == 0 || f.N == 0)
     return cp;
-  if (const char* env = getenv("FLARE_B200_FP16_TENSOR"))
-    if (env[0] == '0') return cp;
+  if (!f16_on_tensor_kernels()) return cp;
   *b = *a;
   flare_fwd_args_t& g = b->fwd;
   g.dtype = FLARE_BF16;

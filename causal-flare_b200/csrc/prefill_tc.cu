@@ -107,7 +107,7 @@ struct Lay {
 constexpr uint32_t TM_COLS = 512;
 
 struct Misc {
-  uint64_t q_full, k_full, k_empty, v_full[2], v_empty[2];
+  uint64_t q_full, k_full, k_empty, v_full[2], v_empty[2], v_conv[2];
   uint64_t s_ready, s_free, kap_done, p1_done, u_done, w_ready, p2_done, y_ready, y_free;
   uint64_t pmax[4], psum[4];  // pair barriers of the two latent half-groups, one per lane quarter
   uint64_t xfull[4], xfree[4];  // on-chip merge of two latent groups, per token warp: the partner's rows have arrived /
@@ -156,7 +156,7 @@ __device__ __forceinline__ uint4 pack_piece(const uint32_t (&r)[32], int ch) {
 // M=256 D=128 with blocks of 64; the others spill less with store_e (the wide one without groups 0 instead of 36 bytes).
 __device__ __forceinline__ void put_piece(uint8_t* at, const uint4& v) { *reinterpret_cast<uint4*>(at) = v; }
 
-// eight values as fp16 or bf16 pairs (uniform per launch)
+// eight values as fp16 or bf16 pairs
 __device__ __forceinline__ void pack_out(const float (&y)[8], bool f16, uint32_t (&o)[4]) {
   if (f16) {
 #pragma unroll
@@ -180,11 +180,12 @@ __device__ __forceinline__ int latent0() {
 
 }  // namespace
 
-// The kernel instances are compiled in separate translation units (FLARE_TC_UNIT = 0..5: head widths (64, 64) / (128, 128) / (64, 128), without /
-// with the latent-group split) to keep build times short; the unit without FLARE_TC_UNIT holds the host side.
-template <int UNIT>
-int launch_prefill_tc_unit(int lat, int mode, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                           const CUtensorMap& ty, const TcParams& p, dim3 grid, cudaStream_t stream);
+// The kernel instances are compiled in separate translation units (FLARE_TC_UNIT = 0..7: head widths (64, 64) / (128, 128) / (64, 128), without /
+// with the latent-group split, and the wide ones; FLARE_TC_MODE = 0..2) to keep build times short; the unit without
+// FLARE_TC_UNIT holds the host side.
+template <int UNIT, int MODE>
+int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
+                           const TcParams& p, dim3 grid, cudaStream_t stream);
 
 #ifdef FLARE_TC_UNIT
 
@@ -212,16 +213,19 @@ int launch_prefill_tc_unit(int lat, int mode, const CUtensorMap& tq, const CUten
 //       SMs in one wave.  Differences: U and Y are 128 columns wide; W and Y0 = R^T U_bf16 come out of ONE product of
 //       width 256 ([E | U_bf16] as one B operand, [W | Y] adjacent in tensor memory), so R is read once for both; W
 //       shares the columns of S; E and R are single-buffered.
-// Y16: the wide instance writes y as fp16 (the others look at p.y_f16; here that choice, in registers of the epilogue, cost
-//       the bf16 calls 5 to 8 %)
-template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, bool Y16>
+// FL:   0 = bf16, every row N tokens long; 1 = bf16 with per-row lengths; 2 = fp16 y (of fp16 inputs, or of bf16 copies:
+//       p.in_f16), with lengths or not.  Instances of their own: as run-time choices they cost every bf16 call 2 to 3 % (B200:
+//       B=8 N=8192 H=16 M=128 D=64 182.3 -> 185.8 us, training B=4 N=4096 H=16 M=64 D=128 411 -> 424 us), and the type of y in
+//       the epilogue of the wide instance 5 to 8 %.
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y, const TcParams p) {
   using L = Lay<DKB, WIDE>;
   constexpr bool PADDED = LAT != 0, PACK = LAT == 2;
   static_assert(!WIDE || (DVB == 2 && !PADDED), "wide instance");
-  static_assert(!Y16 || (WIDE && !KEEP), "fp16 read-out of the wide instance");
+  static_assert(!KEEP || FL == 0, "training forwards are bf16 and know no lengths");
+  constexpr bool LENS = FL != 0, F16 = FL == 2;
   static_assert(!PACK || !SPLIT, "one group of at most 64 latents");
   constexpr int NP = PACK ? 4 : 2;       // token parts of a chunk = latent warps per 32 latents
   constexpr int TOK = C / NP;            // tokens per latent thread
@@ -247,7 +251,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int b = lane_id / p.H, h = lane_id % p.H;
   const int seg_begin = seg * p.seg_len;
   // rows beyond the batch row's own length are right padding: they are not walked
-  const int n_row = p.lens != nullptr ? min(p.N, max(0, p.lens[b])) : p.N;
+  const int n_row = LENS && p.lens != nullptr ? min(p.N, max(0, p.lens[b])) : p.N;
   const int seg_end = max(seg_begin, min(n_row, seg_begin + p.seg_len));
   const int nchunks = (seg_end - seg_begin + C - 1) / C;
 
@@ -258,6 +262,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     for (int i = 0; i < 2; ++i) {
       mbar_init(&misc->v_full[i], 1);
       mbar_init(&misc->v_empty[i], 1);
+      mbar_init(&misc->v_conv[i], 1);
     }
     mbar_init(&misc->s_ready, 1);
     mbar_init(&misc->s_free, 8);
@@ -301,29 +306,87 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   if (warp == 13) {
     // ======================================= TMA producer =======================================
-    if (lane == 0) {
-      prefetch_tensormap(&tm_k);
-      prefetch_tensormap(&tm_v);
-      if (Q_SMEM) {
-        mbar_arrive_expect_tx(&misc->q_full, 16384);
-        tma_load_3d(smem + OFF_Q, &tm_q, &misc->q_full, 0, latent0<ZS, SPLIT>(), h);  // rows beyond M read as zero
-        if (PACK) tma_load_3d(smem + OFF_Q + 8192, &tm_q, &misc->q_full, 0, 0, h);    // (boxes of 64 rows)
+    if constexpr (FL != 2) {
+      if (lane == 0) {
+        prefetch_tensormap(&tm_k);
+        prefetch_tensormap(&tm_v);
+        if (Q_SMEM) {
+          mbar_arrive_expect_tx(&misc->q_full, 16384);
+          tma_load_3d(smem + OFF_Q, &tm_q, &misc->q_full, 0, latent0<ZS, SPLIT>(), h);  // rows beyond M read as zero
+          if (PACK) tma_load_3d(smem + OFF_Q + 8192, &tm_q, &misc->q_full, 0, 0, h);    // (boxes of 64 rows)
+        }
+        const int vc0 = value_col0<ZS, SPLIT>();
+        for (int i = 0; ok && i < nchunks; ++i) {
+          const int t0 = seg_begin + i * C;
+          // K tile: free once the score MMA of the previous chunk has run
+          if (i > 0 && !(ok = wait_or_abort(&misc->k_empty, (i - 1) & 1, misc))) break;
+          mbar_arrive_expect_tx(&misc->k_full, DKB * 16384);
+#pragma unroll
+          for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, &tm_k, &misc->k_full, kb * 64, h, t0, b);
+          // V tile: stage i & 1, free once chunk i - 2 has been folded into Y
+          const int st = i & 1;
+          if (i >= 2 && !(ok = wait_or_abort(&misc->v_empty[st], ((i - 2) >> 1) & 1, misc))) break;
+          mbar_arrive_expect_tx(&misc->v_full[st], VB * 16384);
+#pragma unroll
+          for (int vb = 0; vb < VB; ++vb)
+            tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, &tm_v, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
+        }
       }
-      const int vc0 = value_col0<ZS, SPLIT>();
-      for (int i = 0; ok && i < nchunks; ++i) {
-        const int t0 = seg_begin + i * C;
-        // K tile: free once the score MMA of the previous chunk has run
-        if (i > 0 && !(ok = wait_or_abort(&misc->k_empty, (i - 1) & 1, misc))) break;
-        mbar_arrive_expect_tx(&misc->k_full, DKB * 16384);
-#pragma unroll
-        for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, &tm_k, &misc->k_full, kb * 64, h, t0, b);
-        // V tile: stage i & 1, free once chunk i - 2 has been folded into Y
+    } else {
+      // fp16 inputs: Q and K go to the score product as they are; V, which meets bf16 weights, is rounded to bf16 in place by
+      // this warp (one tile behind the loads, so that the next chunk's K never waits for it).  B200, B=4 N=4096 H=16 M=64 D=128:
+      // 130 us with bf16 copies of K and V made before the kernel (a pass of 42 us over them), 93 us this way.
+      const unsigned active = p.in_f16 ? 0xffffffffu : 1u;  // (bf16 copies: the one thread that issues the loads)
+      auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(active, wait_or_abort(bar, parity, misc)) != 0; };
+      auto convert_v = [&](int i) -> bool {
         const int st = i & 1;
-        if (i >= 2 && !(ok = wait_or_abort(&misc->v_empty[st], ((i - 2) >> 1) & 1, misc))) break;
-        mbar_arrive_expect_tx(&misc->v_full[st], VB * 16384);
+        if (!wait_all(&misc->v_full[st], (i >> 1) & 1)) return false;
+        uint4* tile = reinterpret_cast<uint4*>(smem + OFF_V + st * VB * 16384);
+#pragma unroll 1
+        for (int c = lane; c < VB * 1024; c += 32 * 8) {
+          uint4 x[8];
 #pragma unroll
-        for (int vb = 0; vb < VB; ++vb)
-          tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, &tm_v, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
+          for (int u = 0; u < 8; ++u) x[u] = tile[c + u * 32];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) tile[c + u * 32] = make_uint4(f16x2_to_bf16x2(x[u].x), f16x2_to_bf16x2(x[u].y),
+                                                                    f16x2_to_bf16x2(x[u].z), f16x2_to_bf16x2(x[u].w));
+        }
+        fence_proxy_async_smem();
+        warp_arrive(&misc->v_conv[st], lane);
+        return true;
+      };
+      if (lane == 0 || p.in_f16) {
+        const int vc0 = value_col0<ZS, SPLIT>();
+        if (lane == 0) {
+          prefetch_tensormap(&tm_k);
+          prefetch_tensormap(&tm_v);
+          if (Q_SMEM) {
+            mbar_arrive_expect_tx(&misc->q_full, 16384);
+            tma_load_3d(smem + OFF_Q, &tm_q, &misc->q_full, 0, latent0<ZS, SPLIT>(), h);  // rows beyond M read as zero
+            if (PACK) tma_load_3d(smem + OFF_Q + 8192, &tm_q, &misc->q_full, 0, 0, h);    // (boxes of 64 rows)
+          }
+        }
+        for (int i = 0; ok && i < nchunks; ++i) {
+          const int t0 = seg_begin + i * C;
+          // K tile: free once the score MMA of the previous chunk has run
+          if (i > 0 && !(ok = wait_all(&misc->k_empty, (i - 1) & 1))) break;
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&misc->k_full, DKB * 16384);
+#pragma unroll
+            for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, &tm_k, &misc->k_full, kb * 64, h, t0, b);
+          }
+          if (p.in_f16 && i > 0 && !(ok = convert_v(i - 1))) break;
+          // V tile: stage i & 1, free once chunk i - 2 has been folded into Y
+          const int st = i & 1;
+          if (i >= 2 && !(ok = wait_all(&misc->v_empty[st], ((i - 2) >> 1) & 1))) break;
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&misc->v_full[st], VB * 16384);
+#pragma unroll
+            for (int vb = 0; vb < VB; ++vb)
+              tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, &tm_v, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
+          }
+        }
+        if (p.in_f16 && ok && nchunks > 0) ok = convert_v(nchunks - 1);
       }
     }
   } else if (warp == 12) {
@@ -331,7 +394,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     if (lane == 0) {
       const uint32_t k_addr = smem_u32(smem + OFF_K);
       const uint32_t b16_addr = smem_u32(smem + OFF_B16);
-      constexpr uint32_t ID_S = make_idesc_bf16(128, 128, 0, 0);   // Q (TMEM) x K_c (K-major)
+      // Q (TMEM) x K_c (K-major): both as the caller has them, bf16 or fp16
+      const uint32_t ID_S = F16 && p.in_f16 ? make_idesc_f16(128, 128, 0, 0) : make_idesc_bf16(128, 128, 0, 0);
+      uint64_t* const v_ready = F16 && p.in_f16 ? misc->v_conv : misc->v_full;  // the V tile is in place, as bf16
       constexpr uint32_t ID_U = make_idesc_bf16(128, WIDE ? 128 : 64, 0, 1);  // E (K-major) x V (MN-major)
       constexpr uint32_t ID_DEN = make_idesc_bf16(128, 16, 1, 0);  // R (MN-major) x d tile (K-major)
       constexpr uint32_t ID_Y1 = make_idesc_bf16(128, WIDE ? 128 : 64, 0, 1);  // tril(W) (TMEM) x V (MN-major)
@@ -397,7 +462,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if (!(ok = issue_scores(i + 1))) break;
         }
         if (!(ok = wait_or_abort(&misc->p1_done, par, misc))) break;
-        if (!(ok = wait_or_abort(&misc->v_full[i & 1], (i >> 1) & 1, misc))) break;
+        if (!(ok = wait_or_abort(&v_ready[i & 1], (i >> 1) & 1, misc))) break;
         tc_fence_after_sync();
         TC_TRACE(2, i, 3);
         const uint64_t dek = de_k0, dem = de_mn0, drm = dr_mn0;
@@ -1220,7 +1285,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
                                  f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
               }
-              pack_out(y, Y16, o);
+              pack_out(y, F16, o);
               *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
                   make_uint4(o[0], o[1], o[2], o[3]);
             }
@@ -1265,7 +1330,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             for (int j = 0; j < 4; ++j)  // two columns per multiply
               f2_unpack(f2_mul(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])), inv2), y[2 * j],
                         y[2 * j + 1]);
-            pack_out(y, SPLIT || (WIDE ? Y16 : p.y_f16 != 0), o);
+            pack_out(y, SPLIT || F16, o);
             v[ch] = make_uint4(o[0], o[1], o[2], o[3]);
           }
           if (p.y_tma) {
@@ -1323,10 +1388,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 namespace {
 
-template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE = false, bool Y16 = false>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
 int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
-  auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE, Y16>;
+  auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE, FL>;
   FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer(p.y == nullptr ? "prefill_tc_kernel (state only)" : (WIDE ? "prefill_tc_kernel (wide)" : "prefill_tc_kernel"),
                     stream);
@@ -1353,53 +1418,41 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   return FLARE_OK;
 }
 
-template <int LAT, int DKB, int DVB, bool SPLIT, int MODE>
+template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool WIDE>
 int launch_instance(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
                     const TcParams& p, dim3 grid, cudaStream_t stream) {
-  return p.dump_u != nullptr ? launch_keep<LAT, DKB, DVB, SPLIT, MODE, true>(tq, tk, tv, ty, p, grid, stream)
-                             : launch_keep<LAT, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
+  if (p.dump_u != nullptr)  // training forward that keeps its per-chunk states
+    return launch_keep<LAT, DKB, DVB, SPLIT, MODE, true, WIDE, 0>(tq, tk, tv, ty, p, grid, stream);
+  if (p.y_f16) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 2>(tq, tk, tv, ty, p, grid, stream);
+  if constexpr (MODE != 1) {  // (no lengths in block-causal calls)
+    if (p.lens != nullptr) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 1>(tq, tk, tv, ty, p, grid, stream);
+  }
+  return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 0>(tq, tk, tv, ty, p, grid, stream);
 }
 
 }  // namespace
 
 template <>
-int launch_prefill_tc_unit<FLARE_TC_UNIT>(int lat, int mode, const CUtensorMap& tq, const CUtensorMap& tk,
-                                          const CUtensorMap& tv, const CUtensorMap& ty, const TcParams& p, dim3 grid,
-                                          cudaStream_t stream) {
+int launch_prefill_tc_unit<FLARE_TC_UNIT, FLARE_TC_MODE>(int lat, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                                                         const CUtensorMap& ty, const TcParams& p, dim3 grid,
+                                                         cudaStream_t stream) {
   // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128); units 3..5: the same with the latent-group split;
   // units 6, 7: the wide (128, 128) instance (one CTA for both value blocks) without / with the latent-group split
+  constexpr int MODE = FLARE_TC_MODE;
 #if FLARE_TC_UNIT >= 6
-  constexpr bool WSPLIT = FLARE_TC_UNIT == 7;
   (void)lat;
-  if (p.dump_u != nullptr) {  // training forward that keeps its per-chunk states
-    if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, true, true>(tq, tk, tv, ty, p, grid, stream);
-    if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, true, true>(tq, tk, tv, ty, p, grid, stream);
-    return launch_keep<0, 2, 2, WSPLIT, 0, true, true>(tq, tk, tv, ty, p, grid, stream);
-  }
-  if (p.y_f16 && p.y != nullptr && (!WSPLIT || p.cluster_merge)) {  // (partials in global memory become y in the merge kernel)
-    if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, false, true, true>(tq, tk, tv, ty, p, grid, stream);
-    if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, false, true, true>(tq, tk, tv, ty, p, grid, stream);
-    return launch_keep<0, 2, 2, WSPLIT, 0, false, true, true>(tq, tk, tv, ty, p, grid, stream);
-  }
-  if (mode == 1) return launch_keep<0, 2, 2, WSPLIT, 1, false, true>(tq, tk, tv, ty, p, grid, stream);
-  if (mode == 2) return launch_keep<0, 2, 2, WSPLIT, 2, false, true>(tq, tk, tv, ty, p, grid, stream);
-  return launch_keep<0, 2, 2, WSPLIT, 0, false, true>(tq, tk, tv, ty, p, grid, stream);
+  return launch_instance<0, 2, 2, FLARE_TC_UNIT == 7, MODE, true>(tq, tk, tv, ty, p, grid, stream);
 #else
   constexpr int COMBO = FLARE_TC_UNIT % 3;
   constexpr int DKB = COMBO == 1 ? 2 : 1;
   constexpr int DVB = COMBO == 0 ? 1 : 2;
   constexpr bool SPLIT = FLARE_TC_UNIT >= 3;
   // one instance family per kind of latent bank; the packed one exists for a single group only
-#define FLARE_TC_MODES(LAT)                                                                                \
-  return mode == 1 ? launch_instance<LAT, DKB, DVB, SPLIT, 1>(tq, tk, tv, ty, p, grid, stream)             \
-         : mode == 2 ? launch_instance<LAT, DKB, DVB, SPLIT, 2>(tq, tk, tv, ty, p, grid, stream)           \
-                     : launch_instance<LAT, DKB, DVB, SPLIT, 0>(tq, tk, tv, ty, p, grid, stream)
-  if (lat == 0) FLARE_TC_MODES(0);
+  if (lat == 0) return launch_instance<0, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
   if constexpr (!SPLIT) {
-    if (lat == 2) FLARE_TC_MODES(2);
+    if (lat == 2) return launch_instance<2, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
   }
-  FLARE_TC_MODES(1);
-#undef FLARE_TC_MODES
+  return launch_instance<1, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
 #endif
 }
 
@@ -1407,14 +1460,21 @@ int launch_prefill_tc_unit<FLARE_TC_UNIT>(int lat, int mode, const CUtensorMap& 
 
 __device__ int g_tc_error = 0;
 
-template <> int launch_prefill_tc_unit<0>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<1>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<2>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<3>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<4>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<5>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<6>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
-template <> int launch_prefill_tc_unit<7>(int, int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&, dim3, cudaStream_t);
+#define FLARE_TC_DECLARE(U, MODE)                                                                                            \
+  template <>                                                                                                               \
+  int launch_prefill_tc_unit<U, MODE>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,  \
+                                      const TcParams&, dim3, cudaStream_t);
+#define FLARE_TC_DECLARE_UNIT(U) FLARE_TC_DECLARE(U, 0) FLARE_TC_DECLARE(U, 1) FLARE_TC_DECLARE(U, 2)
+FLARE_TC_DECLARE_UNIT(0)
+FLARE_TC_DECLARE_UNIT(1)
+FLARE_TC_DECLARE_UNIT(2)
+FLARE_TC_DECLARE_UNIT(3)
+FLARE_TC_DECLARE_UNIT(4)
+FLARE_TC_DECLARE_UNIT(5)
+FLARE_TC_DECLARE_UNIT(6)
+FLARE_TC_DECLARE_UNIT(7)
+#undef FLARE_TC_DECLARE_UNIT
+#undef FLARE_TC_DECLARE
 
 // -------------------------------------------------------------------------------------------------
 // host side
@@ -1428,7 +1488,13 @@ bool make_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims
 
 }  // namespace
 
-bool prefill_tc_supported(const flare_fwd_args_t* a) {
+bool prefill_tc_supported(const flare_fwd_args_t* a) { return a->dtype == FLARE_BF16 && prefill_tc_shape(a); }
+
+bool prefill_tc_supported_f16(const flare_fwd_args_t* a) {
+  return a->dtype == FLARE_F16 && a->keep == nullptr && prefill_tc_shape(a);
+}
+
+bool prefill_tc_shape(const flare_fwd_args_t* a) {
   const int bs = a->block_size;
   const bool block_ok = bs == 1 || ((bs == 16 || bs == 32 || bs == 64 || bs == 128) && a->N % bs == 0);
   // the per-block encoder normalisers exist in block-causal mode only; the decode log-sum-exp in every mode
@@ -1442,7 +1508,7 @@ bool prefill_tc_supported(const flare_fwd_args_t* a) {
                              a->q_stride_h, a->q_stride_m};
   for (int64_t st : strides)
     if (st <= 0 || (st % 8) != 0 || st >= (int64_t(1) << 39)) return false;
-  return a->dtype == FLARE_BF16 && variant_ok && block_ok && lse_ok && a->M <= 4 * M && a->M >= 16 &&
+  return variant_ok && block_ok && lse_ok && a->M <= 4 * M && a->M >= 16 &&
          (a->M % 16) == 0 && ((a->Dk == 64 && (a->Dv == 64 || a->Dv == 128)) || (a->Dk == 128 && a->Dv == 128)) && a->q_dec == nullptr &&
          a->k_dec == nullptr && a->mask == nullptr && a->N >= 1;
 }
@@ -1659,20 +1725,15 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   if (const char* env = getenv("FLARE_B200_ROW_STORES"))  // diagnostic: per-thread row stores instead
     if (env[0] == '1' && !p.cluster_merge) p.y_tma = 0;
   const dim3 grid(a->B * a->H, nseg_grid, prefill_tc_grid_z(a, wide));
-  int rc;
   const int combo = a->Dk == 128 ? 1 : (a->Dv == 128 ? 2 : 0);  // (64, 64), (128, 128), (64, 128)
-  if (wide)
-    rc = groups > 1 ? launch_prefill_tc_unit<7>(lat, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<6>(lat, mode, tq, tk, tv, ty, p, grid, stream);
-  else if (combo == 0)
-    rc = groups > 1 ? launch_prefill_tc_unit<3>(lat, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<0>(lat, mode, tq, tk, tv, ty, p, grid, stream);
-  else if (combo == 1)
-    rc = groups > 1 ? launch_prefill_tc_unit<4>(lat, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<1>(lat, mode, tq, tk, tv, ty, p, grid, stream);
-  else
-    rc = groups > 1 ? launch_prefill_tc_unit<5>(lat, mode, tq, tk, tv, ty, p, grid, stream)
-                    : launch_prefill_tc_unit<2>(lat, mode, tq, tk, tv, ty, p, grid, stream);
+  const int unit = wide ? (groups > 1 ? 7 : 6) : combo + (groups > 1 ? 3 : 0);
+  using Launch = int (*)(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&,
+                         dim3, cudaStream_t);
+#define FLARE_TC_UNIT_ROW(U) {launch_prefill_tc_unit<U, 0>, launch_prefill_tc_unit<U, 1>, launch_prefill_tc_unit<U, 2>}
+  static constexpr Launch launch[8][3] = {FLARE_TC_UNIT_ROW(0), FLARE_TC_UNIT_ROW(1), FLARE_TC_UNIT_ROW(2), FLARE_TC_UNIT_ROW(3),
+                                          FLARE_TC_UNIT_ROW(4), FLARE_TC_UNIT_ROW(5), FLARE_TC_UNIT_ROW(6), FLARE_TC_UNIT_ROW(7)};
+#undef FLARE_TC_UNIT_ROW
+  const int rc = launch[unit][mode](lat, tq, tk, tv, ty, p, grid, stream);
   if (rc != FLARE_OK || groups == 1 || p.y == nullptr || p.cluster_merge) return rc;
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);

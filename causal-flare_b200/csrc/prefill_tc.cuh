@@ -5,9 +5,9 @@
 namespace flare {
 
 struct TcParams {
-  void* y;  // bf16 [B, N, H, Dv] (strided) or null
+  void* y;  // bf16 or fp16 [B, N, H, Dv] (strided) or null
   int64_t y_stride_b, y_stride_n, y_stride_h;
-  const void* q;  // bf16 latent bank [H, M, Dk]
+  const void* q;  // bf16 or fp16 latent bank [H, M, Dk]
   int64_t q_stride_h, q_stride_m;
   int N, H;
   int M;   // latents, <= 512; groups of 128 go to separate CTAs
@@ -27,8 +27,8 @@ struct TcParams {
   // the read-out rows leave through tiled bulk stores (set by the launch when the output's strides allow it and no
   // per-row lengths are given); otherwise every thread stores its own row
   int y_tma;
-  int y_f16;  // y is fp16 (a call on bf16 copies of fp16 inputs): rounded once, from the fp32 accumulators
-             // (the wide instance: by its template parameter Y16)
+  int y_f16;   // y is fp16: rounded once, from the fp32 accumulators
+  int in_f16;  // q, k, v are fp16 (a call with fp16 y whose inputs are bf16 copies has y_f16 alone)
   // Two latent groups on the wide instance: the two CTAs of a lane form a thread-block cluster and merge their
   // partial read-outs on chip (each finalises one 64-column value block); no partials in global memory, no merge
   // kernel.  Set by the launch.
@@ -54,7 +54,9 @@ struct TcParams {
   long long* trace;  // optional diagnostic cycle stamps of CTA (0, 0), see TC_TRACE; null in normal use
 };
 
-bool prefill_tc_supported(const flare_fwd_args_t* a);
+bool prefill_tc_supported(const flare_fwd_args_t* a);      // a bf16 call runs on these kernels
+bool prefill_tc_supported_f16(const flare_fwd_args_t* a);  // an fp16 call does, without copies (no training forward)
+bool prefill_tc_shape(const flare_fwd_args_t* a);          // what both ask of sizes, strides and options
 // scratch for the partial read-outs of the latent groups (0 for M <= 128), and the byte offset of the weight-mass
 // array inside it
 size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a);

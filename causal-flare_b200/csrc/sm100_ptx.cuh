@@ -2,6 +2,7 @@
 // mbarrier, TMA tiled loads (no multicast), tcgen05 tensor-memory allocation / MMA / ld / st / commit.
 // Every spin-wait is bounded: a wait that runs out returns false and the caller unwinds.
 #pragma once
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -193,6 +194,10 @@ constexpr uint32_t make_idesc_bf16(int M, int N, int a_mn_major, int b_mn_major)
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) |
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// the same with both operands in fp16
+constexpr uint32_t make_idesc_f16(int M, int N, int a_mn_major, int b_mn_major) {
+  return make_idesc_bf16(M, N, a_mn_major, b_mn_major) & ~((1u << 7) | (1u << 10));
+}
 
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -362,6 +367,10 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+__device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pack_bf16(f.x, f.y);
 }
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
   uint32_t r;

@@ -196,3 +196,31 @@ def test_fp16_through_the_entry_point_that_allocates_nothing():
         want = _ops.forward(q, k, v, scale=D ** -0.5, path=_lib.PATH_AUTO if fits else _lib.PATH_EXACT)[0]
         assert torch.equal(y, want)
     assert _ops.device_status() == 0
+
+
+@pytest.mark.parametrize("variant", ["softmax", "stablemax", "block"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 16, 64, 64), (2, 128, 2, 64, 64, 64), (1, 257, 2, 128, 64, 128), (1, 640, 2, 96, 128, 128),
+                                   (1, 384, 3, 128, 128, 128), (1, 200, 2, 256, 128, 128), (1, 131, 1, 192, 64, 64), (1, 6000, 1, 64, 64, 64)])
+def test_fp16_tensors_read_in_place_and_through_copies(shape, variant):
+    # One head expanded over all of them has a stride of zero, which no tiled copy can express: bf16 copies.  The same numbers
+    # laid out in full are read as they are, with scores from the unrounded q and k: no further from the oracle than the
+    # copies (which round both), to the 2 % that the roundings of the weights, which both share, can fall the other way.
+    B, N, H, M, Dk, Dv = shape
+    if variant == "block":
+        N = max(N // 64, 1) * 64
+    q, k, v = to_dev(*orc.make_inputs(B, N, H, M, Dk, Dv, seed0=31, dtype=F16))
+    k, v = k[:, :, :1].expand(B, N, H, Dk), v[:, :, :1].expand(B, N, H, Dv)
+    kw = dict(scale=Dk ** -0.5)
+    if variant == "stablemax":
+        kw["variant"] = _lib.STABLEMAX
+    if variant == "block":
+        kw["block_size"] = 64
+    copies = _ops.forward(q, k, v, **kw)[0]
+    direct = _ops.forward(q, k.contiguous(), v.contiguous(), **kw)[0]
+    qc, kc, vc = (t.cpu().contiguous() for t in (q, k, v))
+    if variant == "block":
+        ref = orc.semi_ar_forward(qc, kc, vc, block_size=64, scale=Dk ** -0.5)[0]
+    else:
+        ref = orc.ar_forward(qc, kc, vc, scale=Dk ** -0.5, **(dict(variant="stablemax") if variant == "stablemax" else {}))
+    err = [orc.rel_l2(t.float().cpu(), ref) for t in (copies, direct)]
+    assert err[1] <= 1.02 * err[0] + 2e-4 and err[1] <= 5e-3, err
