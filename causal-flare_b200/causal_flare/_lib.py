@@ -79,7 +79,8 @@ ABI_VERSION = 3  # FLARE_ABI_VERSION of include/flare_b200.h
 EXPORTS = (
     "flare_forward_workspace_bytes", "flare_forward", "flare_forward_keep_bytes", "flare_backward_workspace_bytes",
     "flare_backward",
-    "flare_decode_step", "flare_state_merge", "flare_mask_pack", "flare_mask_unpack", "flare_status_string", "flare_last_cuda_error",
+    "flare_decode_step", "flare_state_merge", "flare_mask_pack", "flare_mask_unpack",
+    "flare_forward_masked_workspace_bytes", "flare_forward_masked", "flare_status_string", "flare_last_cuda_error",
     "flare_abi_version", "flare_abi_sizeof", "flare_set_kernel_events", "flare_last_launch_count",
     "flare_forward_uses_tensor_path", "flare_backward_uses_tensor_path", "flare_device_status", "flare_set_trace_buffer",
     "flare_forward_noalloc", "flare_noalloc_scratch_capacity",
@@ -121,6 +122,10 @@ def load() -> C.CDLL:
     lib.flare_forward_keep_bytes.argtypes = [C.POINTER(FwdArgs)]
     lib.flare_forward.restype = C.c_int
     lib.flare_forward.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
+    lib.flare_forward_masked_workspace_bytes.restype = C.c_size_t
+    lib.flare_forward_masked_workspace_bytes.argtypes = [C.POINTER(FwdArgs)]
+    lib.flare_forward_masked.restype = C.c_int
+    lib.flare_forward_masked.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
     lib.flare_backward_workspace_bytes.restype = C.c_size_t
     lib.flare_backward_workspace_bytes.argtypes = [C.POINTER(BwdArgs)]
     lib.flare_backward.restype = C.c_int
@@ -241,12 +246,14 @@ def make_fwd_args(q, k, v, q_dec, k_dec, y, *, scale, variant=SOFTMAX, power=2.0
 
 def run_forward(args: FwdArgs, device) -> None:
     lib = load()
-    need = lib.flare_forward_workspace_bytes(C.byref(args))
+    masked = bool(args.mask)  # on the tensor kernels where the call without its mask would run there
+    need = (lib.flare_forward_masked_workspace_bytes if masked else lib.flare_forward_workspace_bytes)(C.byref(args))
     ws = None
     if need:
         ws = torch.empty(need, dtype=torch.uint8, device=device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), need
-    check(lib.flare_forward(C.byref(args), stream_handle(device)), "flare_forward")
+    run = lib.flare_forward_masked if masked else lib.flare_forward
+    check(run(C.byref(args), stream_handle(device)), "flare_forward")
     # `ws` is stream-ordered torch memory: safe to release after the launches are enqueued.
 
 

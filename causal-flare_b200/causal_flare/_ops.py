@@ -76,11 +76,7 @@ def forward(Q, K, V, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, pow
         if block_size > 1:
             raise ValueError("attention masks are not supported together with block_size > 1 (block-causal read-out)")
         mask = mask.to(device=dev, dtype=torch.int32).contiguous()
-    if mask is not None and B > 0 and N > 0 and _masked_on_tensor_path(q, k, v, qd, kd, y, st_out, scale, variant, power,
-                                                                      block_size, path, want_lse):
-        _forward_compacted(q, k, v, y, mask, scale=scale, variant=variant, power=power, state_in=state_in,
-                           st_out=st_out, path=path)
-    elif B > 0 and N > 0 or want_state:
+    if B > 0 and N > 0 or want_state:
         args = _lib.make_fwd_args(q, k, v, qd, kd, y, scale=scale, variant=variant, power=power,
                                   block_size=block_size, mask=mask, state_in=state_in, state_out=st_out,
                                   lse_dec=lse_dec, lse_enc=lse_enc, path=path)
@@ -102,39 +98,6 @@ def forward(Q, K, V, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, pow
     if want_y:
         out = y_store if out_dtype in (None, dt) else y_store.to(out_dtype)
     return out, st_out, lse_dec, lse_enc
-
-
-def _masked_on_tensor_path(q, k, v, qd, kd, y, st_out, scale, variant, power, block_size, path, want_lse) -> bool:
-    """True when the same call without the mask would run on the tensor-core kernels (they take per-row lengths, not
-    arbitrary masks, so a masked call is served by compacting the valid tokens to the front of every row)."""
-    if path == _lib.PATH_EXACT or want_lse or qd is not None or kd is not None or (y is None and st_out is None):
-        return False
-    probe = _lib.make_fwd_args(q, k, v, None, None, y, scale=scale, variant=variant, power=power, block_size=block_size,
-                               state_out=st_out, path=path)
-    return _lib.load().flare_forward_uses_tensor_path(C.byref(probe)) == 1
-
-
-def _forward_compacted(q, k, v, y, mask, *, scale, variant, power, state_in, st_out, path):
-    """Masked forward on the tensor path: pack the valid tokens of every batch row to the front (original order), run the
-    kernel with per-row lengths, unpack the outputs; masked positions get y = 0 and leave the state as is."""
-    B, N, H, Dk = k.shape
-    Dv = v.shape[-1]
-    lib, dev = _lib.load(), k.device
-    slot = torch.empty((B * (N + 1),), device=dev, dtype=torch.int32)  # slots, then the rows' lengths
-    lens = slot[B * N:]
-    kc = torch.empty((B, N, H, Dk), device=dev, dtype=k.dtype)
-    vc = torch.empty((B, N, H, Dv), device=dev, dtype=k.dtype)
-    yc = torch.empty((B, N, H, Dv), device=dev, dtype=k.dtype) if y is not None else None
-    strides = lambda t: (C.c_int64 * 3)(*t.stride()[:3])  # noqa: E731
-    _lib.check(lib.flare_mask_pack(mask.data_ptr(), k.data_ptr(), strides(k), v.data_ptr(), strides(v), B, N, H, Dk, Dv,
-                                   slot.data_ptr(), lens.data_ptr(), kc.data_ptr(), vc.data_ptr(), _lib.stream_handle(dev)),
-               "flare_mask_pack")
-    args = _lib.make_fwd_args(q, kc, vc, None, None, yc, scale=scale, variant=variant, power=power, state_in=state_in,
-                              state_out=st_out, path=path, lengths=lens)
-    _lib.run_forward(args, dev)
-    if y is not None:
-        _lib.check(lib.flare_mask_unpack(slot.data_ptr(), yc.data_ptr(), y.data_ptr(), strides(y), B, N, H, Dv,
-                                         _lib.stream_handle(dev)), "flare_mask_unpack")
 
 
 def backward(Q, K, V, dY, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, power=2.0, block_size=1,

@@ -55,6 +55,13 @@ static size_t scratch_left(size_t taken) {
 // y of the forward in flight on this thread is fp16 although its inputs are bf16 (copies), see forward_cast
 static thread_local bool g_y_f16 = false;
 
+// masked call in flight on this thread whose packed copies the forward runs on, see forward_masked
+struct MaskedRows {
+  const int32_t* start;
+  const flare_fwd_args_t* call;
+};
+static thread_local const MaskedRows* g_rows = nullptr;
+
 void count_launches(int n) { g_last_launches += n; }
 
 // ---- per-kernel profile records of this thread -----------------------------------------------------------
@@ -263,7 +270,8 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
   if (t.y != nullptr && g_keep.u != nullptr) {
     t.dump_u = g_keep.u; t.dump_c = g_keep.c; t.dump_d = g_keep.d; t.dump_nch = g_keep.nch;
   }
-  return launch_prefill_tc(a, t, nseg_grid, pl.wide, stream);
+  t.row_start = g_rows != nullptr ? g_rows->start : nullptr;
+  return launch_prefill_tc(a, t, nseg_grid, pl.wide, g_rows != nullptr ? g_rows->call : nullptr, stream);
 }
 
 int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaStream_t stream);
@@ -437,6 +445,108 @@ int forward_cast(const flare_fwd_args_t* a, flare_fwd_args_t& b, const CastPlan&
   return FLARE_OK;
 }
 
+// Masked calls on the tensor-core kernels, which take per-row lengths instead of masks.  A row whose valid tokens are its
+// last ones (left padding) is walked where it is; of any other row the valid tokens are packed to the front of a copy, and
+// its outputs unpacked.  Which rows are which is found on the device.  B200, B=8 N=2000 H=16 M=128 D=64 bf16, left-padded
+// rows of 500 to 2000 tokens: 130.9 us with every row packed and unpacked (53 us of copies), 102.8 us this way.
+struct MaskedPlan {
+  bool on;
+  size_t off_lens, off_start, off_k, off_v, off_y, total;
+};
+
+// scratch of the forward on the packed copies (SIZE_MAX: not on the tensor kernels); cast: it is an fp16 call that makes
+// bf16 copies, for a latent bank whose strides a tiled copy cannot express
+size_t masked_inner_bytes(const flare_fwd_args_t* b, bool* cast = nullptr) {
+  const FwdPlan pl = plan_forward(b);
+  if (cast != nullptr) *cast = !pl.use_tc;
+  if (pl.use_tc) return pl.ws_bytes;
+  flare_fwd_args_t c;
+  const CastPlan cp = plan_cast(b, &c);
+  return cp.on ? cp.total + plan_forward(&c).ws_bytes : SIZE_MAX;
+}
+
+MaskedPlan plan_masked(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
+  MaskedPlan mp{false, 0, 0, 0, 0, 0, 0};
+  if (a->mask == nullptr || a->path == FLARE_PATH_EXACT || a->q_dec != nullptr || a->k_dec != nullptr || a->lse_dec != nullptr ||
+      a->lse_enc != nullptr || a->keep != nullptr || a->block_size != 1 || a->B == 0 || a->N == 0 ||
+      (int64_t)a->B * a->N > 0x7fffffff)
+    return mp;
+  *b = *a;
+  b->mask = nullptr;
+  flare_fwd_args_t c;
+  if (!plan_forward(b).use_tc && !plan_cast(b, &c).on) return mp;
+  b->lengths = a->mask;  // (any non-null pointer until the lengths have their place)
+  b->k_stride_h = a->Dk; b->k_stride_n = (int64_t)a->H * a->Dk; b->k_stride_b = (int64_t)a->N * b->k_stride_n;
+  b->v_stride_h = a->Dv; b->v_stride_n = (int64_t)a->H * a->Dv; b->v_stride_b = (int64_t)a->N * b->v_stride_n;
+  b->y_stride_h = b->v_stride_h; b->y_stride_n = b->v_stride_n; b->y_stride_b = b->v_stride_b;
+  if (masked_inner_bytes(b) == SIZE_MAX) return mp;
+  const size_t rows = (size_t)a->B * a->N, es = (size_t)dtype_size(a->dtype);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += align_up(bytes, 256);
+    return o;
+  };
+  mp.on = true;
+  take(rows * sizeof(int32_t));  // slots
+  mp.off_lens = take((size_t)a->B * sizeof(int32_t));
+  mp.off_start = take((size_t)a->B * sizeof(int32_t));
+  mp.off_k = take(rows * a->H * a->Dk * es);
+  mp.off_v = take(rows * a->H * a->Dv * es);
+  mp.off_y = a->y != nullptr ? take(rows * a->H * a->Dv * es) : 0;
+  mp.total = off;
+  return mp;
+}
+
+int forward_masked(const flare_fwd_args_t* a, flare_fwd_args_t& b, const MaskedPlan& mp, cudaStream_t stream) {
+  bool cast = false;
+  const size_t inner = masked_inner_bytes(&b, &cast);
+  if (a->workspace == nullptr || a->workspace_bytes < mp.total + inner || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
+  char* ws = reinterpret_cast<char*>(a->workspace);
+  int32_t* const slot = reinterpret_cast<int32_t*>(ws);
+  int32_t* const lens = reinterpret_cast<int32_t*>(ws + mp.off_lens);
+  int32_t* const start = prefill_tc_rows_in_place(a) ? reinterpret_cast<int32_t*>(ws + mp.off_start) : nullptr;
+  b.k = ws + mp.off_k; b.v = ws + mp.off_v;
+  b.y = a->y != nullptr ? ws + mp.off_y : nullptr;
+  b.lengths = lens;
+  b.workspace = inner > 0 ? ws + mp.total : nullptr;
+  b.workspace_bytes = inner > 0 ? a->workspace_bytes - mp.total : 0;
+  int rc = launch_mask_slots(a->mask, a->B, a->N, slot, lens, start, stream);
+  if (rc != FLARE_OK) return rc;
+  MoveRowsParams p;
+  memset(&p, 0, sizeof(p));
+  p.B = a->B; p.N = a->N; p.H = a->H; p.slot = slot; p.lens = lens; p.start = start;
+  MoveRowsParams u = p;
+  p.in[0] = a->k; p.out[0] = const_cast<void*>(b.k); p.d[0] = a->Dk;
+  p.is_b[0] = a->k_stride_b; p.is_n[0] = a->k_stride_n; p.is_h[0] = a->k_stride_h;
+  p.os_b[0] = b.k_stride_b; p.os_n[0] = b.k_stride_n; p.os_h[0] = b.k_stride_h;
+  p.in[1] = a->v; p.out[1] = const_cast<void*>(b.v); p.d[1] = a->Dv;
+  p.is_b[1] = a->v_stride_b; p.is_n[1] = a->v_stride_n; p.is_h[1] = a->v_stride_h;
+  p.os_b[1] = b.v_stride_b; p.os_n[1] = b.v_stride_n; p.os_h[1] = b.v_stride_h;
+  rc = launch_move_rows(p, 2, stream);
+  if (rc != FLARE_OK) return rc;
+  const MaskedRows rows{start, a};
+  if (cast) {
+    flare_fwd_args_t c;
+    const CastPlan cp = plan_cast(&b, &c);
+    rc = forward_cast(&b, c, cp, stream);
+  } else {
+    g_rows = start != nullptr ? &rows : nullptr;
+    rc = forward_run(&b, stream);
+    g_rows = nullptr;
+  }
+  if (rc != FLARE_OK) return rc;
+  g_last_launches += 2;
+  if (a->y == nullptr) return FLARE_OK;
+  u.unpack = 1;
+  u.in[0] = b.y; u.out[0] = a->y; u.d[0] = a->Dv;
+  u.is_b[0] = b.y_stride_b; u.is_n[0] = b.y_stride_n; u.is_h[0] = b.y_stride_h;
+  u.os_b[0] = a->y_stride_b; u.os_n[0] = a->y_stride_n; u.os_h[0] = a->y_stride_h;
+  rc = launch_move_rows(u, 1, stream);
+  g_last_launches += 1;
+  return rc;
+}
+
 }  // namespace
 
 int forward_keep_states(const flare_fwd_args_t* a, const ChunkStates& keep, int* gate, cudaStream_t stream) {
@@ -550,6 +660,21 @@ int flare_forward(const flare_fwd_args_t* args, flare_stream_t stream) {
     return forward_run(args, stream);  // (planned within what is left, as the size was)
   }
   return forward_run(args, stream);
+}
+
+size_t flare_forward_masked_workspace_bytes(const flare_fwd_args_t* args) {
+  if (check_forward(args) != FLARE_OK) return 0;
+  flare_fwd_args_t b;
+  const MaskedPlan mp = plan_masked(args, &b);
+  return mp.on ? mp.total + masked_inner_bytes(&b) : flare_forward_workspace_bytes(args);
+}
+
+int flare_forward_masked(const flare_fwd_args_t* args, flare_stream_t stream) {
+  const int rc = check_forward(args);
+  if (rc != FLARE_OK) return rc;
+  flare_fwd_args_t b;
+  const MaskedPlan mp = plan_masked(args, &b);
+  return mp.on ? forward_masked(args, b, mp, stream) : flare_forward(args, stream);
 }
 
 static int check_backward(const flare_bwd_args_t* args) {
@@ -732,7 +857,7 @@ int flare_mask_pack(const int32_t* mask, const void* k, const int64_t k_strides_
   if (!mask || !slot || !lengths || !k_strides_bnh || !v_strides_bnh || !rows_ok(k, k_strides_bnh) || !rows_ok(v, v_strides_bnh) ||
       !k_out || !v_out || !aligned16(k_out) || !aligned16(v_out))
     return FLARE_ERR_BAD_POINTER;
-  const int rc = launch_mask_slots(mask, B, N, slot, lengths, stream);
+  const int rc = launch_mask_slots(mask, B, N, slot, lengths, nullptr, stream);
   if (rc != FLARE_OK) return rc;
   MoveRowsParams p;
   memset(&p, 0, sizeof(p));

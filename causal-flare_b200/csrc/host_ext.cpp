@@ -33,6 +33,8 @@ struct Api {
   decltype(&flare_forward_workspace_bytes) forward_workspace_bytes = nullptr;
   decltype(&flare_forward_keep_bytes) forward_keep_bytes = nullptr;
   decltype(&flare_forward) forward = nullptr;
+  decltype(&flare_forward_masked_workspace_bytes) forward_masked_workspace_bytes = nullptr;
+  decltype(&flare_forward_masked) forward_masked = nullptr;
   decltype(&flare_backward_workspace_bytes) backward_workspace_bytes = nullptr;
   decltype(&flare_backward) backward = nullptr;
   decltype(&flare_decode_step) decode_step = nullptr;
@@ -52,6 +54,8 @@ void bind(const py::dict& table) {
   take(api.forward_workspace_bytes, table, "flare_forward_workspace_bytes");
   take(api.forward_keep_bytes, table, "flare_forward_keep_bytes");
   take(api.forward, table, "flare_forward");
+  take(api.forward_masked_workspace_bytes, table, "flare_forward_masked_workspace_bytes");
+  take(api.forward_masked, table, "flare_forward_masked");
   take(api.backward_workspace_bytes, table, "flare_backward_workspace_bytes");
   take(api.backward, table, "flare_backward");
   take(api.decode_step, table, "flare_decode_step");
@@ -197,7 +201,8 @@ struct Forward {
   State out;
 };
 
-Forward run_forward(const Problem& p, const State& in, bool want_state, bool want_lse, bool want_keep) {
+// mask: [B, N] int32, or undefined
+Forward run_forward(const Problem& p, const State& in, bool want_state, bool want_lse, bool want_keep, const Tensor& mask = Tensor()) {
   const auto opts = p.k.options().requires_grad(false);
   const auto f32 = opts.dtype(at::kFloat);
   const int64_t B = p.k.size(0), N = p.k.size(1), H = p.k.size(2), M = p.q.size(1), Dv = p.v.size(3);
@@ -228,12 +233,14 @@ Forward run_forward(const Problem& p, const State& in, bool want_state, bool wan
     a.keep_bytes = keep_bytes;
   }
   Tensor ws;
-  if (const size_t need = api.forward_workspace_bytes(&a)) {
+  if (mask.defined()) a.mask = mask.data_ptr<int32_t>();
+  if (const size_t need = mask.defined() ? api.forward_masked_workspace_bytes(&a) : api.forward_workspace_bytes(&a)) {
     ws = at::empty({(int64_t)need}, opts.dtype(at::kByte));  // stream-ordered memory: free once the launches are enqueued
     a.workspace = ws.data_ptr();
     a.workspace_bytes = need;
   }
-  check(api.forward(&a, c10::cuda::getCurrentCUDAStream(p.k.device().index()).stream()), "flare_forward");
+  const auto stream = c10::cuda::getCurrentCUDAStream(p.k.device().index()).stream();
+  check(mask.defined() ? api.forward_masked(&a, stream) : api.forward(&a, stream), "flare_forward");
   return r;
 }
 
@@ -344,12 +351,21 @@ py::object prefill(const Tensor& q, const Tensor& k, const Tensor& v, const py::
                    const py::object& mask) {
   const int path = path_from_env();
   double sc;
-  if (path < 0 || !mask.is_none() || !plain_qkv(q, k, v) || !to_scale(scale, &sc)) return py::none();
+  if (path < 0 || !plain_qkv(q, k, v) || !to_scale(scale, &sc)) return py::none();
+  Tensor valid;
+  if (!mask.is_none()) {
+    if (!THPVariable_Check(mask.ptr())) return py::none();
+    valid = THPVariable_Unpack(mask.ptr());
+    if (!ordinary(valid) || valid.device() != k.device() || valid.layout() != at::kStrided || valid.dim() != 2 ||
+        valid.size(0) != k.size(0) || valid.size(1) != k.size(1))
+      return py::none();
+  }
   const c10::cuda::CUDAGuard guard(k.device());
+  if (valid.defined()) valid = valid.to(at::kInt).contiguous();
   State in;
   if (!state.is_none() && !plain_state(state, k.size(0), k.size(2), q.size(1), v.size(3), k, &in)) return py::none();
   const Problem p{ready(q), ready(k), ready(v), sc, 2.0, FLARE_SOFTMAX, 1, path};
-  const Forward r = run_forward(p, in, true, false, false);
+  const Forward r = run_forward(p, in, true, false, false, valid);
   return py::make_tuple(r.y, state_dict(r.out));
 }
 

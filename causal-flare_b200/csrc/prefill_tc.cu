@@ -184,7 +184,7 @@ __device__ __forceinline__ int latent0() {
 // with the latent-group split, and the wide ones; FLARE_TC_MODE = 0..2) to keep build times short; the unit without
 // FLARE_TC_UNIT holds the host side.
 template <int UNIT, int MODE>
-int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
+int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty, const CUtensorMap* in,
                            const TcParams& p, dim3 grid, cudaStream_t stream);
 
 #ifdef FLARE_TC_UNIT
@@ -213,14 +213,15 @@ int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk
 //       SMs in one wave.  Differences: U and Y are 128 columns wide; W and Y0 = R^T U_bf16 come out of ONE product of
 //       width 256 ([E | U_bf16] as one B operand, [W | Y] adjacent in tensor memory), so R is read once for both; W
 //       shares the columns of S; E and R are single-buffered.
-// FL:   0 = bf16, every row N tokens long; 1 = bf16 with per-row lengths; 2 = fp16 y (of fp16 inputs, or of bf16 copies:
-//       p.in_f16), with lengths or not.  Instances of their own: as run-time choices they cost every bf16 call 2 to 3 % (B200:
+// FL:   0 = bf16, every row N tokens long; 1 = bf16 with per-row lengths and, of a masked call, rows that were not packed;
+//       2 = fp16 y (of fp16 inputs, or of bf16 copies: p.in_f16), with lengths or not.  Instances of their own: as run-time choices they cost every bf16 call 2 to 3 % (B200:
 //       B=8 N=8192 H=16 M=128 D=64 182.3 -> 185.8 us, training B=4 N=4096 H=16 M=64 D=128 411 -> 424 us), and the type of y in
 //       the epilogue of the wide instance 5 to 8 %.
 template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y, const TcParams p) {
+                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y,
+                  const __grid_constant__ CUtensorMap tm_k_in, const __grid_constant__ CUtensorMap tm_v_in, const TcParams p) {
   using L = Lay<DKB, WIDE>;
   constexpr bool PADDED = LAT != 0, PACK = LAT == 2;
   static_assert(!WIDE || (DVB == 2 && !PADDED), "wide instance");
@@ -306,7 +307,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   if (warp == 13) {
     // ======================================= TMA producer =======================================
-    if constexpr (FL != 2) {
+    if constexpr (FL == 0) {
       if (lane == 0) {
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
@@ -336,7 +337,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // fp16 inputs: Q and K go to the score product as they are; V, which meets bf16 weights, is rounded to bf16 in place by
       // this warp (one tile behind the loads, so that the next chunk's K never waits for it).  B200, B=4 N=4096 H=16 M=64 D=128:
       // 130 us with bf16 copies of K and V made before the kernel (a pass of 42 us over them), 93 us this way.
-      const unsigned active = p.in_f16 ? 0xffffffffu : 1u;  // (bf16 copies: the one thread that issues the loads)
+      const unsigned active = p.in_f16 ? 0xffffffffu : 1u;  // (bf16: the one thread that issues the loads)
       auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(active, wait_or_abort(bar, parity, misc)) != 0; };
       auto convert_v = [&](int i) -> bool {
         const int st = i & 1;
@@ -357,9 +358,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       };
       if (lane == 0 || p.in_f16) {
         const int vc0 = value_col0<ZS, SPLIT>();
+        // a row of a masked call that was not packed: its tokens are the last ones of the caller's row
+        const int row0 = p.row_start != nullptr ? p.row_start[b] : -1;
+        const CUtensorMap* const mk = row0 >= 0 ? &tm_k_in : &tm_k;
+        const CUtensorMap* const mv = row0 >= 0 ? &tm_v_in : &tm_v;
         if (lane == 0) {
-          prefetch_tensormap(&tm_k);
-          prefetch_tensormap(&tm_v);
+          prefetch_tensormap(mk);
+          prefetch_tensormap(mv);
           if (Q_SMEM) {
             mbar_arrive_expect_tx(&misc->q_full, 16384);
             tma_load_3d(smem + OFF_Q, &tm_q, &misc->q_full, 0, latent0<ZS, SPLIT>(), h);  // rows beyond M read as zero
@@ -367,13 +372,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
         }
         for (int i = 0; ok && i < nchunks; ++i) {
-          const int t0 = seg_begin + i * C;
+          const int t0 = seg_begin + i * C + max(row0, 0);
           // K tile: free once the score MMA of the previous chunk has run
           if (i > 0 && !(ok = wait_all(&misc->k_empty, (i - 1) & 1))) break;
           if (lane == 0) {
             mbar_arrive_expect_tx(&misc->k_full, DKB * 16384);
 #pragma unroll
-            for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, &tm_k, &misc->k_full, kb * 64, h, t0, b);
+            for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, mk, &misc->k_full, kb * 64, h, t0, b);
           }
           if (p.in_f16 && i > 0 && !(ok = convert_v(i - 1))) break;
           // V tile: stage i & 1, free once chunk i - 2 has been folded into Y
@@ -383,7 +388,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             mbar_arrive_expect_tx(&misc->v_full[st], VB * 16384);
 #pragma unroll
             for (int vb = 0; vb < VB; ++vb)
-              tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, &tm_v, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
+              tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, mv, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
           }
         }
         if (p.in_f16 && ok && nchunks > 0) ok = convert_v(nchunks - 1);
@@ -1111,6 +1116,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     uint8_t* const stage = smem + L::OFF_STAGE + wq * 2048;
     // latent-group split: dense fp16 partials [group][B][N][H][DV] and log2 weight masses [group][B][N][H]
     const int64_t part_row0 = SPLIT ? (((int64_t)(blockIdx.z / ZS) * (gridDim.x / p.H) + b) * p.N) : 0;
+    const int row0 = LENS && p.row_start != nullptr ? p.row_start[b] : 0;  // (-1: a packed row, whose y goes to the packed copy)
     for (int i = 0; !state_only && ok && i < nchunks; ++i) {
       const uint32_t par = i & 1;
       const int t0 = seg_begin + i * C;
@@ -1333,7 +1339,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             pack_out(y, SPLIT || F16, o);
             v[ch] = make_uint4(o[0], o[1], o[2], o[3]);
           }
-          if (p.y_tma) {
+          if (p.y_tma && (!LENS || row0 >= 0)) {
             // One tiled bulk store per warp and 32 x 32 tile.  A thread storing its own row straight to global
             // memory costs 32 separate 16-byte transactions per instruction; the latent warps' operand stores to
             // shared memory queued behind those and the whole kernel ran 12 % slower.  Rows beyond the sequence end
@@ -1346,7 +1352,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_store_4d(&tm_y, stage, col, h, t0 + wq * 32, SPLIT ? (int)(blockIdx.z / ZS) * (int)(gridDim.x / p.H) + b : b);
+              tma_store_4d(&tm_y, stage, col, h, t0 + row0 + wq * 32, SPLIT ? (int)(blockIdx.z / ZS) * (int)(gridDim.x / p.H) + b : b);
               bulk_commit_group();
             }
           } else if (SPLIT) {
@@ -1389,7 +1395,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 namespace {
 
 template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
-int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
+int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty, const CUtensorMap* in,
                 const TcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = prefill_tc_kernel<LAT, DKB, DVB, SPLIT, MODE, KEEP, WIDE, FL>;
   FLARE_CUDA_CHECK(allow_smem(kern));
@@ -1411,48 +1417,48 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    FLARE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, ty, p));
+    FLARE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, ty, in[0], in[1], p));
   } else {
-    FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NTHREADS), Lay<DKB, WIDE>::SMEM_BYTES, stream, tq, tk, tv, ty, p));
+    FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NTHREADS), Lay<DKB, WIDE>::SMEM_BYTES, stream, tq, tk, tv, ty, in[0], in[1], p));
   }
   return FLARE_OK;
 }
 
 template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool WIDE>
-int launch_instance(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty,
+int launch_instance(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ty, const CUtensorMap* in,
                     const TcParams& p, dim3 grid, cudaStream_t stream) {
   if (p.dump_u != nullptr)  // training forward that keeps its per-chunk states
-    return launch_keep<LAT, DKB, DVB, SPLIT, MODE, true, WIDE, 0>(tq, tk, tv, ty, p, grid, stream);
-  if (p.y_f16) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 2>(tq, tk, tv, ty, p, grid, stream);
+    return launch_keep<LAT, DKB, DVB, SPLIT, MODE, true, WIDE, 0>(tq, tk, tv, ty, in, p, grid, stream);
+  if (p.y_f16) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 2>(tq, tk, tv, ty, in, p, grid, stream);
   if constexpr (MODE != 1) {  // (no lengths in block-causal calls)
-    if (p.lens != nullptr) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 1>(tq, tk, tv, ty, p, grid, stream);
+    if (p.lens != nullptr) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 1>(tq, tk, tv, ty, in, p, grid, stream);
   }
-  return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 0>(tq, tk, tv, ty, p, grid, stream);
+  return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 0>(tq, tk, tv, ty, in, p, grid, stream);
 }
 
 }  // namespace
 
 template <>
 int launch_prefill_tc_unit<FLARE_TC_UNIT, FLARE_TC_MODE>(int lat, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                                                         const CUtensorMap& ty, const TcParams& p, dim3 grid,
-                                                         cudaStream_t stream) {
+                                                         const CUtensorMap& ty, const CUtensorMap* in, const TcParams& p,
+                                                         dim3 grid, cudaStream_t stream) {
   // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128); units 3..5: the same with the latent-group split;
   // units 6, 7: the wide (128, 128) instance (one CTA for both value blocks) without / with the latent-group split
   constexpr int MODE = FLARE_TC_MODE;
 #if FLARE_TC_UNIT >= 6
   (void)lat;
-  return launch_instance<0, 2, 2, FLARE_TC_UNIT == 7, MODE, true>(tq, tk, tv, ty, p, grid, stream);
+  return launch_instance<0, 2, 2, FLARE_TC_UNIT == 7, MODE, true>(tq, tk, tv, ty, in, p, grid, stream);
 #else
   constexpr int COMBO = FLARE_TC_UNIT % 3;
   constexpr int DKB = COMBO == 1 ? 2 : 1;
   constexpr int DVB = COMBO == 0 ? 1 : 2;
   constexpr bool SPLIT = FLARE_TC_UNIT >= 3;
   // one instance family per kind of latent bank; the packed one exists for a single group only
-  if (lat == 0) return launch_instance<0, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
+  if (lat == 0) return launch_instance<0, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, in, p, grid, stream);
   if constexpr (!SPLIT) {
-    if (lat == 2) return launch_instance<2, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
+    if (lat == 2) return launch_instance<2, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, in, p, grid, stream);
   }
-  return launch_instance<1, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, p, grid, stream);
+  return launch_instance<1, DKB, DVB, SPLIT, MODE, false>(tq, tk, tv, ty, in, p, grid, stream);
 #endif
 }
 
@@ -1463,7 +1469,7 @@ __device__ int g_tc_error = 0;
 #define FLARE_TC_DECLARE(U, MODE)                                                                                            \
   template <>                                                                                                               \
   int launch_prefill_tc_unit<U, MODE>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,  \
-                                      const TcParams&, dim3, cudaStream_t);
+                                      const CUtensorMap*, const TcParams&, dim3, cudaStream_t);
 #define FLARE_TC_DECLARE_UNIT(U) FLARE_TC_DECLARE(U, 0) FLARE_TC_DECLARE(U, 1) FLARE_TC_DECLARE(U, 2)
 FLARE_TC_DECLARE_UNIT(0)
 FLARE_TC_DECLARE_UNIT(1)
@@ -1519,8 +1525,10 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* part
                                                                int groups, int64_t rows /* B*N*H */, int N, int H, int dv,
                                                                uint16_t* y, int y_f16, int64_t y_stride_b, int64_t y_stride_n,
                                                                int64_t y_stride_h, float* lse_dec /* [B, H, N] or null */,
-                                                               const int32_t* lens /* [B] or null */, int* gate,
-                                                               int gate_stride, int gate_off) {
+                                                               const int32_t* lens /* [B] or null */,
+                                                               const int32_t* row_start /* [B] or null */, uint16_t* y_in,
+                                                               int64_t yi_stride_b, int64_t yi_stride_n, int64_t yi_stride_h,
+                                                               int* gate, int gate_stride, int gate_off) {
   pdl_begin();
   const int cols8 = dv >> 3;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1567,8 +1575,10 @@ __global__ void __launch_bounds__(256) tc_merge_groups_kernel(const __half* part
   for (int j = 0; j < 8; ++j) acc[j] *= inv;
   uint32_t o[4];
   pack_out(acc, y_f16 != 0, o);
-  *reinterpret_cast<uint4*>(y + b * y_stride_b + (int64_t)n * y_stride_n + (int64_t)h * y_stride_h + c8 * 8) =
-      make_uint4(o[0], o[1], o[2], o[3]);
+  const int row0 = row_start != nullptr ? row_start[b] : -1;  // (>= 0: a row of a masked call that was not packed)
+  uint16_t* const dst = row0 >= 0 ? y_in + b * yi_stride_b + (int64_t)(n + row0) * yi_stride_n + (int64_t)h * yi_stride_h
+                                  : y + b * y_stride_b + (int64_t)n * y_stride_n + (int64_t)h * y_stride_h;
+  *reinterpret_cast<uint4*>(dst + c8 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 
@@ -1653,7 +1663,16 @@ size_t prefill_tc_partial_bytes(const flare_fwd_args_t* a) {
   return prefill_tc_partial_lw_offset(a) + (size_t)groups * a->B * a->N * a->H * sizeof(float);
 }
 
-int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_grid, bool wide, cudaStream_t stream) {
+bool prefill_tc_rows_in_place(const flare_fwd_args_t* a) {
+  if (!prefill_tc_shape(a)) return false;
+  if (a->y == nullptr) return true;
+  for (int64_t st : {a->y_stride_b, a->y_stride_n, a->y_stride_h})
+    if (st <= 0 || (st % 8) != 0 || st >= (int64_t(1) << 39)) return false;
+  return (reinterpret_cast<uintptr_t>(a->y) % 16) == 0;
+}
+
+int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_grid, bool wide, const flare_fwd_args_t* direct,
+                      cudaStream_t stream) {
   TcParams p = p_in;
   {
     const int rc = tc_error_word(&p.err);
@@ -1668,7 +1687,8 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
     p.lse_dec = p.lse_enc = nullptr;
     p.dump_u = nullptr;
   }
-  CUtensorMap tq, tk, tv;
+  if (p.row_start == nullptr) direct = nullptr;
+  CUtensorMap tq, tk, tv, in[2];
   {
     // latent bank (used by the Dk = 64 instances only; any valid map otherwise)
     const uint64_t dims[3] = {(uint64_t)a->Dk, (uint64_t)a->M, (uint64_t)a->H};
@@ -1688,6 +1708,16 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
     if (!make_map(&tk, a->k, 4, dimk, strk, box) || !make_map(&tv, a->v, 4, dimv, strv, box)) {
       set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (keys / values)");
       return FLARE_ERR_CUDA;
+    }
+    in[0] = tk;
+    in[1] = tv;
+    if (direct != nullptr) {
+      const int64_t sk[3] = {direct->k_stride_h, direct->k_stride_n, direct->k_stride_b};
+      const int64_t sv[3] = {direct->v_stride_h, direct->v_stride_n, direct->v_stride_b};
+      if (!make_map(&in[0], direct->k, 4, dimk, sk, box) || !make_map(&in[1], direct->v, 4, dimv, sv, box)) {
+        set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (keys / values of a masked call)");
+        return FLARE_ERR_CUDA;
+      }
     }
   }
   const int groups = prefill_tc_latent_groups(a);
@@ -1722,18 +1752,28 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
       p.y_tma = y_ok && tc::make_map_bf16(&ty, p.y, 4, ydims, str, box, CU_TENSOR_MAP_SWIZZLE_64B) ? 1 : 0;
     }
   }
-  if (const char* env = getenv("FLARE_B200_ROW_STORES"))  // diagnostic: per-thread row stores instead
+  if (direct != nullptr && p.y != nullptr && groups == 1) {
+    // rows of a masked call that stay where they are: their y goes straight to the caller's tensor
+    const uint32_t box[4] = {32, 1, 32, 1};
+    const int64_t str[3] = {direct->y_stride_h, direct->y_stride_n, direct->y_stride_b};
+    const uint64_t ydims[4] = {(uint64_t)a->Dv, (uint64_t)a->H, (uint64_t)a->N, (uint64_t)a->B};
+    if (!tc::make_map_bf16(&ty, direct->y, 4, ydims, str, box, CU_TENSOR_MAP_SWIZZLE_64B)) {
+      set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (output of a masked call)");
+      return FLARE_ERR_CUDA;
+    }
+    p.y_tma = 1;
+  } else if (const char* env = getenv("FLARE_B200_ROW_STORES"))  // diagnostic: per-thread row stores instead
     if (env[0] == '1' && !p.cluster_merge) p.y_tma = 0;
   const dim3 grid(a->B * a->H, nseg_grid, prefill_tc_grid_z(a, wide));
   const int combo = a->Dk == 128 ? 1 : (a->Dv == 128 ? 2 : 0);  // (64, 64), (128, 128), (64, 128)
   const int unit = wide ? (groups > 1 ? 7 : 6) : combo + (groups > 1 ? 3 : 0);
-  using Launch = int (*)(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const TcParams&,
-                         dim3, cudaStream_t);
+  using Launch = int (*)(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap*,
+                         const TcParams&, dim3, cudaStream_t);
 #define FLARE_TC_UNIT_ROW(U) {launch_prefill_tc_unit<U, 0>, launch_prefill_tc_unit<U, 1>, launch_prefill_tc_unit<U, 2>}
   static constexpr Launch launch[8][3] = {FLARE_TC_UNIT_ROW(0), FLARE_TC_UNIT_ROW(1), FLARE_TC_UNIT_ROW(2), FLARE_TC_UNIT_ROW(3),
                                           FLARE_TC_UNIT_ROW(4), FLARE_TC_UNIT_ROW(5), FLARE_TC_UNIT_ROW(6), FLARE_TC_UNIT_ROW(7)};
 #undef FLARE_TC_UNIT_ROW
-  const int rc = launch[unit][mode](lat, tq, tk, tv, ty, p, grid, stream);
+  const int rc = launch[unit][mode](lat, tq, tk, tv, ty, in, p, grid, stream);
   if (rc != FLARE_OK || groups == 1 || p.y == nullptr || p.cluster_merge) return rc;
   const int64_t rows = (int64_t)a->B * a->N * a->H;
   const int64_t threads = rows * (a->Dv / 8);
@@ -1741,7 +1781,9 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   FLARE_CUDA_CHECK(launch_pdl(tc_merge_groups_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream,
                               reinterpret_cast<const __half*>(p.part_y), p.part_lw, groups, rows, a->N, a->H, a->Dv,
                               reinterpret_cast<uint16_t*>(p.y), p.y_f16, p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
-                              p.gate, p.gate_stride, p.gate_off));
+                              p.row_start, direct != nullptr ? reinterpret_cast<uint16_t*>(direct->y) : nullptr,
+                              direct != nullptr ? direct->y_stride_b : 0, direct != nullptr ? direct->y_stride_n : 0,
+                              direct != nullptr ? direct->y_stride_h : 0, p.gate, p.gate_stride, p.gate_off));
   return FLARE_OK;
 }
 

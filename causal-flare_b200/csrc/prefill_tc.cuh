@@ -35,6 +35,9 @@ struct TcParams {
   int cluster_merge;
   int out_mode;  // 0: none, 1: every segment, 2: last segment only
   int nseg_total;
+  // Masked call (with lens): row_start[b] >= 0 says that row b was not packed, because its tokens are the last lens[b] ones of
+  // the caller's row, from token row_start[b] on; K, V and y of such a row are the caller's own.  Null otherwise.
+  const int32_t* row_start;
   const int32_t* lens;       // [B] tokens per batch row (right padding beyond), or null
   int block;                 // 1 = token-causal; 16, 32, 64, 128 = block-causal
   float power;               // stablemax exponent (stablemax encoder only)
@@ -70,8 +73,11 @@ int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide);
 // whatever instance the environment asks for (what a backward sizes by, see keep_layout)
 int prefill_tc_gate_stride(const flare_fwd_args_t* a, int nseg, bool wide);
 int prefill_tc_max_gate_stride(const flare_fwd_args_t* a);
-// launches segments 0 .. nseg_grid-1
-int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, bool wide, cudaStream_t stream);
+// rows of a masked call `a` can stay where they are: tiled copies can express the strides of its k, v and y
+bool prefill_tc_rows_in_place(const flare_fwd_args_t* a);
+// launches segments 0 .. nseg_grid-1; direct: the masked call whose packed copies `a` holds (with p.row_start, else null)
+int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, bool wide, const flare_fwd_args_t* direct,
+                      cudaStream_t stream);
 // device address (current device) of the error word shared by all tensor-core kernels
 int tc_error_word(int** device_address);
 // reads (and optionally clears) the device-side error flag of the tensor-core kernels; synchronises

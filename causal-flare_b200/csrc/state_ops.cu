@@ -140,15 +140,16 @@ __global__ void __launch_bounds__(256) cast_rows_kernel(const __grid_constant__ 
 }
 
 // One CTA per batch row: ranks by ballots within a warp, then over the warps.
-__global__ void __launch_bounds__(1024) mask_slots_kernel(const int* mask, int N, int* slot, int* lens) {
+__global__ void __launch_bounds__(1024) mask_slots_kernel(const int* mask, int N, int* slot, int* lens, int* start) {
   pdl_begin();
-  __shared__ int sums[32];
+  __shared__ int sums[32], firsts[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * N;
-  int base = 0;
+  int base = 0, first = N;  // first valid token among this thread's
   for (int n0 = 0; n0 < N; n0 += 1024) {
     const int n = n0 + threadIdx.x;
     const bool on = n < N && mask[row + n] != 0;
+    if (on && n < first) first = n;
     const unsigned votes = __ballot_sync(0xffffffffu, on);
     __syncthreads();  // (the sums of the tile before have been read)
     if (lane == 0) sums[warp] = __popc(votes);
@@ -162,51 +163,75 @@ __global__ void __launch_bounds__(1024) mask_slots_kernel(const int* mask, int N
     base += all;
   }
   if (threadIdx.x == 0) lens[blockIdx.x] = base;
+  if (start != nullptr) {
+    first = __reduce_min_sync(0xffffffffu, first);
+    if (lane == 0) firsts[warp] = first;
+    __syncthreads();
+    if (warp == 0) {
+      first = __reduce_min_sync(0xffffffffu, firsts[lane]);
+      if (lane == 0) start[blockIdx.x] = first == N - base ? first : -1;
+    }
+  }
 }
 
-// A streaming copy of 16-byte pieces, both tensors of a pack in one launch (blockIdx.y).  Bound by memory: every valid row is
-// read and written once.  One block per token, so that the index arithmetic is a few 32-bit operations.
-__global__ void __launch_bounds__(128) move_rows_kernel(const MoveRowsParams p) {
+// A streaming copy of 16-byte pieces, both tensors of a pack in one launch (blockIdx.z).  Bound by memory: every valid row is
+// read and written once.  One block takes kMoveTokens tokens of a batch row (blockIdx.y): a call whose rows all stay where
+// they are is a few hundred blocks that return at once, and the index arithmetic stays a few 32-bit operations.
+constexpr int kMoveTokens = 16;
+__global__ void __launch_bounds__(256) move_rows_kernel(const MoveRowsParams p) {
   pdl_begin();
-  const int w = blockIdx.y;
-  const int64_t bn = blockIdx.x;
-  const int b = (int)(bn / p.N), n = (int)(bn - (int64_t)b * p.N);
-  const int s = p.slot[bn];
+  const int w = blockIdx.z, b = blockIdx.y;
+  const int first = p.start != nullptr ? p.start[b] : -1;
+  const int n0 = blockIdx.x * kMoveTokens, n1 = min(p.N, n0 + kMoveTokens);
+  if (first >= 0 && (!p.unpack || n0 >= first)) return;
   const uint16_t* in = reinterpret_cast<const uint16_t*>(p.in[w]) + b * p.is_b[w];
   uint16_t* out = reinterpret_cast<uint16_t*>(p.out[w]) + b * p.os_b[w];
+  const int* slot = p.slot + (int64_t)b * p.N;
   const int c8n = p.d[w] >> 3, pieces = p.H * c8n;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   const int len = p.unpack ? 0 : p.lens[b];
-  const bool tail = !p.unpack && n >= len && n < (len + 127) / 128 * 128;
-  if (!p.unpack && s < 0 && !tail) return;
-  for (int i = threadIdx.x; i < pieces; i += 128) {
-    const int h = i / c8n, c = (i - h * c8n) * 8;
+  for (int i = threadIdx.x; i < (n1 - n0) * pieces; i += 256) {
+    const int t = i / pieces, n = n0 + t, r = i - t * pieces;
+    const int h = r / c8n, c = (r - h * c8n) * 8;
+    const int s = slot[n];
     const uint16_t* src = in + h * p.is_h[w] + c;
     uint16_t* dst = out + h * p.os_h[w] + c;
     if (p.unpack) {
-      *reinterpret_cast<uint4*>(dst + n * p.os_n[w]) = s >= 0 ? *reinterpret_cast<const uint4*>(src + s * p.is_n[w]) : zero;
+      if (s < 0) *reinterpret_cast<uint4*>(dst + n * p.os_n[w]) = zero;
+      else if (first < 0) *reinterpret_cast<uint4*>(dst + n * p.os_n[w]) = *reinterpret_cast<const uint4*>(src + s * p.is_n[w]);
     } else {
       if (s >= 0) *reinterpret_cast<uint4*>(dst + s * p.os_n[w]) = *reinterpret_cast<const uint4*>(src + n * p.is_n[w]);
-      if (tail) *reinterpret_cast<uint4*>(dst + n * p.os_n[w]) = zero;
+      if (n >= len && n < (len + 127) / 128 * 128) *reinterpret_cast<uint4*>(dst + n * p.os_n[w]) = zero;
     }
   }
 }
 
 }  // namespace
 
-int launch_mask_slots(const int* mask, int B, int N, int* slot, int* lens, cudaStream_t stream) {
+int launch_mask_slots(const int* mask, int B, int N, int* slot, int* lens, int* start, cudaStream_t stream) {
   LaunchTimer timer("mask_slots_kernel", stream);
-  FLARE_CUDA_CHECK(launch_pdl(mask_slots_kernel, dim3((unsigned)B), dim3(1024), 0, stream, mask, N, slot, lens));
+  FLARE_CUDA_CHECK(launch_pdl(mask_slots_kernel, dim3((unsigned)B), dim3(1024), 0, stream, mask, N, slot, lens, start));
   return FLARE_OK;
 }
 
 int launch_move_rows(const MoveRowsParams& p, int tensors, cudaStream_t stream) {
-  const int64_t tokens = (int64_t)p.B * p.N;
-  if (tokens > 0x7fffffff) return FLARE_ERR_UNSUPPORTED;
+  if ((int64_t)p.B * p.N > 0x7fffffff) return FLARE_ERR_UNSUPPORTED;
   for (int w = 0; w < tensors; ++w)
     if (p.d[w] % 8) return FLARE_ERR_BAD_SHAPE;
   LaunchTimer timer(p.unpack ? "move_rows_kernel (unpack)" : "move_rows_kernel (pack)", stream);
-  FLARE_CUDA_CHECK(launch_pdl(move_rows_kernel, dim3((unsigned)tokens, tensors), dim3(128), 0, stream, p));
+  const unsigned blocks = (unsigned)((p.N + kMoveTokens - 1) / kMoveTokens);
+  MoveRowsParams q = p;
+  for (int b0 = 0; b0 < p.B; b0 += 65535) {  // (what grid.y holds)
+    q.B = p.B - b0 < 65535 ? p.B - b0 : 65535;
+    FLARE_CUDA_CHECK(launch_pdl(move_rows_kernel, dim3(blocks, (unsigned)q.B, tensors), dim3(256), 0, stream, q));
+    q.slot += (int64_t)65535 * p.N;
+    if (q.lens != nullptr) q.lens += 65535;
+    if (q.start != nullptr) q.start += 65535;
+    for (int w = 0; w < tensors; ++w) {
+      q.in[w] = reinterpret_cast<const uint16_t*>(q.in[w]) + 65535 * p.is_b[w];
+      q.out[w] = reinterpret_cast<uint16_t*>(q.out[w]) + 65535 * p.os_b[w];
+    }
+  }
   return FLARE_OK;
 }
 

@@ -38,7 +38,9 @@ int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t s
 
 // Compaction of masked rows (2-byte elements, head widths that are multiples of 8, 16-byte aligned rows).
 // slot[b][n] = number of valid tokens before token n of row b, or -1 for a masked token; lens[b] = valid tokens of the row.
-int launch_mask_slots(const int* mask, int B, int N, int* slot, int* lens, cudaStream_t stream);
+// start (may be null): start[b] = N - lens[b] for a row whose valid tokens are its last ones (left padding, or none), else -1.
+int launch_mask_slots(const int* mask, int B, int N, int* slot, int* lens, int* start, cudaStream_t stream);
+// Rows with start[b] >= 0 (start may be null: none) stay where they are: pack skips them, unpack only zeroes their padding.
 // pack: out[b][slot[n]] = in[b][n] for the valid tokens of up to two tensors; rows lens[b] .. up to the end of their 128-token
 // chunk become zero, later rows stay as they are.  unpack: out[b][n] = in[b][slot[n]], zero for masked tokens.
 struct MoveRowsParams {
@@ -47,7 +49,7 @@ struct MoveRowsParams {
   int64_t is_b[2], is_n[2], is_h[2], os_b[2], os_n[2], os_h[2];
   int d[2];
   int B, N, H, unpack;
-  const int *slot, *lens;
+  const int *slot, *lens, *start;
 };
 int launch_move_rows(const MoveRowsParams& p, int tensors, cudaStream_t stream);
 

@@ -223,6 +223,15 @@ int flare_mask_pack(const int32_t* mask, const void* k, const int64_t k_strides_
 int flare_mask_unpack(const int32_t* slot, const void* y_in, void* y, const int64_t y_strides_bnh[3], int32_t B, int32_t N,
                       int32_t H, int32_t Dv, flare_stream_t stream);
 
+/*
+ * flare_forward, with masked calls on the tensor-core kernels wherever the same call without its mask would run there (no
+ * log-sum-exps wanted, no keep buffer).  What the two functions above do by hand happens inside, and a batch row whose valid
+ * tokens are its last ones (left padding, or none) is not copied at all.  Such calls have no exact kernels standing by.
+ * Everything else is flare_forward itself.  The workspace is that of flare_forward_masked_workspace_bytes.
+ */
+size_t flare_forward_masked_workspace_bytes(const flare_fwd_args_t* args);
+int flare_forward_masked(const flare_fwd_args_t* args, flare_stream_t stream);
+
 const char* flare_status_string(int status);
 const char* flare_last_cuda_error(void);
 /* Version of the structs and functions above.  It grows with every change that a caller compiled against an older header

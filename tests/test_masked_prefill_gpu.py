@@ -85,3 +85,45 @@ def test_rows_beyond_a_length_are_left_alone(monkeypatch, M, Dk, wide, dtype):
         assert torch.equal(y[b, n:], before[b, n:]), f"row {b}"
         if n:
             assert_bf16_gate(y[b:b + 1, :n], orc.ar_forward(q, k[b:b + 1, :n], v[b:b + 1, :n], scale=Dk ** -0.5), f"row {b}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("wide", [None, "1 merge kernel"])
+@pytest.mark.parametrize("B,N,H,M,D", [(3, 127, 2, 64, 64), (3, 128, 2, 128, 64), (3, 129, 1, 192, 64), (2, 513, 2, 128, 128),
+                                       (2, 300, 2, 256, 128), (2, 5000, 1, 64, 64)])
+def test_left_padded_rows_stay_where_they_are(monkeypatch, B, N, H, M, D, wide, dtype):
+    # y of the valid tokens and the state agree with those of the unpadded prompts on their own, and the padding, whatever it
+    # holds, is not touched.  Edges of a chunk, latent groups (their merge kernel moves the rows), wide heads, a carried
+    # state, sequence segments, an output in another layout.
+    choose(monkeypatch, wide)
+    q, k, v = orc.make_inputs(B, N, H, M, D, seed0=13, dtype=dtype)
+    pads = [0, N // 3, N - 1][:B]
+    mask = (torch.arange(N)[None, :] >= torch.tensor(pads)[:, None]).cuda()
+    qc, kc, vc = to_dev(q, k, v)
+    _, st0 = cf.flare_autoregressive_prefill_triton(qc, kc[:, :40], vc[:, :40], scale=D ** -0.5)
+    kc, vc = kc.masked_fill(~mask[..., None, None], float("nan")), vc.masked_fill(~mask[..., None, None], float("inf"))
+    for bhnd in (False, True):
+        if bhnd:
+            kc, vc = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (kc, vc))
+        y, st, _, _ = _ops.forward(qc, kc, vc, scale=D ** -0.5, mask=mask, state_in=st0, want_state=True, out_bhnd=bhnd)
+        y = y.transpose(1, 2) if bhnd else y
+        for b, pad in enumerate(pads):
+            assert not y[b, :pad].any()
+            one = {key: t[b:b + 1] for key, t in st0.items()}
+            ref, ref_st = cf.flare_autoregressive_prefill_triton(qc, kc[b:b + 1, pad:].contiguous(), vc[b:b + 1, pad:].contiguous(),
+                                                                 state=one, scale=D ** -0.5)
+            # (another number of segments sums in another order, one rounding of the 16-bit outputs and operands apart)
+            assert_bf16_gate(y[b:b + 1, pad:], ref, f"row {b}")
+            assert_bf16_gate((st["u"] / st["d"][..., None])[b:b + 1], ref_st["u"] / ref_st["d"][..., None], f"state {b}")
+
+
+def test_masked_fp16_with_a_bank_expanded_over_the_heads():
+    # (a stride of zero, which no tiled copy can express: bf16 copies of the packed rows)
+    B, N, H, M, D = 2, 200, 2, 64, 64
+    q, k, v = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=14, dtype=torch.float16))
+    mask = torch.rand(B, N, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) < 0.7
+    shared = q[:1].expand(H, M, D)
+    a = cf.flare_autoregressive_prefill_triton(shared, k, v, scale=D ** -0.5, attention_mask=mask)
+    b = cf.flare_autoregressive_prefill_triton(shared.contiguous(), k, v, scale=D ** -0.5, attention_mask=mask)
+    assert_bf16_gate(a[0], b[0], "y")
+    assert_bf16_gate(a[1]["u"] / a[1]["d"][..., None], b[1]["u"] / b[1]["d"][..., None], "state")
