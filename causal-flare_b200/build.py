@@ -28,6 +28,7 @@ UNITS = [
     ("walk_exact.cu", [], "walk_exact_dispatch"),
     *[("walk_exact.cu", [f"-DFLARE_WALK_MM={mm}"], f"walk_exact_mm{mm}") for mm in (2, 8, 16, 32, 64)],
     ("narrow_exact.cu", [], "narrow_exact"),
+    ("narrow_mma.cu", [], "narrow_mma"),
     ("decode_step.cu", [], "decode_step"),
     ("state_ops.cu", [], "state_ops"),
     ("prefill_tc.cu", [], "prefill_tc_host"),

@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include "narrow_exact.cuh"
+#include "narrow_mma.cuh"
 #include "walk_device.cuh"
 #include "walk_exact.cuh"
 
@@ -1147,14 +1148,18 @@ __global__ void __launch_bounds__(256) bwd_seg_scan_kernel(float* seg_b, float* 
   }
 }
 
+constexpr size_t kGateBytes = 256;
+
 size_t bwd_exact_workspace_bytes(const flare_bwd_args_t& a) {
   if (a.fwd.B == 0 || a.fwd.N == 0) return 0;
-  return plan_backward(a).total;
+  const size_t exact = plan_backward(a).total;
+  if (!narrow_mma_backward_supported(a)) return exact;
+  const size_t mma = narrow_mma_backward_bytes(a);  // (shares its space with the pass standing by; the gate word comes first)
+  return kGateBytes + (mma > exact ? mma : exact);
 }
 
 static int bwd_narrow(const flare_bwd_args_t& a, const BwdPlan& pl, cudaStream_t stream, const int* gate) {
   const flare_fwd_args_t& f = a.fwd;
-  if (gate != nullptr) return FLARE_ERR_UNSUPPORTED;  // (never: the tensor kernels, which it gates, take no narrow heads)
   char* ws = reinterpret_cast<char*>(f.workspace);
   auto at = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
   NarrowBwdParams p;
@@ -1169,12 +1174,13 @@ static int bwd_narrow(const flare_bwd_args_t& a, const BwdPlan& pl, cudaStream_t
   p.E = at(pl.off_E); p.G = at(pl.off_G); p.W2 = at(pl.off_W2); p.P = at(pl.off_P);
   p.seg_len = pl.seg_len; p.nseg = pl.nseg;
   p.dk = a.dk; p.dv = a.dv; p.dq_part = at(pl.off_part_q);
+  p.gate = gate;
   int rc;
   if (pl.nseg > 1) {
     p.in_m = at(pl.off_seg_m); p.in_d = at(pl.off_seg_d); p.in_u = at(pl.off_seg_u);
     p.seg_b = at(pl.off_seg_b); p.seg_c = at(pl.off_seg_c); p.seg_gam = at(pl.off_seg_gam);
     rc = segment_prefix_states(&f, pl.nseg, pl.seg_len, at(pl.off_seg_m), at(pl.off_seg_d), at(pl.off_seg_u), nullptr, stream,
-                               nullptr);
+                               gate);
     if (rc != FLARE_OK) return rc;
   }
   rc = launch_narrow_replay(p, stream);
@@ -1184,14 +1190,14 @@ static int bwd_narrow(const flare_bwd_args_t& a, const BwdPlan& pl, cudaStream_t
     LaunchTimer timer("bwd_seg_scan_kernel", stream);
     FLARE_CUDA_CHECK(launch_pdl(bwd_seg_scan_kernel, dim3((unsigned)((nscan + 255) / 256)), dim3(256), 0, stream, p.seg_b, p.seg_c,
                                 p.seg_gam, pl.nseg, pl.seg_len, lanes, f.N, f.M, f.Dv, p.E, nullptr, 1, nullptr, nullptr, nullptr,
-                                1, nullptr, nullptr, nullptr, nullptr, nullptr));
+                                1, nullptr, nullptr, nullptr, nullptr, gate));
   }
   rc = launch_narrow_reverse(p, stream);
   if (rc != FLARE_OK) return rc;
   const int64_t lat_n = (int64_t)f.H * f.M * f.Dk;
   LaunchTimer timer("bwd_sum_splits_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(bwd_sum_splits_kernel, dim3((unsigned)((lat_n + 255) / 256)), dim3(256), 0, stream, a.dq, a.dq_dtype,
-                              p.dq_part, lat_n, f.B * pl.nseg, nullptr));
+                              p.dq_part, lat_n, f.B * pl.nseg, gate));
   return FLARE_OK;
 }
 
@@ -1199,6 +1205,19 @@ int bwd_exact(const flare_bwd_args_t& a, cudaStream_t stream, const int* gate) {
   const flare_fwd_args_t& f = a.fwd;
   if (f.B == 0 || f.N == 0) return FLARE_OK;
   if (f.M > 512) return FLARE_ERR_UNSUPPORTED;
+  if (gate == nullptr && narrow_mma_backward_supported(a)) {
+    if (f.workspace == nullptr || f.workspace_bytes < bwd_exact_workspace_bytes(a) || (reinterpret_cast<uintptr_t>(f.workspace) & 15u))
+      return FLARE_ERR_WORKSPACE;
+    char* ws = reinterpret_cast<char*>(f.workspace);
+    int* word = reinterpret_cast<int*>(ws);
+    const int rc = narrow_mma_backward(a, ws + kGateBytes, word, stream);
+    if (rc != FLARE_OK) return rc;
+    flare_bwd_args_t ex = a;  // standing by: every kernel returns at once unless the word is set
+    ex.fwd.path = FLARE_PATH_EXACT;
+    ex.fwd.workspace = ws + kGateBytes;
+    ex.fwd.workspace_bytes = f.workspace_bytes - kGateBytes;
+    return bwd_exact(ex, stream, word);
+  }
   const BwdPlan pl = plan_backward(a);
   if (f.workspace == nullptr || f.workspace_bytes < pl.total || (reinterpret_cast<uintptr_t>(f.workspace) & 15u))
     return FLARE_ERR_WORKSPACE;

@@ -8,6 +8,7 @@
 #include "decode_step.cuh"
 #include "flare_common.cuh"
 #include "narrow_exact.cuh"
+#include "narrow_mma.cuh"
 #include "prefill_tc.cuh"
 #include "state_ops.cuh"
 #include "walk_exact.cuh"
@@ -159,6 +160,7 @@ struct FwdPlan {
   // runs the exact kernels for the flagged lanes.
   int gate_stride;
   size_t gate_off, gate_bytes;
+  bool narrow_mma;  // narrow heads on the tensor cores (narrow_mma.cu), with gate words as above
 };
 
 // fp16 calls may run on the tensor kernels (FLARE_B200_FP16_TENSOR=0 keeps them on the exact ones, which multiply q, k, v at
@@ -169,7 +171,7 @@ bool f16_on_tensor_kernels() {
 }
 
 FwdPlan plan_forward(const flare_fwd_args_t* a) {
-  FwdPlan pl{false, false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, false, 1, a->N > 0 ? a->N : 1, 0, 0, 0, 0, 0, 0, 0, false};
   if (a->B == 0 || a->N == 0) return pl;
   const int64_t lanes = (int64_t)a->B * a->H;
   pl.state_floats = (size_t)2 * a->M + (size_t)a->M * a->Dv;
@@ -192,6 +194,17 @@ FwdPlan plan_forward(const flare_fwd_args_t* a) {
       pl.gate_bytes = align_up((size_t)(1 + lanes * pl.gate_stride) * sizeof(int), 256);
       pl.ws_bytes += pl.gate_bytes;
     }
+    return pl;
+  }
+  if (narrow_mma_forward_supported(a) && align_up((size_t)(1 + lanes) * sizeof(int), 256) <= scratch_left(0)) {
+    const size_t room = scratch_left(0) / ((size_t)lanes * pl.state_floats * 4);
+    pl.narrow_mma = true;
+    narrow_mma_segments(lanes, a->N, a->M, false, room < 1 ? 1 : (room > 64 ? 64 : (int64_t)room), &pl.nseg, &pl.seg_len);
+    pl.ws_bytes = pl.nseg > 1 ? align_up((size_t)lanes * pl.nseg * pl.state_floats * 4, 256) : 0;
+    pl.gate_stride = pl.nseg;
+    pl.gate_off = pl.ws_bytes;
+    pl.gate_bytes = align_up((size_t)(1 + lanes * pl.nseg) * sizeof(int), 256);
+    pl.ws_bytes += pl.gate_bytes;
     return pl;
   }
   if (narrow_shape(a->M, a->Dk, a->Dv, a->block_size, a->q_dec != nullptr || a->k_dec != nullptr)) {
@@ -334,6 +347,12 @@ int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaSt
   if (pl.ws_bytes > 0 && (a->workspace == nullptr || a->workspace_bytes < pl.ws_bytes || !aligned16(a->workspace)))
     return FLARE_ERR_WORKSPACE;
   const int64_t lanes = (int64_t)a->B * a->H;
+  if (pl.narrow_mma) {
+    float* const seg_m = reinterpret_cast<float*>(a->workspace);
+    float* const seg_d = seg_m + (size_t)lanes * pl.nseg * a->M;
+    g_last_launches = pl.nseg > 1 ? 2 : 1;
+    return narrow_mma_forward(*a, seg_m, seg_d, seg_d + (size_t)lanes * pl.nseg * a->M, pl.nseg, pl.seg_len, g_gate, stream);
+  }
   const bool have_out = a->state_out.u != nullptr;
   WalkParams w;
   fill_walk(w, a);
@@ -575,7 +594,7 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
   memset(&a.state_in, 0, sizeof(a.state_in));
   memset(&a.state_out, 0, sizeof(a.state_out));
   a.state_out.m = seg_m; a.state_out.d = seg_d; a.state_out.u = seg_u;  // marks "a state is wanted" for the checks
-  FwdPlan pl{false, false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0};
+  FwdPlan pl{false, false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0, false};
   pl.use_tc = a.path != FLARE_PATH_EXACT && (seg_len % 128) == 0 && prefill_tc_supported(&a);
   const int64_t lanes = (int64_t)a.B * a.H;
   if (pl.use_tc) {

@@ -9,7 +9,8 @@
 // and 3 shuffles for 4 columns.  The per-latent statistics run with one latent per lane.  The latents of a warp are
 // touched by no other warp, so only the decode softmax and the cross-latent sums need CTA barriers.
 // Bound by the latency and issue of the fp32 passes; one CTA (M / 32 warps) per (lane, segment), segments so short that
-// about twelve warps per SM are in flight.  B200: training step B=8 N=2048 H=16 M=64 D=32 4007 us with the general kernels,
+// about twelve warps per SM are in flight.  bf16 softmax calls run on the tensor cores at the same precision (narrow_mma.cu);
+// these kernels serve the rest (fp32, fp16, stablemax, states, masks) and stand by behind those.  B200: training step B=8 N=2048 H=16 M=64 D=32 4007 us with the general kernels,
 // 1823 us with these.
 #include "narrow_exact.cuh"
 
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(128, 4) walk_narrow_kernel(const WalkParams p)
 template <bool STABLE>
 __global__ void __launch_bounds__(128, 3) narrow_replay_kernel(const NarrowBwdParams p) {
   pdl_begin();
+  if (p.gate != nullptr && *p.gate == 0) return;
   extern __shared__ __align__(16) float smem_raw[];
   const int nw = blockDim.x >> 5, ms = nw * 32;
   float* ks = smem_raw;
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(128, 3) narrow_replay_kernel(const NarrowBwdPa
 template <bool STABLE>
 __global__ void __launch_bounds__(128, 4) narrow_reverse_kernel(const NarrowBwdParams p) {
   pdl_begin();
+  if (p.gate != nullptr && *p.gate == 0) return;
   extern __shared__ __align__(16) float smem_raw[];
   const int nw = blockDim.x >> 5, ms = nw * 32;
   float* ks = smem_raw;

@@ -28,6 +28,7 @@ struct NarrowBwdParams {
   float *seg_b, *seg_c, *seg_gam;    // replay: carries of the segment alone; reverse: the carries that enter it
   void *dk, *dv;                     // [B, N, H, D] contiguous, input dtype
   float* dq_part;                    // [B * nseg][H][M][Dk]
+  const int* gate;                   // optional: nothing is done unless *gate != 0
 };
 int launch_narrow_replay(const NarrowBwdParams& p, cudaStream_t stream);
 int launch_narrow_reverse(const NarrowBwdParams& p, cudaStream_t stream);

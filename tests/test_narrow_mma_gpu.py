@@ -1,0 +1,76 @@
+"""Narrow heads on the tensor cores (bf16, softmax): as close to 64 bits as the fp32 kernels, and theirs where it leaves its domain."""
+import pytest
+import torch
+
+import causal_flare as cf
+from oracle import flare_oracle as orc
+from util import to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def step(monkeypatch, path, q, k, v, dy):
+    monkeypatch.setenv("FLARE_B200_PATH", path)
+    ql, kl, vl = (t.detach().requires_grad_() for t in (q, k, v))
+    y = cf.flare_autoregressive_triton(ql, kl, vl)
+    return (y.detach(),) + torch.autograd.grad(y, (ql, kl, vl), dy)
+
+
+# one token; a tile of 16 and its neighbours; a block of 32 and its neighbours; the second segment's first token; a ragged end of
+# many segments; one warp, an odd number of warps and eight of them; unequal widths; more lanes than are cut into segments
+SHAPES = [(1, 1, 1, 16, 16, 16), (2, 15, 2, 32, 32, 32), (1, 16, 3, 48, 16, 32), (1, 17, 1, 64, 32, 16), (2, 31, 1, 128, 32, 32),
+          (1, 33, 2, 96, 32, 32), (1, 65, 2, 64, 32, 32), (1, 1999, 2, 80, 32, 32), (2, 1024, 2, 128, 32, 16), (40, 130, 16, 32, 32, 32)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_no_further_from_64_bits_than_the_fp32_kernels(monkeypatch, shape):
+    # Both round the same sums to bf16.  Operands of the products carry 16 mantissa bits: 2^-17 relative per factor, against
+    # 2^-9 of the outputs' own rounding, so the two distances differ by what roundings that fall the other way make of it: below
+    # 1 % of the distance plus, for outputs of few entries, a fraction of one rounding.
+    B, N, H, M, Dk, Dv = shape
+    q, k, v, dy = orc.make_inputs(B, N, H, M, Dk, Dv, seed0=21, dtype=torch.bfloat16, with_dy=True)
+    n = min(B, 2)
+    if B > 2:  # equal batch rows: the oracle looks at the first ones
+        k, v, dy = (t.clone() for t in (k, v, dy))
+        k[1:], v[1:], dy[1:] = k[:1], v[:1], dy[:1]
+    y_ref = orc.ar_forward(q, k[:n], v[:n])
+    ref = orc.ar_backward_closed_form(q, k[:n], v[:n], dy[:n])
+    want = (y_ref, ref["dQ"], ref["dK"], ref["dV"])
+    got = {path: step(monkeypatch, path, *to_dev(q, k, v, dy)) for path in ("auto", "exact")}
+    for i, name in enumerate(("y", "dQ", "dK", "dV")):
+        err = {}
+        for path, out in got.items():
+            x = out[i].float().cpu()
+            x = x * (n / B) if name == "dQ" else x[:n]
+            # (a single token has no gradient but dV: what is left there are differences of equal fp32 numbers)
+            err[path] = orc.rel_l2(x, want[i]) if N > 1 or name in ("y", "dV") else orc.max_abs(x, want[i])
+        assert err["auto"] <= 1.01 * err["exact"] + 2.0 ** -9 / want[i].numel() ** 0.5 + 1e-5, f"{name}: {err}"
+
+
+@pytest.mark.parametrize("std", [4.0, 24.0])
+def test_sharp_scores(monkeypatch, std):
+    # at 24 the running maximum grows by hundreds of powers of two inside tiles: the fp32 kernels standing by redo those lanes
+    B, N, H, M, D = 2, 200, 4, 32, 32
+    q, k, v, dy = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=22, dtype=torch.bfloat16, with_dy=True))
+    a, b = (step(monkeypatch, path, q * std, k, v, dy) for path in ("auto", "exact"))
+    for name, x, y in zip(("y", "dQ", "dK", "dV"), a, b):
+        assert torch.isfinite(x.float()).all(), name
+        assert orc.rel_l2(x.float().cpu(), y.float().cpu()) <= 2.0 ** -8, name
+
+
+@pytest.mark.parametrize("where", ["v", "k"])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(monkeypatch, where):
+    B, N, H, M, D = 1, 100, 2, 64, 32
+    q, k, v, dy = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=23, dtype=torch.bfloat16, with_dy=True))
+    (v if where == "v" else k)[0, 43, 1, 5] = float("inf")
+    a, b = (step(monkeypatch, path, q, k, v, dy)[0] for path in ("auto", "exact"))
+    assert torch.isfinite(a[:, :43].float()).all() and torch.isfinite(a[:, :, 0].float()).all()
+    assert torch.equal(torch.isfinite(a), torch.isfinite(b))
+
+
+def test_head_slices(monkeypatch):
+    B, N, H, M, D = 2, 300, 3, 64, 32
+    q, k, v, dy = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=24, dtype=torch.bfloat16, with_dy=True))
+    k2, v2, dy2 = (torch.cat([t, t], dim=2)[:, :, :H] for t in (k, v, dy))
+    for x, y in zip(step(monkeypatch, "auto", q, k, v, dy), step(monkeypatch, "auto", q, k2, v2, dy2)):
+        assert torch.equal(x, y)
