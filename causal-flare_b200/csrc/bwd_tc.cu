@@ -41,7 +41,7 @@ using tc::bf16_hi;
 using tc::bf16_lo;
 using tc::kmaj_step;
 using tc::mnmaj_step;
-using tc::sigma_fast;
+using tc::sigma8;
 using tc::swz_chunk_off;
 using tc::warp_arrive;
 
@@ -144,10 +144,23 @@ __device__ __forceinline__ float unpack8(const uint4& v, int j) {
   return (j & 1) ? bf16_hi(w) : bf16_lo(w);
 }
 // slope sigma'(s) / sigma(s) = p / (1 + |s|) recovered from the (rounded) weight: 1 + |s| = E^(1/p) for s >= 0
-// (E >= 1) and E^(-1/p) for s < 0
-__device__ __forceinline__ float slope_from_sigma(float e, float p) {
-  const float l = __log2f(e) * (1.0f / p);
-  return p * ex2_approx(e >= 1.0f ? -l : l);
+// (E >= 1) and E^(-1/p) for s < 0; eight weights at a time, so that the power is looked at once for all of them.  The default
+// power takes one reciprocal square root instead of a logarithm and an exponential (a weight of zero stays a slope of zero).
+__device__ __forceinline__ void slope8_from_sigma(const float (&e)[8], float p, float (&slope)[8]) {
+  if (p == 2.0f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float r = rsqrtf(fmaxf(e[j], 1e-37f));
+      slope[j] = 2.0f * (e[j] >= 1.0f ? r : e[j] * r);
+    }
+  } else {
+    const float inv_p = 1.0f / p;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float l = __log2f(e[j]) * inv_p;
+      slope[j] = p * ex2_approx(e[j] >= 1.0f ? -l : l);
+    }
+  }
 }
 
 }  // namespace
@@ -521,13 +534,17 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch) {
           float e[8];
+          if constexpr (STABLE) {
+            float x[8];
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) x[jj] = __uint_as_float(rs[ch * 8 + jj]) * p.scale;
+            sigma8(x, p.power, e);
+          }
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
             const int k = ch * 8 + jj;
-            const float sv = __uint_as_float(rs[k]);
-            float x = STABLE ? sigma_fast(sv * p.scale, p.power) : ex2_approx(fmaf(sv, sc2, -c_i));
-            if (!fast) x = k < lim ? x : 0.f;
-            e[jj] = x;
+            if constexpr (!STABLE) e[jj] = ex2_approx(fmaf(__uint_as_float(rs[k]), sc2, -c_i));
+            if (!fast) e[jj] = k < lim ? e[jj] : 0.f;
           }
           uint4 v;
           v.x = pack_bf16(e[0], e[1]); v.y = pack_bf16(e[2], e[3]); v.z = pack_bf16(e[4], e[5]); v.w = pack_bf16(e[6], e[7]);
@@ -686,12 +703,15 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
             for (int c2 = 1; c2 >= 0; --c2) {
               const int ch = blk * 2 + c2;
               const uint4 ev = *reinterpret_cast<const uint4*>(e_row + swz_chunk_off(m, ch0 + ch));
-              float ds[8];
+              float ds[8], e8[8], slope[8];
+#pragma unroll
+              for (int jj = 0; jj < 8; ++jj) e8[jj] = unpack8(ev, jj);
+              if constexpr (STABLE) slope8_from_sigma(e8, p.power, slope);
 #pragma unroll
               for (int jj = 7; jj >= 0; --jj) {
                 const int k = ch * 8 + jj;
                 const float x = __uint_as_float(xr[c2 * 8 + jj]);
-                const float eb = unpack8(ev, jj);
+                const float eb = e8[jj];
                 float csub;
                 if constexpr (BLOCK) {
                   csub = ccg[ch >> 1];
@@ -701,7 +721,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                   csub = cc;
                 }
                 float enc = eb * (x - csub);
-                if constexpr (STABLE) enc *= slope_from_sigma(eb, p.power);
+                if constexpr (STABLE) enc *= slope[jj];
                 ds[jj] = __uint_as_float(pd[k]) + ((STABLE && eb == 0.f) ? 0.f : enc);
               }
               // dS = hi + lo, two bf16 values: the dK / dQ products then see it with 16 mantissa bits

@@ -136,7 +136,7 @@ struct Misc {
 
 using tc::swz_chunk_off;
 using tc::warp_arrive;
-using tc::sigma_fast;
+using tc::sigma8;
 
 // bounded wait that also gives up as soon as another role of the CTA has given up
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, Misc* misc) {
@@ -694,16 +694,23 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if constexpr (PACK) *reinterpret_cast<uint4*>(e_row + 8192 + swz_chunk_off(m, ch0 + ch)) = v;
       };
       if constexpr (STABLE) {
-        // encoder weights sigma(s): packed and stored 8 tokens at a time; the raw scores stay in ra / rb for phase b
+        // encoder weights sigma(s): packed and stored 8 tokens at a time; the raw scores stay in ra / rb for phase b (packed:
+        // rb is free there and keeps the weights)
 #pragma unroll
         for (int ch = 0; ch < TOK / 8; ++ch) {
-          float sg[8];
+          float sg[8], x[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float raw = __uint_as_float(ch < 4 ? ra[ch * 8 + j] : rb[(ch - 4) * 8 + j]);
             if (tok0 + ch * 8 + j < nvalid) cma = fmaxf(cma, raw * sc2 - c_new);
-            sg[j] = (tok0 + ch * 8 + j < nvalid) ? sigma_fast(raw * p.scale, p.power) : 0.f;
+            x[j] = raw * p.scale;
+          }
+          sigma8(x, p.power, sg);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (tok0 + ch * 8 + j >= nvalid) sg[j] = 0.f;
             tot0 += sg[j];
+            if constexpr (PACK) rb[ch * 8 + j] = __float_as_uint(sg[j]);
           }
           store_e(ch, make_uint4(pack_bf16(sg[0], sg[1]), pack_bf16(sg[2], sg[3]), pack_bf16(sg[4], sg[5]), pack_bf16(sg[6], sg[7])));
         }
@@ -818,24 +825,31 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (state_only) {
         // no read-out: R is not needed
       } else if constexpr (STABLE) {
-        // phase b, stablemax: D = running sum of sigma (recomputed), decode numerator exp2(s - c) a_m, R = numerator / D
+        // phase b, stablemax: D = running sum of sigma (kept, or recomputed), decode numerator exp2(s - c) a_m, R = numerator / D
 #pragma unroll
-        for (int blk = 0; blk < TOK / 32; ++blk) {
-          uint32_t rp[16];
+        for (int ch = 0; ch < TOK / 8; ++ch) {
+          float s[8], sg[8], r[8];
 #pragma unroll
-          for (int k = 0; k < 32; k += 2) {
-            const float s0 = __uint_as_float(blk ? rb[k] : ra[k]), s1 = __uint_as_float(blk ? rb[k + 1] : ra[k + 1]);
-            const int tk = tok0 + blk * 32 + k;
-            run += (tk < nvalid) ? sigma_fast(s0 * p.scale, p.power) : 0.f;
-            const float r0 = ex2_approx(s0 * sc2 - c_new) * (a_m * rcp_approx(run));
-            run += (tk + 1 < nvalid) ? sigma_fast(s1 * p.scale, p.power) : 0.f;
-            const float r1 = ex2_approx(s1 * sc2 - c_new) * (a_m * rcp_approx(run));
-            rp[k >> 1] = pack_bf16(r0, r1);
+          for (int j = 0; j < 8; ++j) s[j] = __uint_as_float(ch < 4 ? ra[ch * 8 + j] : rb[(ch - 4) * 8 + j]);
+          if constexpr (PACK) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sg[j] = __uint_as_float(rb[ch * 8 + j]);
+          } else {
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = s[j] * p.scale;
+            sigma8(x, p.power, sg);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (tok0 + ch * 8 + j >= nvalid) sg[j] = 0.f;
           }
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch)
-            *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + blk * 4 + ch)) =
-                make_uint4(rp[ch * 4], rp[ch * 4 + 1], rp[ch * 4 + 2], rp[ch * 4 + 3]);
+          for (int j = 0; j < 8; ++j) {
+            run += sg[j];
+            r[j] = ex2_approx(s[j] * sc2 - c_new) * (a_m * rcp_approx(run));
+          }
+          *reinterpret_cast<uint4*>(r_row + swz_chunk_off(m, ch0 + ch)) =
+              make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7]));
         }
       } else if constexpr (!BLOCK) {
         // phase b: D = running denominator, R = E a_m / D, R operand rows.  Reciprocals run on the special-function

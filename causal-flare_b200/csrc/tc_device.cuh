@@ -63,6 +63,22 @@ __device__ __forceinline__ float sigma_fast(float x, float p) {
   return x >= 0.0f ? r : rcp_approx(r);
 }
 
+// The weights of eight scores.  The power is the same for a whole launch, but a test of it for every element stays a branch
+// for every element: it is taken once here, with the operator's default power in line.  B200, training steps with the default
+// power: B=4 N=4096 H=16 M=64 D=128 560 -> 470 us, B=8 N=2048 H=16 M=128 D=64 589 -> 462 us (with the slopes of the backward).
+__device__ __forceinline__ void sigma8(const float (&x)[8], float p, float (&w)[8]) {
+  if (p == 2.0f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float base = 1.0f + fabsf(x[j]), r = base * base;
+      w[j] = x[j] >= 0.0f ? r : rcp_approx(r);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = sigma_fast(x[j], p);
+  }
+}
+
 __device__ __forceinline__ float bf16_lo(uint32_t pk) { return __uint_as_float(pk << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t pk) { return __uint_as_float(pk & 0xffff0000u); }
 
