@@ -73,7 +73,7 @@ int prefill_tc_grid_z(const flare_fwd_args_t* a, bool wide);
 // whatever instance the environment asks for (what a backward sizes by, see keep_layout)
 int prefill_tc_gate_stride(const flare_fwd_args_t* a, int nseg, bool wide);
 int prefill_tc_max_gate_stride(const flare_fwd_args_t* a);
-// rows of a masked call `a` can stay where they are: tiled copies can express the strides of its k, v and y
+// rows of a masked call can stay where they are: tiled copies can express the strides of its k, v and y (a: without the mask)
 bool prefill_tc_rows_in_place(const flare_fwd_args_t* a);
 // launches segments 0 .. nseg_grid-1; direct: the masked call whose packed copies `a` holds (with p.row_start, else null)
 int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p, int nseg_grid, bool wide, const flare_fwd_args_t* direct,
