@@ -38,6 +38,7 @@ UNITS = [
     *[("bwd_tc.cu", [f"-DFLARE_BT_UNIT={u}"], f"bwd_tc_unit{u}") for u in range(6)],
     ("bwd_exact.cu", [], "bwd_exact_dispatch"),
     *[("bwd_exact.cu", [f"-DFLARE_WALK_MM={mm}"], f"bwd_exact_mm{mm}") for mm in (2, 8, 16, 32, 64)],
+    *[("bwd_standby.cu", [f"-DFLARE_WALK_MM={mm}"], f"bwd_standby_mm{mm}") for mm in (64, 32, 16, 8, 2)],
 ]
 
 

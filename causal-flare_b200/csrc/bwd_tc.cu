@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
                                                                   int64_t y_sn, int64_t y_sh, const float* lse,
                                                                   int B, int N, int H, int Dv, int npad, float* tok_l2,
                                                                   float* tok_delta, const int* fwd_gate,
-                                                                  int fwd_gate_words, int* gate) {
+                                                                  int fwd_gate_words, int* gate, int* sync) {
   pdl_begin();
   __shared__ float delta_s[ST_HEADS][ST_TOK + 1];
   if (blockIdx.x == 0) {
@@ -983,6 +983,7 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
     for (int i = threadIdx.x; i < words; i += 256) raised |= fwd_gate[1 + i];
     raised = __syncthreads_or(raised);
     if (threadIdx.x == 0) *gate = raised ? 1 : 0;
+    if (threadIdx.x < kBwdSyncWords) sync[threadIdx.x] = 0;
   }
   // Dv / 8 threads per (token, head) row (8 or 16, a divisor of the warp size), one 16-byte piece of dY and of y each
   const int tpr = Dv >> 3, rows_per_pass = 256 / tpr;
@@ -1377,7 +1378,8 @@ TcBwdPlan plan_tc(const flare_bwd_args_t& a) {
   const bool saved = have_saved(a);
   pl.fwd_ws = saved ? 0 : align_up(flare_forward_workspace_bytes(&probe), 256);
   pl.gate_words = saved ? 1 : forward_gate_words(&probe);
-  pl.gate_bytes = align_up(pl.gate_words * sizeof(int), 256);
+  // (and the counters of the pass standing by, 256 bytes that the token statistics zero)
+  pl.gate_bytes = align_up(pl.gate_words * sizeof(int), 256) + 256;
   size_t off = pl.gate_bytes + pl.fwd_ws;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -1474,6 +1476,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
   char* ws = reinterpret_cast<char*>(f.workspace);
   const int64_t lanes = (int64_t)f.B * f.H;
   int* gate = reinterpret_cast<int*>(ws);
+  int* sync = reinterpret_cast<int*>(ws + pl.gate_bytes - 256);
   const bool saved = have_saved(a);
   const int* fwd_gate;
   int fwd_gate_words;
@@ -1522,7 +1525,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     FLARE_CUDA_CHECK(launch_pdl(bwd_tc_token_stats_kernel, dim3((unsigned)(pl.npad / ST_TOK) * (unsigned)f.B), dim3(256), 0, stream,
                                 reinterpret_cast<const __nv_bfloat16*>(a.dy), a.dy_stride_b, a.dy_stride_n, a.dy_stride_h,
                                 reinterpret_cast<const __nv_bfloat16*>(y), y_sb, y_sn, y_sh, lse, f.B, f.N, f.H, f.Dv, pl.npad,
-                                tok_l2, tok_delta, fwd_gate, fwd_gate_words, gate));
+                                tok_l2, tok_delta, fwd_gate, fwd_gate_words, gate, sync));
     count_launches(1);
   }
   int* err = nullptr;
@@ -1618,14 +1621,14 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
                                 f.B * pl.nsplit, n4, a.dq, a.dq_dtype));
     count_launches(2);
   }
-  // (5) path AUTO: the exact pass stands by.  Each of its kernels looks at the gate word and returns at once unless the
-  // tensor kernels above found the inputs outside their numeric domain, in which case it rewrites dq, dk, dv.
+  // (5) path AUTO: the exact pass stands by.  Its kernel looks at the gate word and returns at once unless the tensor
+  // kernels above found the inputs outside their numeric domain, in which case it rewrites dq, dk, dv.
   if (f.path == FLARE_PATH_AUTO) {
     flare_bwd_args_t ex = a;
     ex.fwd.path = FLARE_PATH_EXACT;
     ex.fwd.workspace = ws + pl.gate_bytes;
     ex.fwd.workspace_bytes = pl.total - pl.gate_bytes;
-    const int rc = bwd_exact(ex, stream, gate);
+    const int rc = bwd_exact(ex, stream, gate, sync);
     if (rc != FLARE_OK) return rc;
   }
   return FLARE_OK;

@@ -587,19 +587,46 @@ size_t forward_gate_words(const flare_fwd_args_t* a) {
   return 1 + (size_t)a->B * a->H * prefill_tc_max_gate_stride(a);
 }
 
+// a forward problem reduced to the states at its segment boundaries
+static void segment_states(const flare_fwd_args_t* f, int nseg, int seg_len, float* seg_m, float* seg_d, float* seg_u,
+                           const flare_state_t* init, flare_fwd_args_t* a, WalkParams* w, FoldParams* fp) {
+  *a = *f;
+  a->y = nullptr;
+  a->mask = nullptr;
+  a->lse_dec = a->lse_enc = nullptr;
+  a->block_size = 1;  // the state at a segment boundary does not depend on the read-out mode
+  memset(&a->state_in, 0, sizeof(a->state_in));
+  memset(&a->state_out, 0, sizeof(a->state_out));
+  a->state_out.m = seg_m; a->state_out.d = seg_d; a->state_out.u = seg_u;  // marks "a state is wanted" for the checks
+  fill_walk(*w, a);
+  w->seg_len = seg_len;
+  w->nseg_total = nseg;
+  w->y = nullptr; w->write_y = 0;
+  w->out_m = seg_m; w->out_d = seg_d; w->out_u = seg_u;
+  w->out_lane_stride = nseg; w->out_seg_stride = 1; w->out_mode = 1;
+  memset(fp, 0, sizeof(*fp));
+  if (init != nullptr) {
+    fp->a_m = init->m; fp->a_d = init->d; fp->a_u = init->u;
+  }
+  fp->s_m = seg_m; fp->s_d = seg_d; fp->s_u = seg_u;
+  fp->lane_stride = nseg; fp->seg_stride = 1; fp->count = nseg; fp->mode = 0;
+  fp->lanes = (int64_t)a->B * a->H; fp->M = a->M; fp->Dv = a->Dv; fp->stablemax = a->variant == FLARE_STABLEMAX;
+}
+
+void segment_state_params(const flare_fwd_args_t* f, int nseg, int seg_len, float* seg_m, float* seg_d, float* seg_u, WalkParams* w,
+                          FoldParams* fold) {
+  flare_fwd_args_t a;
+  segment_states(f, nseg, seg_len, seg_m, seg_d, seg_u, nullptr, &a, w, fold);
+}
+
 int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, float* seg_m, float* seg_d, float* seg_u,
                           const flare_state_t* init, cudaStream_t stream, const int* gate) {
-  flare_fwd_args_t a = *f;
-  a.y = nullptr;
-  a.mask = nullptr;
-  a.lse_dec = a.lse_enc = nullptr;
-  a.block_size = 1;  // the state at a segment boundary does not depend on the read-out mode
-  memset(&a.state_in, 0, sizeof(a.state_in));
-  memset(&a.state_out, 0, sizeof(a.state_out));
-  a.state_out.m = seg_m; a.state_out.d = seg_d; a.state_out.u = seg_u;  // marks "a state is wanted" for the checks
+  flare_fwd_args_t a;
+  WalkParams w;
+  FoldParams fp;
+  segment_states(f, nseg, seg_len, seg_m, seg_d, seg_u, init, &a, &w, &fp);
   FwdPlan pl{false, false, nseg, seg_len, (size_t)2 * a.M + (size_t)a.M * a.Dv, 0, 0, 0, 0, 0, 0, false};
   pl.use_tc = a.path != FLARE_PATH_EXACT && (seg_len % 128) == 0 && prefill_tc_supported(&a);
-  const int64_t lanes = (int64_t)a.B * a.H;
   if (pl.use_tc) {
     // the wide instance where the two-slice grid would not fit the SMs in one wave
     int n = 1;
@@ -607,26 +634,11 @@ int segment_prefix_states(const flare_fwd_args_t* f, int nseg, int seg_len, floa
     one.B = (int32_t)(a.B * nseg);
     prefill_tc_plan(&one, SIZE_MAX, &n, &pl.wide);
   }
-  WalkParams w;
-  fill_walk(w, &a);
-  w.seg_len = seg_len;
-  w.nseg_total = nseg;
-  w.y = nullptr; w.write_y = 0;
-  w.out_m = seg_m; w.out_d = seg_d; w.out_u = seg_u;
-  w.out_lane_stride = nseg; w.out_seg_stride = 1; w.out_mode = 1;
   w.gate = gate; w.gate_stride = 0; w.gate_count = 1;  // (a gated pass always runs on the exact kernels: its caller forces that path)
   if (nseg > 1) {
     const int rc = launch_walk(&a, pl, w, nseg - 1, stream);  // local states of all segments but the last
     if (rc != FLARE_OK) return rc;
   }
-  FoldParams fp;
-  memset(&fp, 0, sizeof(fp));
-  if (init != nullptr) {
-    fp.a_m = init->m; fp.a_d = init->d; fp.a_u = init->u;
-  }
-  fp.s_m = seg_m; fp.s_d = seg_d; fp.s_u = seg_u;
-  fp.lane_stride = nseg; fp.seg_stride = 1; fp.count = nseg; fp.mode = 0;
-  fp.lanes = lanes; fp.M = a.M; fp.Dv = a.Dv; fp.stablemax = a.variant == FLARE_STABLEMAX;
   fp.gate = gate;
   return launch_fold(fp, stream);  // exclusive scan from the initial (or empty) state
 }
