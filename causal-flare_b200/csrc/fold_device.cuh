@@ -5,7 +5,7 @@
 namespace flare {
 namespace fold {
 
-constexpr int DCH = 4;  // value columns per lane per pass (32 * DCH columns per pass)
+constexpr int DCH = 8;  // value columns per lane per pass (32 * DCH columns per pass)
 
 __device__ __forceinline__ void merge_factors(float ma, float mb, float& mn, float& fa, float& fb) {
   mn = fmaxf(ma, mb);
@@ -18,12 +18,10 @@ __device__ __forceinline__ void merge_factors(float ma, float mb, float& mn, flo
   }
 }
 
-// Bound by latency: every state waits for the one before it only in a few multiplications, but a loop that loads a state where
-// it needs it waits for memory `count` times.  The next kAhead states are in registers before they are folded.
-constexpr int kAhead = 4;
+// (The next four states fetched ahead measured the same at nine segments of 64 KB and 7 us slower at eight of 8 KB, where the
+// larger code has to come from memory for every call.)
 __device__ __forceinline__ void fold_row(const FoldParams& p, int64_t lane_id, int m, int lane) {
   const int M = p.M, Dv = p.Dv;
-  const int have = p.mode == 1 ? p.count : p.count - 1;  // states that are folded (a scan does not need the last)
   for (int dv0 = 0; dv0 < Dv; dv0 += 32 * DCH) {
     float rm = p.a_m ? p.a_m[lane_id * M + m] : (p.stablemax ? 0.f : kNegInf);
     float rd = p.a_d ? p.a_d[lane_id * M + m] : 0.f;
@@ -35,46 +33,39 @@ __device__ __forceinline__ void fold_row(const FoldParams& p, int64_t lane_id, i
     }
     // the statistics are rewritten only in the last column pass: earlier passes still need the originals
     const bool first = (dv0 + 32 * DCH >= Dv) && lane == 0;
-    for (int j0 = 0; j0 < p.count; j0 += kAhead) {
-      float bm[kAhead], bd[kAhead], bu[kAhead][DCH];
-#pragma unroll
-      for (int a = 0; a < kAhead; ++a) {
-        const int64_t sidx = lane_id * p.lane_stride + (int64_t)(j0 + a) * p.seg_stride;
-        const bool on = j0 + a < have;
-        bm[a] = on ? p.s_m[sidx * M + m] : kNegInf;
-        bd[a] = on ? p.s_d[sidx * M + m] : 0.f;
+    for (int j = 0; j < p.count; ++j) {
+      const int64_t sidx = lane_id * p.lane_stride + (int64_t)j * p.seg_stride;
+      const bool have_b = (p.mode == 1) || (j < p.count - 1);
+      float bm = kNegInf, bd = 0.f, bu[DCH];
+      if (have_b) {
+        bm = p.s_m[sidx * M + m];
+        bd = p.s_d[sidx * M + m];
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
           const int dv = dv0 + lane + 32 * c;
-          bu[a][c] = on && dv < Dv ? p.s_u[(sidx * M + m) * Dv + dv] : 0.f;
+          bu[c] = dv < Dv ? p.s_u[(sidx * M + m) * Dv + dv] : 0.f;
         }
       }
-      // all lanes of the warp have read the slots before anyone overwrites them
-      if (p.mode == 0) __syncwarp();
-#pragma unroll
-      for (int a = 0; a < kAhead; ++a) {
-        const int j = j0 + a;
-        if (j >= p.count) break;
-        if (p.mode == 0) {
-          const int64_t sidx = lane_id * p.lane_stride + (int64_t)j * p.seg_stride;
-          if (first) {
-            p.s_m[sidx * M + m] = rm;
-            p.s_d[sidx * M + m] = rd;
-          }
-#pragma unroll
-          for (int c = 0; c < DCH; ++c) {
-            const int dv = dv0 + lane + 32 * c;
-            if (dv < Dv) p.s_u[(sidx * M + m) * Dv + dv] = ru[c];
-          }
+      if (p.mode == 0) {
+        // all lanes of the warp have read slot j before anyone overwrites it
+        __syncwarp();
+        if (first) {
+          p.s_m[sidx * M + m] = rm;
+          p.s_d[sidx * M + m] = rd;
         }
-        if (j < have) {
-          float mn, fa, fb;
-          merge_factors(rm, bm[a], mn, fa, fb);
-          rm = mn;
-          rd = rd * fa + bd[a] * fb;
 #pragma unroll
-          for (int c = 0; c < DCH; ++c) ru[c] = ru[c] * fa + bu[a][c] * fb;
+        for (int c = 0; c < DCH; ++c) {
+          const int dv = dv0 + lane + 32 * c;
+          if (dv < Dv) p.s_u[(sidx * M + m) * Dv + dv] = ru[c];
         }
+      }
+      if (have_b) {
+        float mn, fa, fb;
+        merge_factors(rm, bm, mn, fa, fb);
+        rm = mn;
+        rd = rd * fa + bd * fb;
+#pragma unroll
+        for (int c = 0; c < DCH; ++c) ru[c] = ru[c] * fa + bu[c] * fb;
       }
     }
     if (p.mode == 1) {
