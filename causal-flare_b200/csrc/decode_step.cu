@@ -2,11 +2,14 @@
 //
 // Per lane the kernel reads and writes u [M, Dv] fp32 once (128-bit accesses, streaming cache hints so the
 // shared latent bank Q stays resident in L2), plus m, d [M].  Phases inside a CTA (one CTA per lane):
-//   0. issue the first batch of state loads so they are in flight while scores are computed
+//   0. issue the first batch of state loads so they are in flight while scores are computed (few lanes: all of them, the lane's
+//      value columns shared by the CTAs of a cluster)
 //   1. scores s[m] = scale <q_m, k>, 8 lanes per latent, 16-byte loads of Q, 3-step shuffle reduction
 //   2. running max / denominator update per latent, decode softmax over the M latents (block reductions)
 //   3. stream u: u' = gamma u + eta v,  y += (softmax / d') u'; thread-private y columns, reduced once
 #include "decode_step.cuh"
+
+#include "sm100_ptx.cuh"
 
 namespace flare {
 
@@ -27,31 +30,49 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
   return r;
 }
 
-// scores of all M latents against one token vector held in shared memory (fp32)
+// scores of latents mb .. me - 1 against one token vector held in shared memory (fp32), AHEAD latent rows in flight per thread;
+// SLICED: into the same place of every CTA of the cluster
+template <int AHEAD, bool SLICED>
 __device__ __forceinline__ void lane_scores(float* out, const float* tok, const void* lat, int dtype, int64_t lat_off,
-                                            int64_t lat_stride_m, int M, int Dk, float scale) {
+                                            int64_t lat_stride_m, int mb, int me, int Dk, float scale, int slices) {
   const int grp = threadIdx.x >> 3, gl = threadIdx.x & 7;
-  for (int m = grp; m < M; m += NT / 8) {
-    float acc = 0.f;
-    const int64_t row = lat_off + (int64_t)m * lat_stride_m;
-    for (int d0 = gl * 8; d0 < Dk; d0 += 64) {
-      float qv[8];
-      load8(lat, dtype, row + d0, qv);
+  for (int m0 = mb; m0 < me; m0 += AHEAD * (NT / 8)) {
+    float acc[AHEAD];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc += qv[i] * tok[d0 + i];
+    for (int a = 0; a < AHEAD; ++a) acc[a] = 0.f;
+    for (int d0 = gl * 8; d0 < Dk; d0 += 64) {
+      float qv[AHEAD][8];
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+        load8(lat, dtype, lat_off + (int64_t)min(m0 + a * (NT / 8) + grp, me - 1) * lat_stride_m + d0, qv[a]);
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[a] += qv[a][i] * tok[d0 + i];
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    if (gl == 0) out[m] = acc * scale;
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a) {
+      acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 4);
+      acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 2);
+      acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 1);
+      const int m = m0 + a * (NT / 8) + grp;
+      if (m >= me) continue;
+      if constexpr (SLICED) {
+        if (gl < slices) sm100::st_cluster_f32(sm100::mapa_shared(sm100::smem_u32(out + m), gl), acc[a] * scale);
+      } else if (gl == 0) {
+        out[m] = acc[a] * scale;
+      }
+    }
   }
 }
 
 }  // namespace
 
 // PRE: state vectors per thread issued before the score phase; UNR: state vectors in flight per thread in the
-// streaming loop; MINB: CTAs per SM the register budget is held to
-template <int PRE, int UNR, int MINB>
+// streaming loop; MINB: CTAs per SM the register budget is held to; AHEAD: latent rows in flight per thread in the scores
+// SLICED: the lane's value columns are shared by the CTAs of a cluster (blockIdx.y).  Each computes the scores of its part of the
+// latents and sends them to the others; the statistics are the business of all of them and written by the first.
+template <int PRE, int UNR, int MINB, int AHEAD, bool SLICED>
 __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParams p) {
   extern __shared__ __align__(16) float smem[];
   const int lane_id = blockIdx.x;
@@ -60,9 +81,10 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   const int M = p.M, Dk = p.Dk, Dv = p.Dv;
   const int tid = threadIdx.x;
   const int dtype = p.dtype;
-  const int dv4 = Dv >> 2;
-  const int rows_per_pass = NT / dv4;
-  const int col4 = tid % dv4, row0 = tid / dv4;
+  const int slices = SLICED ? (int)gridDim.y : 1, slice = SLICED ? (int)blockIdx.y : 0;
+  const int dv4 = Dv >> 2, cols = dv4 / slices;
+  const int rows_per_pass = NT / cols;
+  const int col4 = slice * cols + tid % cols, row0 = tid / cols;
 
   float* s_sc = smem;           // [M] encode scores -> eta
   float* a_sc = s_sc + M;       // [M] decode scores -> read-out weight
@@ -75,19 +97,27 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
 
   if (p.mask != nullptr && p.mask[b] == 0) {
     // masked lane: state untouched, y = 0
-    for (int i = tid; i < Dv; i += NT) store1(p.y, dtype, (int64_t)lane_id * Dv + i, 0.f);
+    if (slice == 0)
+      for (int i = tid; i < Dv; i += NT) store1(p.y, dtype, (int64_t)lane_id * Dv + i, 0.f);
     return;
   }
 
-  float4* u4 = reinterpret_cast<float4*>(p.u + (int64_t)lane_id * M * Dv);
-  const int total4 = M * dv4;
+  if constexpr (SLICED) sm100::cluster_arrive();  // (a CTA may be written to once it runs)
+  float4* u4 = reinterpret_cast<float4*>(p.u + (int64_t)lane_id * M * Dv) + col4;
 
-  // phase 0: first state vectors in flight
+  // phase 0: first state vectors in flight, and the statistics of this thread's first latent
   float4 pre[PRE];
 #pragma unroll
   for (int i = 0; i < PRE; ++i) {
-    const int idx = tid + i * NT;
-    pre[i] = idx < total4 ? load_streaming(u4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int r = row0 + i * rows_per_pass;
+    pre[i] = r < M ? load_streaming(u4 + (int64_t)r * dv4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float* gm = p.m + (int64_t)lane_id * M;
+  float* gd = p.d + (int64_t)lane_id * M;
+  float m_first = 0.f, d_first = 0.f;
+  if (SLICED && tid < M) {
+    m_first = gm[tid];
+    d_first = gd[tid];
   }
 
   // token vectors -> smem fp32
@@ -97,16 +127,20 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   }
   for (int i = tid; i < Dv; i += NT) vtok[i] = load1(p.v, dtype, (int64_t)b * p.v_stride_b + (int64_t)h * p.v_stride_h + i);
   __syncthreads();
+  if constexpr (SLICED) sm100::cluster_wait();
 
   // phase 1: scores
-  lane_scores(s_sc, ktok, p.q, dtype, (int64_t)h * p.q_stride_h, p.q_stride_m, M, Dk, p.scale);
+  const int ms = SLICED ? (M + slices - 1) / slices : M, mb = slice * ms, me = min(M, mb + ms);
+  lane_scores<AHEAD, SLICED>(s_sc, ktok, p.q, dtype, (int64_t)h * p.q_stride_h, p.q_stride_m, mb, me, Dk, p.scale, slices);
   const bool shared_w = p.qd == nullptr && p.kd == nullptr;
   if (!shared_w) {
-    lane_scores(a_sc, p.qd ? qtok : ktok, p.kd ? p.kd : p.q, dtype,
-                p.kd ? (int64_t)h * p.kd_stride_h : (int64_t)h * p.q_stride_h, p.kd ? p.kd_stride_m : p.q_stride_m, M,
-                Dk, p.scale);
+    lane_scores<AHEAD, SLICED>(a_sc, p.qd ? qtok : ktok, p.kd ? p.kd : p.q, dtype,
+                               p.kd ? (int64_t)h * p.kd_stride_h : (int64_t)h * p.q_stride_h, p.kd ? p.kd_stride_m : p.q_stride_m,
+                               mb, me, Dk, p.scale, slices);
   }
-  __syncthreads();
+  // (sliced: every CTA of the lane has all scores, and has read the statistics that the first one rewrites below)
+  if constexpr (SLICED) sm100::cluster_sync_all();
+  else __syncthreads();
 
   // phase 2: decode softmax over latents and per-latent statistics
   float amax = kNegInf;
@@ -120,17 +154,17 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   }
   asum = block_reduce(asum, red, false);
   const float ainv = 1.0f / asum;
-  float* gm = p.m + (int64_t)lane_id * M;
-  float* gd = p.d + (int64_t)lane_id * M;
   for (int m = tid; m < M; m += NT) {
     const float s = s_sc[m];
-    const float mo = gm[m], dold = gd[m];
+    const float mo = SLICED ? m_first : gm[m], dold = SLICED ? d_first : gd[m];
     const float mn = fmaxf(mo, s);
     const float g = (mo == kNegInf) ? 0.f : __expf(mo - mn);
     const float eta = __expf(s - mn);
     const float dn = dold * g + eta;
-    gm[m] = mn;
-    gd[m] = dn;
+    if (slice == 0) {
+      gm[m] = mn;
+      gd[m] = dn;
+    }
     gam[m] = g;
     s_sc[m] = eta;
     a_sc[m] = a_sc[m] * ainv / (dn > 0.f ? dn : 1.f);
@@ -140,13 +174,13 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   // phase 3: stream the state
   const float4 v4 = reinterpret_cast<const float4*>(vtok)[col4];
   float4 yacc = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto apply = [&](float4 x, int row, int idx) {
+  auto apply = [&](float4 x, int row) {
     const float g = gam[row], e = s_sc[row], w = a_sc[row];
     x.x = x.x * g + e * v4.x;
     x.y = x.y * g + e * v4.y;
     x.z = x.z * g + e * v4.z;
     x.w = x.w * g + e * v4.w;
-    __stcs(u4 + idx, x);
+    __stcs(u4 + (int64_t)row * dv4, x);
     yacc.x += w * x.x;
     yacc.y += w * x.y;
     yacc.z += w * x.z;
@@ -154,32 +188,29 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   };
 #pragma unroll
   for (int i = 0; i < PRE; ++i) {
-    const int idx = tid + i * NT;
-    if (idx < total4) apply(pre[i], row0 + i * rows_per_pass, idx);
+    const int r = row0 + i * rows_per_pass;
+    if (r < M) apply(pre[i], r);
   }
-  int base = PRE * NT;
-  for (; base + UNR * NT <= total4; base += UNR * NT) {
+  int r = row0 + PRE * rows_per_pass;
+  for (; r + (UNR - 1) * rows_per_pass < M; r += UNR * rows_per_pass) {
     float4 x[UNR];
 #pragma unroll
-    for (int i = 0; i < UNR; ++i) x[i] = load_streaming(u4 + base + tid + i * NT);
+    for (int i = 0; i < UNR; ++i) x[i] = load_streaming(u4 + (int64_t)(r + i * rows_per_pass) * dv4);
 #pragma unroll
-    for (int i = 0; i < UNR; ++i) apply(x[i], (base + tid + i * NT) / dv4, base + tid + i * NT);
+    for (int i = 0; i < UNR; ++i) apply(x[i], r + i * rows_per_pass);
   }
-  for (; base < total4; base += NT) {
-    const int idx = base + tid;
-    if (idx < total4) apply(load_streaming(u4 + idx), idx / dv4, idx);
-  }
+  for (; r < M; r += rows_per_pass) apply(load_streaming(u4 + (int64_t)r * dv4), r);
 
   // reduce y over the row groups that share a column
   ypart[tid] = yacc;
   __syncthreads();
-  if (tid < dv4) {
+  if (tid < cols) {
     float4 acc = ypart[tid];
     for (int r = 1; r < rows_per_pass; ++r) {
-      const float4 x = ypart[tid + r * dv4];
+      const float4 x = ypart[tid + r * cols];
       acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
     }
-    store4(p.y, dtype, (int64_t)lane_id * Dv + tid * 4, acc.x, acc.y, acc.z, acc.w);
+    store4(p.y, p.dtype, (int64_t)lane_id * Dv + col4 * 4, acc.x, acc.y, acc.z, acc.w);
   }
 }
 
@@ -190,23 +221,51 @@ bool decode_step_supported(int M, int Dk, int Dv) {
   return smem <= 200 * 1024;
 }
 
-template <int PRE, int UNR, int MINB>
-static int launch_variant(const DecodeParams& p, size_t smem, cudaStream_t stream) {
-  auto kern = decode_step_kernel<PRE, UNR, MINB>;
+template <int PRE, int UNR, int MINB, int AHEAD, bool SLICED>
+static int launch_variant(const DecodeParams& p, size_t smem, int slices, cudaStream_t stream) {
+  auto kern = decode_step_kernel<PRE, UNR, MINB, AHEAD, SLICED>;
   if (smem > 48 * 1024) FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("decode_step_kernel", stream);
-  FLARE_CUDA_CHECK(launch_pdl(kern, dim3(p.B * p.H), dim3(NT), smem, stream, p));
+  if constexpr (SLICED) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.B * p.H, slices);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = slices;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    FLARE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, p));
+  } else {
+    FLARE_CUDA_CHECK(launch_pdl(kern, dim3(p.B * p.H), dim3(NT), smem, stream, p));
+  }
   return FLARE_OK;
 }
 
 int launch_decode_step(const DecodeParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)(3 * p.M + 2 * p.Dk + p.Dv + NW) * 4 + NT * 16;
-  // Measured on B200 at B=64, H=32, M=256, D=128 (us per step): <2,4,8> 112.0, <8,8,4> 113.8, <4,8,4> 115.6,
-  // <4,4,6> 116.8, <4,8,1> 141.9, <4,16,2> 157.8: occupancy (8 CTAs of 32 registers per SM) beats deeper unrolling.
-  // Also measured and rejected: 128-thread CTAs at 16 per SM (121.7), and moving the state with bulk async copies
-  // through a shared-memory ring (4 x 8 KB: 115.5, 4 x 16 KB: 131.3, 8 x 16 KB: 207.2) - the per-lane score and
-  // softmax phases are hidden best by many resident CTAs, not by more bytes in flight per CTA.
-  return launch_variant<2, 4, 8>(p, smem, stream);
+  // What counts is how much of the state is on its way: a thread needs registers for the vectors that it has asked for.  At 32
+  // registers (eight CTAs per SM, the choice before) the compiler asks for one at a time.  Per step, us on B200 with the state
+  // cold, <2, 4, 8> of 32 registers / <4, 4, 4> / <8, 8, 2> / the sliced one:
+  //   2048 lanes of 128 KB 121 / 97 / 99 / 108     2048 lanes of 64 KB 65 / 52 / 56 / 69     768 lanes of 32 KB 19 / 16 / 18 / 23
+  //    256 lanes of 128 KB  49 / 21 / 17 / 18        96 lanes of 64 KB 12.4 / 10.9 / 8.0 / 7.8     16 lanes of 128 KB 16.6 / 11.2 / 9.3 / 6.8
+  // So: four CTAs per SM while there are lanes for more than two, else two with twice the vectors, and a lane whose state does
+  // not fit the vectors asked for ahead is cut into column slices (128 bytes wide at least) while two per SM hold them all.
+  // Measured and rejected on the largest shape: one kernel for the coefficients of all lanes and one that only streams (98 to
+  // 103), 128-thread CTAs (121.7 against 112), bulk async copies through a shared-memory ring (115.5 to 207).
+  const int64_t lanes = (int64_t)p.B * p.H, slots = 2 * (int64_t)sm_count();
+  if (lanes > slots) return launch_variant<4, 4, 4, 4, false>(p, smem, 1, stream);
+  constexpr int PRE = 8;
+  int slices = 1;
+  while (p.M <= NT && p.M * (p.Dv / 4) > slices * PRE * NT && lanes * slices * 2 <= slots && p.Dv / 4 % (slices * 16) == 0) slices *= 2;
+  return slices == 1 ? launch_variant<PRE, 8, 2, 4, false>(p, smem, 1, stream)
+                     : launch_variant<PRE, 8, 2, 4, true>(p, smem, slices, stream);
 }
 
 }  // namespace flare
