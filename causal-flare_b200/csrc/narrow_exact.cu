@@ -73,10 +73,11 @@ __device__ __forceinline__ float reduce_latents(float (&v)[4], int lane) {
   return v[0];
 }
 
-// scores of the tile for this thread's latent (its bank row in registers)
-__device__ __forceinline__ void score_rows(float (&s)[BT], const float* ks, const float (&q)[W], float scale) {
+// scores of TS tokens for this thread's latent (its bank row in registers)
+template <int TS>
+__device__ __forceinline__ void score_rows(float (&s)[TS], const float* ks, const float (&q)[W], float scale) {
 #pragma unroll
-  for (int t = 0; t < BT; ++t) {
+  for (int t = 0; t < TS; ++t) {
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll
     for (int c = 0; c < W; c += 4) {
@@ -90,10 +91,11 @@ __device__ __forceinline__ void score_rows(float (&s)[BT], const float* ks, cons
   }
 }
 
-// Maximum of v[t] over the lanes of the warp; lane l keeps that of token l & 15 (16 shuffles for 16 tokens).
-__device__ __forceinline__ float reduce_max(float (&v)[BT], int lane) {
+// Maximum of v[t] over the lanes of the warp; lane l keeps that of token l % TS (16 shuffles for 16 tokens).
+template <int TS>
+__device__ __forceinline__ float reduce_max(float (&v)[TS], int lane) {
 #pragma unroll
-  for (int s = BT / 2; s >= 1; s >>= 1) {
+  for (int s = TS / 2; s >= 1; s >>= 1) {
     const bool upper = (lane & s) != 0;
 #pragma unroll
     for (int k = 0; k < s; ++k) {
@@ -101,38 +103,42 @@ __device__ __forceinline__ float reduce_max(float (&v)[BT], int lane) {
       v[k] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, s));
     }
   }
-  return fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 16));
+  float r = v[0];
+#pragma unroll
+  for (int o = TS; o < 32; o <<= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+  return r;
 }
 
-// Decode softmax of the tile's tokens over all latents: a[t] = weight of this thread's latent.  red: [2][nw][BT] floats.
-// Contains two CTA barriers.
-__device__ __forceinline__ void decode_weights(float (&a)[BT], const float (&s)[BT], bool live, float* red, float* lse, int t0,
+// Decode softmax of TS tokens over all latents: a[t] = weight of this thread's latent.  red: [2][nw] rows of BT floats, of which
+// these tokens have their own.  Contains two CTA barriers.
+template <int TS>
+__device__ __forceinline__ void decode_weights(float (&a)[TS], const float (&s)[TS], bool live, float* red, float* lse, int t0,
                                                int t_end, const int* valid) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-  for (int t = 0; t < BT; ++t) a[t] = live ? s[t] : kNegInf;
-  const float mx = reduce_max(a, lane);
-  if (lane < BT) red[warp * BT + lane] = mx;
+  for (int t = 0; t < TS; ++t) a[t] = live ? s[t] : kNegInf;
+  const float mx = reduce_max<TS>(a, lane);
+  if (lane < TS) red[warp * BT + lane] = mx;
   __syncthreads();
-  float e[BT];
+  float e[TS];
 #pragma unroll
-  for (int t = 0; t < BT; ++t) {
+  for (int t = 0; t < TS; ++t) {
     float m = red[t];
     for (int w = 1; w < nw; ++w) m = fmaxf(m, red[w * BT + t]);
     a[t] = live ? __expf(s[t] - m) : 0.f;
     e[t] = a[t];
   }
-  walk::warp_reduce_scatter<BT>(e, lane);
+  walk::warp_reduce_scatter<TS>(e, lane);
   float* sums = red + nw * BT;
-  if (lane < BT) sums[warp * BT + lane] = e[0];
+  if (lane < TS) sums[warp * BT + lane] = e[0];
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < BT; ++t) {
+  for (int t = 0; t < TS; ++t) {
     float sum = sums[t];
     for (int w = 1; w < nw; ++w) sum += sums[w * BT + t];
     a[t] *= 1.0f / sum;
   }
-  if (lse != nullptr && threadIdx.x < BT && t0 + (int)threadIdx.x < t_end) {
+  if (lse != nullptr && threadIdx.x < TS && t0 + (int)threadIdx.x < t_end) {
     const int t = threadIdx.x;
     float m = red[t], sum = sums[t];
     for (int w = 1; w < nw; ++w) {
@@ -171,6 +177,11 @@ __device__ __forceinline__ void decay_state(float (&U)[8][4], const float* gam_r
 // ---------------------------------------------------------------------------------------------
 // forward walk
 // ---------------------------------------------------------------------------------------------
+// Scores and statistics are taken for eight tokens at a time and the state is walked without unrolling.  Unrolled for the 16 tokens
+// of a tile the code was most of the time of a CTA that walks two tiles (half of the warps' cycles waited for an instruction),
+// and held more registers: B200, fp32 B=1 N=256 H=8 M=64 D=32 47.2 -> 43.1 us, B=8 N=4096 H=16 1256 -> 1124 us, fp16 B=4
+// N=2048 H=16 M=128 637 -> 568 us.  (Four tokens at a time: 44.3, 1148, 579.)
+constexpr int TS = 8;
 template <bool STABLE>
 __global__ void __launch_bounds__(128, 4) walk_narrow_kernel(const WalkParams p) {
   pdl_begin();
@@ -222,32 +233,35 @@ __global__ void __launch_bounds__(128, 4) walk_narrow_kernel(const WalkParams p)
     stage_rows(ks, p.k, p.dtype, k_off, p.k_stride_n, t0, seg_end, p.Dk);
     stage_rows(vs, p.v, p.dtype, v_off, p.v_stride_n, t0, seg_end, p.Dv);
     __syncthreads();
-    float sv[BT], aw[BT];
-    score_rows(sv, ks, q, p.scale);
-    if (write_y)
-      decode_weights(aw, sv, live, red, p.lse_dec != nullptr ? p.lse_dec + (int64_t)lane_id * p.N + t0 : nullptr, t0, seg_end,
-                     valid);
-    // running statistics of this thread's latent
+#pragma unroll 1
+    for (int t1 = 0; t1 < BT; t1 += TS) {
+      float sv[TS], aw[TS];
+      score_rows<TS>(sv, ks + t1 * W, q, p.scale);
+      if (write_y)
+        decode_weights<TS>(aw, sv, live, red + t1, p.lse_dec != nullptr ? p.lse_dec + (int64_t)lane_id * p.N + t0 + t1 : nullptr,
+                           t0 + t1, seg_end, valid + t1);
+      // running statistics of this thread's latent
 #pragma unroll
-    for (int t = 0; t < BT; ++t) {
-      const bool on = valid[t] != 0;
-      float gam = 1.f, eta;
-      if constexpr (STABLE) {
-        eta = on ? stablemax_sigma(sv[t], p.power) : 0.f;
-        dr += eta;
-      } else {
-        const float mn = on ? fmaxf(mr, sv[t]) : mr;
-        if (on) gam = (mr == kNegInf) ? 0.f : __expf(mr - mn);
-        eta = on ? __expf(sv[t] - mn) : 0.f;
-        dr = dr * gam + eta;
-        mr = mn;
+      for (int t = 0; t < TS; ++t) {
+        const bool on = valid[t1 + t] != 0;
+        float gam = 1.f, eta;
+        if constexpr (STABLE) {
+          eta = on ? stablemax_sigma(sv[t], p.power) : 0.f;
+          dr += eta;
+        } else {
+          const float mn = on ? fmaxf(mr, sv[t]) : mr;
+          if (on) gam = (mr == kNegInf) ? 0.f : __expf(mr - mn);
+          eta = on ? __expf(sv[t] - mn) : 0.f;
+          dr = dr * gam + eta;
+          mr = mn;
+        }
+        if (write_y) w_s[(t1 + t) * ms + m] = aw[t] * (1.0f / (dr > 0.f ? dr : 1.f));
+        if constexpr (!STABLE) g_s[(t1 + t) * ms + m] = gam;
+        s_s[(t1 + t) * ms + m] = eta;
       }
-      if (write_y) w_s[t * ms + m] = aw[t] * (1.0f / (dr > 0.f ? dr : 1.f));
-      if constexpr (!STABLE) g_s[t * ms + m] = gam;
-      s_s[t * ms + m] = eta;
     }
     __syncwarp();
-#pragma unroll 4
+#pragma unroll 1
     for (int t = 0; t < BT; ++t) {
       float y[4] = {0.f, 0.f, 0.f, 0.f};
       if (valid[t]) {
@@ -353,8 +367,8 @@ __global__ void __launch_bounds__(128, 3) narrow_replay_kernel(const NarrowBwdPa
     stage_rows(dos, p.dy, p.dtype, dy_off, p.dy_stride_n, t0, tend, p.Dv);
     __syncthreads();
     float sv[BT], aw[BT];
-    score_rows(sv, ks, q, p.scale);
-    decode_weights(aw, sv, live, red, nullptr, t0, tend, nullptr);
+    score_rows<BT>(sv, ks, q, p.scale);
+    decode_weights<BT>(aw, sv, live, red, nullptr, t0, tend, nullptr);
 #pragma unroll
     for (int t = 0; t < BT; ++t) {
       if (t >= nt) break;
