@@ -17,7 +17,8 @@
 // (4) latents: per-split partial dQ / dK_dec = dS^T Rows; (5) fixed-order sum of the partials
 // (deterministic: no atomics anywhere).
 // Heads up to 32 wide take narrow_exact.cu instead: its replay also forms the segment carries, its reverse walk also dK
-// and dQ, so (3), (4) and the dS planes fall away.
+// and dQ, so (3), (4) and the dS planes fall away; bf16 softmax calls among those take narrow_mma.cu.  The kernels' bodies are in
+// bwd_cta.cuh: behind the tensor-core backward they stand by as the tasks of one kernel (bwd_standby.cu).
 #include "bwd_exact.cuh"
 
 #include <string.h>
