@@ -7,9 +7,10 @@
 //   backward  P = U dY^T + E A     X = G V^T + R A^T    dS = g (P / D - delta) + E (X - C - suffix sum of R P / D)
 //             dV = E^T G + (E^T R) dY    dK = dS^T Q    dQ += dS K    G += R dY    C += sum of R P / D
 // (A, W and E^T R masked to the causal half), the algebra of the kernels for wide heads.  The products run as bf16
-// mma.sync.m16n8k16: every operand that is not the caller's own bf16 tensor (E, R, W, A, U, G, dS) enters as a pair hi + lo of
-// bf16 values (16 mantissa bits), with all terms of a product but lo x lo, sums in fp32.  The accumulator layout of
-// one product is the A operand layout of the next one; the transposes that are left are movmatrix on the packed pairs.
+// mma.sync.m16n8k16: every operand that is not the caller's own bf16 tensor (E, R, W, A, U, G, dS) enters as the sum of three
+// bf16 values, all the 24 bits of its mantissa; terms below 2^-24 of a product are left out, and what lives over many tiles (U, G,
+// dQ, the carries) takes a tile's product in one rounded fp32 addition.  The accumulator layout of one product is the A operand
+// layout of the next one; the transposes that are left are movmatrix on the packed pairs.
 // Why not tcgen05: the smallest product it takes is 64 rows against tensor memory, and a tile here is 16 x 16 x 32 with a scan
 // over the tokens between every two products; per token and latent the work is the exponentials and the packing.
 // The recurrence walked token by token (narrow_exact.cu) has a chain of 16 dependent steps where this has one.
@@ -22,8 +23,15 @@
 // flush weights that still count; that, and any non-finite result, raises the CTA's gate word and the fp32 kernels standing
 // by redo the lane (forward) or the call (backward).
 //
-// B200, training step B=8 N=2048 H=16 M=64 D=32: 1827 us on the fp32 kernels, 385 us on these.  Distance of y, dQ, dK, dV from
-// 64 bits over M = 32 .. 128, N = 300 .. 700: 1.5e-3 to 1.7e-3 (the rounding to bf16) on both, equal to five digits.
+// Precision: the distances of the bf16 outputs from 64 bits equal those of the fp32 kernels to 1 part in 10^6, either way, over
+// M = 32 .. 128, N = 128 .. 4096, and 0.1 % of the outputs at most are rounded the other way, as there.  (Two values per operand
+// were faster, 386 us for the step below, but left 0.1 to 0.5 % of the outputs rounded the other way and an fp32 dQ ten times
+// as far from 64 bits.)  What is left is the tensor cores' own addition, which cuts off instead of rounding: 3.7e-7 of an fp32
+// dQ whatever N is, where the fp32 kernels have 2.8e-7 (N = 128) to 5.2e-7 (N = 4096).  A caller that wants dQ in fp32 gets
+// the fp32 kernels.
+//
+// B200, training step B=8 N=2048 H=16 M=64 D=32: 1823 us on the fp32 kernels, 473 us on these; the forward alone 632
+// and 132 us.
 #include "narrow_mma.cuh"
 
 #include <string.h>
@@ -85,35 +93,71 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 
 // Thread (g, q) = (lane / 4, lane % 4).  An accumulator x[j] covers rows g (elements 0, 1) and g + 8 (2, 3) and columns
 // 8 j + 2 q, + 1.  A 16 x 16 operand is the four 8 x 8 blocks (rows 0-7 | 8-15, columns 0-7), (rows 0-7 | 8-15, columns 8-15).
-struct Pair {
-  uint32_t hi[4], lo[4];
+struct Split {
+  uint32_t hi[4], mid[4], lo[4];
 };
-__device__ __forceinline__ void split(float x, float y, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = pack_bf16(x, y);
-  lo = pack_bf16(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
+  x -= __uint_as_float(hi << 16);
+  y -= __uint_as_float(hi & 0xffff0000u);
+  mid = pack_bf16(x, y);
+  lo = pack_bf16(x - __uint_as_float(mid << 16), y - __uint_as_float(mid & 0xffff0000u));
 }
 // accumulators of columns 0-7 and 8-15 as an A operand
-__device__ __forceinline__ void split_tile(Pair& p, const float (&x0)[4], const float (&x1)[4]) {
-  split(x0[0], x0[1], p.hi[0], p.lo[0]);
-  split(x0[2], x0[3], p.hi[1], p.lo[1]);
-  split(x1[0], x1[1], p.hi[2], p.lo[2]);
-  split(x1[2], x1[3], p.hi[3], p.lo[3]);
+__device__ __forceinline__ void split_tile(Split& p, const float (&x0)[4], const float (&x1)[4]) {
+  split(x0[0], x0[1], p.hi[0], p.mid[0], p.lo[0]);
+  split(x0[2], x0[3], p.hi[1], p.mid[1], p.lo[1]);
+  split(x1[0], x1[1], p.hi[2], p.mid[2], p.lo[2]);
+  split(x1[2], x1[3], p.hi[3], p.mid[3], p.lo[3]);
 }
 // the transposed 16 x 16 operand in A order; as B operand of a product over its own rows: columns 0-7 = blocks 0, 2 and
 // columns 8-15 = blocks 1, 3 of this
-__device__ __forceinline__ void transpose_tile(Pair& t, const Pair& p) {
-  t.hi[0] = transpose8(p.hi[0]); t.hi[1] = transpose8(p.hi[2]); t.hi[2] = transpose8(p.hi[1]); t.hi[3] = transpose8(p.hi[3]);
-  t.lo[0] = transpose8(p.lo[0]); t.lo[1] = transpose8(p.lo[2]); t.lo[2] = transpose8(p.lo[1]); t.lo[3] = transpose8(p.lo[3]);
+__device__ __forceinline__ void transpose_blocks(uint32_t (&t)[4], const uint32_t (&p)[4]) {
+  t[0] = transpose8(p[0]); t[1] = transpose8(p[2]); t[2] = transpose8(p[1]); t[3] = transpose8(p[3]);
 }
-// d += a b: both split (all terms but lo x lo), or b exact
-__device__ __forceinline__ void mma3(float (&d)[4], const Pair& a, uint32_t bh0, uint32_t bh1, uint32_t bl0, uint32_t bl1) {
-  mma(d, a.lo, bh0, bh1);
-  mma(d, a.hi, bl0, bl1);
-  mma(d, a.hi, bh0, bh1);
+__device__ __forceinline__ void transpose_tile(Split& t, const Split& p) {
+  transpose_blocks(t.hi, p.hi);
+  transpose_blocks(t.mid, p.mid);
+  transpose_blocks(t.lo, p.lo);
 }
-__device__ __forceinline__ void mma2(float (&d)[4], const Pair& a, uint32_t b0, uint32_t b1) {
+// d += a b, small terms first: b exact, or both split (what is left out is below 2^-24 of the product)
+__device__ __forceinline__ void mma_exact(float (&d)[4], const Split& a, uint32_t b0, uint32_t b1) {
   mma(d, a.lo, b0, b1);
+  mma(d, a.mid, b0, b1);
   mma(d, a.hi, b0, b1);
+}
+struct Col {  // eight columns of a split B operand
+  uint32_t hi0, hi1, mid0, mid1, lo0, lo1;
+};
+__device__ __forceinline__ void mma_split(float (&d)[4], const Split& a, const Col& b) {
+  mma(d, a.lo, b.hi0, b.hi1);
+  mma(d, a.hi, b.lo0, b.lo1);
+  mma(d, a.mid, b.mid0, b.mid1);
+  mma(d, a.mid, b.hi0, b.hi1);
+  mma(d, a.hi, b.mid0, b.mid1);
+  mma(d, a.hi, b.hi0, b.hi1);
+}
+template <int I>  // columns 8 I .. + 7 of an operand in the order above
+__device__ __forceinline__ Col col(const Split& t) {
+  return Col{t.hi[I], t.hi[I + 2], t.mid[I], t.mid[I + 2], t.lo[I], t.lo[I + 2]};
+}
+// an accumulator (16 rows, 8 columns) as B operand of a product over its rows
+__device__ __forceinline__ Col as_col(const float (&x)[4]) {
+  Col c;
+  split(x[0], x[1], c.hi0, c.mid0, c.lo0);
+  split(x[2], x[3], c.hi1, c.mid1, c.lo1);
+  c.hi0 = transpose8(c.hi0); c.hi1 = transpose8(c.hi1);
+  c.mid0 = transpose8(c.mid0); c.mid1 = transpose8(c.mid1);
+  c.lo0 = transpose8(c.lo0); c.lo1 = transpose8(c.lo1);
+  return c;
+}
+// Sums that live over many tiles take a tile's product in one rounded addition: the tensor cores cut off what does not fit
+// the accumulator, always towards zero.
+__device__ __forceinline__ void add_product(float (&sum)[4], const Split& a, uint32_t b0, uint32_t b1) {
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  mma_exact(d, a, b0, b1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sum[i] += d[i];
 }
 
 // rows of a staged tile (16 tokens): f[h][piece] = tokens 8 h .. + 7, columns 8 piece .. + 7.  B operand of a product over the
@@ -344,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) narrow_mma_forward_ker
       rescale(u, alpha);
       uint32_t vt[4][2];
       load_cols(vt, vs, lane);
-      Pair ep;
+      Split ep;
       split_tile(ep, e[0], e[1]);
       if constexpr (WRITE_Y) {
         float den[2][4];
@@ -367,7 +411,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) narrow_mma_forward_ker
           sum_s[t] = sum;
           kap_s[t] = summed_frame(kap, lane);
         }
-        Pair rp, rt, et;
+        Split rp, rt, et;
         split_tile(rp, r[0], r[1]);
         transpose_tile(rt, rp);  // A operand: tokens x latents
         transpose_tile(et, ep);  // B operand over the latents
@@ -376,24 +420,19 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) narrow_mma_forward_ker
         {
           float w[2][4];
           zero(w);
-          mma3(w[0], rt, et.hi[0], et.hi[2], et.lo[0], et.lo[2]);
-          mma3(w[1], rt, et.hi[1], et.hi[3], et.lo[1], et.lo[3]);
+          mma_split(w[0], rt, col<0>(et));
+          mma_split(w[1], rt, col<1>(et));
 #pragma unroll
           for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? w[j][i] : 0.f;
-          Pair wp;
+          Split wp;
           split_tile(wp, w[0], w[1]);
 #pragma unroll
-          for (int n = 0; n < 4; ++n) mma2(y[n], wp, vt[n][0], vt[n][1]);
+          for (int n = 0; n < 4; ++n) mma_exact(y[n], wp, vt[n][0], vt[n][1]);
         }
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          uint32_t h0, h1, l0, l1;
-          split(u[n][0], u[n][1], h0, l0);
-          split(u[n][2], u[n][3], h1, l1);
-          mma3(y[n], rt, transpose8(h0), transpose8(h1), transpose8(l0), transpose8(l1));
-        }
+        for (int n = 0; n < 4; ++n) mma_split(y[n], rt, as_col(u[n]));
         float* const dst = ypart + (warp * BT + tile * 16 + g) * LDP + q2;
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
@@ -405,7 +444,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) narrow_mma_forward_ker
         for (int r = 0; r < 2; ++r) d[r] += quad_sum((e[0][2 * r] + e[0][2 * r + 1]) + (e[1][2 * r] + e[1][2 * r + 1]));
       }
 #pragma unroll
-      for (int n = 0; n < 4; ++n) mma2(u[n], ep, vt[n][0], vt[n][1]);
+      for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
     }
     if constexpr (WRITE_Y) {
       __syncthreads();
@@ -576,7 +615,7 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_replay_kern
             r[j][i] = rcp_approx(den[j][i]);  // 1 / D
           }
         }
-      Pair ep;
+      Split ep;
       split_tile(ep, e[0], e[1]);
       uint32_t vf[2][4], df[2][4];
       load_rows(vf, ks + STAGE, lane);
@@ -598,17 +637,17 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_replay_kern
         for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int i = 0; i < 4; ++i) at[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? at[j][i] : 0.f;
-        Pair ap;
+        Split ap;
         split_tile(ap, at[0], at[1]);  // blocks (t 0-7 | 8-15, tau 0-7), (t 0-7 | 8-15, tau 8-15)
-        mma3(pp[0], ep, ap.hi[0], ap.hi[2], ap.lo[0], ap.lo[2]);
-        mma3(pp[1], ep, ap.hi[1], ap.hi[3], ap.lo[1], ap.lo[3]);
+        mma_split(pp[0], ep, col<0>(ap));
+        mma_split(pp[1], ep, col<1>(ap));
       }
 #pragma unroll
       for (int k2 = 0; k2 < 2; ++k2) {
-        Pair up;
+        Split up;
         split_tile(up, u[2 * k2], u[2 * k2 + 1]);
-        mma2(pp[0], up, df[0][2 * k2], df[0][2 * k2 + 1]);
-        mma2(pp[1], up, df[1][2 * k2], df[1][2 * k2 + 1]);
+        mma_exact(pp[0], up, df[0][2 * k2], df[0][2 * k2 + 1]);
+        mma_exact(pp[1], up, df[1][2 * k2], df[1][2 * k2 + 1]);
       }
       float part[2][2];
 #pragma unroll
@@ -628,7 +667,7 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_replay_kern
         uint32_t vt[4][2];
         load_cols(vt, ks + STAGE, lane);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma2(u[n], ep, vt[n][0], vt[n][1]);
+        for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
       }
       if (carries) {
         // in the frame before the segment (the frames only grow, so the factors stay below 1)
@@ -640,12 +679,12 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_replay_kern
             r[j][i] *= f[i >> 1];
             c0[i >> 1] = fmaf(r[j][i], pp[j][i], c0[i >> 1]);
           }
-        Pair rp;
+        Split rp;
         split_tile(rp, r[0], r[1]);
         uint32_t dt[4][2];
         load_cols(dt, ks + 2 * STAGE, lane);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma2(b0[n], rp, dt[n][0], dt[n][1]);
+        for (int n = 0; n < 4; ++n) add_product(b0[n], rp, dt[n][0], dt[n][1]);
       }
     }
   }
@@ -781,9 +820,9 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
             }
           }
       }
-      Pair ep, rpair;
+      Split ep, rs;
       split_tile(ep, e[0], e[1]);
-      split_tile(rpair, r[0], r[1]);
+      split_tile(rs, r[0], r[1]);
       uint32_t vf[2][4], dt[4][2];
       load_rows(vf, ks + STAGE, lane);
       load_cols(dt, ks + 2 * STAGE, lane);
@@ -807,16 +846,16 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
         for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int i = 0; i < 4; ++i) a[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? a[j][i] : 0.f;  // row tau, column t
-        Pair ap;
+        Split ap;
         split_tile(ap, a[0], a[1]);  // blocks (tau 0-7 | 8-15, t 0-7), (tau 0-7 | 8-15, t 8-15)
-        mma3(x[0], rpair, ap.hi[0], ap.hi[2], ap.lo[0], ap.lo[2]);
-        mma3(x[1], rpair, ap.hi[1], ap.hi[3], ap.lo[1], ap.lo[3]);
+        mma_split(x[0], rs, col<0>(ap));
+        mma_split(x[1], rs, col<1>(ap));
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2) {
-          Pair gp;
+          Split gp;
           split_tile(gp, gr[2 * k2], gr[2 * k2 + 1]);
-          mma2(x[0], gp, vf[0][2 * k2], vf[0][2 * k2 + 1]);
-          mma2(x[1], gp, vf[1][2 * k2], vf[1][2 * k2 + 1]);
+          mma_exact(x[0], gp, vf[0][2 * k2], vf[0][2 * k2 + 1]);
+          mma_exact(x[1], gp, vf[1][2 * k2], vf[1][2 * k2 + 1]);
         }
         // encoder part: C + sum of R p from the token on
 #pragma unroll
@@ -838,7 +877,7 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
           cc[i] = behind;
         }
       }
-      Pair et;
+      Split et;
       transpose_tile(et, ep);
       float out[4][4];
       zero(out);
@@ -846,26 +885,21 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
         // dV = E^T G + (E^T R masked) dY
         float w[2][4];
         zero(w);
-        Pair rt;
-        transpose_tile(rt, rpair);
-        mma3(w[0], et, rt.hi[0], rt.hi[2], rt.lo[0], rt.lo[2]);
-        mma3(w[1], et, rt.hi[1], rt.hi[3], rt.lo[1], rt.lo[3]);
+        Split rt;
+        transpose_tile(rt, rs);
+        mma_split(w[0], et, col<0>(rt));
+        mma_split(w[1], et, col<1>(rt));
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? w[j][i] : 0.f;
-        Pair wp;
+        Split wp;
         split_tile(wp, w[0], w[1]);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma2(out[n], wp, dt[n][0], dt[n][1]);
+        for (int n = 0; n < 4; ++n) mma_exact(out[n], wp, dt[n][0], dt[n][1]);
       }
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        uint32_t h0, h1, l0, l1;
-        split(gr[n][0], gr[n][1], h0, l0);
-        split(gr[n][2], gr[n][3], h1, l1);
-        mma3(out[n], et, transpose8(h0), transpose8(h1), transpose8(l0), transpose8(l1));
-      }
+      for (int n = 0; n < 4; ++n) mma_split(out[n], et, as_col(gr[n]));
       float* dst = part + (warp * BT + tile * 16 + g) * LDP + q2;
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
@@ -874,13 +908,13 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
       }
       // G += R dY, then into the frame of the tile before
 #pragma unroll
-      for (int n = 0; n < 4; ++n) mma2(gr[n], rpair, dt[n][0], dt[n][1]);
+      for (int n = 0; n < 4; ++n) add_product(gr[n], rs, dt[n][0], dt[n][1]);
       const float phi[2] = {ex2_approx(c_prev[0] - c[0]), ex2_approx(c_prev[1] - c[1])};
       rescale(gr, phi);
       cc[0] *= phi[0];
       cc[1] *= phi[1];
       // dK = dS^T Q, dQ += dS K
-      Pair dsp, dst_t;
+      Split dsp, dst_t;
       split_tile(dsp, ds[0], ds[1]);
       transpose_tile(dst_t, dsp);
       {
@@ -888,7 +922,7 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
         load_cols(qf, qs + m0 * LD, lane);
         zero(out);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma2(out[n], dst_t, qf[n][0], qf[n][1]);
+        for (int n = 0; n < 4; ++n) mma_exact(out[n], dst_t, qf[n][0], qf[n][1]);
       }
       dst += nw * BT * LDP;
 #pragma unroll
@@ -900,7 +934,7 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
         uint32_t kt[4][2];
         load_cols(kt, ks, lane);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma2(dq[n], dsp, kt[n][0], kt[n][1]);
+        for (int n = 0; n < 4; ++n) add_product(dq[n], dsp, kt[n][0], kt[n][1]);
       }
     }
     __syncthreads();
@@ -1030,7 +1064,8 @@ bool narrow_mma_forward_supported(const flare_fwd_args_t* a) {
 
 bool narrow_mma_backward_supported(const flare_bwd_args_t& a) {
   const bool span = a.carry_b || a.carry_c || a.carry_rho || a.span_b0 || a.span_c0 || a.span_gam || a.span_rho_first || a.phase != 0;
-  return shape_ok(a.fwd) && !span && (reinterpret_cast<uintptr_t>(a.dy) & 15u) == 0 && a.dy_stride_b % 8 == 0 &&
+  // (dQ in fp32: nothing would hide how the tensor cores add, see above)
+  return shape_ok(a.fwd) && a.dq_dtype != FLARE_F32 && !span && (reinterpret_cast<uintptr_t>(a.dy) & 15u) == 0 && a.dy_stride_b % 8 == 0 &&
          a.dy_stride_n % 8 == 0 && a.dy_stride_h % 8 == 0;
 }
 

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import causal_flare as cf
+from causal_flare import _lib, _ops
 from oracle import flare_oracle as orc
 from util import to_dev
 
@@ -24,8 +25,7 @@ SHAPES = [(1, 1, 1, 16, 16, 16), (2, 15, 2, 32, 32, 32), (1, 16, 3, 48, 16, 32),
 
 @pytest.mark.parametrize("shape", SHAPES)
 def test_no_further_from_64_bits_than_the_fp32_kernels(monkeypatch, shape):
-    # Both round the same sums to bf16.  Operands of the products carry 16 mantissa bits: 2^-17 relative per factor, against
-    # 2^-9 of the outputs' own rounding, so the two distances differ by what roundings that fall the other way make of it: below
+    # Both round the same sums to bf16, so the two distances differ by what roundings that fall the other way make of it: below
     # 1 % of the distance plus, for outputs of few entries, a fraction of one rounding.
     B, N, H, M, Dk, Dv = shape
     q, k, v, dy = orc.make_inputs(B, N, H, M, Dk, Dv, seed0=21, dtype=torch.bfloat16, with_dy=True)
@@ -45,6 +45,32 @@ def test_no_further_from_64_bits_than_the_fp32_kernels(monkeypatch, shape):
             # (a single token has no gradient but dV: what is left there are differences of equal fp32 numbers)
             err[path] = orc.rel_l2(x, want[i]) if N > 1 or name in ("y", "dV") else orc.max_abs(x, want[i])
         assert err["auto"] <= 1.01 * err["exact"] + 2.0 ** -9 / want[i].numel() ** 0.5 + 1e-5, f"{name}: {err}"
+
+
+def test_roundings_are_those_of_the_exact_values():
+    # A relative error e of a sum moves its rounding to bf16 with the probability 2 e / 2^-8 on average.  fp32 sums of terms that
+    # cancel (dK, dQ) stay within 2^-20: 2^-11, and twice that for the spread over the entries.  Operands of 16 bits (2^-17 per
+    # factor) move five times as many.
+    B, N, H, M, D = 2, 1024, 4, 64, 32
+    q, k, v, dy = orc.make_inputs(B, N, H, M, D, seed0=25, dtype=torch.bfloat16, with_dy=True)
+    ql, kl, vl = (t.detach().cuda().requires_grad_() for t in (q, k, v))
+    got = torch.autograd.grad(cf.flare_autoregressive_triton(ql, kl, vl), (ql, kl, vl), dy.cuda())
+    ref = orc.ar_backward_closed_form(q, k, v, dy)
+    for x, name in zip(got[1:], ("dK", "dV")):
+        moved = (x.cpu() != ref[name].to(torch.bfloat16)).float().mean().item()
+        assert moved <= 2.0 ** -10, f"{name}: {moved}"
+
+
+def test_dq_in_fp32_is_that_of_the_fp32_kernels():
+    # B N terms summed in fp32: one rounding each, 2^-24, which add up like their square root
+    B, N, H, M, D = 2, 1000, 4, 64, 32
+    q, k, v, dy = orc.make_inputs(B, N, H, M, D, seed0=26, dtype=torch.bfloat16, with_dy=True)
+    auto, exact = (_ops.backward(*to_dev(q, k, v, dy), scale=D ** -0.5, path=path) for path in (_lib.PATH_AUTO, _lib.PATH_EXACT))
+    for x, y in zip(auto[:3], exact[:3]):
+        assert torch.equal(x, y)
+    assert auto[0].dtype == torch.float32
+    want = orc.ar_backward_closed_form(q, k, v, dy)["dQ"]
+    assert orc.rel_l2(auto[0].cpu(), want) <= 2.0 ** -24 * (B * N) ** 0.5
 
 
 @pytest.mark.parametrize("std", [4.0, 24.0])
