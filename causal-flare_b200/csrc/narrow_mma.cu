@@ -19,22 +19,28 @@
 // decode frame) and partial dV, dK are summed over the warps there.  Segments of the sequence run concurrently: states of the
 // segments alone, folded by every CTA for itself; the backward's replay leaves the carries of the segments alone the same way.
 //
-// Domain: the frame is the maximum through the tile, so a running maximum that grows by more than 2^57 inside a tile would
-// flush weights that still count; that, and any non-finite result, raises the CTA's gate word and the fp32 kernels standing
-// by redo the lane (forward) or the call (backward).
+// Sharp scores: the frame is the maximum through the tile, so a running maximum that grows by more than 2^57 inside a tile would
+// flush weights that still count.  Such a tile is taken in windows, each with a frame of its own, that end before the token that
+// outgrows them (at worst one token each); the reverse sweep finds the same windows again from the frame before the tile.  So only
+// results that are not finite raise the CTA's gate word and let the fp32 kernels standing by redo the lane (forward) or the call
+// (backward).  One CTA walks a whole lane there: before tiles were taken in windows, B=2 N=1000 H=4 M=64 D=32 with a standard
+// deviation of 200 of the scores took 611 us forward and 950 us a step; 63 and 320 us in windows (85 and 383 us on the fp32 kernels).
+// Code of its own for the tile that is one window: with one for both, every step took 5 % longer (516 us the one below).
 //
 // Precision: the distances of the bf16 outputs from 64 bits equal those of the fp32 kernels to 1 part in 10^6, either way, over
 // M = 32 .. 128, N = 128 .. 4096, and 0.1 % of the outputs at most are rounded the other way, as there.  (Two values per operand
-// were faster, 386 us for the step below, but left 0.1 to 0.5 % of the outputs rounded the other way and an fp32 dQ ten times
+// were faster, 386 us for the step below, where three took 472 before the windows, but left 0.1 to 0.5 % of the outputs rounded the other way and an fp32 dQ ten times
 // as far from 64 bits.)  What is left is the tensor cores' own addition, which cuts off instead of rounding: 3.7e-7 of an fp32
 // dQ whatever N is, where the fp32 kernels have 2.8e-7 (N = 128) to 5.2e-7 (N = 4096).  A caller that wants dQ in fp32 gets
 // the fp32 kernels.
 //
-// B200, training step B=8 N=2048 H=16 M=64 D=32: 1823 us on the fp32 kernels, 473 us on these; the forward alone 632
+// B200, training step B=8 N=2048 H=16 M=64 D=32: 1823 us on the fp32 kernels, 493 us on these; the forward alone 632
 // and 132 us.
 #include "narrow_mma.cuh"
 
 #include <string.h>
+
+#include <type_traits>
 
 #include "bwd_exact.cuh"
 #include "sm100_ptx.cuh"
@@ -53,7 +59,7 @@ constexpr int LD = 40;         // bf16 per staged row: 80 bytes, so that the eig
 constexpr int LDP = 40;        // floats per row of a warp's partial outputs
 constexpr int STAGE = BT * LD; // bf16 elements of a staged tensor
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-constexpr float kGrowth = 57.f;  // growth of the running maximum inside a tile (log2 units) up to which nothing is lost: a
+constexpr float kGrowth = 57.f;  // growth of the running maximum inside a window (log2 units) up to which nothing is lost: a
                                  // weight flushed to zero (below 2^-126) then stood for less than 2^-69 of its row's sum
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool on) {
@@ -204,36 +210,77 @@ __device__ __forceinline__ void scores(float (&s)[2][4], const uint32_t (&qa)[2]
   }
 }
 
-// frame through the tile: c becomes the running maximum, alpha the factor from the old frame; false: grown too far for it
-__device__ __forceinline__ bool advance_frame(const float (&s)[2][4], float (&c)[2], float (&alpha)[2], int nvalid, int lane) {
+// running maximum cn of the rows through the tokens [lo, end) of the tile
+__device__ __forceinline__ void maximum_through(float (&cn)[2], const float (&s)[2][4], const float (&c)[2], int lo, int end, int lane) {
   const int q2 = (lane & 3) * 2;
-  bool ok = true;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     float top = kNegInf;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
-        if (8 * j + q2 + x < nvalid) top = fmaxf(top, s[j][2 * r + x]);
+      for (int x = 0; x < 2; ++x) {
+        const int t = 8 * j + q2 + x;
+        if (t >= lo && t < end) top = fmaxf(top, s[j][2 * r + x]);
+      }
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-    const float first = __shfl_sync(0xffffffffu, s[0][2 * r], lane & ~3);
-    const float cn = fmaxf(c[r], top);
-    ok = ok && cn - fmaxf(c[r], first) <= kGrowth;  // (false for a NaN as well)
-    alpha[r] = ex2_approx(c[r] - cn);               // (an empty state: 0)
-    c[r] = cn;
+    cn[r] = fmaxf(c[r], top);
   }
-  return ok;
 }
+__device__ __forceinline__ void change_frame(float (&c)[2], float (&alpha)[2], const float (&cn)[2]) {
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    alpha[r] = ex2_approx(c[r] - cn[r]);  // (an empty state: 0)
+    c[r] = cn[r];
+  }
+}
+// Frame through the tile: c becomes the running maximum, alpha the factor from the old frame.  False, and nothing done, where one
+// frame may not hold the tile (the first tile of all among them, which has nothing to grow from).
+__device__ __forceinline__ bool tile_frame(const float (&s)[2][4], float (&c)[2], float (&alpha)[2], int nvalid, int lane) {
+  float cn[2];
+  maximum_through(cn, s, c, 0, nvalid, lane);
+  if (__any_sync(0xffffffffu, cn[0] - c[0] > kGrowth || cn[1] - c[1] > kGrowth)) return false;
+  change_frame(c, alpha, cn);
+  return true;
+}
+// The same for a window of the tile that begins at token lo.  Returns its end: the first token that outgrows it, else nvalid.
+__device__ __forceinline__ int window_frame(const float (&s)[2][4], float (&c)[2], float (&alpha)[2], int lo, int nvalid, int lane) {
+  const int q2 = (lane & 3) * 2;
+  float low[2], cn[2];  // what the window grows from, its maximum
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float mine = (lo & 8) ? ((lo & 1) ? s[1][2 * r + 1] : s[1][2 * r]) : ((lo & 1) ? s[0][2 * r + 1] : s[0][2 * r]);
+    low[r] = fmaxf(c[r], __shfl_sync(0xffffffffu, mine, (lane & ~3) + ((lo >> 1) & 3)));
+  }
+  int end = nvalid;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = 8 * j + q2 + (i & 1);
+      if (t > lo && t < end && s[j][i] - low[i >> 1] > kGrowth) end = t;
+    }
+  end = __reduce_min_sync(0xffffffffu, end);
+  maximum_through(cn, s, c, lo, end, lane);
+  change_frame(c, alpha, cn);
+  return end;
+}
+// whether a token is of a window that is the whole tile (then all that is checked is the sequence's end), or a part of it
+template <bool WHOLE>
+__device__ __forceinline__ bool in_window(int t, int lo, int hi) { return WHOLE ? t < hi : t >= lo && t < hi; }
 
-// encoder weights in the frame c, zero from token nvalid on
-__device__ __forceinline__ void encode(float (&e)[2][4], const float (&s)[2][4], const float (&c)[2], int nvalid, int lane) {
+// encoder weights in the frame c of the window [lo, hi), zero outside
+template <bool WHOLE>
+__device__ __forceinline__ void encode(float (&e)[2][4], const float (&s)[2][4], const float (&c)[2], int lo, int hi, int lane) {
   const int q2 = (lane & 3) * 2;
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) e[j][i] = 8 * j + q2 + (i & 1) < nvalid ? ex2_approx(s[j][i] - c[i >> 1]) : 0.f;
+    for (int i = 0; i < 4; ++i) {
+      const int t = 8 * j + q2 + (i & 1);
+      e[j][i] = in_window<WHOLE>(t, lo, hi) ? ex2_approx(s[j][i] - c[i >> 1]) : 0.f;
+    }
 }
 
 // den = base + running sum over the tokens; base becomes the sum through the tile
@@ -286,6 +333,18 @@ __device__ __forceinline__ void decode_frame(float (&kap)[2][2], const float (&s
 }
 __device__ __forceinline__ float summed_frame(const float (&kap)[2][2], int lane) {  // that of summed_token
   return (lane & 16) ? ((lane & 8) ? kap[1][1] : kap[1][0]) : ((lane & 8) ? kap[0][1] : kap[0][0]);
+}
+
+// a warp's partial rows of a tile: this thread's pieces of rows g and g + 8; windows after the first one add theirs
+__device__ __forceinline__ void put_rows(float* dst, const float (&x)[4], bool add) {
+  float2 *const a = reinterpret_cast<float2*>(dst), *const b = reinterpret_cast<float2*>(dst + 8 * LDP);
+  float2 p = make_float2(x[0], x[1]), q = make_float2(x[2], x[3]);
+  if (add) {
+    const float2 p0 = *a, q0 = *b;
+    p.x += p0.x; p.y += p0.y; q.x += q0.x; q.y += q0.y;
+  }
+  *a = p;
+  *b = q;
 }
 
 template <int ROWS>
@@ -375,76 +434,96 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) narrow_mma_forward_ker
       if (nvalid <= 0) break;
       const __nv_bfloat16* const ks = kv + buf * 2 * STAGE + tile * 16 * LD;
       const __nv_bfloat16* const vs = ks + STAGE;
-      float s[2][4], e[2][4], alpha[2];
-      {
+      auto tile_scores = [&](float (&s)[2][4]) {
         uint32_t kf[2][4];
         load_rows(kf, ks, lane);
         scores(s, qa, kf, sc2);
-      }
-      ok = advance_frame(s, c, alpha, nvalid, lane) && ok;
-      encode(e, s, c, nvalid, lane);
-      d[0] *= alpha[0];
-      d[1] *= alpha[1];
-      rescale(u, alpha);
-      uint32_t vt[4][2];
-      load_cols(vt, vs, lane);
-      Split ep;
-      split_tile(ep, e[0], e[1]);
-      if constexpr (WRITE_Y) {
-        float den[2][4];
-        scan(den, e, d, lane);
-        // decode weights in the warp's own frame, their sum, R
-        float kap[2][2], part[2][2], r[2][4];
-        decode_frame(kap, s);
+      };
+      // the window [lo, hi) of the tile, whose frame is c
+      auto window = [&](auto whole, const float (&s)[2][4], const float (&alpha)[2], int lo, int hi) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        float e[2][4];
+        encode<WHOLE>(e, s, c, lo, hi, lane);
+        d[0] *= alpha[0];
+        d[1] *= alpha[1];
+        rescale(u, alpha);
+        uint32_t vt[4][2];
+        load_cols(vt, vs, lane);
+        Split ep;
+        split_tile(ep, e[0], e[1]);
+        if constexpr (WRITE_Y) {
+          float den[2][4];
+          scan(den, e, d, lane);
+          // decode weights in the warp's own frame, their sum, R
+          float kap[2][2], part[2][2], r[2][4];
+          decode_frame(kap, s);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+          for (int j = 0; j < 2; ++j) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) r[j][i] = ex2_approx(s[j][i] - kap[j][i & 1]);
-          part[j][0] = r[j][0] + r[j][2];
-          part[j][1] = r[j][1] + r[j][3];
+            for (int i = 0; i < 4; ++i) r[j][i] = ex2_approx(s[j][i] - kap[j][i & 1]);
+            part[j][0] = r[j][0] + r[j][2];
+            part[j][1] = r[j][1] + r[j][3];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) r[j][i] = 8 * j + q2 + (i & 1) < nvalid ? r[j][i] * rcp_approx(den[j][i]) : 0.f;
+            for (int i = 0; i < 4; ++i) {
+              const int t = 8 * j + q2 + (i & 1);
+              r[j][i] = in_window<WHOLE>(t, lo, hi) ? r[j][i] * rcp_approx(den[j][i]) : 0.f;
+            }
+          }
+          const float sum = sum_latents(part, lane);
+          if (!(lane & 4)) {
+            const int t = warp * BT + tile * 16 + summed_token(lane);
+            sum_s[t] = sum;
+            kap_s[t] = summed_frame(kap, lane);
+          }
+          Split rp, rt, et;
+          split_tile(rp, r[0], r[1]);
+          transpose_tile(rt, rp);  // A operand: tokens x latents
+          transpose_tile(et, ep);  // B operand over the latents
+          float y[4][4];
+          zero(y);
+          {
+            float w[2][4];
+            zero(w);
+            mma_split(w[0], rt, col<0>(et));
+            mma_split(w[1], rt, col<1>(et));
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? w[j][i] : 0.f;
+            Split wp;
+            split_tile(wp, w[0], w[1]);
+#pragma unroll
+            for (int n = 0; n < 4; ++n) mma_exact(y[n], wp, vt[n][0], vt[n][1]);
+          }
+#pragma unroll
+          for (int n = 0; n < 4; ++n) mma_split(y[n], rt, as_col(u[n]));
+          float* const dst = ypart + (warp * BT + tile * 16 + g) * LDP + q2;
+#pragma unroll
+          for (int n = 0; n < 4; ++n) put_rows(dst + 8 * n, y[n], !WHOLE && lo > 0);
+        } else {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) d[r] += quad_sum((e[0][2 * r] + e[0][2 * r + 1]) + (e[1][2 * r] + e[1][2 * r + 1]));
         }
-        const float sum = sum_latents(part, lane);
-        if (!(lane & 4)) {
-          const int t = warp * BT + tile * 16 + summed_token(lane);
-          sum_s[t] = sum;
-          kap_s[t] = summed_frame(kap, lane);
-        }
-        Split rp, rt, et;
-        split_tile(rp, r[0], r[1]);
-        transpose_tile(rt, rp);  // A operand: tokens x latents
-        transpose_tile(et, ep);  // B operand over the latents
-        float y[4][4];
-        zero(y);
-        {
-          float w[2][4];
-          zero(w);
-          mma_split(w[0], rt, col<0>(et));
-          mma_split(w[1], rt, col<1>(et));
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? w[j][i] : 0.f;
-          Split wp;
-          split_tile(wp, w[0], w[1]);
-#pragma unroll
-          for (int n = 0; n < 4; ++n) mma_exact(y[n], wp, vt[n][0], vt[n][1]);
-        }
-#pragma unroll
-        for (int n = 0; n < 4; ++n) mma_split(y[n], rt, as_col(u[n]));
-        float* const dst = ypart + (warp * BT + tile * 16 + g) * LDP + q2;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(y[n][0], y[n][1]);
-          *reinterpret_cast<float2*>(dst + 8 * LDP + 8 * n) = make_float2(y[n][2], y[n][3]);
-        }
+        for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
+      };
+      float s[2][4], alpha[2];
+      tile_scores(s);
+      if constexpr (!WRITE_Y) {  // (what is lost in a frame too high counts for nothing at the segment's end)
+        float cn[2];
+        maximum_through(cn, s, c, 0, nvalid, lane);
+        change_frame(c, alpha, cn);
+        window(std::true_type(), s, alpha, 0, nvalid);
+      } else if (tile_frame(s, c, alpha, nvalid, lane)) {
+        window(std::true_type(), s, alpha, 0, nvalid);
       } else {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) d[r] += quad_sum((e[0][2 * r] + e[0][2 * r + 1]) + (e[1][2 * r] + e[1][2 * r + 1]));
+#pragma unroll 1
+        for (int lo = 0, hi; lo < nvalid; lo = hi) {
+          tile_scores(s);
+          hi = window_frame(s, c, alpha, lo, nvalid, lane);
+          window(std::false_type(), s, alpha, lo, hi);
+        }
       }
-#pragma unroll
-      for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
     }
     if constexpr (WRITE_Y) {
       __syncthreads();
@@ -583,109 +662,135 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_replay_kern
       if (nvalid <= 0) break;
       const int64_t tile_id = (int64_t)lane_id * p.ntiles + (t0 >> 4) + tile;
       const __nv_bfloat16* const ks = block + tile * 16 * LD;
-      float s[2][4], e[2][4], den[2][4], r[2][4], alpha[2];
-      {
+      auto tile_scores = [&](float (&s)[2][4]) {
         uint32_t kf[2][4];
         load_rows(kf, ks, lane);
         scores(s, qa, kf, sc2);
-      }
-      ok = advance_frame(s, c, alpha, nvalid, lane) && ok;
-      encode(e, s, c, nvalid, lane);
-      d[0] *= alpha[0];
-      d[1] *= alpha[1];
-      rescale(u, alpha);
-      if ((lane & 3) == 0) {
+      };
+      auto window = [&](auto whole, const float (&s)[2][4], const float (&alpha)[2], int lo, int hi) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        float e[2][4], den[2][4], r[2][4];
+        encode<WHOLE>(e, s, c, lo, hi, lane);
+        if ((WHOLE || lo == 0) && (lane & 3) == 0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          p.stat_c[tile_id * p.M + m0 + g + 8 * i] = c[i];
-          p.stat_d[tile_id * p.M + m0 + g + 8 * i] = d[i];
+          for (int i = 0; i < 2; ++i) p.stat_d[tile_id * p.M + m0 + g + 8 * i] = !WHOLE && hi < nvalid ? -d[i] : d[i];
         }
-      }
-      scan(den, e, d, lane);
-      float dec[2][4];
+        d[0] *= alpha[0];
+        d[1] *= alpha[1];
+        rescale(u, alpha);
+        scan(den, e, d, lane);
+        float dec[2][4];
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const int t = 8 * j + q2 + x;
-          const float l = __shfl_sync(0xffffffffu, l2, tile * 16 + t);
+          for (int x = 0; x < 2; ++x) {
+            const int t = 8 * j + q2 + x;
+            const float l = __shfl_sync(0xffffffffu, l2, tile * 16 + t);
 #pragma unroll
-          for (int i = x; i < 4; i += 2) {
-            dec[j][i] = t < nvalid ? ex2_approx(s[j][i] - l) : 0.f;
-            r[j][i] = rcp_approx(den[j][i]);  // 1 / D
+            for (int i = x; i < 4; i += 2) {
+              dec[j][i] = t < nvalid ? ex2_approx(s[j][i] - l) : 0.f;
+              r[j][i] = in_window<WHOLE>(t, lo, hi) ? rcp_approx(den[j][i]) : 0.f;  // 1 / D
+            }
           }
+        Split ep;
+        split_tile(ep, e[0], e[1]);
+        uint32_t vf[2][4], df[2][4];
+        load_rows(vf, ks + STAGE, lane);
+        load_rows(df, ks + 2 * STAGE, lane);
+        float pp[2][4];
+        zero(pp);
+        {
+          // A^T = dY V^T, masked to tau <= t, as B operand of a product over tau
+          float at[2][4];
+          zero(at);
+#pragma unroll
+          for (int k2 = 0; k2 < 2; ++k2) {
+            uint32_t a[4];
+            as_rows(a, df, k2);
+            mma(at[0], a, vf[0][2 * k2], vf[0][2 * k2 + 1]);
+            mma(at[1], a, vf[1][2 * k2], vf[1][2 * k2 + 1]);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) at[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? at[j][i] : 0.f;
+          Split ap;
+          split_tile(ap, at[0], at[1]);  // blocks (t 0-7 | 8-15, tau 0-7), (t 0-7 | 8-15, tau 8-15)
+          mma_split(pp[0], ep, col<0>(ap));
+          mma_split(pp[1], ep, col<1>(ap));
         }
-      Split ep;
-      split_tile(ep, e[0], e[1]);
-      uint32_t vf[2][4], df[2][4];
-      load_rows(vf, ks + STAGE, lane);
-      load_rows(df, ks + 2 * STAGE, lane);
-      float pp[2][4];
-      zero(pp);
-      {
-        // A^T = dY V^T, masked to tau <= t, as B operand of a product over tau
-        float at[2][4];
-        zero(at);
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2) {
-          uint32_t a[4];
-          as_rows(a, df, k2);
-          mma(at[0], a, vf[0][2 * k2], vf[0][2 * k2 + 1]);
-          mma(at[1], a, vf[1][2 * k2], vf[1][2 * k2 + 1]);
+          Split up;
+          split_tile(up, u[2 * k2], u[2 * k2 + 1]);
+          mma_exact(pp[0], up, df[0][2 * k2], df[0][2 * k2 + 1]);
+          mma_exact(pp[1], up, df[1][2 * k2], df[1][2 * k2 + 1]);
         }
+        float part[2][2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) at[j][i] = 8 * j + q2 + (i & 1) <= g + (i >> 1) * 8 ? at[j][i] : 0.f;
-        Split ap;
-        split_tile(ap, at[0], at[1]);  // blocks (t 0-7 | 8-15, tau 0-7), (t 0-7 | 8-15, tau 8-15)
-        mma_split(pp[0], ep, col<0>(ap));
-        mma_split(pp[1], ep, col<1>(ap));
-      }
-#pragma unroll
-      for (int k2 = 0; k2 < 2; ++k2) {
-        Split up;
-        split_tile(up, u[2 * k2], u[2 * k2 + 1]);
-        mma_exact(pp[0], up, df[0][2 * k2], df[0][2 * k2 + 1]);
-        mma_exact(pp[1], up, df[1][2 * k2], df[1][2 * k2 + 1]);
-      }
-      float part[2][2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          pp[j][i] *= r[j][i];   // p
-          r[j][i] *= dec[j][i];  // R
-        }
-        part[j][0] = dec[j][0] * pp[j][0] + dec[j][2] * pp[j][2];
-        part[j][1] = dec[j][1] * pp[j][1] + dec[j][3] * pp[j][3];
-        p.p[((tile_id * nw + warp) * 2 + j) * 32 + lane] = make_float4(pp[j][0], pp[j][1], pp[j][2], pp[j][3]);
-      }
-      const float sum = sum_latents(part, lane);
-      if (!(lane & 4)) del_s[(buf * nw + warp) * BT + tile * 16 + summed_token(lane)] = sum;
-      {
-        uint32_t vt[4][2];
-        load_cols(vt, ks + STAGE, lane);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
-      }
-      if (carries) {
-        // in the frame before the segment (the frames only grow, so the factors stay below 1)
-        const float f[2] = {ex2_approx(c_start[0] - c[0]), ex2_approx(c_start[1] - c[1])};
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            r[j][i] *= f[i >> 1];
-            c0[i >> 1] = fmaf(r[j][i], pp[j][i], c0[i >> 1]);
+            pp[j][i] *= r[j][i];   // p
+            r[j][i] *= dec[j][i];  // R
           }
-        Split rp;
-        split_tile(rp, r[0], r[1]);
-        uint32_t dt[4][2];
-        load_cols(dt, ks + 2 * STAGE, lane);
+          part[j][0] = dec[j][0] * pp[j][0] + dec[j][2] * pp[j][2];
+          part[j][1] = dec[j][1] * pp[j][1] + dec[j][3] * pp[j][3];
+          // (zero outside the window)
+          float4* const out = p.p + ((tile_id * nw + warp) * 2 + j) * 32 + lane;
+          float4 x = make_float4(pp[j][0], pp[j][1], pp[j][2], pp[j][3]);
+          if (!WHOLE && lo > 0) {
+            const float4 y = *out;
+            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+          }
+          *out = x;
+        }
+        const float sum = sum_latents(part, lane);
+        if (!(lane & 4)) {
+          float* const out = del_s + (buf * nw + warp) * BT + tile * 16 + summed_token(lane);
+          *out = !WHOLE && lo > 0 ? *out + sum : sum;
+        }
+        {
+          uint32_t vt[4][2];
+          load_cols(vt, ks + STAGE, lane);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) add_product(b0[n], rp, dt[n][0], dt[n][1]);
+          for (int n = 0; n < 4; ++n) add_product(u[n], ep, vt[n][0], vt[n][1]);
+        }
+        if (carries) {
+          // in the frame before the segment (the frames only grow, so the factors stay below 1)
+          const float f[2] = {ex2_approx(c_start[0] - c[0]), ex2_approx(c_start[1] - c[1])};
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              r[j][i] *= f[i >> 1];
+              c0[i >> 1] = fmaf(r[j][i], pp[j][i], c0[i >> 1]);
+            }
+          Split rp;
+          split_tile(rp, r[0], r[1]);
+          uint32_t dt[4][2];
+          load_cols(dt, ks + 2 * STAGE, lane);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) add_product(b0[n], rp, dt[n][0], dt[n][1]);
+        }
+      };
+      float s[2][4], alpha[2];
+      tile_scores(s);
+      if (tile_frame(s, c, alpha, nvalid, lane)) {
+        window(std::true_type(), s, alpha, 0, nvalid);
+      } else {
+#pragma unroll 1
+        for (int lo = 0, hi; lo < nvalid; lo = hi) {
+          tile_scores(s);
+          hi = window_frame(s, c, alpha, lo, nvalid, lane);
+          window(std::false_type(), s, alpha, lo, hi);
+        }
       }
+      if ((lane & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) p.stat_c[tile_id * p.M + m0 + g + 8 * i] = c[i];
+      }
+      ok = ok && c[0] < INFINITY && c[1] < INFINITY;
     }
   }
   const int bad = __syncthreads_or(!ok);
@@ -790,151 +895,176 @@ __global__ void __launch_bounds__(THREADS, 384 / THREADS) narrow_mma_reverse_ker
       if (nvalid <= 0) continue;
       const int64_t tile_id = (int64_t)lane_id * p.ntiles + (t0 >> 4) + tile;
       const __nv_bfloat16* const ks = block + tile * 16 * LD;
-      const float4 p0 = p.p[((tile_id * nw + warp) * 2) * 32 + lane], p1 = p.p[((tile_id * nw + warp) * 2 + 1) * 32 + lane];
+      const float4* const pt = p.p + ((tile_id * nw + warp) * 2) * 32 + lane;
       const int64_t so = tile_id * p.M + m0 + g;
-      const float c[2] = {p.stat_c[so], p.stat_c[so + 8]};
-      float run[2] = {p.stat_d[so], p.stat_d[so + 8]};
-      const bool more = t0 + tile * 16 > tbeg;
-      const float c_prev[2] = {more ? p.stat_c[so - p.M] : c[0], more ? p.stat_c[so - p.M + 8] : c[1]};
-      const float pv[2][4] = {{p0.x, p0.y, p0.z, p0.w}, {p1.x, p1.y, p1.z, p1.w}};
-      float e[2][4], r[2][4], ds[2][4], rp[2][4];
-      {
-        float s[2][4], den[2][4];
-        uint32_t kf[2][4];
-        load_rows(kf, ks, lane);
-        scores(s, qa, kf, sc2);
-        encode(e, s, c, nvalid, lane);
-        scan(den, e, run, lane);
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const int t = 8 * j + q2 + x;
-            const float l = __shfl_sync(0xffffffffu, l2, tile * 16 + t), dl = __shfl_sync(0xffffffffu, delta, tile * 16 + t);
-#pragma unroll
-            for (int i = x; i < 4; i += 2) {
-              const float dec = t < nvalid ? ex2_approx(s[j][i] - l) : 0.f;
-              r[j][i] = dec * rcp_approx(den[j][i]);
-              rp[j][i] = r[j][i] * pv[j][i];
-              ds[j][i] = dec * (pv[j][i] - dl);  // decode part
+      // frame before the tile
+      const float* const cb = t0 + tile * 16 > tbeg ? p.stat_c + so - p.M : p.start_c + ((int64_t)lane_id * p.nseg + seg) * p.M + m0 + g;
+      // the window of the tile that ends at `end`; returns its begin
+      auto window = [&](auto whole, int end) -> int {
+        constexpr bool WHOLE = decltype(whole)::value;
+        int begin = 0;
+        float e[2][4], r[2][4], ds[2][4], rp[2][4], phi[2];  // (phi: the factor to the frame before the window)
+        {
+          const float4 p0 = pt[0], p1 = pt[32];
+          const float pv[2][4] = {{p0.x, p0.y, p0.z, p0.w}, {p1.x, p1.y, p1.z, p1.w}};
+          float c[2] = {cb[0], cb[8]}, run[2] = {p.stat_d[so], p.stat_d[so + 8]};
+          float s[2][4], den[2][4];
+          uint32_t kf[2][4];
+          load_rows(kf, ks, lane);
+          scores(s, qa, kf, sc2);
+          if constexpr (WHOLE) {
+            const float cn[2] = {p.stat_c[so], p.stat_c[so + 8]};
+            change_frame(c, phi, cn);
+          } else {
+            run[0] = fabsf(run[0]);
+            run[1] = fabsf(run[1]);
+#pragma unroll 1
+            for (;;) {
+              const int hi = window_frame(s, c, phi, begin, nvalid, lane);
+              if (hi >= end) break;
+              encode<false>(e, s, c, begin, hi, lane);
+              run[0] *= phi[0];
+              run[1] *= phi[1];
+              scan(den, e, run, lane);
+              begin = hi;
             }
           }
-      }
-      Split ep, rs;
-      split_tile(ep, e[0], e[1]);
-      split_tile(rs, r[0], r[1]);
-      uint32_t vf[2][4], dt[4][2];
-      load_rows(vf, ks + STAGE, lane);
-      load_cols(dt, ks + 2 * STAGE, lane);
-      {
-        // X = G V^T + R (A masked)^T
-        float x[2][4], a[2][4];
-        zero(x);
-        zero(a);
+          encode<WHOLE>(e, s, c, begin, end, lane);
+          run[0] *= phi[0];
+          run[1] *= phi[1];
+          scan(den, e, run, lane);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              const int t = 8 * j + q2 + x;
+              const float l = __shfl_sync(0xffffffffu, l2, tile * 16 + t), dl = __shfl_sync(0xffffffffu, delta, tile * 16 + t);
+#pragma unroll
+              for (int i = x; i < 4; i += 2) {
+                const bool on = in_window<WHOLE>(t, begin, end);
+                const float dec = on ? ex2_approx(s[j][i] - l) : 0.f;
+                r[j][i] = WHOLE || on ? dec * rcp_approx(den[j][i]) : 0.f;
+                rp[j][i] = r[j][i] * pv[j][i];
+                ds[j][i] = dec * (pv[j][i] - dl);  // decode part
+              }
+            }
+        }
+        Split ep, rs;
+        split_tile(ep, e[0], e[1]);
+        split_tile(rs, r[0], r[1]);
+        uint32_t vf[2][4], dt[4][2];
+        load_rows(vf, ks + STAGE, lane);
+        load_cols(dt, ks + 2 * STAGE, lane);
         {
-          uint32_t df[2][4];
-          load_rows(df, ks + 2 * STAGE, lane);
+          // X = G V^T + R (A masked)^T
+          float x[2][4], a[2][4];
+          zero(x);
+          zero(a);
+          {
+            uint32_t df[2][4];
+            load_rows(df, ks + 2 * STAGE, lane);
+#pragma unroll
+            for (int k2 = 0; k2 < 2; ++k2) {
+              uint32_t va[4];
+              as_rows(va, vf, k2);
+              mma(a[0], va, df[0][2 * k2], df[0][2 * k2 + 1]);
+              mma(a[1], va, df[1][2 * k2], df[1][2 * k2 + 1]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? a[j][i] : 0.f;  // row tau, column t
+          Split ap;
+          split_tile(ap, a[0], a[1]);  // blocks (tau 0-7 | 8-15, t 0-7), (tau 0-7 | 8-15, t 8-15)
+          mma_split(x[0], rs, col<0>(ap));
+          mma_split(x[1], rs, col<1>(ap));
 #pragma unroll
           for (int k2 = 0; k2 < 2; ++k2) {
-            uint32_t va[4];
-            as_rows(va, vf, k2);
-            mma(a[0], va, df[0][2 * k2], df[0][2 * k2 + 1]);
-            mma(a[1], va, df[1][2 * k2], df[1][2 * k2 + 1]);
+            Split gp;
+            split_tile(gp, gr[2 * k2], gr[2 * k2 + 1]);
+            mma_exact(x[0], gp, vf[0][2 * k2], vf[0][2 * k2 + 1]);
+            mma_exact(x[1], gp, vf[1][2 * k2], vf[1][2 * k2 + 1]);
+          }
+          // encoder part: C + sum of R p from the token on
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            float behind = cc[i];
+#pragma unroll
+            for (int j = 1; j >= 0; --j) {
+              float suf = rp[j][2 * i] + rp[j][2 * i + 1];
+              float t = __shfl_down_sync(0xffffffffu, suf, 1, 4);
+              if (q <= 2) suf += t;
+              t = __shfl_down_sync(0xffffffffu, suf, 2, 4);
+              if (q <= 1) suf += t;
+              const float later = __shfl_down_sync(0xffffffffu, suf, 1, 4), total = __shfl_sync(0xffffffffu, suf, 0, 4);
+              const float from1 = (q <= 2 ? behind + later : behind) + rp[j][2 * i + 1], from0 = from1 + rp[j][2 * i];
+              ds[j][2 * i] = fmaf(e[j][2 * i], x[j][2 * i] - from0, ds[j][2 * i]);
+              ds[j][2 * i + 1] = fmaf(e[j][2 * i + 1], x[j][2 * i + 1] - from1, ds[j][2 * i + 1]);
+              behind += total;
+            }
+            cc[i] = behind;
           }
         }
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) a[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? a[j][i] : 0.f;  // row tau, column t
-        Split ap;
-        split_tile(ap, a[0], a[1]);  // blocks (tau 0-7 | 8-15, t 0-7), (tau 0-7 | 8-15, t 8-15)
-        mma_split(x[0], rs, col<0>(ap));
-        mma_split(x[1], rs, col<1>(ap));
-#pragma unroll
-        for (int k2 = 0; k2 < 2; ++k2) {
-          Split gp;
-          split_tile(gp, gr[2 * k2], gr[2 * k2 + 1]);
-          mma_exact(x[0], gp, vf[0][2 * k2], vf[0][2 * k2 + 1]);
-          mma_exact(x[1], gp, vf[1][2 * k2], vf[1][2 * k2 + 1]);
-        }
-        // encoder part: C + sum of R p from the token on
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          float behind = cc[i];
-#pragma unroll
-          for (int j = 1; j >= 0; --j) {
-            float suf = rp[j][2 * i] + rp[j][2 * i + 1];
-            float t = __shfl_down_sync(0xffffffffu, suf, 1, 4);
-            if (q <= 2) suf += t;
-            t = __shfl_down_sync(0xffffffffu, suf, 2, 4);
-            if (q <= 1) suf += t;
-            const float later = __shfl_down_sync(0xffffffffu, suf, 1, 4), total = __shfl_sync(0xffffffffu, suf, 0, 4);
-            const float from1 = (q <= 2 ? behind + later : behind) + rp[j][2 * i + 1], from0 = from1 + rp[j][2 * i];
-            ds[j][2 * i] = fmaf(e[j][2 * i], x[j][2 * i] - from0, ds[j][2 * i]);
-            ds[j][2 * i + 1] = fmaf(e[j][2 * i + 1], x[j][2 * i + 1] - from1, ds[j][2 * i + 1]);
-            behind += total;
-          }
-          cc[i] = behind;
-        }
-      }
-      Split et;
-      transpose_tile(et, ep);
-      float out[4][4];
-      zero(out);
-      {
-        // dV = E^T G + (E^T R masked) dY
-        float w[2][4];
-        zero(w);
-        Split rt;
-        transpose_tile(rt, rs);
-        mma_split(w[0], et, col<0>(rt));
-        mma_split(w[1], et, col<1>(rt));
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? w[j][i] : 0.f;
-        Split wp;
-        split_tile(wp, w[0], w[1]);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) mma_exact(out[n], wp, dt[n][0], dt[n][1]);
-      }
-#pragma unroll
-      for (int n = 0; n < 4; ++n) mma_split(out[n], et, as_col(gr[n]));
-      float* dst = part + (warp * BT + tile * 16 + g) * LDP + q2;
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(out[n][0], out[n][1]);
-        *reinterpret_cast<float2*>(dst + 8 * LDP + 8 * n) = make_float2(out[n][2], out[n][3]);
-      }
-      // G += R dY, then into the frame of the tile before
-#pragma unroll
-      for (int n = 0; n < 4; ++n) add_product(gr[n], rs, dt[n][0], dt[n][1]);
-      const float phi[2] = {ex2_approx(c_prev[0] - c[0]), ex2_approx(c_prev[1] - c[1])};
-      rescale(gr, phi);
-      cc[0] *= phi[0];
-      cc[1] *= phi[1];
-      // dK = dS^T Q, dQ += dS K
-      Split dsp, dst_t;
-      split_tile(dsp, ds[0], ds[1]);
-      transpose_tile(dst_t, dsp);
-      {
-        uint32_t qf[4][2];
-        load_cols(qf, qs + m0 * LD, lane);
+        Split et;
+        transpose_tile(et, ep);
+        float out[4][4];
         zero(out);
+        {
+          // dV = E^T G + (E^T R masked) dY
+          float w[2][4];
+          zero(w);
+          Split rt;
+          transpose_tile(rt, rs);
+          mma_split(w[0], et, col<0>(rt));
+          mma_split(w[1], et, col<1>(rt));
 #pragma unroll
-        for (int n = 0; n < 4; ++n) mma_exact(out[n], dst_t, qf[n][0], qf[n][1]);
-      }
-      dst += nw * BT * LDP;
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        *reinterpret_cast<float2*>(dst + 8 * n) = make_float2(out[n][0], out[n][1]);
-        *reinterpret_cast<float2*>(dst + 8 * LDP + 8 * n) = make_float2(out[n][2], out[n][3]);
-      }
-      {
-        uint32_t kt[4][2];
-        load_cols(kt, ks, lane);
+            for (int i = 0; i < 4; ++i) w[j][i] = 8 * j + q2 + (i & 1) >= g + (i >> 1) * 8 ? w[j][i] : 0.f;
+          Split wp;
+          split_tile(wp, w[0], w[1]);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) add_product(dq[n], dsp, kt[n][0], kt[n][1]);
+          for (int n = 0; n < 4; ++n) mma_exact(out[n], wp, dt[n][0], dt[n][1]);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) mma_split(out[n], et, as_col(gr[n]));
+        float* dst = part + (warp * BT + tile * 16 + g) * LDP + q2;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) put_rows(dst + 8 * n, out[n], !WHOLE && end < nvalid);
+        // G += R dY, then into the frame before the window
+#pragma unroll
+        for (int n = 0; n < 4; ++n) add_product(gr[n], rs, dt[n][0], dt[n][1]);
+        rescale(gr, phi);
+        cc[0] *= phi[0];
+        cc[1] *= phi[1];
+        // dK = dS^T Q, dQ += dS K
+        Split dsp, dst_t;
+        split_tile(dsp, ds[0], ds[1]);
+        transpose_tile(dst_t, dsp);
+        {
+          uint32_t qf[4][2];
+          load_cols(qf, qs + m0 * LD, lane);
+          zero(out);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) mma_exact(out[n], dst_t, qf[n][0], qf[n][1]);
+        }
+        dst += nw * BT * LDP;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) put_rows(dst + 8 * n, out[n], !WHOLE && end < nvalid);
+        {
+          uint32_t kt[4][2];
+          load_cols(kt, ks, lane);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) add_product(dq[n], dsp, kt[n][0], kt[n][1]);
+        }
+        return begin;
+      };
+      if (!signbit(p.stat_d[so])) {
+        window(std::true_type(), nvalid);
+      } else {  // (the tile was taken in several windows: from the last to the first)
+#pragma unroll 1
+        for (int end = nvalid; end > 0;) end = window(std::false_type(), end);
       }
     }
     __syncthreads();

@@ -23,7 +23,8 @@ struct NarrowMmaParams {
   int gate_stride;                    // forward: words per lane, behind a leading one
   // backward
   int ntiles;                         // tiles of 16 tokens in a lane
-  float *stat_c, *stat_d;             // [lanes][ntiles][M]: frame of the tile (log2 units), denominator before it in that frame
+  float *stat_c, *stat_d;             // [lanes][ntiles][M]: frame after the tile (log2 units); denominator before the tile, in the frame
+                                      // before it, with a minus sign where the tile was taken in several windows
   float *start_c;                     // [lanes][nseg][M]: frame before the segment
   float4* p;                          // [lanes][ntiles][M / 16][2][32]: p = <z_t[m], dY_t>, in the order of a warp's registers
   float *tok_l2, *tok_delta;          // [lanes][ntiles * 16]: decode log-sum-exp (log2 units), <dY_t, y_t>

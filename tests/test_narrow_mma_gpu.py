@@ -1,4 +1,4 @@
-"""Narrow heads on the tensor cores (bf16, softmax): as close to 64 bits as the fp32 kernels, and theirs where it leaves its domain."""
+"""Narrow heads on the tensor cores (bf16, softmax): as close to 64 bits as the fp32 kernels, sharp scores, values that are not finite."""
 import pytest
 import torch
 
@@ -75,7 +75,7 @@ def test_dq_in_fp32_is_that_of_the_fp32_kernels():
 
 @pytest.mark.parametrize("std", [4.0, 24.0])
 def test_sharp_scores(monkeypatch, std):
-    # at 24 the running maximum grows by hundreds of powers of two inside tiles: the fp32 kernels standing by redo those lanes
+    # at 24 the running maximum grows by hundreds of powers of two inside tiles, which are taken in several windows
     B, N, H, M, D = 2, 200, 4, 32, 32
     q, k, v, dy = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=22, dtype=torch.bfloat16, with_dy=True))
     a, b = (step(monkeypatch, path, q * std, k, v, dy) for path in ("auto", "exact"))
@@ -100,3 +100,38 @@ def test_head_slices(monkeypatch):
     k2, v2, dy2 = (torch.cat([t, t], dim=2)[:, :, :H] for t in (k, v, dy))
     for x, y in zip(step(monkeypatch, "auto", q, k, v, dy), step(monkeypatch, "auto", q, k2, v2, dy2)):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("shape, sharp", [((2, 77, 2, 32, 32, 32), 1.0), ((1, 300, 2, 128, 32, 32), 20.0), ((1, 16, 1, 16, 16, 32), 20.0)])
+def test_windows(monkeypatch, shape, sharp):
+    # One latent's score rises by 60 nats at ten tokens: next to one another, at edges of tiles, two in one tile; the others are
+    # sharp by themselves or not.  (600 nats in all: 64 bits hold 700.)  As close to 64 bits as the fp32 kernels.
+    B, N, H, M, Dk, Dv = shape
+    q, k, v, dy = orc.make_inputs(B, N, H, M, Dk, Dv, seed0=27, dtype=torch.bfloat16, with_dy=True)
+    q = (q.float() * sharp).bfloat16()
+    steps = torch.zeros(N)
+    steps[[t for t in (1, 2, 9, 15, 16, 31, 33, 47, 60, 70) if t < N]] = 1
+    q[:, 0], q[:, 1:, 0], k[..., 0] = 0, 0, steps.cumsum(0).bfloat16()[None, :, None]
+    q[:, 0, 0] = 60 * Dk ** 0.5
+    want = (orc.ar_forward(q, k, v),) + tuple(orc.ar_backward_closed_form(q, k, v, dy)[n] for n in ("dQ", "dK", "dV"))
+    got = {path: step(monkeypatch, path, *to_dev(q, k, v, dy)) for path in ("auto", "exact")}
+    for i, name in enumerate(("y", "dQ", "dK", "dV")):
+        err = {path: orc.rel_l2(out[i].float().cpu(), want[i]) for path, out in got.items()}
+        assert err["auto"] <= 1.05 * err["exact"] + 2.0 ** -9 / want[i].numel() ** 0.5, f"{name}: {err}"
+
+
+def test_sharp_scores_stay_on_the_tensor_cores():
+    # (the kernels standing by walk a lane with one CTA: 20 times the call's time)
+    q, k, v = to_dev(*orc.make_inputs(2, 1000, 4, 64, 32, seed0=28, dtype=torch.bfloat16))
+    def best(q):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                cf.flare_autoregressive_triton(q, k, v)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    assert best(q * 200) <= 4 * best(q)
