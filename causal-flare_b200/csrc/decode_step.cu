@@ -58,6 +58,7 @@ __device__ __forceinline__ void lane_scores(float* out, const float* tok, const 
       const int m = m0 + a * (NT / 8) + grp;
       if (m >= me) continue;
       if constexpr (SLICED) {
+        // (one thread of the latent's eight for every CTA of the cluster: eight at most)
         if (gl < slices) sm100::st_cluster_f32(sm100::mapa_shared(sm100::smem_u32(out + m), gl), acc[a] * scale);
       } else if (gl == 0) {
         out[m] = acc[a] * scale;
@@ -262,8 +263,8 @@ int launch_decode_step(const DecodeParams& p, cudaStream_t stream) {
   const int64_t lanes = (int64_t)p.B * p.H, slots = 2 * (int64_t)sm_count();
   if (lanes > slots) return launch_variant<4, 4, 4, 4, false>(p, smem, 1, stream);
   constexpr int PRE = 8;
-  int slices = 1;
-  while (p.M <= NT && p.M * (p.Dv / 4) > slices * PRE * NT && lanes * slices * 2 <= slots && p.Dv / 4 % (slices * 16) == 0) slices *= 2;
+  int slices = 1;  // (eight at most: what a cluster may have without being asked for more, and what lane_scores serves)
+  while (slices < 8 && p.M <= NT && p.M * (p.Dv / 4) > slices * PRE * NT && lanes * slices * 2 <= slots && p.Dv / 4 % (slices * 16) == 0) slices *= 2;
   return slices == 1 ? launch_variant<PRE, 8, 2, 4, false>(p, smem, 1, stream)
                      : launch_variant<PRE, 8, 2, 4, true>(p, smem, slices, stream);
 }

@@ -8,6 +8,10 @@ from util import assert_close, to_dev
 
 pytestmark = pytest.mark.gpu
 
+# Widths above 128: eight slices, where a lane doubles to them and just below; as many as are allowed of wider ones, which would
+# double further (512 and 1024 columns); few latents, or too few columns per slice, that stop earlier.
+WIDE = [(1, 2, 256, 128, 256), (1, 3, 144, 64, 256), (2, 1, 128, 64, 256), (1, 2, 256, 128, 512), (1, 2, 144, 32, 512), (1, 1, 256, 64, 1024),
+        (1, 2, 80, 64, 1024), (2, 1, 16, 64, 1024), (19, 1, 256, 64, 512)]
 # four slices; four with a number of latents that they do not share evenly by 32; two (64 columns); too many latents to slice; a lane
 # whose state just fits what is asked for ahead, and one latent group more; more lanes than two CTAs per SM, with and without a
 # remainder of the streaming loop
@@ -17,7 +21,7 @@ SHAPES = [(1, 2, 256, 128, 128), (2, 3, 208, 128, 128), (1, 1, 144, 64, 64), (1,
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("separate", [False, True])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + WIDE)
 def test_step(shape, separate, dtype):
     # fp32: about 2^8 terms summed in another order, exponentials of the fast unit: 1e-5.  bf16: one rounding of y.
     B, H, M, Dk, Dv = shape
