@@ -36,7 +36,9 @@ template <int AHEAD, bool SLICED>
 __device__ __forceinline__ void lane_scores(float* out, const float* tok, const void* lat, int dtype, int64_t lat_off,
                                             int64_t lat_stride_m, int mb, int me, int Dk, float scale, int slices) {
   const int grp = threadIdx.x >> 3, gl = threadIdx.x & 7;
-  for (int m0 = mb; m0 < me; m0 += AHEAD * (NT / 8)) {
+  // (latents come in multiples of 16, so a warp's four rows are all there, or its part of a slice ends inside it)
+  constexpr bool ALL_THERE = AHEAD == 1 && !SLICED;
+  for (int m0 = mb; m0 + (grp & ~3) < me; m0 += AHEAD * (NT / 8)) {  // (whole warps: the shuffles below)
     float acc[AHEAD];
 #pragma unroll
     for (int a = 0; a < AHEAD; ++a) acc[a] = 0.f;
@@ -44,7 +46,7 @@ __device__ __forceinline__ void lane_scores(float* out, const float* tok, const 
       float qv[AHEAD][8];
 #pragma unroll
       for (int a = 0; a < AHEAD; ++a)
-        load8(lat, dtype, lat_off + (int64_t)min(m0 + a * (NT / 8) + grp, me - 1) * lat_stride_m + d0, qv[a]);
+        load8(lat, dtype, lat_off + (int64_t)(ALL_THERE ? m0 + grp : min(m0 + a * (NT / 8) + grp, me - 1)) * lat_stride_m + d0, qv[a]);
 #pragma unroll
       for (int a = 0; a < AHEAD; ++a)
 #pragma unroll
@@ -56,7 +58,7 @@ __device__ __forceinline__ void lane_scores(float* out, const float* tok, const 
       acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 2);
       acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 1);
       const int m = m0 + a * (NT / 8) + grp;
-      if (m >= me) continue;
+      if (!ALL_THERE && m >= me) continue;
       if constexpr (SLICED) {
         // (one thread of the latent's eight for every CTA of the cluster: eight at most)
         if (gl < slices) sm100::st_cluster_f32(sm100::mapa_shared(sm100::smem_u32(out + m), gl), acc[a] * scale);
@@ -70,7 +72,8 @@ __device__ __forceinline__ void lane_scores(float* out, const float* tok, const 
 }  // namespace
 
 // PRE: state vectors per thread issued before the score phase; UNR: state vectors in flight per thread in the
-// streaming loop; MINB: CTAs per SM the register budget is held to; AHEAD: latent rows in flight per thread in the scores
+// streaming loop (0: PRE vectors are all there is); MINB: CTAs per SM the register budget is held to; AHEAD: latent rows in flight per
+// thread in the scores
 // SLICED: the lane's value columns are shared by the CTAs of a cluster (blockIdx.y).  Each computes the scores of its part of the
 // latents and sends them to the others; the statistics are the business of all of them and written by the first.
 template <int PRE, int UNR, int MINB, int AHEAD, bool SLICED>
@@ -104,14 +107,16 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   }
 
   if constexpr (SLICED) sm100::cluster_arrive();  // (a CTA may be written to once it runs)
-  float4* u4 = reinterpret_cast<float4*>(p.u + (int64_t)lane_id * M * Dv) + col4;
+  // rows row0, row0 + rows_per_pass, ... of this thread's columns: NT * slices vectors apart, a constant for a whole lane
+  float4* const u4 = reinterpret_cast<float4*>(p.u + (int64_t)lane_id * M * Dv) + (SLICED ? row0 * dv4 + col4 : tid);
+  const int step = NT * slices;
 
   // phase 0: first state vectors in flight, and the statistics of this thread's first latent
   float4 pre[PRE];
 #pragma unroll
   for (int i = 0; i < PRE; ++i) {
     const int r = row0 + i * rows_per_pass;
-    pre[i] = r < M ? load_streaming(u4 + (int64_t)r * dv4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pre[i] = r < M ? load_streaming(u4 + i * step) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float* gm = p.m + (int64_t)lane_id * M;
   float* gd = p.d + (int64_t)lane_id * M;
@@ -175,13 +180,13 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
   // phase 3: stream the state
   const float4 v4 = reinterpret_cast<const float4*>(vtok)[col4];
   float4 yacc = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto apply = [&](float4 x, int row) {
+  auto apply = [&](float4 x, int row, int at) {
     const float g = gam[row], e = s_sc[row], w = a_sc[row];
     x.x = x.x * g + e * v4.x;
     x.y = x.y * g + e * v4.y;
     x.z = x.z * g + e * v4.z;
     x.w = x.w * g + e * v4.w;
-    __stcs(u4 + (int64_t)row * dv4, x);
+    __stcs(u4 + at, x);
     yacc.x += w * x.x;
     yacc.y += w * x.y;
     yacc.z += w * x.z;
@@ -190,17 +195,29 @@ __global__ void __launch_bounds__(NT, MINB) decode_step_kernel(const DecodeParam
 #pragma unroll
   for (int i = 0; i < PRE; ++i) {
     const int r = row0 + i * rows_per_pass;
-    if (r < M) apply(pre[i], r);
+    if (r < M) apply(pre[i], r, i * step);
   }
-  int r = row0 + PRE * rows_per_pass;
-  for (; r + (UNR - 1) * rows_per_pass < M; r += UNR * rows_per_pass) {
-    float4 x[UNR];
+  if constexpr (UNR > 0) {
+    int r = row0 + PRE * rows_per_pass, at = PRE * step;
+    for (; r + (UNR - 1) * rows_per_pass < M; r += UNR * rows_per_pass, at += UNR * step) {
+      float4 x[UNR];
 #pragma unroll
-    for (int i = 0; i < UNR; ++i) x[i] = load_streaming(u4 + (int64_t)(r + i * rows_per_pass) * dv4);
+      for (int i = 0; i < UNR; ++i) x[i] = load_streaming(u4 + at + i * step);
 #pragma unroll
-    for (int i = 0; i < UNR; ++i) apply(x[i], r + i * rows_per_pass);
+      for (int i = 0; i < UNR; ++i) apply(x[i], r + i * rows_per_pass, at + i * step);
+    }
+    if constexpr (MINB == 4) {  // what is left, together too (the registers of the others do not allow it, or the code costs more)
+      float4 x[UNR - 1];
+#pragma unroll
+      for (int i = 0; i < UNR - 1; ++i)
+        if (r + i * rows_per_pass < M) x[i] = load_streaming(u4 + at + i * step);
+#pragma unroll
+      for (int i = 0; i < UNR - 1; ++i)
+        if (r + i * rows_per_pass < M) apply(x[i], r + i * rows_per_pass, at + i * step);
+    } else {
+      for (; r < M; r += rows_per_pass, at += step) apply(load_streaming(u4 + at), r, at);
+    }
   }
-  for (; r < M; r += rows_per_pass) apply(load_streaming(u4 + (int64_t)r * dv4), r);
 
   // reduce y over the row groups that share a column
   ypart[tid] = yacc;
@@ -249,24 +266,46 @@ static int launch_variant(const DecodeParams& p, size_t smem, int slices, cudaSt
   return FLARE_OK;
 }
 
+template <int PRE, int UNR, int MINB, bool SLICED>
+static int launch_ahead(const DecodeParams& p, size_t smem, int slices, cudaStream_t stream) {
+  // rows of 32 latents per round of the scores: as many as there are, or what loads the fewest of them twice
+  const int rows = ((p.M + slices - 1) / slices + 31) / 32;
+  constexpr int MOST = MINB == 8 ? 2 : 4;  // (more do not fit 32 registers)
+  const int ahead = rows <= MOST ? rows : (MOST == 2 ? 2 : (rows % 4 == 1 || rows % 4 == 2 ? 3 : 4));
+  if (ahead == 1) return launch_variant<PRE, UNR, MINB, 1, SLICED>(p, smem, slices, stream);
+  if (ahead == 2) return launch_variant<PRE, UNR, MINB, 2, SLICED>(p, smem, slices, stream);
+  if constexpr (MOST == 4) {
+    if (ahead == 3) return launch_variant<PRE, UNR, MINB, 3, SLICED>(p, smem, slices, stream);
+    return launch_variant<PRE, UNR, MINB, 4, SLICED>(p, smem, slices, stream);
+  }
+  return FLARE_ERR_UNSUPPORTED;
+}
+
 int launch_decode_step(const DecodeParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)(3 * p.M + 2 * p.Dk + p.Dv + NW) * 4 + NT * 16;
   // What counts is how much of the state is on its way: a thread needs registers for the vectors that it has asked for.  At 32
-  // registers (eight CTAs per SM, the choice before) the compiler asks for one at a time.  Per step, us on B200 with the state
-  // cold, <2, 4, 8> of 32 registers / <4, 4, 4> / <8, 8, 2> / the sliced one:
-  //   2048 lanes of 128 KB 121 / 97 / 99 / 108     2048 lanes of 64 KB 65 / 52 / 56 / 69     768 lanes of 32 KB 19 / 16 / 18 / 23
+  // registers (eight CTAs per SM) the compiler asks for one at a time.  Per step, us on B200 with the state cold, eight CTAs / four /
+  // two, in columns of their own / sliced:
+  //   2048 lanes of 128 KB 121 / 97 / 99 / 108     2048 lanes of 64 KB 65 / 52 / 56 / 69      768 lanes of 32 KB 19 / 16 / 18 / 23
   //    256 lanes of 128 KB  49 / 21 / 17 / 18        96 lanes of 64 KB 12.4 / 10.9 / 8.0 / 7.8     16 lanes of 128 KB 16.6 / 11.2 / 9.3 / 6.8
   // So: four CTAs per SM while there are lanes for more than two, else two with twice the vectors, and a lane whose state does
   // not fit the vectors asked for ahead is cut into column slices (128 bytes wide at least) while two per SM hold them all.
+  // Small states of many lanes have little to ask for; there eight CTAs per SM, which hide the phases before the state, are the
+  // better ones (us a step among others, eight / four): 2048 lanes of 8 KB (M = 32, D = 64) 15.2 / 17.4, 1024 lanes 9.1 / 9.7, M = 16 with keys 512 wide 18.3 / 23.2; of 16 KB
+  // (M = 64) 21.1 / 21.6 with 2048 lanes, 12.4 / 12.1 with 1024.
+  // The rows of the latent bank in flight follow the latents that there are: four CTAs with four rows were 19.1 us at M = 32.
   // Measured and rejected on the largest shape: one kernel for the coefficients of all lanes and one that only streams (98 to
   // 103), 128-thread CTAs (121.7 against 112), bulk async copies through a shared-memory ring (115.5 to 207).
-  const int64_t lanes = (int64_t)p.B * p.H, slots = 2 * (int64_t)sm_count();
-  if (lanes > slots) return launch_variant<4, 4, 4, 4, false>(p, smem, 1, stream);
+  const int64_t lanes = (int64_t)p.B * p.H, sms = sm_count();
+  const int vectors = p.M * (p.Dv / 4);
+  if (lanes > 4 * sms && vectors <= 2 * NT) return launch_ahead<2, 0, 8, false>(p, smem, 1, stream);
+  if (lanes > 8 * sms && vectors <= 4 * NT) return launch_ahead<2, 4, 8, false>(p, smem, 1, stream);
+  if (lanes > 2 * sms) return launch_ahead<4, 4, 4, false>(p, smem, 1, stream);
   constexpr int PRE = 8;
   int slices = 1;  // (eight at most: what a cluster may have without being asked for more, and what lane_scores serves)
-  while (slices < 8 && p.M <= NT && p.M * (p.Dv / 4) > slices * PRE * NT && lanes * slices * 2 <= slots && p.Dv / 4 % (slices * 16) == 0) slices *= 2;
-  return slices == 1 ? launch_variant<PRE, 8, 2, 4, false>(p, smem, 1, stream)
-                     : launch_variant<PRE, 8, 2, 4, true>(p, smem, slices, stream);
+  while (slices < 8 && p.M <= NT && vectors > slices * PRE * NT && lanes * slices * 2 <= 2 * sms && p.Dv / 4 % (slices * 16) == 0)
+    slices *= 2;
+  return slices == 1 ? launch_ahead<PRE, 8, 2, false>(p, smem, 1, stream) : launch_ahead<PRE, 8, 2, true>(p, smem, slices, stream);
 }
 
 }  // namespace flare

@@ -12,6 +12,10 @@ pytestmark = pytest.mark.gpu
 # double further (512 and 1024 columns); few latents, or too few columns per slice, that stop earlier.
 WIDE = [(1, 2, 256, 128, 256), (1, 3, 144, 64, 256), (2, 1, 128, 64, 256), (1, 2, 256, 128, 512), (1, 2, 144, 32, 512), (1, 1, 256, 64, 1024),
         (1, 2, 80, 64, 1024), (2, 1, 16, 64, 1024), (19, 1, 256, 64, 512)]
+# Many lanes: a state of 8 KB at most, just above it, of 16 KB with more than eight lanes per SM and just above that, of 24 KB, whose last
+# vectors are a batch of their own; one to eight rows of latents, an odd number of them; a key wider than a round of its columns.
+MANY = [(38, 16, 32, 64, 64), (38, 16, 48, 64, 64), (75, 16, 64, 64, 64), (75, 16, 80, 64, 64), (38, 16, 96, 64, 64), (75, 16, 16, 512, 64),
+        (38, 16, 128, 32, 16), (19, 16, 160, 64, 64), (19, 16, 176, 64, 32), (38, 16, 208, 64, 32), (1, 2, 96, 64, 64), (1, 3, 16, 96, 64)]
 # four slices; four with a number of latents that they do not share evenly by 32; two (64 columns); too many latents to slice; a lane
 # whose state just fits what is asked for ahead, and one latent group more; more lanes than two CTAs per SM, with and without a
 # remainder of the streaming loop
@@ -21,7 +25,7 @@ SHAPES = [(1, 2, 256, 128, 128), (2, 3, 208, 128, 128), (1, 1, 144, 64, 64), (1,
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("separate", [False, True])
-@pytest.mark.parametrize("shape", SHAPES + WIDE)
+@pytest.mark.parametrize("shape", SHAPES + WIDE + MANY)
 def test_step(shape, separate, dtype):
     # fp32: about 2^8 terms summed in another order, exponentials of the fast unit: 1e-5.  bf16: one rounding of y.
     B, H, M, Dk, Dv = shape
