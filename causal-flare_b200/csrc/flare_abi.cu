@@ -3,6 +3,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <initializer_list>
+
 #include "bwd_exact.cuh"
 #include "bwd_tc.cuh"
 #include "decode_step.cuh"
@@ -53,9 +55,6 @@ ScratchLimit::~ScratchLimit() { g_scratch_limit = before; }
 static size_t scratch_left(size_t taken) {
   return g_scratch_limit == SIZE_MAX ? SIZE_MAX : (g_scratch_limit > taken ? g_scratch_limit - taken : 0);
 }
-// y of the forward in flight on this thread is fp16 although its inputs are bf16 (copies), see forward_cast
-static thread_local bool g_y_f16 = false;
-
 // masked call in flight on this thread whose packed copies the forward runs on, see forward_masked
 struct MaskedRows {
   const int32_t* start;
@@ -274,8 +273,7 @@ int launch_walk(const flare_fwd_args_t* a, const FwdPlan& pl, const WalkParams& 
     t.part_lw = reinterpret_cast<float*>(reinterpret_cast<char*>(t.part_y) + prefill_tc_partial_lw_offset(a));
   }
   t.trace = g_trace;
-  t.in_f16 = a->dtype == FLARE_F16 ? 1 : 0;
-  t.y_f16 = t.in_f16 || g_y_f16 ? 1 : 0;
+  t.f16 = a->dtype == FLARE_F16 ? 1 : 0;
   t.gate = g_gate;
   t.gate_stride = pl.gate_stride;
   // (the state pass over all segments but the last comes first)
@@ -309,10 +307,7 @@ int launch_guard_walk(const flare_fwd_args_t* a, const int* lane_gates, int gate
   return launch_walk_exact(w, 1, stream);
 }
 
-// `orig`: the fp16 call behind one that runs on bf16 copies (forward_cast below).  The standby walk of the flagged lanes takes
-// the caller's own fp16 tensors, so that the lanes whose score spreads left the tensor kernels' domain - where the rounding
-// of q and k to bf16 would move the scores most - are computed from the unrounded inputs.
-int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, const flare_fwd_args_t* orig = nullptr) {
+int forward_run(const flare_fwd_args_t* a, cudaStream_t stream) {
   const FwdPlan pl = plan_forward(a);
   if (g_keep.u != nullptr) return forward_tensor_or_exact(a, pl, stream);  // the backward's own replay of the forward
   int* gate = nullptr;
@@ -336,7 +331,7 @@ int forward_run(const flare_fwd_args_t* a, cudaStream_t stream, const flare_fwd_
   g_keep = ChunkStates{nullptr, nullptr, nullptr, 0};
   if (rc != FLARE_OK) return rc;
   if (a->path == FLARE_PATH_AUTO && a->lengths == nullptr) {
-    rc = launch_guard_walk(orig != nullptr ? orig : a, gate + 1, pl.gate_stride, stream);
+    rc = launch_guard_walk(a, gate + 1, pl.gate_stride, stream);
     g_last_launches += 1;
   }
   return rc;
@@ -403,64 +398,90 @@ int forward_tensor_or_exact(const flare_fwd_args_t* a, const FwdPlan& pl, cudaSt
   return launch_walk(a, pl, w, pl.nseg, stream);
 }
 
-// fp16 inputs on the tensor-core kernels.  The forward kernels take them as they are (prefill_tc_supported_f16).  What is left
-// for copies are the tensors whose strides a tiled copy cannot express (expanded over heads, say): q, k, v are copied to
-// dense bf16 in the workspace and the bf16 forward runs on those and writes y as fp16, which is 40 to 60 times faster than the
-// exact walk the call would otherwise take.  Lanes that the kernels flag as outside their numeric domain are recomputed
-// by the exact kernels from the fp16 tensors themselves, either way.  States and log-sum-exps are fp32 and go straight
-// to the caller's buffers.  Not for the training forward (no state is kept for a backward) and not with separate decode
-// weights or a mask, which the tensor kernels do not take.
-struct CastPlan {
-  bool on;
-  size_t off_q, off_k, off_v, total;
+// fp16 inputs on the tensor-core kernels.  The forward kernels take them as they are (prefill_tc_supported_f16), where a tiled copy
+// can express their strides.  Of a tensor whose strides it cannot (expanded over heads, say) a dense copy is made in the
+// workspace first, which is 40 to 60 times faster than the exact walk the call would otherwise take.  Not for the training
+// forward (no state is kept for a backward) and not with separate decode weights or a mask, which the tensor kernels do not
+// take.  (Dense copies in bf16 of all three, and kernels that told them from fp16 inputs at run time, were 146 us at B=4 N=4096
+// H=16 M=64 D=128 with a bank expanded over the heads.)
+struct CopyPlan {
+  bool on;  // an fp16 call for the tensor kernels, with copies (of q, k, v) or without
+  bool copy[3];
+  size_t off[3], total;
 };
 
-CastPlan plan_cast(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
-  CastPlan cp{false, 0, 0, 0, 0};
+CopyPlan plan_copies(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
+  CopyPlan cp;
+  memset(&cp, 0, sizeof(cp));
   if (a->dtype != FLARE_F16 || a->path == FLARE_PATH_EXACT || a->keep != nullptr || a->q_dec != nullptr ||
       a->k_dec != nullptr || a->mask != nullptr || a->B == 0 || a->N == 0 || !f16_on_tensor_kernels())
     return cp;
   *b = *a;
-  b->dtype = FLARE_BF16;
-  b->q_stride_m = a->Dk; b->q_stride_h = (int64_t)a->M * a->Dk;
-  b->k_stride_h = a->Dk; b->k_stride_n = (int64_t)a->H * a->Dk; b->k_stride_b = (int64_t)a->N * b->k_stride_n;
-  b->v_stride_h = a->Dv; b->v_stride_n = (int64_t)a->H * a->Dv; b->v_stride_b = (int64_t)a->N * b->v_stride_n;
-  if (!prefill_tc_supported(b)) return cp;
+  auto tiled = [](std::initializer_list<int64_t> strides) {
+    for (int64_t st : strides)
+      if (!prefill_tc_stride(st)) return false;
+    return true;
+  };
+  if (!tiled({a->q_stride_h, a->q_stride_m})) {
+    cp.copy[0] = true;
+    b->q_stride_m = a->Dk; b->q_stride_h = (int64_t)a->M * a->Dk;
+  }
+  if (!tiled({a->k_stride_b, a->k_stride_n, a->k_stride_h})) {
+    cp.copy[1] = true;
+    b->k_stride_h = a->Dk; b->k_stride_n = (int64_t)a->H * a->Dk; b->k_stride_b = (int64_t)a->N * b->k_stride_n;
+  }
+  if (!tiled({a->v_stride_b, a->v_stride_n, a->v_stride_h})) {
+    cp.copy[2] = true;
+    b->v_stride_h = a->Dv; b->v_stride_n = (int64_t)a->H * a->Dv; b->v_stride_b = (int64_t)a->N * b->v_stride_n;
+  }
+  if (!prefill_tc_supported_f16(b)) return cp;
   const size_t rows = (size_t)a->B * a->N * a->H;
   cp.on = true;
-  cp.off_q = 0;
-  cp.off_k = align_up((size_t)a->H * a->M * a->Dk * 2, 256);
-  cp.off_v = cp.off_k + align_up(rows * a->Dk * 2, 256);
-  // (The size that callers plan with: it has room for a y in bf16, which nothing uses, and a call without copies asks for it too.)
-  cp.total = cp.off_v + align_up(rows * a->Dv * 2, 256) * (a->y != nullptr ? 2 : 1);
+  cp.off[1] = align_up((size_t)a->H * a->M * a->Dk * 2, 256);
+  cp.off[2] = cp.off[1] + align_up(rows * a->Dk * 2, 256);
+  // The size that callers plan with does not depend on the strides: it has room for copies of q, k, v and of y, used or not
+  // (flare_forward_noalloc chooses between the tensor and the exact kernels by it).
+  cp.total = cp.off[2] + align_up(rows * a->Dv * 2, 256) * (a->y != nullptr ? 2 : 1);
   return cp;
 }
 
-int forward_cast(const flare_fwd_args_t* a, flare_fwd_args_t& b, const CastPlan& cp, cudaStream_t stream) {
+int forward_copied(const flare_fwd_args_t* a, flare_fwd_args_t& b, const CopyPlan& cp, cudaStream_t stream) {
   const ScratchLimit limit(scratch_left(cp.total));
   const size_t inner = plan_forward(&b).ws_bytes;
   if (a->workspace == nullptr || a->workspace_bytes < cp.total + inner || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
   char* ws = reinterpret_cast<char*>(a->workspace);
-  b.q = ws + cp.off_q; b.k = ws + cp.off_k; b.v = ws + cp.off_v;
   b.workspace = inner > 0 ? ws + cp.total : nullptr;
   b.workspace_bytes = inner > 0 ? a->workspace_bytes - cp.total : 0;
   CastParams c[3];
   memset(c, 0, sizeof(c));
-  c[0].in = a->q; c[0].out = const_cast<void*>(b.q); c[0].n0 = 1; c[0].n1 = a->H; c[0].n2 = a->M; c[0].d = a->Dk;
-  c[0].is1 = a->q_stride_h; c[0].is2 = a->q_stride_m; c[0].os1 = b.q_stride_h; c[0].os2 = b.q_stride_m;
-  c[1].in = a->k; c[1].out = const_cast<void*>(b.k); c[1].n0 = a->B; c[1].n1 = a->N; c[1].n2 = a->H; c[1].d = a->Dk;
-  c[1].is0 = a->k_stride_b; c[1].is1 = a->k_stride_n; c[1].is2 = a->k_stride_h;
-  c[1].os0 = b.k_stride_b; c[1].os1 = b.k_stride_n; c[1].os2 = b.k_stride_h;
-  c[2].in = a->v; c[2].out = const_cast<void*>(b.v); c[2].n0 = a->B; c[2].n1 = a->N; c[2].n2 = a->H; c[2].d = a->Dv;
-  c[2].is0 = a->v_stride_b; c[2].is1 = a->v_stride_n; c[2].is2 = a->v_stride_h;
-  c[2].os0 = b.v_stride_b; c[2].os1 = b.v_stride_n; c[2].os2 = b.v_stride_h;
-  int rc = launch_cast_rows(c, 3, false, stream);
+  int count = 0;
+  if (cp.copy[0]) {
+    CastParams& t = c[count++];
+    b.q = ws + cp.off[0];
+    t.in = a->q; t.out = const_cast<void*>(b.q); t.n0 = 1; t.n1 = a->H; t.n2 = a->M; t.d = a->Dk;
+    t.is1 = a->q_stride_h; t.is2 = a->q_stride_m; t.os1 = b.q_stride_h; t.os2 = b.q_stride_m;
+  }
+  if (cp.copy[1]) {
+    CastParams& t = c[count++];
+    b.k = ws + cp.off[1];
+    t.in = a->k; t.out = const_cast<void*>(b.k); t.n0 = a->B; t.n1 = a->N; t.n2 = a->H; t.d = a->Dk;
+    t.is0 = a->k_stride_b; t.is1 = a->k_stride_n; t.is2 = a->k_stride_h;
+    t.os0 = b.k_stride_b; t.os1 = b.k_stride_n; t.os2 = b.k_stride_h;
+  }
+  if (cp.copy[2]) {
+    CastParams& t = c[count++];
+    b.v = ws + cp.off[2];
+    t.in = a->v; t.out = const_cast<void*>(b.v); t.n0 = a->B; t.n1 = a->N; t.n2 = a->H; t.d = a->Dv;
+    t.is0 = a->v_stride_b; t.is1 = a->v_stride_n; t.is2 = a->v_stride_h;
+    t.os0 = b.v_stride_b; t.os1 = b.v_stride_n; t.os2 = b.v_stride_h;
+  }
+  if (count > 0) {
+    const int rc = launch_cast_rows(c, count, CAST_COPY, stream);
+    if (rc != FLARE_OK) return rc;
+  }
+  const int rc = forward_run(&b, stream);
   if (rc != FLARE_OK) return rc;
-  g_y_f16 = true;
-  rc = forward_run(&b, stream, a);  // gate words in b's workspace
-  g_y_f16 = false;
-  if (rc != FLARE_OK) return rc;
-  g_last_launches += 1;
+  g_last_launches += count > 0 ? 1 : 0;
   return FLARE_OK;
 }
 
@@ -474,14 +495,14 @@ struct MaskedPlan {
   size_t off_lens, off_start, off_k, off_v, off_y, total;
 };
 
-// scratch of the forward on the packed copies (SIZE_MAX: not on the tensor kernels); cast: it is an fp16 call that makes
-// bf16 copies, for a latent bank whose strides a tiled copy cannot express
-size_t masked_inner_bytes(const flare_fwd_args_t* b, bool* cast = nullptr) {
+// scratch of the forward on the packed copies (SIZE_MAX: not on the tensor kernels); copied: it is an fp16 call that copies a
+// latent bank whose strides a tiled copy cannot express
+size_t masked_inner_bytes(const flare_fwd_args_t* b, bool* copied = nullptr) {
   const FwdPlan pl = plan_forward(b);
-  if (cast != nullptr) *cast = !pl.use_tc;
+  if (copied != nullptr) *copied = !pl.use_tc;
   if (pl.use_tc) return pl.ws_bytes;
   flare_fwd_args_t c;
-  const CastPlan cp = plan_cast(b, &c);
+  const CopyPlan cp = plan_copies(b, &c);
   return cp.on ? cp.total + plan_forward(&c).ws_bytes : SIZE_MAX;
 }
 
@@ -494,7 +515,7 @@ MaskedPlan plan_masked(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
   *b = *a;
   b->mask = nullptr;
   flare_fwd_args_t c;
-  if (!plan_forward(b).use_tc && !plan_cast(b, &c).on) return mp;
+  if (!plan_forward(b).use_tc && !plan_copies(b, &c).on) return mp;
   b->lengths = a->mask;  // (any non-null pointer until the lengths have their place)
   b->k_stride_h = a->Dk; b->k_stride_n = (int64_t)a->H * a->Dk; b->k_stride_b = (int64_t)a->N * b->k_stride_n;
   b->v_stride_h = a->Dv; b->v_stride_n = (int64_t)a->H * a->Dv; b->v_stride_b = (int64_t)a->N * b->v_stride_n;
@@ -519,8 +540,8 @@ MaskedPlan plan_masked(const flare_fwd_args_t* a, flare_fwd_args_t* b) {
 }
 
 int forward_masked(const flare_fwd_args_t* a, flare_fwd_args_t& b, const MaskedPlan& mp, cudaStream_t stream) {
-  bool cast = false;
-  const size_t inner = masked_inner_bytes(&b, &cast);
+  bool copied = false;
+  const size_t inner = masked_inner_bytes(&b, &copied);
   if (a->workspace == nullptr || a->workspace_bytes < mp.total + inner || !aligned16(a->workspace)) return FLARE_ERR_WORKSPACE;
   char* ws = reinterpret_cast<char*>(a->workspace);
   int32_t* const slot = reinterpret_cast<int32_t*>(ws);
@@ -548,10 +569,10 @@ int forward_masked(const flare_fwd_args_t* a, flare_fwd_args_t& b, const MaskedP
   rc = launch_move_rows(p, 2, stream);
   if (rc != FLARE_OK) return rc;
   const MaskedRows rows{start, a};
-  if (cast) {
+  if (copied) {
     flare_fwd_args_t c;
-    const CastPlan cp = plan_cast(&b, &c);
-    rc = forward_cast(&b, c, cp, stream);
+    const CopyPlan cp = plan_copies(&b, &c);
+    rc = forward_copied(&b, c, cp, stream);
   } else {
     g_rows = start != nullptr ? &rows : nullptr;
     rc = forward_run(&b, stream);
@@ -652,7 +673,7 @@ extern "C" {
 size_t flare_forward_workspace_bytes(const flare_fwd_args_t* args) {
   if (check_forward(args) != FLARE_OK) return 0;
   flare_fwd_args_t b;
-  const CastPlan cp = plan_cast(args, &b);
+  const CopyPlan cp = plan_copies(args, &b);
   if (cp.on) {
     const ScratchLimit limit(scratch_left(cp.total));
     return cp.total + plan_forward(&b).ws_bytes;
@@ -686,13 +707,8 @@ int flare_forward(const flare_fwd_args_t* args, flare_stream_t stream) {
     return FLARE_OK;
   }
   flare_fwd_args_t b;
-  const CastPlan cp = plan_cast(args, &b);
-  if (cp.on && !prefill_tc_supported_f16(args)) return forward_cast(args, b, cp, stream);
-  if (cp.on) {  // nothing is copied, but a workspace that would not have held the copies is refused all the same
-    const ScratchLimit limit(scratch_left(cp.total));
-    if (args->workspace == nullptr || args->workspace_bytes < cp.total + plan_forward(&b).ws_bytes) return FLARE_ERR_WORKSPACE;
-    return forward_run(args, stream);  // (planned within what is left, as the size was)
-  }
+  const CopyPlan cp = plan_copies(args, &b);
+  if (cp.on) return forward_copied(args, b, cp, stream);
   return forward_run(args, stream);
 }
 
@@ -800,7 +816,7 @@ int backward_cast(const flare_bwd_args_t* a, flare_bwd_args_t& b, const BwdCastP
     t.is0 = is[i][0]; t.is1 = is[i][1]; t.is2 = is[i][2];
     t.os0 = os[i][0]; t.os1 = os[i][1]; t.os2 = os[i][2];
   }
-  int rc = launch_cast_rows(c, 4, false, stream);
+  int rc = launch_cast_rows(c, 4, CAST_TO_BF16, stream);
   if (rc != FLARE_OK) return rc;
   rc = bwd_tc(b, stream);
   if (rc != FLARE_OK) return rc;
@@ -809,7 +825,7 @@ int backward_cast(const flare_bwd_args_t* a, flare_bwd_args_t& b, const BwdCastP
   c[0].in = b.dk; c[0].out = a->dk; c[0].is0 = c[0].os0; c[0].is1 = c[0].os1; c[0].is2 = c[0].os2;
   c[1] = c[2];
   c[1].in = b.dv; c[1].out = a->dv; c[1].is0 = c[1].os0; c[1].is1 = c[1].os1; c[1].is2 = c[1].os2;
-  rc = launch_cast_rows(c, 2, true, stream);
+  rc = launch_cast_rows(c, 2, CAST_TO_F16, stream);
   if (rc != FLARE_OK) return rc;
   g_last_launches += 2;
   return FLARE_OK;
@@ -965,7 +981,7 @@ void flare_set_trace_buffer(void* device_buffer) { g_trace = static_cast<long lo
 int flare_forward_uses_tensor_path(const flare_fwd_args_t* args) {
   if (check_forward(args) != FLARE_OK) return 0;
   flare_fwd_args_t b;
-  if (plan_cast(args, &b).on) return 1;
+  if (plan_copies(args, &b).on) return 1;
   return plan_forward(args).use_tc ? 1 : 0;
 }
 

@@ -32,8 +32,8 @@ int flare_forward_noalloc(const flare_fwd_args_t* args, flare_stream_t stream) {
   const flare::ScratchLimit limit(FLARE_NOALLOC_SCRATCH_BYTES);
   size_t need = flare_forward_workspace_bytes(&a);
   if (need > sizeof(g_flare_noalloc_scratch) && a.dtype == FLARE_F16 && a.path != FLARE_PATH_EXACT) {
-    // the tensor-core route of an fp16 call asks for room for bf16 copies of its tensors; when those do not fit the
-    // built-in scratch the call runs on the exact kernels
+    // the tensor-core route of an fp16 call asks for room for copies of its tensors (which it makes where no tiled copy can
+    // express their strides); when those do not fit the built-in scratch the call runs on the exact kernels
     a.path = FLARE_PATH_EXACT;
     need = flare_forward_workspace_bytes(&a);
   }

@@ -214,7 +214,7 @@ int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk
 //       width 256 ([E | U_bf16] as one B operand, [W | Y] adjacent in tensor memory), so R is read once for both; W
 //       shares the columns of S; E and R are single-buffered.
 // FL:   0 = bf16, every row N tokens long; 1 = bf16 with per-row lengths and, of a masked call, rows that were not packed;
-//       2 = fp16 y (of fp16 inputs, or of bf16 copies: p.in_f16), with lengths or not.  Instances of their own: as run-time choices they cost every bf16 call 2 to 3 % (B200:
+//       2 = fp16, with lengths or not.  Instances of their own: as run-time choices they cost every bf16 call 2 to 3 % (B200:
 //       B=8 N=8192 H=16 M=128 D=64 182.3 -> 185.8 us, training B=4 N=4096 H=16 M=64 D=128 411 -> 424 us), and the type of y in
 //       the epilogue of the wide instance 5 to 8 %.
 template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
@@ -337,7 +337,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // fp16 inputs: Q and K go to the score product as they are; V, which meets bf16 weights, is rounded to bf16 in place by
       // this warp (one tile behind the loads, so that the next chunk's K never waits for it).  B200, B=4 N=4096 H=16 M=64 D=128:
       // 130 us with bf16 copies of K and V made before the kernel (a pass of 42 us over them), 93 us this way.
-      const unsigned active = p.in_f16 ? 0xffffffffu : 1u;  // (bf16: the one thread that issues the loads)
+      constexpr unsigned active = F16 ? 0xffffffffu : 1u;  // (bf16: the one thread that issues the loads)
       auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(active, wait_or_abort(bar, parity, misc)) != 0; };
       auto convert_v = [&](int i) -> bool {
         const int st = i & 1;
@@ -356,7 +356,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         warp_arrive(&misc->v_conv[st], lane);
         return true;
       };
-      if (lane == 0 || p.in_f16) {
+      if (lane == 0 || F16) {
         const int vc0 = value_col0<ZS, SPLIT>();
         // a row of a masked call that was not packed: its tokens are the last ones of the caller's row
         const int row0 = p.row_start != nullptr ? p.row_start[b] : -1;
@@ -380,7 +380,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
             for (int kb = 0; kb < DKB; ++kb) tma_load_4d(smem + OFF_K + kb * 16384, mk, &misc->k_full, kb * 64, h, t0, b);
           }
-          if (p.in_f16 && i > 0 && !(ok = convert_v(i - 1))) break;
+          if (F16 && i > 0 && !(ok = convert_v(i - 1))) break;
           // V tile: stage i & 1, free once chunk i - 2 has been folded into Y
           const int st = i & 1;
           if (i >= 2 && !(ok = wait_all(&misc->v_empty[st], ((i - 2) >> 1) & 1))) break;
@@ -391,7 +391,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               tma_load_4d(smem + OFF_V + (st * VB + vb) * 16384, mv, &misc->v_full[st], vc0 + vb * 64, h, t0, b);
           }
         }
-        if (p.in_f16 && ok && nchunks > 0) ok = convert_v(nchunks - 1);
+        if (F16 && ok && nchunks > 0) ok = convert_v(nchunks - 1);
       }
     }
   } else if (warp == 12) {
@@ -400,8 +400,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const uint32_t k_addr = smem_u32(smem + OFF_K);
       const uint32_t b16_addr = smem_u32(smem + OFF_B16);
       // Q (TMEM) x K_c (K-major): both as the caller has them, bf16 or fp16
-      const uint32_t ID_S = F16 && p.in_f16 ? make_idesc_f16(128, 128, 0, 0) : make_idesc_bf16(128, 128, 0, 0);
-      uint64_t* const v_ready = F16 && p.in_f16 ? misc->v_conv : misc->v_full;  // the V tile is in place, as bf16
+      constexpr uint32_t ID_S = F16 ? make_idesc_f16(128, 128, 0, 0) : make_idesc_bf16(128, 128, 0, 0);
+      uint64_t* const v_ready = F16 ? misc->v_conv : misc->v_full;  // the V tile is in place, as bf16
       constexpr uint32_t ID_U = make_idesc_bf16(128, WIDE ? 128 : 64, 0, 1);  // E (K-major) x V (MN-major)
       constexpr uint32_t ID_DEN = make_idesc_bf16(128, 16, 1, 0);  // R (MN-major) x d tile (K-major)
       constexpr uint32_t ID_Y1 = make_idesc_bf16(128, WIDE ? 128 : 64, 0, 1);  // tril(W) (TMEM) x V (MN-major)
@@ -1443,7 +1443,7 @@ int launch_instance(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
                     const TcParams& p, dim3 grid, cudaStream_t stream) {
   if (p.dump_u != nullptr)  // training forward that keeps its per-chunk states
     return launch_keep<LAT, DKB, DVB, SPLIT, MODE, true, WIDE, 0>(tq, tk, tv, ty, in, p, grid, stream);
-  if (p.y_f16) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 2>(tq, tk, tv, ty, in, p, grid, stream);
+  if (p.f16) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 2>(tq, tk, tv, ty, in, p, grid, stream);
   if constexpr (MODE != 1) {  // (no lengths in block-causal calls)
     if (p.lens != nullptr) return launch_keep<LAT, DKB, DVB, SPLIT, MODE, false, WIDE, 1>(tq, tk, tv, ty, in, p, grid, stream);
   }
@@ -1508,6 +1508,8 @@ bool make_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims
 
 }  // namespace
 
+bool prefill_tc_stride(int64_t st) { return st > 0 && (st % 8) == 0 && st < (int64_t(1) << 39); }
+
 bool prefill_tc_supported(const flare_fwd_args_t* a) { return a->dtype == FLARE_BF16 && prefill_tc_shape(a); }
 
 bool prefill_tc_supported_f16(const flare_fwd_args_t* a) {
@@ -1522,12 +1524,11 @@ bool prefill_tc_shape(const flare_fwd_args_t* a) {
   if (a->lengths != nullptr && bs > 1) return false;  // per-row lengths: token-causal only
   // stablemax encoder weights: token-causal only
   const bool variant_ok = a->variant == FLARE_SOFTMAX || (a->variant == FLARE_STABLEMAX && bs == 1 && a->power > 0.f);
-  // the tiled copies need positive strides whose byte size is a multiple of 16 and stays below 2^40; anything else
-  // (a tensor expanded over heads with stride 0, say) is served by the exact kernels
+  // (of a tensor expanded over heads, with a stride of 0, fp16 calls make a copy; bf16 ones are served by the exact kernels)
   const int64_t strides[] = {a->k_stride_b, a->k_stride_n, a->k_stride_h, a->v_stride_b, a->v_stride_n, a->v_stride_h,
                              a->q_stride_h, a->q_stride_m};
   for (int64_t st : strides)
-    if (st <= 0 || (st % 8) != 0 || st >= (int64_t(1) << 39)) return false;
+    if (!prefill_tc_stride(st)) return false;
   return variant_ok && block_ok && lse_ok && a->M <= 4 * M && a->M >= 16 &&
          (a->M % 16) == 0 && ((a->Dk == 64 && (a->Dv == 64 || a->Dv == 128)) || (a->Dk == 128 && a->Dv == 128)) && a->q_dec == nullptr &&
          a->k_dec == nullptr && a->mask == nullptr && a->N >= 1;
@@ -1681,7 +1682,7 @@ bool prefill_tc_rows_in_place(const flare_fwd_args_t* a) {
   if (!prefill_tc_shape(a)) return false;
   if (a->y == nullptr) return true;
   for (int64_t st : {a->y_stride_b, a->y_stride_n, a->y_stride_h})
-    if (st <= 0 || (st % 8) != 0 || st >= (int64_t(1) << 39)) return false;
+    if (!prefill_tc_stride(st)) return false;
   return (reinterpret_cast<uintptr_t>(a->y) % 16) == 0;
 }
 
@@ -1748,7 +1749,7 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
     const uint32_t box[4] = {32, 1, 32, 1};
     const int64_t str[3] = {p.y_stride_h, p.y_stride_n, p.y_stride_b};
     bool y_ok = (reinterpret_cast<uintptr_t>(p.y) % 16) == 0;
-    for (int64_t st : str) y_ok = y_ok && st > 0 && (st % 8) == 0 && st < (int64_t(1) << 39);
+    for (int64_t st : str) y_ok = y_ok && prefill_tc_stride(st);
     const uint64_t ydims[4] = {(uint64_t)a->Dv, (uint64_t)a->H, (uint64_t)a->N, (uint64_t)a->B};
     // wide instance with exactly two latent groups: the two CTAs of a lane merge on chip (thread-block cluster) and
     // store y themselves.  FLARE_B200_CLUSTER=0 keeps the partials in global memory and the merge kernel.
@@ -1794,7 +1795,7 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
   LaunchTimer timer("tc_merge_groups_kernel", stream);
   FLARE_CUDA_CHECK(launch_pdl(tc_merge_groups_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream,
                               reinterpret_cast<const __half*>(p.part_y), p.part_lw, groups, rows, a->N, a->H, a->Dv,
-                              reinterpret_cast<uint16_t*>(p.y), p.y_f16, p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
+                              reinterpret_cast<uint16_t*>(p.y), p.f16, p.y_stride_b, p.y_stride_n, p.y_stride_h, p.lse_dec, p.lens,
                               p.row_start, direct != nullptr ? reinterpret_cast<uint16_t*>(direct->y) : nullptr,
                               direct != nullptr ? direct->y_stride_b : 0, direct != nullptr ? direct->y_stride_n : 0,
                               direct != nullptr ? direct->y_stride_h : 0, p.gate, p.gate_stride, p.gate_off));

@@ -27,8 +27,7 @@ struct TcParams {
   // the read-out rows leave through tiled bulk stores (set by the launch when the output's strides allow it and no
   // per-row lengths are given); otherwise every thread stores its own row
   int y_tma;
-  int y_f16;   // y is fp16: rounded once, from the fp32 accumulators
-  int in_f16;  // q, k, v are fp16 (a call with fp16 y whose inputs are bf16 copies has y_f16 alone)
+  int f16;  // q, k, v and y are fp16 (y: rounded once, from the fp32 accumulators)
   // Two latent groups on the wide instance: the two CTAs of a lane form a thread-block cluster and merge their
   // partial read-outs on chip (each finalises one 64-column value block); no partials in global memory, no merge
   // kernel.  Set by the launch.
@@ -57,6 +56,8 @@ struct TcParams {
   long long* trace;  // optional diagnostic cycle stamps of CTA (0, 0), see TC_TRACE; null in normal use
 };
 
+// a tiled copy can express this stride (elements): positive, a multiple of 16 bytes, below 2^40 bytes
+bool prefill_tc_stride(int64_t st);
 bool prefill_tc_supported(const flare_fwd_args_t* a);      // a bf16 call runs on these kernels
 bool prefill_tc_supported_f16(const flare_fwd_args_t* a);  // an fp16 call does, without copies (no training forward)
 bool prefill_tc_shape(const flare_fwd_args_t* a);          // what both ask of sizes, strides and options

@@ -29,7 +29,7 @@ struct CastList {
 
 // blockIdx.y = tensor.  Bound by memory; a tensor that is one dense run needs no index arithmetic (three 64-bit divisions for
 // every 16-byte piece otherwise).
-template <bool TO_F16>
+template <Cast CAST>
 __global__ void __launch_bounds__(256) cast_rows_kernel(const __grid_constant__ CastList list) {
   pdl_begin();
   const CastParams& p = list.t[blockIdx.y];
@@ -54,11 +54,11 @@ __global__ void __launch_bounds__(256) cast_rows_kernel(const __grid_constant__ 
     uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (TO_F16) {
+      if (CAST == CAST_TO_F16) {
         const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
         const __half2 h = __floats2half2_rn(f.x, f.y);
         w[j] = *reinterpret_cast<const uint32_t*>(&h);
-      } else {
+      } else if (CAST == CAST_TO_BF16) {
         const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
         const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
         w[j] = *reinterpret_cast<const uint32_t*>(&h);
@@ -164,7 +164,7 @@ int launch_move_rows(const MoveRowsParams& p, int tensors, cudaStream_t stream) 
   return FLARE_OK;
 }
 
-int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t stream) {
+int launch_cast_rows(const CastParams* p, int count, Cast cast, cudaStream_t stream) {
   CastList list;
   memset(&list, 0, sizeof(list));
   int64_t most = 0;
@@ -186,9 +186,11 @@ int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t s
   int64_t blocks = (most + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  LaunchTimer timer(to_f16 ? "cast_rows_kernel<bf16 to fp16>" : "cast_rows_kernel<fp16 to bf16>", stream);
-  FLARE_CUDA_CHECK(launch_pdl(to_f16 ? cast_rows_kernel<true> : cast_rows_kernel<false>, dim3((unsigned)blocks, count), dim3(256),
-                              0, stream, list));
+  const char* const names[] = {"cast_rows_kernel<fp16 to bf16>", "cast_rows_kernel<bf16 to fp16>", "cast_rows_kernel<copy>"};
+  auto* const kernel = cast == CAST_COPY ? cast_rows_kernel<CAST_COPY>
+                                         : (cast == CAST_TO_F16 ? cast_rows_kernel<CAST_TO_F16> : cast_rows_kernel<CAST_TO_BF16>);
+  LaunchTimer timer(names[cast], stream);
+  FLARE_CUDA_CHECK(launch_pdl(kernel, dim3((unsigned)blocks, count), dim3(256), 0, stream, list));
   return FLARE_OK;
 }
 

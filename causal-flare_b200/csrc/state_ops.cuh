@@ -23,7 +23,7 @@ struct FoldParams {
 
 int launch_fold(const FoldParams& p, cudaStream_t stream);
 
-// fp16 <-> bf16 copy of a tensor of rows: n0 x n1 x n2 rows of d contiguous 2-byte elements (d a multiple of 8, row
+// Copy of a tensor of rows, fp16 <-> bf16 or as it is: n0 x n1 x n2 rows of d contiguous 2-byte elements (d a multiple of 8, row
 // starts 16-byte aligned), row (i0, i1, i2) at element offset i0 * s0 + i1 * s1 + i2 * s2 on either side.
 struct CastParams {
   const void* in;
@@ -33,8 +33,9 @@ struct CastParams {
   int64_t os0, os1, os2;
 };
 
-// up to four tensors in one launch, all in one direction
-int launch_cast_rows(const CastParams* p, int count, bool to_f16, cudaStream_t stream);
+enum Cast { CAST_TO_BF16 = 0, CAST_TO_F16 = 1, CAST_COPY = 2 };
+// up to four tensors in one launch, all alike
+int launch_cast_rows(const CastParams* p, int count, Cast cast, cudaStream_t stream);
 
 // Compaction of masked rows (2-byte elements, head widths that are multiples of 8, 16-byte aligned rows).
 // slot[b][n] = number of valid tokens before token n of row b, or -1 for a masked token; lens[b] = valid tokens of the row.

@@ -259,7 +259,7 @@ int flare_profile_entry(int i, const char** name, float* ms);
 void flare_set_trace_buffer(void* device_buffer);
 
 /* 1 when flare_forward would take the tcgen05 tensor-core path for this problem, else 0.  That is: path AUTO or
- * TENSOR, bf16 (or fp16 without args->keep: read as they are, or through bf16 copies in the workspace where a tiled copy cannot
+ * TENSOR, bf16 (or fp16 without args->keep: read as they are, or copied to the workspace first where a tiled copy cannot
  * express their strides; flare_forward_workspace_bytes has room for the copies either way), 16 <= M <= 512 (multiple of 16), (Dk, Dv) = (64, 64), (128, 128) or (64, 128), shared decode weights (q_dec = k_dec = NULL),
  * mask = NULL, and either the softmax encoder with block_size 1 / 16 / 32 / 64 / 128 (N a multiple of it) or the
  * stablemax encoder with block_size 1; lse_enc only with block_size > 1; lengths only with block_size 1. */

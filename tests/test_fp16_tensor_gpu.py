@@ -1,5 +1,5 @@
-"""fp16 inputs on the tensor-core prefill: the library rounds q, k, v to bf16 copies in its workspace, runs the bf16
-kernels on them and writes y back as fp16.  Every case is held to the oracle on the fp16 inputs with the bf16 gate
+"""fp16 inputs on the tensor-core kernels: the forward reads q, k, v as they are (tensors that no tiled copy can express are
+copied first), rounds V to bf16 on chip and writes y as fp16; the backward runs on bf16 copies.  Every case is held to the oracle on the fp16 inputs with the bf16 gate
 (the products inside the kernels are bf16 for every input type), and to the exact kernels, which read fp16 directly."""
 import ctypes as C
 
@@ -180,8 +180,8 @@ def test_fp16_training_step_through_autograd():
 
 
 def test_fp16_through_the_entry_point_that_allocates_nothing():
-    # the bf16 copies live in the library's built-in scratch when they fit it (same bits as flare_forward with a
-    # workspace); when they do not, the call runs on the exact kernels, which read fp16 directly
+    # a call whose workspace, with room for copies of its tensors, fits the built-in scratch gives the same bits as
+    # flare_forward with a workspace; any other runs on the exact kernels
     lib = _lib.load()
     cap = lib.flare_noalloc_scratch_capacity()
     stream = torch.cuda.current_stream().cuda_stream
@@ -202,9 +202,8 @@ def test_fp16_through_the_entry_point_that_allocates_nothing():
 @pytest.mark.parametrize("shape", [(1, 1, 1, 16, 64, 64), (2, 128, 2, 64, 64, 64), (1, 257, 2, 128, 64, 128), (1, 640, 2, 96, 128, 128),
                                    (1, 384, 3, 128, 128, 128), (1, 200, 2, 256, 128, 128), (1, 131, 1, 192, 64, 64), (1, 6000, 1, 64, 64, 64)])
 def test_fp16_tensors_read_in_place_and_through_copies(shape, variant):
-    # One head expanded over all of them has a stride of zero, which no tiled copy can express: bf16 copies.  The same numbers
-    # laid out in full are read as they are, with scores from the unrounded q and k: no further from the oracle than the
-    # copies (which round both), to the 2 % that the roundings of the weights, which both share, can fall the other way.
+    # One head expanded over all of them has a stride of zero, which no tiled copy can express: it is copied first.  The same
+    # numbers laid out in full are read as they are.
     B, N, H, M, Dk, Dv = shape
     if variant == "block":
         N = max(N // 64, 1) * 64
@@ -224,3 +223,18 @@ def test_fp16_tensors_read_in_place_and_through_copies(shape, variant):
         ref = orc.ar_forward(qc, kc, vc, scale=Dk ** -0.5, **(dict(variant="stablemax") if variant == "stablemax" else {}))
     err = [orc.rel_l2(t.float().cpu(), ref) for t in (copies, direct)]
     assert err[1] <= 1.02 * err[0] + 2e-4 and err[1] <= 5e-3, err
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "qkv"])
+@pytest.mark.parametrize("shape", [(2, 130, 3, 64, 64, 64), (1, 640, 2, 256, 128, 128), (1, 4096, 2, 96, 64, 128)])
+def test_fp16_expanded_tensors_are_copied_as_they_are(shape, which):
+    # the same numbers through the same kernel: the same bits, whichever of the tensors is copied
+    B, N, H, M, Dk, Dv = shape
+    q, k, v = to_dev(*orc.make_inputs(B, N, H, M, Dk, Dv, seed0=58, dtype=F16))
+    one = dict(q=q[:1].expand(H, M, Dk), k=k[:, :, :1].expand(B, N, H, Dk), v=v[:, :, :1].expand(B, N, H, Dv))
+    args = [one[name] if name in which else t for name, t in (("q", q), ("k", k), ("v", v))]
+    y, st, lse, _ = run(*args, want_state=True, want_lse=True)
+    y2, st2, lse2, _ = run(*(t.contiguous() for t in args), want_state=True, want_lse=True)
+    assert torch.equal(y, y2) and torch.equal(lse, lse2)
+    for key in ("m", "d", "u"):
+        assert torch.equal(st[key], st2[key]), key

@@ -118,7 +118,7 @@ def test_left_padded_rows_stay_where_they_are(monkeypatch, B, N, H, M, D, wide, 
 
 
 def test_masked_fp16_with_a_bank_expanded_over_the_heads():
-    # (a stride of zero, which no tiled copy can express: bf16 copies of the packed rows)
+    # (a stride of zero, which no tiled copy can express: the bank is copied, the packed rows are not)
     B, N, H, M, D = 2, 200, 2, 64, 64
     q, k, v = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=14, dtype=torch.float16))
     mask = torch.rand(B, N, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) < 0.7
