@@ -990,7 +990,7 @@ struct StandbyParams {
   // tasks of every phase, in the order above (sizes of a grid in x, y, z; scan, sum: blocks of 256 elements in x)
   int nx[kStandbyPhases], ny[kStandbyPhases], nz[kStandbyPhases];
   const int* gate;
-  int* sync;  // [1 + kStandbyPhases] words, zero before the launch: tasks handed out, tasks done of every phase
+  int* sync;  // kBwdSyncWords words, zero before the launch: tasks handed out, tasks done of every phase, someone has given up
   int* err;
 };
 // defined once per MM_MAX in {2, 8, 16, 32, 64}, each in its own translation unit
