@@ -1,4 +1,6 @@
 """Masked prefill on the tensor kernels: packing and unpacking of the valid tokens, and an fp16 read-out."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -127,3 +129,31 @@ def test_masked_fp16_with_a_bank_expanded_over_the_heads():
     b = cf.flare_autoregressive_prefill_triton(shared.contiguous(), k, v, scale=D ** -0.5, attention_mask=mask)
     assert_bf16_gate(a[0], b[0], "y")
     assert_bf16_gate(a[1]["u"] / a[1]["d"][..., None], b[1]["u"] / b[1]["d"][..., None], "state")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,N,H,Dk,Dv", [(1, 1, 1, 8, 8), (4, 127, 2, 64, 32), (4, 129, 3, 16, 128), (5, 1030, 1, 64, 64)])
+def test_pack_and_unpack_on_their_own(B, N, H, Dk, Dv, dtype):
+    # the two entry points for callers that run the kernels on lengths themselves: copies, so bit for bit
+    g = torch.Generator().manual_seed(N)
+    mask = torch.rand(B, N, generator=g) < 0.5
+    for row, keep in enumerate((torch.ones(N), torch.zeros(N), torch.arange(N) >= N // 3, torch.arange(N) < N // 2)[:B]):
+        mask[row] = keep.bool()
+    k, v = (torch.randn(B, N, 2, H, D, generator=g).to(dtype).cuda()[:, :, 1] for D in (Dk, Dv))  # (strides of a fused projection)
+    m = mask.int().cuda()
+    slot, lens = torch.full((B, N), -7, dtype=torch.int32, device="cuda"), torch.empty(B, dtype=torch.int32, device="cuda")
+    kp, vp = (torch.full((B, N, H, D), float("nan"), dtype=dtype, device="cuda") for D in (Dk, Dv))
+    strides = lambda t: (C.c_int64 * 3)(*t.stride()[:3])  # noqa: E731
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    assert lib.flare_mask_pack(m.data_ptr(), k.data_ptr(), strides(k), v.data_ptr(), strides(v), B, N, H, Dk, Dv, slot.data_ptr(),
+                               lens.data_ptr(), kp.data_ptr(), vp.data_ptr(), stream) == 0
+    assert torch.equal(lens.cpu(), mask.sum(1).int())
+    assert torch.equal(slot.cpu(), torch.where(mask, mask.cumsum(1) - 1, -1).int())
+    for b in range(B):
+        n = int(mask[b].sum())
+        for src, out in ((k, kp), (v, vp)):
+            assert torch.equal(out[b, :n], src[b][mask[b].cuda()])
+            assert not out[b, n:min(N, -(-n // 128) * 128)].any()
+    y = torch.full((B, N, H, Dv), float("nan"), dtype=dtype, device="cuda")
+    assert lib.flare_mask_unpack(slot.data_ptr(), vp.data_ptr(), y.data_ptr(), strides(y), B, N, H, Dv, stream) == 0
+    assert torch.equal(y, torch.where(mask.cuda()[..., None, None], v, torch.zeros_like(v)))
