@@ -291,8 +291,8 @@ int launch_decode_step(const DecodeParams& p, cudaStream_t stream) {
   // So: four CTAs per SM while there are lanes for more than two, else two with twice the vectors, and a lane whose state does
   // not fit the vectors asked for ahead is cut into column slices (128 bytes wide at least) while two per SM hold them all.
   // Small states of many lanes have little to ask for; there eight CTAs per SM, which hide the phases before the state, are the
-  // better ones (us a step among others, eight / four): 2048 lanes of 8 KB (M = 32, D = 64) 15.2 / 17.4, 1024 lanes 9.1 / 9.7, M = 16 with keys 512 wide 18.3 / 23.2; of 16 KB
-  // (M = 64) 21.1 / 21.6 with 2048 lanes, 12.4 / 12.1 with 1024.
+  // better ones.  Us a step among others, eight / four: 2048 lanes of 8 KB (M = 32, D = 64) 15.2 / 17.4, 1024 lanes 9.1 / 9.7, 2048 lanes
+  // with M = 16 and keys 512 wide 18.3 / 23.2; of 16 KB (M = 64) 21.1 / 21.6 with 2048 lanes, 12.4 / 12.1 with 1024.
   // The rows of the latent bank in flight follow the latents that there are: four CTAs with four rows were 19.1 us at M = 32.
   // Measured and rejected on the largest shape: one kernel for the coefficients of all lanes and one that only streams (98 to
   // 103), 128-thread CTAs (121.7 against 112), bulk async copies through a shared-memory ring (115.5 to 207).

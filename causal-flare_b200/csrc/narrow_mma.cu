@@ -29,10 +29,10 @@
 //
 // Precision: the distances of the bf16 outputs from 64 bits equal those of the fp32 kernels to 1 part in 10^6, either way, over
 // M = 32 .. 128, N = 128 .. 4096, and 0.1 % of the outputs at most are rounded the other way, as there.  (Two values per operand
-// were faster, 386 us for the step below, where three took 472 before the windows, but left 0.1 to 0.5 % of the outputs rounded the other way and an fp32 dQ ten times
-// as far from 64 bits.)  What is left is the tensor cores' own addition, which cuts off instead of rounding: 3.7e-7 of an fp32
-// dQ whatever N is, where the fp32 kernels have 2.8e-7 (N = 128) to 5.2e-7 (N = 4096).  A caller that wants dQ in fp32 gets
-// the fp32 kernels.
+// were faster, 386 us for the step below where three took 472 before the windows, but left 0.1 to 0.5 % of the outputs rounded
+// the other way and an fp32 dQ ten times as far from 64 bits.)  What is left is the tensor cores' own addition, which cuts off
+// instead of rounding: 3.7e-7 of an fp32 dQ whatever N is, where the fp32 kernels have 2.8e-7 (N = 128) to 5.2e-7 (N = 4096).  A
+// caller that wants dQ in fp32 gets the fp32 kernels.
 //
 // B200, training step B=8 N=2048 H=16 M=64 D=32: 1823 us on the fp32 kernels, 493 us on these; the forward alone 632
 // and 132 us.

@@ -130,7 +130,8 @@ size_t flare_noalloc_scratch_capacity(void);
  * Nothing but the inputs is needed from the forward: intermediates are recomputed.  Two implementations: the
  * tensor-core one (bwd_tc.cu: a forward that keeps per-chunk states, then a reverse chunk sweep on tcgen05 and a
  * tensor-core dK / dQ product) for the shapes flare_backward_uses_tensor_path accepts, and the exact fp32 one
- * (bwd_exact.cu) for everything else; fwd.path = FLARE_PATH_EXACT forces the latter.
+ * (bwd_exact.cu) for everything else; fwd.path = FLARE_PATH_EXACT forces the latter.  bf16 softmax problems with heads up to 32
+ * wide run on tensor-core kernels of their own (narrow_mma.cu) unless dq is wanted in fp32, which the exact ones sum more exactly.
  * dq / dk_dec are [H, M, Dk] (summed over the batch in fp32; dk_dec is fp32, dq as dq_dtype says); dk, dv, dq_dec have the input dtype and the
  * input's shape, densely packed.  With weight sharing (q_dec/k_dec NULL) the decode-side gradients are
  * folded into dk / dq and dq_dec / dk_dec must be NULL.
