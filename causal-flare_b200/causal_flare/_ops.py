@@ -101,9 +101,11 @@ def forward(Q, K, V, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, pow
 
 
 def backward(Q, K, V, dY, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX, power=2.0, block_size=1,
-             dy_bhnd=False, path=None, saved=None):
+             dy_bhnd=False, path=None, saved=None, dq_dtype=torch.float32):
     """Run flare_backward.  ``saved``: what a forward with ``keep_for_backward`` left behind (or None / empty: the
-    backward replays the forward itself).  Returns fp32 dQ, input-dtype dK, dV, and dQ_dec / dK_dec (or None)."""
+    backward replays the forward itself).  ``dq_dtype``: what the caller makes of dQ; the library rounds it once from its
+    fp32 sum if that is the inputs' type (bf16 narrow heads run on the tensor cores only then).  Returns dQ in it, else in
+    fp32, input-dtype dK, dV, and dQ_dec / dK_dec (or None)."""
     _lib.load()
     if path is None:
         path = default_path()
@@ -117,7 +119,7 @@ def backward(Q, K, V, dY, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX
     dy = _prep(dy, dt)
     # the kernels write every element of every gradient; only an empty problem needs explicit zeros
     alloc = torch.empty if (B > 0 and N > 0) else torch.zeros
-    dq = alloc((H, M, Dk), device=dev, dtype=torch.float32)
+    dq = alloc((H, M, Dk), device=dev, dtype=dt if dq_dtype == dt else torch.float32)
     dk = alloc((B, N, H, Dk), device=dev, dtype=dt)
     dv = alloc((B, N, H, Dv), device=dev, dtype=dt)
     dqd = alloc((B, N, H, Dk), device=dev, dtype=dt) if qd is not None else None
@@ -129,6 +131,7 @@ def backward(Q, K, V, dY, *, scale, Q_dec=None, K_dec=None, variant=_lib.SOFTMAX
         a.dy = dy.data_ptr()
         a.dy_stride_b, a.dy_stride_n, a.dy_stride_h = dy.stride(0), dy.stride(1), dy.stride(2)
         a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
+        a.dq_dtype = _lib.dtype_code(dq.dtype)
         a.dq_dec, a.dk_dec = _lib.ptr(dqd), _lib.ptr(dkd)
         if saved:
             ys = saved["y"]

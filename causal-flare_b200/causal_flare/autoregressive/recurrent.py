@@ -57,7 +57,8 @@ class RecurrentFLARE(autograd.Function):
         rest = saved[3:]
         Q_dec = rest.pop(0) if ctx.sep_q else None
         K_dec = rest.pop(0) if ctx.sep_k else None
-        dq, dk, dv, dqd, dkd = _ops.backward(Q, K, V, dY, scale=ctx.scale, Q_dec=Q_dec, K_dec=K_dec, dy_bhnd=True)
+        dq, dk, dv, dqd, dkd = _ops.backward(Q, K, V, dY, scale=ctx.scale, Q_dec=Q_dec, K_dec=K_dec, dy_bhnd=True,
+                                             dq_dtype=Q.dtype)
         return (
             dq.to(Q.dtype), dk.to(K.dtype), dv.to(V.dtype), None, None, None,
             None if dqd is None else dqd.to(Q_dec.dtype), None if dkd is None else dkd.to(K_dec.dtype), None,

@@ -86,7 +86,7 @@ class AutoRegressiveFLARE(autograd.Function):
         prof = ctx.profile_timings
         dq, dk, dv, dqd, dkd = _timed(
             K.device, prof["backward"] if prof is not None else None, "flare_backward",
-            lambda: _ops.backward(Q, K, V, dO, scale=ctx.scale, Q_dec=Q_dec, K_dec=K_dec, saved=kept),
+            lambda: _ops.backward(Q, K, V, dO, scale=ctx.scale, Q_dec=Q_dec, K_dec=K_dec, saved=kept, dq_dtype=Q.dtype),
         )
         if prof is not None:
             _refresh_profile_totals(prof)

@@ -73,6 +73,21 @@ def test_dq_in_fp32_is_that_of_the_fp32_kernels():
     assert orc.rel_l2(auto[0].cpu(), want) <= 2.0 ** -24 * (B * N) ** 0.5
 
 
+@pytest.mark.parametrize("shape", [(2, 300, 4, 64, 32), (1, 33, 2, 32, 16)])
+def test_every_entry_point_that_rounds_dq_takes_these_kernels(shape):
+    # the autograd functions in Python and the recurrent operator give the gradients of the native layer, bit for bit
+    B, N, H, M, D = shape
+    q, k, v, dy = to_dev(*orc.make_inputs(B, N, H, M, D, seed0=29, dtype=torch.bfloat16, with_dy=True))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    want = torch.autograd.grad(cf.flare_autoregressive_triton(*leaves), leaves, dy)
+    y, _ = cf.flare_autoregressive_triton(*leaves, profile=True)
+    for x, ref in zip(torch.autograd.grad(y, leaves, dy), want):
+        assert x.dtype == torch.bfloat16 and torch.equal(x, ref)
+    y = cf.flare_recurrent_triton(*leaves)
+    for x, ref in zip(torch.autograd.grad(y, leaves, dy.permute(0, 2, 1, 3)), want):
+        assert torch.equal(x, ref)
+
+
 @pytest.mark.parametrize("std", [4.0, 24.0])
 def test_sharp_scores(monkeypatch, std):
     # at 24 the running maximum grows by hundreds of powers of two inside tiles, which are taken in several windows
