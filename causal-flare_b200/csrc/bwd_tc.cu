@@ -15,15 +15,15 @@
 //   dS   = R (P - D delta_t)  +  E slope (X - Cc - sum_{t' >= t} R p)          slope = 1 | sigma'/sigma
 //   dV   = E^T G + (E^T R . vis) dY
 //   G   += R dY,  Cc += sum_t R p,  then both are rescaled by exp2(c_{i-1} - c_i) for the next chunk.
-// dS is written per latent as a hi and a lo bf16 row over the tokens ([lane][2][m][t], dS = hi + lo: a latent thread's
-// eight tokens are one 16-byte store each); a second tensor-core kernel forms dK = scale dS^T Q per chunk and
-// dQ = scale sum_t dS K per (lane, split) (fp32 partials, summed in fixed order: no atomics, deterministic).
+// dS is written per latent as a hi and a lo bf16 row over the tokens ([lane][2][m][t], dS = hi + lo); a second tensor-core
+// kernel forms dK = scale dS^T Q per chunk and dQ = scale sum_t dS K per (lane, split) (fp32 partials, summed in fixed order:
+// no atomics, deterministic).
 //
-// Main kernel, one CTA per (lane, group of 128 latents, sequence segment), 22 warps: 0-15 latent group (thread = latent = TMEM
+// Main kernel, one CTA per (lane, group of 128 latents, sequence segment), 23 warps: 0-15 latent group (thread = latent = TMEM
 // lane, the four warps of a lane quarter take 32 tokens each; packed: see PACK), 16-19 token group (thread = token = TMEM lane:
-// causal masks of A and E^T R, dV store), 20 MMA issuer, 21 TMA producer (elected threads: with lane 0 of the warp issuing, a
-// training step B=4 N=4096 H=16 M=128 D=64 takes 496 instead of 484 us).  Ten MMAs per chunk; every operand that the latent / token
-// threads produce (E, R, masked A, G as bf16) is written once into a 128-byte-swizzled buffer and read K-major or
+// causal masks of A and E^T R, dV store), 20 MMA issuer, 21 TMA producer, 22 stores of dS (elected threads: with lane 0
+// of the issuer and the producer, a training step B=4 N=4096 H=16 M=128 D=64 took 496 instead of 484 us).  Ten MMAs per chunk; every
+// operand that the latent / token threads produce (E, R, masked A, G as bf16) is written once into a 128-byte-swizzled buffer and read K-major or
 // MN-major as the product needs, so there is no transposition pass.
 #include "bwd_tc.cuh"
 
@@ -58,7 +58,6 @@ struct BwdTcParams {
   float scale, power;
   const float *chunk_c, *chunk_d;  // [lanes][nch][M]
   const float *tok_l2, *tok_delta;  // [lanes][npad]
-  void* ds;      // bf16 [lanes][2][M][npad]: dS of every latent as a hi row and a lo row over the tokens (dS = hi + lo)
   void* dv;      // bf16 [B, N, H, Dv] contiguous, or (more than one latent group) bf16 [groups][B][N][H][Dv]
   int groups;
   // Sequence segments (grid.z = the segments from seg_first on, segment s = chunks seg_begin[s] .. seg_begin[s + 1] - 1).
@@ -85,14 +84,14 @@ struct GradTcParams {
 // one instance family per head-width combination, compiled in its own translation unit
 template <int UNIT>
 int launch_bwd_tc_unit(int mode, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy, const CUtensorMap& tu,
-                       const BwdTcParams& p, dim3 grid, cudaStream_t stream);
+                       const CUtensorMap& tds, const CUtensorMap& tdv, const BwdTcParams& p, dim3 grid, cudaStream_t stream);
 
 namespace {
 
 constexpr int C = 128;
 constexpr int LW = 4;                           // latent warps per lane quarter
-constexpr int NT_MAIN = (4 * LW + 4 + 2) * 32;  // latent warps, token warps, MMA issuer, TMA producer
-constexpr int W_TOKEN = 4 * LW, W_MMA = 4 * LW + 4, W_TMA = 4 * LW + 5;  // first token warp, issuer, producer
+constexpr int NT_MAIN = (4 * LW + 4 + 3) * 32;  // latent warps, token warps, MMA issuer, TMA producer, dS stores
+constexpr int W_TOKEN = 4 * LW, W_MMA = 4 * LW + 4, W_TMA = 4 * LW + 5, W_OUT = 4 * LW + 6;  // first token warp, issuer, producer, dS stores
 constexpr float kLog2e = 1.4426950408889634f;
 
 // shared memory map of the main kernel (bytes; every operand buffer 1024-aligned for the 128B swizzle)
@@ -116,7 +115,7 @@ constexpr uint32_t T0 = 0, T1 = 128, T2 = 256, TQ = 320, TG = 384, TM_COLS = 512
 struct Misc {
   uint64_t k_full, v_full, dy_full, u_full, q_ready;
   uint64_t s_ready, a_ready, px_ready, g_ready, wt_ready, dv_ready;
-  uint64_t er_done, am_done, p_free, x_done, wm_done, dv_free, gc_done;
+  uint64_t er_done, am_done, p_free, x_done, wm_done, dv_free, gc_done, ds_out, dv_out;
   uint64_t psum[4], prp[4];
   uint32_t tmem_base;
   volatile int abort_flag;
@@ -178,7 +177,8 @@ __device__ __forceinline__ void slope8_from_sigma(const float (&e)[8], float p, 
 template <int DKB, int DVB, int MODE, bool PACK>
 __global__ void __launch_bounds__(NT_MAIN, 1)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-              const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_u, const BwdTcParams p) {
+              const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_u,
+              const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_dv, const BwdTcParams p) {
   using L = BL<DVB>;
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int DV = DVB * 64;
@@ -187,6 +187,14 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   constexpr int NG = TOK / 16;            // groups of 16 tokens among them
   constexpr int NCH = TOK / 8;            // 16-byte pieces of its operand rows
   constexpr int XL = PACK ? 64 : 128;     // latents of an exchange row
+  // dS and dV leave through tiled bulk stores.  A thread storing its own row straight to global memory costs a transaction for every
+  // 16 bytes, 4 096 (dS) and 2 048 (dV) a chunk at M = D = 128, and everything else that goes through the load / store unit waits
+  // behind them: at M = 64, D = 128 the descending pass took 4 400 of a chunk's 15 700 cycles and the dV rows 4 200.
+  // dS is laid down where E (hi) and R (lo) were: packed, in their second copies, which are free when P, X and G have been formed;
+  // else in place, when the chunk's last product has run.  dV goes through R's first copy (packed) or the unused half of U's slot
+  // (Dv = 64); at Dv = 128 without packing there is no room and its rows are stored as they are.  B200, us a training step: B=4
+  // N=4096 H=16 M=128 D=64 482 -> 450, M=64 D=128 376 -> 362, B=8 M=64 D=64 432 -> 392, B=2 N=2048 M=256 D=128 304 -> 289.
+  constexpr bool DV_TILES = PACK || DVB == 1;
   pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -228,6 +236,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_init(&misc->wm_done, 4);
     mbar_init(&misc->dv_free, 4);
     mbar_init(&misc->gc_done, 4 * LW);
+    mbar_init(&misc->ds_out, 1);
+    mbar_init(&misc->dv_out, 4);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&misc->psum[i], NP);
       mbar_init(&misc->prp[i], NP);
@@ -374,6 +384,26 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         tc_commit(&misc->dv_ready);
       }
     }
+  } else if (warp == W_OUT) {
+    // ======================================= dS stores =======================================
+    if (elect_one()) {
+      prefetch_tensormap(&tm_ds);
+      for (int j = 0; ok && j < steps; ++j) {
+        const int i = first - 1 - j;
+        if (!(ok = wait_or_abort(&misc->x_done, j & 1, misc))) break;
+        if (i >= full_end) continue;
+        constexpr int COPY = PACK ? 8192 : 0;
+#pragma unroll
+        for (int tb = 0; tb < 2; ++tb) {  // (rows beyond M are clipped)
+          tma_store_4d(&tm_ds, smem + L::OFF_E + tb * 16384 + COPY, i * C + tb * 64, group * 128, 0, lane_id);
+          tma_store_4d(&tm_ds, smem + L::OFF_R + tb * 16384 + COPY, i * C + tb * 64, group * 128, 1, lane_id);
+        }
+        bulk_commit_group();
+        bulk_wait_group_read0();
+        mbar_arrive(&misc->ds_out);
+      }
+      bulk_wait_group0();
+    }
   } else if (warp < 4 * LW) {
     // ======== latent group: thread = (latent = TMEM lane, part of the chunk's tokens); 4 warps per lane quarter ========
     const int tq = warp >> 2, q = warp & 3;
@@ -415,10 +445,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
     float cc_carry = 0.f;  // Cc: sum over later chunks of R p, in the current chunk's frame
     const int64_t stat0 = (int64_t)lane_id * nch * p.M + mg;
-    // dS rows of this latent: element (part, latent, token t) of the lane at (part * M + latent) * npad + t.  Token-wise rows
-    // over the latents took a 2-byte store per element and plane, 64 instead of 8 stores per thread and chunk.
-    __nv_bfloat16* const ds_row = reinterpret_cast<__nv_bfloat16*>(p.ds) +
-                                  ((int64_t)lane_id * 2 * p.M + (live ? mg : 0)) * p.npad + tok0;
     // value columns of G this warp rescales and repacks
     constexpr int GCOLS = DV / NP;
     const int gcol = tp * GCOLS;
@@ -510,6 +536,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       for (int j = 0; ok && j < steps; ++j) {
         const int i = first - 1 - j, t0 = i * C;
         const uint32_t par = j & 1, pp = (j - 1) & 1;
+        const uint32_t fpar = (j - (first - full_end)) & 1;  // parity among the full chunks
         const int nvalid = min(C, p.N - t0);
         const int lim = live ? nvalid - tok0 : 0;  // tokens of this thread's part that exist (may be <= 0)
         const bool fast = __all_sync(0xffffffffu, lim >= TOK);
@@ -524,6 +551,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         const float dl_pre = i > 0 ? ld_pinned(dl_row + (int64_t)(i - 1) * C) : 0.f;
         // E / R buffers: the previous chunk's products have read them
         if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
+        const bool after_full = i + 1 < full_end && j > 0;  // and the previous (full) chunk's dS has left them
+        if (after_full && !(ok = wait_or_abort(&misc->ds_out, fpar ^ 1, misc))) break;
         if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
         tc_fence_after_sync();
         if (tid == 0) BT_TRACE(0, j, 0);
@@ -585,6 +614,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           for (int g = 0; g < NG; ++g) invg[g] = rcp_approx(dend[g]);
         }
         // ---- phase 1b: R = g / D rows (bf16)
+        if (PACK && after_full && !(ok = wait_or_abort(&misc->dv_out, fpar ^ 1, misc))) break;  // (the dV rows have left R)
         {
           float run = base_run;
 #pragma unroll
@@ -675,6 +705,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 
         // ---- phase 2b (descending): encoder part, dS rows to global memory as a hi + lo pair
         if (i < full_end) {
+          // dS may be laid down: see DV_TILES
+          if (!(ok = PACK ? wait_or_abort(&misc->g_ready, par, misc) : wait_or_abort(&misc->dv_ready, par, misc))) break;
           float ccg[NG];  // block-causal: Cc + sum of R p from the start of the group's block on
           float cc = cc_carry + rp_later;
           if constexpr (BLOCK) {
@@ -695,7 +727,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
               for (int g = 0; g < NG; ++g) ccg[g] = tot;
             }
           }
-          __nv_bfloat16* const dst = ds_row + t0;
 #pragma unroll
           for (int blk = NG - 1; blk >= 0; --blk) {
             uint32_t xr[16];
@@ -732,12 +763,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                 hi[jj >> 1] = pack_bf16(ds[jj], ds[jj + 1]);
                 lo[jj >> 1] = pack_bf16(ds[jj] - bf16_lo(hi[jj >> 1]), ds[jj + 1] - bf16_hi(hi[jj >> 1]));
               }
-              if (live) {
-                *reinterpret_cast<uint4*>(dst + ch * 8) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(dst + (int64_t)p.M * p.npad + ch * 8) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-              }
+              constexpr int COPY = PACK ? 8192 : 0;
+              *reinterpret_cast<uint4*>(e_row + COPY + swz_chunk_off(m, ch0 + ch)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+              *reinterpret_cast<uint4*>(r_row + COPY + swz_chunk_off(m, ch0 + ch)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
           }
+          fence_proxy_async_smem();
         }
         if (tid == 0) BT_TRACE(3, j, 5);
         tc_fence_before_sync();
@@ -802,6 +833,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const uint32_t tl = tmem + ((uint32_t)(wq * 32) << 16);
     const int tt = wq * 32 + lane;
     const int lo = BLOCK ? (tt & ~(p.block - 1)) : tt;  // first column (token) this row keeps
+    uint8_t* const dv_stage = smem + (PACK ? L::OFF_R + (wq >> 1) * 16384 + (wq & 1) * 4096 : L::OFF_UR + 16384 + wq * 4096);
     __nv_bfloat16* dv_base;
     int64_t dv_stride_n;
     {
@@ -887,29 +919,51 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       if (!(ok = wait_or_abort(&misc->dv_ready, par, misc))) break;
       tc_fence_after_sync();
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 4);
+      // (packed: the latent group has read R)
+      if (PACK && !(ok = wait_or_abort(&misc->x_done, par, misc))) break;
 #pragma unroll
       for (int half = 0; half < DV / 32; ++half) {
         uint32_t r[32];
         tmem_ld32(tl + T0 + half * 32, r);
         tmem_wait_ld();
         tmem_fence_regs(r);
-        if (tt < nvalid) {
+        if (half == DV / 32 - 1) {
+          tc_fence_before_sync();
+          warp_arrive(&misc->dv_free, lane);
+        }
+        uint4 v[4];
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          v[ch] = make_uint4(pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1])),
+                             pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3])),
+                             pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5])),
+                             pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7])));
+        if constexpr (DV_TILES) {
+          // two 32 x 32 tiles per warp (64-byte swizzle), stored in turn; rows beyond the sequence end are clipped
+          uint8_t* const tile = dv_stage + (half & 1) * 2048;
+          if (lane == 0) bulk_wait_group_read1();
+          __syncwarp();
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) *reinterpret_cast<uint4*>(tile + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) = v[ch];
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_4d(&tm_dv, tile, half * 32, h, t0 + wq * 32, group * (int)(gridDim.x / p.H) + b);
+            bulk_commit_group();
+          }
+        } else if (tt < nvalid) {
           uint4* dst = reinterpret_cast<uint4*>(dv_base + (int64_t)(t0 + tt) * dv_stride_n + half * 32);
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            uint4 v;
-            v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]), __uint_as_float(r[ch * 8 + 1]));
-            v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3]));
-            v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5]));
-            v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7]));
-            dst[ch] = v;
-          }
+          for (int ch = 0; ch < 4; ++ch) dst[ch] = v[ch];
         }
       }
-      tc_fence_before_sync();
-      warp_arrive(&misc->dv_free, lane);
+      if constexpr (PACK) {
+        if (lane == 0) bulk_wait_group_read0();
+        warp_arrive(&misc->dv_out, lane);
+      }
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 5);
     }
+    if (DV_TILES && lane == 0) bulk_wait_group0();
   }
   if (!ok) {
     misc->abort_flag = 1;
@@ -924,11 +978,11 @@ namespace {
 
 template <int DKB, int DVB, int MODE, bool PACK>
 int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy, const CUtensorMap& tu,
-                const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
+                const CUtensorMap& tds, const CUtensorMap& tdv, const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = bwd_tc_kernel<DKB, DVB, MODE, PACK>;
   FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("bwd_tc_kernel", stream);
-  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_MAIN), BL<DVB>::SMEM_BYTES, stream, tk, tv, tdy, tu, p));
+  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_MAIN), BL<DVB>::SMEM_BYTES, stream, tk, tv, tdy, tu, tds, tdv, p));
   return FLARE_OK;
 }
 
@@ -936,25 +990,31 @@ int launch_main(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap&
 
 template <>
 int launch_bwd_tc_unit<FLARE_BT_UNIT>(int mode, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdy,
-                                      const CUtensorMap& tu, const BwdTcParams& p, dim3 grid, cudaStream_t stream) {
+                                      const CUtensorMap& tu, const CUtensorMap& tds, const CUtensorMap& tdv, const BwdTcParams& p,
+                                      dim3 grid, cudaStream_t stream) {
   // units 0..2: (Dk, Dv) = (64, 64), (128, 128), (64, 128); units 3..5: the same, packed
   constexpr int W = FLARE_BT_UNIT % 3;
   constexpr int DKB = W == 1 ? 2 : 1;
   constexpr int DVB = W == 0 ? 1 : 2;
   constexpr bool PACK = FLARE_BT_UNIT >= 3;
-  if (mode == 1) return launch_main<DKB, DVB, 1, PACK>(tk, tv, tdy, tu, p, grid, stream);
-  if (mode == 2) return launch_main<DKB, DVB, 2, PACK>(tk, tv, tdy, tu, p, grid, stream);
-  return launch_main<DKB, DVB, 0, PACK>(tk, tv, tdy, tu, p, grid, stream);
+  if (mode == 1) return launch_main<DKB, DVB, 1, PACK>(tk, tv, tdy, tu, tds, tdv, p, grid, stream);
+  if (mode == 2) return launch_main<DKB, DVB, 2, PACK>(tk, tv, tdy, tu, tds, tdv, p, grid, stream);
+  return launch_main<DKB, DVB, 0, PACK>(tk, tv, tdy, tu, tds, tdv, p, grid, stream);
 }
 
 #else  // host side, the dK / dQ kernel and the small helper kernels
 
-template <> int launch_bwd_tc_unit<0>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
-template <> int launch_bwd_tc_unit<1>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
-template <> int launch_bwd_tc_unit<2>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
-template <> int launch_bwd_tc_unit<3>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
-template <> int launch_bwd_tc_unit<4>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
-template <> int launch_bwd_tc_unit<5>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
+#define FLARE_BT_DECLARE(U)                                                                                                    \
+  template <>                                                                                                               \
+  int launch_bwd_tc_unit<U>(int, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, \
+                            const CUtensorMap&, const BwdTcParams&, dim3, cudaStream_t);
+FLARE_BT_DECLARE(0)
+FLARE_BT_DECLARE(1)
+FLARE_BT_DECLARE(2)
+FLARE_BT_DECLARE(3)
+FLARE_BT_DECLARE(4)
+FLARE_BT_DECLARE(5)
+#undef FLARE_BT_DECLARE
 
 namespace {
 
@@ -1536,7 +1596,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
   }
   // (3) reverse chunk sweep: dV and the dS plane
   const bool pack = f.M <= 64;
-  CUtensorMap tk, tv, tdy, tu, tds, tq;
+  CUtensorMap tk, tv, tdy, tu, tds, tds_out, tdv, tq;
   {
     const uint64_t dimk[4] = {(uint64_t)f.Dk, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B};
     const uint64_t dimv[4] = {(uint64_t)f.Dv, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B};
@@ -1549,13 +1609,19 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     const uint32_t boxu[4] = {64, pack ? 64u : 128u, 1, 1};
     const uint64_t dims[4] = {(uint64_t)pl.npad, (uint64_t)f.M, 2, (uint64_t)lanes};
     const int64_t strs[3] = {pl.npad, (int64_t)f.M * pl.npad, 2 * (int64_t)f.M * pl.npad};
-    const uint32_t boxs[4] = {64, 128, 1, 1};
+    const uint32_t boxs[4] = {64, 128, 1, 1}, boxo[4] = {64, pack ? 64u : 128u, 1, 1};
+    // dV rows, or with several latent groups their dense partials
+    void* const dv = pl.groups > 1 ? static_cast<void*>(ws + pl.off_dvp) : a.dv;
+    const uint64_t dimdv[4] = {(uint64_t)f.Dv, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B * pl.groups};
+    const int64_t strdv[3] = {f.Dv, (int64_t)f.H * f.Dv, (int64_t)f.N * f.H * f.Dv};
+    const uint32_t boxdv[4] = {32, 1, 32, 1};
     const uint64_t dimq[3] = {(uint64_t)f.Dk, (uint64_t)f.M, (uint64_t)f.H};
     const int64_t strq[2] = {f.q_stride_m, f.q_stride_h};
     const uint32_t boxq[3] = {64, 128, 1};
     if (!tc::make_map_bf16(&tk, f.k, 4, dimk, strk, box) || !tc::make_map_bf16(&tv, f.v, 4, dimv, strv, box) ||
         !tc::make_map_bf16(&tdy, a.dy, 4, dimv, strd, box) || !tc::make_map_bf16(&tu, keep.u, 4, dimu, stru, boxu) ||
-        !tc::make_map_bf16(&tds, ws + pl.off_ds, 4, dims, strs, boxs) || !tc::make_map_bf16(&tq, f.q, 3, dimq, strq, boxq)) {
+        !tc::make_map_bf16(&tds, ws + pl.off_ds, 4, dims, strs, boxs) || !tc::make_map_bf16(&tds_out, ws + pl.off_ds, 4, dims, strs, boxo) ||
+        !tc::make_map_bf16(&tdv, dv, 4, dimdv, strdv, boxdv, CU_TENSOR_MAP_SWIZZLE_64B) || !tc::make_map_bf16(&tq, f.q, 3, dimq, strq, boxq)) {
       set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (backward operands)");
       return FLARE_ERR_CUDA;
     }
@@ -1567,7 +1633,6 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     p.N = f.N; p.H = f.H; p.M = f.M; p.nch = pl.nch; p.npad = pl.npad; p.block = f.block_size;
     p.scale = f.scale; p.power = f.power;
     p.chunk_c = keep.c; p.chunk_d = keep.d; p.tok_l2 = tok_l2; p.tok_delta = tok_delta;
-    p.ds = ws + pl.off_ds;
     p.groups = pl.groups;
     p.dv = pl.groups > 1 ? static_cast<void*>(ws + pl.off_dvp) : a.dv;
     p.err = err;
@@ -1585,7 +1650,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
       const auto launch = f.Dk == 128   ? (pack ? launch_bwd_tc_unit<4> : launch_bwd_tc_unit<1>)
                           : f.Dv == 128 ? (pack ? launch_bwd_tc_unit<5> : launch_bwd_tc_unit<2>)
                                         : (pack ? launch_bwd_tc_unit<3> : launch_bwd_tc_unit<0>);
-      return launch(mode, tk, tv, tdy, tu, p, grid, stream);
+      return launch(mode, tk, tv, tdy, tu, tds_out, tdv, p, grid, stream);
     };
     int rc = FLARE_OK;
     if (pl.seg.n > 1 && !pl.seg.lead) {
