@@ -76,7 +76,7 @@ struct GradTcParams {
   int nch, npad, groups;
   int nsplit, chunks_per_split;
   float scale;
-  void* dk;        // bf16 [B, N, H, Dk] contiguous
+  int plane, nds, nk;  // bytes of a dS plane of the ring, stages (see grad_rings)
   float* dq_part;  // fp32 [B * nsplit][H][M][Dk]
   int* err;
 };
@@ -1129,36 +1129,58 @@ __global__ void __launch_bounds__(256) bwd_tc_sum_dq_kernel(const float* part, i
 // One CTA per (lane, split), 6 warps: 0 TMA producer, 1 MMA issuer, 2-5 epilogue (thread = TMEM lane).
 // -------------------------------------------------------------------------------------------------
 constexpr int NT_GRAD = 192;
-constexpr int GRAD_MAXG = 4;
 
-template <int DKB>
-struct GL {
-  static constexpr int OFF_DS = 0;                         // 2 stages x [2 t-blocks][128 m][64 t]
-  static constexpr int OFF_K = 65536;                      // 2 stages x [DKB][128 t][64]
-  static constexpr int OFF_Q = OFF_K + 2 * DKB * 16384;    // groups x [DKB][128 m][64]
-  static constexpr int off_misc(int groups) { return OFF_Q + groups * DKB * 16384; }
-  static constexpr int smem_bytes(int groups) { return off_misc(groups) + 256 + 1024; }
-  static constexpr uint32_t TM_DK = 0;                     // 2 buffers x Dk columns
-  static constexpr uint32_t TM_DQ = 2 * DKB * 64;          // groups x Dk columns
+constexpr int GRAD_MAXST = 8;  // stages of a ring
+
+// Shared memory: rings of nds dS planes ([2 t-blocks][rows m][64 t], rows = 64 for banks of at most 64 latents, else 128) and of nk K
+// tiles ([DKB][128 t][64]), the latent bank (groups x [DKB][128 m][64]), two 32 x 32 tiles of dK rows per epilogue warp.  A streaming
+// kernel: as many stages as fit, about two planes for a K tile.  B=4 N=4096 H=16 M=64 D=128 (200 MB, 31 us at the copy rate): 33 us; 45
+// with two stages of each, planes of 128 rows whatever the bank, and dK rows stored by their threads in 16-byte pieces.
+struct GradRings {
+  int plane, nds, nk, smem;
 };
+GradRings grad_rings(int M, int dkb) {
+  const int groups = (M + 127) / 128, tile = dkb * 16384, fixed = groups * tile + 16384 + 512 + 1024;
+  GradRings r;
+  r.plane = M <= 64 ? 16384 : 32768;
+  for (r.nk = 4;; --r.nk) {
+    r.nds = (232448 - fixed - r.nk * tile) / r.plane;
+    if (r.nk == 2 || r.nds >= 2 * r.nk - 1) break;
+  }
+  if (r.nds > GRAD_MAXST) r.nds = GRAD_MAXST;
+  r.smem = fixed + r.nk * tile + r.nds * r.plane;
+  return r;
+}
 
 struct GradMisc {
-  uint64_t q_full, ds_full[2], ds_empty[2], k_full[2], k_empty[2], dk_ready[2], dk_free[2], dq_ready;
+  uint64_t q_full, ds_full[GRAD_MAXST], ds_empty[GRAD_MAXST], k_full[4], k_empty[4], dk_ready[2], dk_free[2], dq_ready;
   uint32_t tmem_base;
   volatile int abort_flag;
+};
+static_assert(sizeof(GradMisc) <= 512, "GradMisc");
+// the next stage of a ring, and the parity of its phase
+struct Stage {
+  int s = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++s == n) s = 0, phase ^= 1;
+  }
 };
 
 template <int DKB>
 __global__ void __launch_bounds__(NT_GRAD, 1)
 bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_q, const GradTcParams p) {
-  using L = GL<DKB>;
+                    const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_dk, const GradTcParams p) {
   constexpr int DK = DKB * 64;
+  constexpr uint32_t TM_DK = 0, TM_DQ = 2 * DK;  // tensor-memory columns: two buffers of dK, then dQ of every group
   pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  const int G = p.groups;
-  GradMisc* misc = reinterpret_cast<GradMisc*>(smem + L::off_misc(G));
+  const int G = p.groups, plane = p.plane, nds = p.nds, nk = p.nk;
+  uint8_t* const k_ring = smem + nds * plane;
+  uint8_t* const q_bank = k_ring + nk * DKB * 16384;
+  uint8_t* const stage = q_bank + G * DKB * 16384;
+  GradMisc* misc = reinterpret_cast<GradMisc*>(stage + 16384);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lane_id = blockIdx.x, split = blockIdx.y;
   const int b = lane_id / p.H, h = lane_id % p.H;
@@ -1168,11 +1190,15 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
 
   if (tid == 0) {
     mbar_init(&misc->q_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < GRAD_MAXST; ++i) {
       mbar_init(&misc->ds_full[i], 1);
       mbar_init(&misc->ds_empty[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&misc->k_full[i], 1);
       mbar_init(&misc->k_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&misc->dk_ready[i], 1);
       mbar_init(&misc->dk_free[i], 4);
     }
@@ -1198,23 +1224,20 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
       mbar_arrive_expect_tx(&misc->q_full, G * DKB * 16384);
       for (int g = 0; g < G; ++g)
         for (int kb = 0; kb < DKB; ++kb)
-          tma_load_3d(smem + L::OFF_Q + (g * DKB + kb) * 16384, &tm_q, &misc->q_full, kb * 64, g * 128, h);
-      int it = 0;
-      for (int cc = 0; ok && cc < ncs; ++cc) {
+          tma_load_3d(q_bank + (g * DKB + kb) * 16384, &tm_q, &misc->q_full, kb * 64, g * 128, h);
+      Stage ks, ds;  // (a fresh ring's stages are empty: the phase before the first one counts as complete)
+      for (int cc = 0; ok && cc < ncs; ++cc, ks.next(nk)) {
         const int t0 = (c_begin + cc) * C;
-        const int ks = cc & 1;
-        if (cc >= 2 && !(ok = wait(&misc->k_empty[ks], ((cc - 2) >> 1) & 1))) break;
-        mbar_arrive_expect_tx(&misc->k_full[ks], DKB * 16384);
+        if (!(ok = wait(&misc->k_empty[ks.s], ks.phase ^ 1))) break;
+        mbar_arrive_expect_tx(&misc->k_full[ks.s], DKB * 16384);
         for (int kb = 0; kb < DKB; ++kb)
-          tma_load_4d(smem + L::OFF_K + (ks * DKB + kb) * 16384, &tm_k, &misc->k_full[ks], kb * 64, h, t0, b);
-        for (int gp = 0; ok && gp < 2 * G; ++gp, ++it) {  // (group, hi | lo plane)
+          tma_load_4d(k_ring + (ks.s * DKB + kb) * 16384, &tm_k, &misc->k_full[ks.s], kb * 64, h, t0, b);
+        for (int gp = 0; ok && gp < 2 * G; ++gp, ds.next(nds)) {  // (group, hi | lo plane)
           const int g = gp >> 1, part = gp & 1;
-          const int s = it & 1;
-          if (it >= 2 && !(ok = wait(&misc->ds_empty[s], ((it - 2) >> 1) & 1))) break;
-          mbar_arrive_expect_tx(&misc->ds_full[s], 32768);
+          if (!(ok = wait(&misc->ds_empty[ds.s], ds.phase ^ 1))) break;
+          mbar_arrive_expect_tx(&misc->ds_full[ds.s], plane);
           for (int tb = 0; tb < 2; ++tb)  // (rows beyond M read as zero)
-            tma_load_4d(smem + L::OFF_DS + s * 32768 + tb * 16384, &tm_ds, &misc->ds_full[s], t0 + tb * 64, g * 128, part,
-                        lane_id);
+            tma_load_4d(smem + ds.s * plane + tb * (plane >> 1), &tm_ds, &misc->ds_full[ds.s], t0 + tb * 64, g * 128, part, lane_id);
         }
       }
       pdl_trigger();
@@ -1224,34 +1247,35 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
       constexpr uint32_t ID_DK = make_idesc_bf16(128, DK, 1, 1);  // dS (MN-major: tokens contiguous) x Q (MN-major)
       constexpr uint32_t ID_DQ = make_idesc_bf16(128, DK, 0, 1);  // dS (K-major: rows = latents) x K tile (MN-major)
       ok = wait(&misc->q_full, 0);
-      int it = 0;
-      for (int cc = 0; ok && cc < ncs; ++cc) {
-        const int ks = cc & 1, kb = cc & 1;
-        if (!(ok = wait(&misc->k_full[ks], (cc >> 1) & 1))) break;
+      Stage ks, ds;
+      for (int cc = 0; ok && cc < ncs; ++cc, ks.next(nk)) {
+        const int kb = cc & 1;
+        if (!(ok = wait(&misc->k_full[ks.s], ks.phase))) break;
         if (cc >= 2 && !(ok = wait(&misc->dk_free[kb], ((cc - 2) >> 1) & 1))) break;
         tc_fence_after_sync();
-        const uint64_t d_k_mn = make_desc_sw128(smem_u32(smem + L::OFF_K + ks * DKB * 16384), 16384, 1024);
-        for (int gp = 0; ok && gp < 2 * G; ++gp, ++it) {  // (group, hi | lo plane): lo accumulates on top of hi
+        const uint64_t d_k_mn = make_desc_sw128(smem_u32(k_ring + ks.s * DKB * 16384), 16384, 1024);
+        for (int gp = 0; ok && gp < 2 * G; ++gp, ds.next(nds)) {  // (group, hi | lo plane): lo accumulates on top of hi
           const int g = gp >> 1;
-          const int s = it & 1;
-          if (!(ok = wait(&misc->ds_full[s], (it >> 1) & 1))) break;
+          if (!(ok = wait(&misc->ds_full[ds.s], ds.phase))) break;
           tc_fence_after_sync();
-          const uint32_t ds_addr = smem_u32(smem + L::OFF_DS + s * 32768);
-          const uint64_t d_ds_mn = make_desc_sw128(ds_addr, 16384, 1024), d_ds_k = make_desc_sw128(ds_addr, 16, 1024);
-          const uint64_t d_q_mn = make_desc_sw128(smem_u32(smem + L::OFF_Q + g * DKB * 16384), 16384, 1024);
+          const uint32_t ds_addr = smem_u32(smem + ds.s * plane);
+          const uint64_t d_ds_mn = make_desc_sw128(ds_addr, plane >> 1, 1024), d_ds_k = make_desc_sw128(ds_addr, 16, 1024);
+          const uint64_t d_q_mn = make_desc_sw128(smem_u32(q_bank + g * DKB * 16384), 16384, 1024);
           const int rows = min(128, p.M - g * 128);
           const int ksm = (rows + 15) >> 4;
           for (int st = 0; st < ksm; ++st)  // contraction over the latents of the group
-            mma_ss(tmem + L::TM_DK + kb * DK, mnmaj_step(d_ds_mn, st), mnmaj_step(d_q_mn, st), ID_DK, (gp > 0 || st > 0) ? 1u : 0u);
+            mma_ss(tmem + TM_DK + kb * DK, mnmaj_step(d_ds_mn, st), mnmaj_step(d_q_mn, st), ID_DK, (gp > 0 || st > 0) ? 1u : 0u);
+          // contraction over the tokens of the chunk.  (Planes of 64 rows: the product's upper 64 rows come from whatever lies behind
+          // the block; they belong to no latent and are not read.)
 #pragma unroll
-          for (int st = 0; st < 8; ++st)  // contraction over the tokens of the chunk
-            mma_ss(tmem + L::TM_DQ + g * DK, kmaj_step(d_ds_k, st), mnmaj_step(d_k_mn, st), ID_DQ,
-                   (cc > 0 || (gp & 1) || st > 0) ? 1u : 0u);
-          tc_commit(&misc->ds_empty[s]);
+          for (int st = 0; st < 8; ++st)
+            mma_ss(tmem + TM_DQ + g * DK, d_ds_k + (uint64_t)(((st >> 2) * (plane >> 1) + (st & 3) * 32) >> 4), mnmaj_step(d_k_mn, st),
+                   ID_DQ, (cc > 0 || (gp & 1) || st > 0) ? 1u : 0u);
+          tc_commit(&misc->ds_empty[ds.s]);
         }
         if (!ok) break;
         tc_commit(&misc->dk_ready[kb]);
-        tc_commit(&misc->k_empty[ks]);
+        tc_commit(&misc->k_empty[ks.s]);
       }
       if (ok) tc_commit(&misc->dq_ready);
     }
@@ -1259,34 +1283,42 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
     const int wq = warp & 3;  // TMEM lane quarter of this warp
     const uint32_t tl = tmem + ((uint32_t)(wq * 32) << 16);
     const int tt = wq * 32 + lane;
-    __nv_bfloat16* dk_base = reinterpret_cast<__nv_bfloat16*>(p.dk) + ((int64_t)b * p.N * p.H + h) * DK;
     for (int cc = 0; ok && cc < ncs; ++cc) {
       const int kb = cc & 1;
-      const int t = (c_begin + cc) * C + tt;
       if (!(ok = wait(&misc->dk_ready[kb], (cc >> 1) & 1))) break;
       tc_fence_after_sync();
 #pragma unroll
       for (int half = 0; half < DK / 32; ++half) {
         uint32_t r[32];
-        tmem_ld32(tl + L::TM_DK + kb * DK + half * 32, r);
+        tmem_ld32(tl + TM_DK + kb * DK + half * 32, r);
         tmem_wait_ld();
         tmem_fence_regs(r);
-        if (t < p.N) {
-          uint4* dst = reinterpret_cast<uint4*>(dk_base + (int64_t)t * p.H * DK + half * 32);
+        if (half == DK / 32 - 1) {
+          tc_fence_before_sync();
+          warp_arrive(&misc->dk_free[kb], lane);
+        }
+        // two 32 x 32 tiles (64-byte swizzle), stored in turn; rows beyond the sequence end are clipped
+        uint8_t* const tile = stage + wq * 4096 + (half & 1) * 2048;
+        if (lane == 0) bulk_wait_group_read1();
+        __syncwarp();
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            uint4 v;
-            v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]) * p.scale, __uint_as_float(r[ch * 8 + 1]) * p.scale);
-            v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]) * p.scale, __uint_as_float(r[ch * 8 + 3]) * p.scale);
-            v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]) * p.scale, __uint_as_float(r[ch * 8 + 5]) * p.scale);
-            v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]) * p.scale, __uint_as_float(r[ch * 8 + 7]) * p.scale);
-            dst[ch] = v;
-          }
+        for (int ch = 0; ch < 4; ++ch) {
+          uint4 v;
+          v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]) * p.scale, __uint_as_float(r[ch * 8 + 1]) * p.scale);
+          v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]) * p.scale, __uint_as_float(r[ch * 8 + 3]) * p.scale);
+          v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]) * p.scale, __uint_as_float(r[ch * 8 + 5]) * p.scale);
+          v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]) * p.scale, __uint_as_float(r[ch * 8 + 7]) * p.scale);
+          *reinterpret_cast<uint4*>(tile + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) = v;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_4d(&tm_dk, tile, half * 32, h, (c_begin + cc) * C + wq * 32, b);
+          bulk_commit_group();
         }
       }
-      tc_fence_before_sync();
-      warp_arrive(&misc->dk_free[kb], lane);
     }
+    if (lane == 0) bulk_wait_group0();
     // this split's part of dQ
     float* part = p.dq_part + (((int64_t)(b * p.nsplit + split) * p.H + h) * p.M) * DK;
     if (ncs > 0) ok = ok && wait(&misc->dq_ready, 0);
@@ -1297,7 +1329,7 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
       for (int half = 0; half < DK / 32; ++half) {
         uint32_t r[32];
         if (ncs > 0 && ok) {
-          tmem_ld32(tl + L::TM_DQ + g * DK + half * 32, r);
+          tmem_ld32(tl + TM_DQ + g * DK + half * 32, r);
           tmem_wait_ld();
           tmem_fence_regs(r);
         } else {
@@ -1324,13 +1356,14 @@ bwd_tc_grads_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_cons
 }
 
 template <int DKB>
-int launch_grads(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMap& tq, const GradTcParams& p, dim3 grid,
-                 cudaStream_t stream) {
+int launch_grads(const CUtensorMap& tds, const CUtensorMap& tk, const CUtensorMap& tq, const CUtensorMap& tdk, GradTcParams p,
+                 dim3 grid, cudaStream_t stream) {
   auto kern = bwd_tc_grads_kernel<DKB>;
-  const int smem = GL<DKB>::smem_bytes(p.groups);
+  const GradRings r = grad_rings(p.M, DKB);
+  p.plane = r.plane; p.nds = r.nds; p.nk = r.nk;
   FLARE_CUDA_CHECK(allow_smem(kern));
   LaunchTimer timer("bwd_tc_grads_kernel", stream);
-  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_GRAD), smem, stream, tds, tk, tq, p));
+  FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NT_GRAD), r.smem, stream, tds, tk, tq, tdk, p));
   return FLARE_OK;
 }
 
@@ -1596,7 +1629,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
   }
   // (3) reverse chunk sweep: dV and the dS plane
   const bool pack = f.M <= 64;
-  CUtensorMap tk, tv, tdy, tu, tds, tds_out, tdv, tq;
+  CUtensorMap tk, tv, tdy, tu, tds, tdv, tdk, tq;
   {
     const uint64_t dimk[4] = {(uint64_t)f.Dk, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B};
     const uint64_t dimv[4] = {(uint64_t)f.Dv, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B};
@@ -1609,18 +1642,20 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     const uint32_t boxu[4] = {64, pack ? 64u : 128u, 1, 1};
     const uint64_t dims[4] = {(uint64_t)pl.npad, (uint64_t)f.M, 2, (uint64_t)lanes};
     const int64_t strs[3] = {pl.npad, (int64_t)f.M * pl.npad, 2 * (int64_t)f.M * pl.npad};
-    const uint32_t boxs[4] = {64, 128, 1, 1}, boxo[4] = {64, pack ? 64u : 128u, 1, 1};
+    const uint32_t boxs[4] = {64, pack ? 64u : 128u, 1, 1};
     // dV rows, or with several latent groups their dense partials
     void* const dv = pl.groups > 1 ? static_cast<void*>(ws + pl.off_dvp) : a.dv;
     const uint64_t dimdv[4] = {(uint64_t)f.Dv, (uint64_t)f.H, (uint64_t)f.N, (uint64_t)f.B * pl.groups};
     const int64_t strdv[3] = {f.Dv, (int64_t)f.H * f.Dv, (int64_t)f.N * f.H * f.Dv};
+    const int64_t strdk[3] = {f.Dk, (int64_t)f.H * f.Dk, (int64_t)f.N * f.H * f.Dk};
     const uint32_t boxdv[4] = {32, 1, 32, 1};
     const uint64_t dimq[3] = {(uint64_t)f.Dk, (uint64_t)f.M, (uint64_t)f.H};
     const int64_t strq[2] = {f.q_stride_m, f.q_stride_h};
     const uint32_t boxq[3] = {64, 128, 1};
     if (!tc::make_map_bf16(&tk, f.k, 4, dimk, strk, box) || !tc::make_map_bf16(&tv, f.v, 4, dimv, strv, box) ||
         !tc::make_map_bf16(&tdy, a.dy, 4, dimv, strd, box) || !tc::make_map_bf16(&tu, keep.u, 4, dimu, stru, boxu) ||
-        !tc::make_map_bf16(&tds, ws + pl.off_ds, 4, dims, strs, boxs) || !tc::make_map_bf16(&tds_out, ws + pl.off_ds, 4, dims, strs, boxo) ||
+        !tc::make_map_bf16(&tds, ws + pl.off_ds, 4, dims, strs, boxs) ||
+        !tc::make_map_bf16(&tdk, a.dk, 4, dimk, strdk, boxdv, CU_TENSOR_MAP_SWIZZLE_64B) ||
         !tc::make_map_bf16(&tdv, dv, 4, dimdv, strdv, boxdv, CU_TENSOR_MAP_SWIZZLE_64B) || !tc::make_map_bf16(&tq, f.q, 3, dimq, strq, boxq)) {
       set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (backward operands)");
       return FLARE_ERR_CUDA;
@@ -1650,7 +1685,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
       const auto launch = f.Dk == 128   ? (pack ? launch_bwd_tc_unit<4> : launch_bwd_tc_unit<1>)
                           : f.Dv == 128 ? (pack ? launch_bwd_tc_unit<5> : launch_bwd_tc_unit<2>)
                                         : (pack ? launch_bwd_tc_unit<3> : launch_bwd_tc_unit<0>);
-      return launch(mode, tk, tv, tdy, tu, tds_out, tdv, p, grid, stream);
+      return launch(mode, tk, tv, tdy, tu, tds, tdv, p, grid, stream);
     };
     int rc = FLARE_OK;
     if (pl.seg.n > 1 && !pl.seg.lead) {
@@ -1676,10 +1711,10 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     memset(&g, 0, sizeof(g));
     g.N = f.N; g.H = f.H; g.M = f.M; g.B = f.B; g.nch = pl.nch; g.npad = pl.npad; g.groups = pl.groups;
     g.nsplit = pl.nsplit; g.chunks_per_split = pl.chunks_per_split; g.scale = f.scale;
-    g.dk = a.dk; g.dq_part = reinterpret_cast<float*>(ws + pl.off_dqp);
+    g.dq_part = reinterpret_cast<float*>(ws + pl.off_dqp);
     g.err = err;
     const dim3 grid((unsigned)lanes, pl.nsplit, 1);
-    const int rc = f.Dk == 128 ? launch_grads<2>(tds, tk, tq, g, grid, stream) : launch_grads<1>(tds, tk, tq, g, grid, stream);
+    const int rc = f.Dk == 128 ? launch_grads<2>(tds, tk, tq, tdk, g, grid, stream) : launch_grads<1>(tds, tk, tq, tdk, g, grid, stream);
     if (rc != FLARE_OK) return rc;
     const int64_t n4 = (int64_t)f.H * f.M * f.Dk / 4;
     LaunchTimer timer("bwd_tc_sum_dq_kernel", stream);

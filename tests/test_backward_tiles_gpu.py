@@ -1,6 +1,6 @@
-"""GPU: dS and dV of the tensor-core backward leave in tiles of 64 and 32 tokens that are clipped at the sequence's and the latent
+"""GPU: dS, dV and dK of the tensor-core backward leave in tiles of 64 and 32 tokens that are clipped at the sequence's and the latent
 bank's end.  Lengths and banks around the tiles' edges, against the oracle's closed form (not one token: its y is v whatever q and k
-are, so that dQ = 0 has no relative error); nothing around dV is touched."""
+are, so that dQ = 0 has no relative error); nothing around dV and dK is touched."""
 import ctypes as C
 
 import pytest
@@ -23,16 +23,18 @@ def test_rows_that_leave_in_tiles(B, N, H, M, Dk, Dv, bs):
     ref = orc.ar_backward_closed_form(q, k, v, dy, block_size=bs)
     qc, kc, vc, dyc = to_dev(q, k, v, dy)
     guard, size = 4096, B * N * H * Dv
-    dv_all = torch.full((size + 2 * guard,), 7.0, dtype=torch.bfloat16, device="cuda")
-    dq, dk = torch.empty(q.shape, dtype=torch.bfloat16, device="cuda"), torch.empty_like(kc)
+    ksize = B * N * H * Dk
+    dv_all, dk_all = (torch.full((n + 2 * guard,), 7.0, dtype=torch.bfloat16, device="cuda") for n in (size, ksize))
+    dq = torch.empty(q.shape, dtype=torch.bfloat16, device="cuda")
     a = _lib.BwdArgs()
     a.fwd = _lib.make_fwd_args(qc, kc, vc, None, None, None, scale=Dk ** -0.5, block_size=bs)
     a.dy = dyc.data_ptr()
     a.dy_stride_b, a.dy_stride_n, a.dy_stride_h = dyc.stride()[:3]
-    a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv_all[guard:].data_ptr()
+    a.dq, a.dk, a.dv = dq.data_ptr(), dk_all[guard:].data_ptr(), dv_all[guard:].data_ptr()
     a.dq_dtype = 1
     assert _lib.load().flare_backward_uses_tensor_path(C.byref(a)) == 1
     _lib.run_backward(a, dyc.device)
-    got = dict(dQ=dq, dK=dk, dV=dv_all[guard:guard + size].view(B, N, H, Dv))
+    got = dict(dQ=dq, dK=dk_all[guard:guard + ksize].view(B, N, H, Dk), dV=dv_all[guard:guard + size].view(B, N, H, Dv))
     check_gate(got, ref, f"tiles {(B, N, H, M, Dk, Dv, bs)}", rel_l2=SWEEP)
-    assert bool((dv_all[:guard] == 7).all()) and bool((dv_all[guard + size:] == 7).all())
+    for x, n in ((dv_all, size), (dk_all, ksize)):
+        assert bool((x[:guard] == 7).all()) and bool((x[guard + n:] == 7).all())
