@@ -1022,12 +1022,13 @@ namespace {
 // per-token statistics: delta_t = <dY_t, y_t> and the decode log-sum-exp in log2 units, rows padded to whole chunks
 // (delta = 0, log-sum-exp = +inf there, which makes every decode weight of a padding token exactly zero)
 // -------------------------------------------------------------------------------------------------
-// One block per (16 tokens, batch row), 16 heads at a time: dY and y of a token lie head by head behind one another, so a block
-// streams them in long runs with four pieces of each in flight per thread; its results, which lie token by token, go through
-// shared memory into rows of 16.  (One piece of each per thread and results scattered as they come: 41 us at B=4 N=4096 H=16
-// D=128, 134 MB to read.)
-constexpr int ST_TOK = 16, ST_HEADS = 16;
-__global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bfloat16* dy, int64_t dy_sb,
+// One block per (8 tokens, batch row), 16 heads at a time: dY and y of a token lie head by head behind one another, so a block
+// streams them in long runs with two pieces of each in flight per thread, eight blocks to an SM; its results, which lie token by
+// token, go through shared memory into rows of 8.  B=4 N=4096 H=16 D=128, 134 MB to read, us with the launch: 31; 35 with 16
+// tokens and four pieces (its grid is 1.7 waves), 33 with 4 tokens or one piece, 41 with 16 tokens and eight pieces, 41 with one
+// piece and results scattered as they come.
+constexpr int ST_TOK = 8, ST_HEADS = 16, ST_LOADS = 2;
+__global__ void __launch_bounds__(256, 8) bwd_tc_token_stats_kernel(const __nv_bfloat16* dy, int64_t dy_sb,
                                                                   int64_t dy_sn, int64_t dy_sh,
                                                                   const __nv_bfloat16* y, int64_t y_sb,
                                                                   int64_t y_sn, int64_t y_sh, const float* lse,
@@ -1054,17 +1055,17 @@ __global__ void __launch_bounds__(256) bwd_tc_token_stats_kernel(const __nv_bflo
   const __nv_bfloat16* const y_b = y + b * y_sb + sub * 8;
   for (int h0 = 0; h0 < H; h0 += ST_HEADS) {
     const int heads = min(ST_HEADS, H - h0);
-    for (int r0 = row0; r0 < ST_TOK * heads; r0 += 4 * rows_per_pass) {  // (the same for all rows of a warp)
-      uint4 a[4], c[4];
+    for (int r0 = row0; r0 < ST_TOK * heads; r0 += ST_LOADS * rows_per_pass) {  // (the same for all rows of a warp)
+      uint4 a[ST_LOADS], c[ST_LOADS];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < ST_LOADS; ++u) {
         const int r = r0 + u * rows_per_pass, t = r / heads, h = h0 + (r - t * heads), n = n0 + t;
         const bool on = t < ST_TOK && n < N;
         a[u] = on ? *reinterpret_cast<const uint4*>(dy_b + (int64_t)n * dy_sn + h * dy_sh) : make_uint4(0, 0, 0, 0);
         c[u] = on ? *reinterpret_cast<const uint4*>(y_b + (int64_t)n * y_sn + h * y_sh) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < ST_LOADS; ++u) {
         float acc = (bf16_lo(a[u].x) * bf16_lo(c[u].x) + bf16_hi(a[u].x) * bf16_hi(c[u].x)) +
                     (bf16_lo(a[u].y) * bf16_lo(c[u].y) + bf16_hi(a[u].y) * bf16_hi(c[u].y)) +
                     (bf16_lo(a[u].z) * bf16_lo(c[u].z) + bf16_hi(a[u].z) * bf16_hi(c[u].z)) +
