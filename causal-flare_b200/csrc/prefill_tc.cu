@@ -60,7 +60,8 @@ namespace {
 constexpr int C = 128;    // tokens per chunk
 constexpr int M = 128;    // latents
 constexpr int D = 64;     // value columns per CTA, and width of one 128-byte operand block
-constexpr int NTHREADS = 448;
+// (keep: a warp that stores the kept states)
+constexpr int nthreads(bool keep) { return keep ? 480 : 448; }
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -95,8 +96,11 @@ struct Lay {
   // wide, two latent groups merged on chip: the partner CTA's normalised partial rows of the value block this CTA
   // finalises, [128 t][64] fp16 (16-byte pieces swizzled by row), and the log2 weight mass per row
   static constexpr int OFF_XCH = OFF_STAGE + 8192;         //                                          16 KB + 512 B
-  static constexpr int SMEM_BYTES = OFF_XCH + (WIDE ? 16384 + 512 : 0) + 1024;  // + slack for manual 1024-byte alignment
-  static_assert(SMEM_BYTES <= 232448, "shared memory");
+  static constexpr int OFF_KEEP = (OFF_XCH + 1023) / 1024 * 1024;  // training (not wide): the chunk's kept state, [128 m][64] bf16
+  static constexpr int smem_bytes(bool keep) {  // + slack for manual 1024-byte alignment
+    return (keep ? OFF_KEEP + 16384 : OFF_XCH + (WIDE ? 16384 + 512 : 0)) + 1024;
+  }
+  static_assert(smem_bytes(!WIDE) <= 232448, "shared memory");
   // tensor-memory columns.  [W | Y | Den] are adjacent (one product writes them); single accumulators, handed back by
   // the token group as soon as it has them in registers.  Wide: W shares the columns of S (the latent group has the
   // next chunk's scores in registers before W of this chunk is written) and U takes 128 columns.
@@ -108,7 +112,7 @@ constexpr uint32_t TM_COLS = 512;
 
 struct Misc {
   uint64_t q_full, k_full, k_empty, v_full[2], v_empty[2], v_conv[2];
-  uint64_t s_ready, s_free, kap_done, p1_done, u_done, w_ready, p2_done, y_ready, y_free;
+  uint64_t keep_free, s_ready, s_free, kap_done, p1_done, u_done, w_ready, p2_done, y_ready, y_free;
   uint64_t pmax[4], psum[4];  // pair barriers of the two latent half-groups, one per lane quarter
   uint64_t xfull[4], xfree[4];  // on-chip merge of two latent groups, per token warp: the partner's rows have arrived /
                                 // the partner has read the rows this CTA sent
@@ -218,7 +222,7 @@ int launch_prefill_tc_unit(int lat, const CUtensorMap& tq, const CUtensorMap& tk
 //       B=8 N=8192 H=16 M=128 D=64 182.3 -> 185.8 us, training B=4 N=4096 H=16 M=64 D=128 411 -> 424 us), and the type of y in
 //       the epilogue of the wide instance 5 to 8 %.
 template <int LAT, int DKB, int DVB, bool SPLIT, int MODE, bool KEEP, bool WIDE, int FL>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(nthreads(KEEP && !WIDE), 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_y,
                   const __grid_constant__ CUtensorMap tm_k_in, const __grid_constant__ CUtensorMap tm_v_in, const TcParams p) {
@@ -228,6 +232,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   static_assert(!KEEP || FL == 0, "training forwards are bf16 and know no lengths");
   constexpr bool LENS = FL != 0, F16 = FL == 2;
   static_assert(!PACK || !SPLIT, "one group of at most 64 latents");
+  // The kept states leave through a bulk store of the chunk's tile by a warp of its own (its tensor map comes as tm_k_in, which no
+  // training forward needs).  Stored by the latent threads, 32 bytes of a row each (512 transactions a chunk, packed), they made
+  // the state pass of a chunk 1 300 instead of 350 cycles.  B200, us a training step: B=4 N=4096 H=16 M=128 D=64 442 -> 432, M=64
+  // D=128 354 -> 348, B=2 N=2048 M=256 D=128 288 -> 283.  (Wide: no room for the tile.)
+  constexpr bool KEEP_TILE = KEEP && !WIDE;
+  constexpr int NTHREADS = nthreads(KEEP_TILE);
   constexpr int NP = PACK ? 4 : 2;       // token parts of a chunk = latent warps per 32 latents
   constexpr int TOK = C / NP;            // tokens per latent thread
   constexpr int ROWS = PACK ? 64 : 128;  // latent rows of the operand buffers that the products over the latents read
@@ -270,6 +280,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_init(&misc->v_empty[i], 1);
       mbar_init(&misc->v_conv[i], 1);
     }
+    mbar_init(&misc->keep_free, 1);
     mbar_init(&misc->s_ready, 1);
     mbar_init(&misc->s_free, 8);
     mbar_init(&misc->kap_done, 4);
@@ -398,6 +409,19 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         if (F16 && ok && nchunks > 0) ok = convert_v(nchunks - 1);
       }
+    }
+  } else if (KEEP_TILE && warp == 14) {
+    // ======================================= kept states =======================================
+    if (elect_one()) {
+      prefetch_tensormap(&tm_k_in);
+      for (int i = 0; ok && i < nchunks; ++i) {
+        if (!(ok = wait_or_abort(&misc->p1_done, i & 1, misc))) break;
+        tma_store_4d(&tm_k_in, smem + L::OFF_KEEP, value_col0<ZS, SPLIT>(), latent0<ZS, SPLIT>(), seg_begin / C + i, lane_id);
+        bulk_commit_group();
+        bulk_wait_group_read0();
+        mbar_arrive(&misc->keep_free);
+      }
+      bulk_wait_group0();
     }
   } else if (warp == 12) {
     // ======================================= MMA issuer =======================================
@@ -1059,19 +1083,18 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               c_true = fmaxf(c2, xmax_all(par));
               fin = ex2_approx(c2 - c_true);
             }
+            if (i > 0 && !(ok = wait_or_abort(&misc->keep_free, (i - 1) & 1, misc))) break;  // the tile has been read
+#pragma unroll
+            for (int ch = 0; ch < NU / 8; ++ch) {  // (rows beyond M are clipped)
+              uint4 v;
+              v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]) * fin, __uint_as_float(r[ch * 8 + 1]) * fin);
+              v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]) * fin, __uint_as_float(r[ch * 8 + 3]) * fin);
+              v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]) * fin, __uint_as_float(r[ch * 8 + 5]) * fin);
+              v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]) * fin, __uint_as_float(r[ch * 8 + 7]) * fin);
+              *reinterpret_cast<uint4*>(smem + L::OFF_KEEP + swz_chunk_off(m, (ucol >> 3) + ch)) = v;
+            }
             if (live) {
               const int64_t o = ((int64_t)lane_id * p.dump_nch + (seg_begin / C + i)) * p.M + latent0<ZS, SPLIT>() + m;
-              uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dump_u) + o * DV +
-                                                    value_col0<ZS, SPLIT>() + ucol);
-#pragma unroll
-              for (int ch = 0; ch < NU / 8; ++ch) {
-                uint4 v;
-                v.x = pack_bf16(__uint_as_float(r[ch * 8 + 0]) * fin, __uint_as_float(r[ch * 8 + 1]) * fin);
-                v.y = pack_bf16(__uint_as_float(r[ch * 8 + 2]) * fin, __uint_as_float(r[ch * 8 + 3]) * fin);
-                v.z = pack_bf16(__uint_as_float(r[ch * 8 + 4]) * fin, __uint_as_float(r[ch * 8 + 5]) * fin);
-                v.w = pack_bf16(__uint_as_float(r[ch * 8 + 6]) * fin, __uint_as_float(r[ch * 8 + 7]) * fin);
-                dst[ch] = v;
-              }
               if (tp == 0 && value_col0<ZS, SPLIT>() == 0) {
                 p.dump_c[o] = c_true;          // log2 units (unused for the stablemax encoder)
                 p.dump_d[o] = d_carry * fin;   // denominator before the chunk in that frame
@@ -1424,8 +1447,8 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     // the two latent-group CTAs of a lane (adjacent in grid.z) as one thread-block cluster
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = Lay<DKB, WIDE>::SMEM_BYTES;
+    cfg.blockDim = dim3(nthreads(KEEP && !WIDE));
+    cfg.dynamicSmemBytes = Lay<DKB, WIDE>::smem_bytes(KEEP && !WIDE);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1438,7 +1461,7 @@ int launch_keep(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     cfg.numAttrs = 2;
     FLARE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, ty, in[0], in[1], p));
   } else {
-    FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(NTHREADS), Lay<DKB, WIDE>::SMEM_BYTES, stream, tq, tk, tv, ty, in[0], in[1], p));
+    FLARE_CUDA_CHECK(launch_pdl(kern, grid, dim3(nthreads(KEEP && !WIDE)), Lay<DKB, WIDE>::smem_bytes(KEEP && !WIDE), stream, tq, tk, tv, ty, in[0], in[1], p));
   }
   return FLARE_OK;
 }
@@ -1738,6 +1761,16 @@ int launch_prefill_tc(const flare_fwd_args_t* a, const TcParams& p_in, int nseg_
         set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (keys / values of a masked call)");
         return FLARE_ERR_CUDA;
       }
+    }
+  }
+  if (p.dump_u != nullptr && !wide) {
+    // kept states [lanes][chunks][M][Dv], a value slice of a latent group at a time
+    const uint64_t dims[4] = {(uint64_t)a->Dv, (uint64_t)a->M, (uint64_t)p.dump_nch, (uint64_t)a->B * a->H};
+    const int64_t str[3] = {a->Dv, (int64_t)a->M * a->Dv, (int64_t)p.dump_nch * a->M * a->Dv};
+    const uint32_t box[4] = {64, a->M <= 64 ? 64u : 128u, 1, 1};
+    if (!tc::make_map_bf16(&in[0], p.dump_u, 4, dims, str, box)) {
+      set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (kept states)");
+      return FLARE_ERR_CUDA;
     }
   }
   const int groups = prefill_tc_latent_groups(a);
