@@ -1159,6 +1159,74 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // latent-group split: dense fp16 partials [group][B][N][H][DV] and log2 weight masses [group][B][N][H]
     const int64_t part_row0 = SPLIT ? (((int64_t)(blockIdx.z / ZS) * (gridDim.x / p.H) + b) * p.N) : 0;
     const int row0 = LENS && p.row_start != nullptr ? p.row_start[b] : 0;  // (-1: a packed row, whose y goes to the packed copy)
+    // Two latent groups merged on chip: a chunk's own rows wait in registers and are merged with the partner's behind the next chunk's
+    // mask, while that chunk's tril(W) V runs and the rows are long there.  B200, B=2 N=65536 H=32 M=256 D=128 blocks of 64: 1 899
+    // us, 1 967 with the merge at the end of its own chunk (a chunk's period 6 200 and 6 800 cycles).
+    constexpr bool XM = WIDE && SPLIT;
+    uint32_t own[XM ? 2 : 1][XM ? 32 : 1];
+    float lw_own = 0.f, inv_own = 0.f;
+    auto receive = [&](int i) {
+      if constexpr (XM) {
+        const int t0 = seg_begin + i * C, nvalid = min(C, seg_end - t0);
+        const uint32_t rank = cluster_ctarank();
+                  if (!(ok = tc::wait_or_abort_cluster(&misc->xfull[wq], i & 1, &misc->abort_flag))) return;
+                  const float lw_p = *reinterpret_cast<const float*>(smem + L::OFF_XCH + 16384 + tt * 4);
+                  uint4 xp[8];
+        #pragma unroll
+                  for (int ch = 0; ch < 8; ++ch)  // [warp][32-column half][32 rows x 64 bytes, 16-byte pieces swizzled as in the staging tile]
+                    xp[ch] = *reinterpret_cast<const uint4*>(smem + L::OFF_XCH + wq * 4096 + (ch >> 2) * 2048 + lane * 64 +
+                                                             (((ch & 3) ^ ((lane >> 1) & 3)) << 4));
+                  const float mx = fmaxf(lw_own, lw_p);
+                  float ca = 0.f, cb = 0.f;  // coefficients of the raw accumulator values and of the partner's normalised rows
+                  if (mx == -INFINITY) {
+                    // every group's weights underflowed: outside the numeric domain of this path
+                    if (rank == 0 && tt < nvalid) {
+                      atomicOr(p.err, 2);
+                      misc->out_of_domain = 1;
+                    }
+                  } else {
+                    const float wa = ex2_approx(lw_own - mx), wb = ex2_approx(lw_p - mx);
+                    const float iw = rcp_approx(wa + wb);
+                    ca = wa * iw * inv_own;
+                    cb = wb * iw;
+                    if (rank == 0 && p.lse_dec != nullptr && tt < nvalid)
+                      p.lse_dec[(int64_t)lane_id * p.N + t0 + tt] = (mx + __log2f(wa + wb)) * kLn2;
+                  }
+                  // The merged rows go out from the exchange tile itself (its layout is the bulk store's 64-byte swizzle and
+                  // the partner's rows are in registers by now): both 32-column tiles are stored without waiting on each other.
+                  uint8_t* const xt = smem + L::OFF_XCH + wq * 4096;
+        #pragma unroll
+                  for (int half = 0; half < 2; ++half) {
+                    const uint32_t(&r)[32] = own[half];
+        #pragma unroll
+                    for (int ch = 0; ch < 4; ++ch) {
+                      const uint4 x = xp[half * 4 + ch];
+                      const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+                      uint32_t o[4];
+                      float y[8];
+        #pragma unroll
+                      for (int j = 0; j < 4; ++j) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[j]));
+                        // own raw values * ca + partner's normalised values * cb, two columns per instruction
+                        f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
+                                         f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
+                      }
+                      pack_out(y, F16, o);
+                      *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
+                          make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                  }
+                  fence_proxy_async_smem();
+                  __syncwarp();
+                  if (lane == 0) {
+                    tma_store_4d(&tm_y, xt, (int)rank * 64, h, t0 + wq * 32, b);
+                    tma_store_4d(&tm_y, xt + 2048, (int)rank * 64 + 32, h, t0 + wq * 32, b);
+                    bulk_commit_group();
+                  }
+                  // (the partner learns that the tile is free when the next chunk's epilogue begins, see above: by then the
+                  // stores have long read it; it does not send before its own next epilogue anyway)
+      }
+    };
     for (int i = 0; !state_only && ok && i < nchunks; ++i) {
       const uint32_t par = i & 1;
       const int t0 = seg_begin + i * C;
@@ -1174,6 +1242,37 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint64_t rs2 = f2_pack(0.f, 0.f);  // row sum of the bf16-rounded masked W (the values the read-out MMA multiplies), as a pair of partial sums
       // last column (token of the chunk) this row may see: itself, or the end of its block
       const int be = BLOCK ? (tt | (p.block - 1)) : tt;
+      if constexpr (XM) {  // (the rows of the chunk before are in registers: 16 columns at a time)
+#pragma unroll 1
+        for (int j = 0; j < 8; ++j) {
+          uint32_t wp[8];
+          const int last = BLOCK ? be : tt;  // last column this row may see
+          if (__any_sync(0xffffffffu, j * 16 <= last)) {
+            uint32_t r[16];
+            tmem_read(tl + TM_W + j * 16, r);
+            if (__all_sync(0xffffffffu, j * 16 + 15 <= last)) {
+#pragma unroll
+              for (int k = 0; k < 16; k += 2) {
+                const uint32_t pk = pack_bf16(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+                wp[k >> 1] = pk;
+                rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < 16; k += 2) {
+                const uint32_t pk = pack_bf16(j * 16 + k <= last ? __uint_as_float(r[k]) : 0.f,
+                                              j * 16 + k + 1 <= last ? __uint_as_float(r[k + 1]) : 0.f);
+                wp[k >> 1] = pk;
+                rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
+              }
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) wp[k] = 0u;
+          }
+          tmem_st8(tl + TM_W + j * 8, wp);
+        }
+      } else {
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         uint32_t wp[16];
@@ -1205,11 +1304,16 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         tmem_st16(tl + TM_W + j * 16, wp);
       }
+      }
       tmem_wait_st();
       tc_fence_before_sync();
       warp_arrive(&misc->p2_done, lane);
       if (tid == 256) TC_TRACE(1, i, 1);
 
+      if (XM && xmerge && i > 0) {
+        receive(i - 1);
+        if (!ok) break;
+      }
       // normalise and store (wide: the first of the two value blocks; two accumulator phases per chunk)
       if (!(ok = wait_or_abort(&misc->y_ready, par, misc))) break;
       tc_fence_after_sync();
@@ -1244,8 +1348,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           // partial of the OTHER block (fp16) and the log2 of its weight mass into the partner's shared memory,
           // takes the partner's rows for its own block, and stores y = sum_g w_g y_g / sum_g w_g.
           const uint32_t rank = cluster_ctarank(), peer = rank ^ 1u;
-          const float lw_own = den_ok ? kap_i + __log2f(den) : -INFINITY;
-          uint32_t ra[32], rb[32], pk[32];
+          lw_own = den_ok ? kap_i + __log2f(den) : -INFINITY;
+          inv_own = inv;
+          uint32_t pk[32];
+          uint32_t(&ra)[32] = own[0], (&rb)[32] = own[1];
           // The exchange tile was the source of the previous chunk's bulk stores: once they have read it the partner
           // may send this chunk's rows (32 rows x 128 bytes and 32 weight masses per warp), which the barrier counts.
           if (lane == 0) {
@@ -1289,64 +1395,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             st_async_b32(mapa_shared(smem_u32(smem + L::OFF_XCH + 16384 + tt * 4), peer), __float_as_uint(lw_own), xbar);
           }
           if (tid == 256) TC_TRACE(1, i, 4);
-          // (2) receive the partner's rows of this CTA's block
-          if (!(ok = tc::wait_or_abort_cluster(&misc->xfull[wq], par, &misc->abort_flag))) break;
-          if (tid == 256) TC_TRACE(1, i, 5);
-          const float lw_p = *reinterpret_cast<const float*>(smem + L::OFF_XCH + 16384 + tt * 4);
-          uint4 xp[8];
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch)  // [warp][32-column half][32 rows x 64 bytes, 16-byte pieces swizzled as in the staging tile]
-            xp[ch] = *reinterpret_cast<const uint4*>(smem + L::OFF_XCH + wq * 4096 + (ch >> 2) * 2048 + lane * 64 +
-                                                     (((ch & 3) ^ ((lane >> 1) & 3)) << 4));
-          const float mx = fmaxf(lw_own, lw_p);
-          float ca = 0.f, cb = 0.f;  // coefficients of the raw accumulator values and of the partner's normalised rows
-          if (mx == -INFINITY) {
-            // every group's weights underflowed: outside the numeric domain of this path
-            if (rank == 0 && tt < nvalid) {
-              atomicOr(p.err, 2);
-              misc->out_of_domain = 1;
-            }
-          } else {
-            const float wa = ex2_approx(lw_own - mx), wb = ex2_approx(lw_p - mx);
-            const float iw = rcp_approx(wa + wb);
-            ca = wa * iw * inv;
-            cb = wb * iw;
-            if (rank == 0 && p.lse_dec != nullptr && tt < nvalid)
-              p.lse_dec[(int64_t)lane_id * p.N + t0 + tt] = (mx + __log2f(wa + wb)) * kLn2;
-          }
-          // The merged rows go out from the exchange tile itself (its layout is the bulk store's 64-byte swizzle and
-          // the partner's rows are in registers by now): both 32-column tiles are stored without waiting on each other.
-          uint8_t* const xt = smem + L::OFF_XCH + wq * 4096;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const uint32_t(&r)[32] = half ? rb : ra;
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch) {
-              const uint4 x = xp[half * 4 + ch];
-              const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
-              uint32_t o[4];
-              float y[8];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[j]));
-                // own raw values * ca + partner's normalised values * cb, two columns per instruction
-                f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
-                                 f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
-              }
-              pack_out(y, F16, o);
-              *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
-                  make_uint4(o[0], o[1], o[2], o[3]);
-            }
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_4d(&tm_y, xt, (int)rank * 64, h, t0 + wq * 32, b);
-            tma_store_4d(&tm_y, xt + 2048, (int)rank * 64 + 32, h, t0 + wq * 32, b);
-            bulk_commit_group();
-          }
-          // (the partner learns that the tile is free when the next chunk's epilogue begins, see above: by then the
-          // stores have long read it; it does not send before its own next epilogue anyway)
           if (tid == 256) TC_TRACE(1, i, 3);
           continue;
         }
@@ -1415,6 +1463,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (!ok) break;
       if (tid == 256) TC_TRACE(1, i, 3);
     }
+    if (XM && xmerge && !state_only && ok && nchunks > 0) receive(nchunks - 1);
     if (lane == 0) bulk_wait_group0();  // the bulk stores of this warp are complete
   }
   if (!ok) {
