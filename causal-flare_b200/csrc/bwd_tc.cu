@@ -58,7 +58,6 @@ struct BwdTcParams {
   float scale, power;
   const float *chunk_c, *chunk_d;  // [lanes][nch][M]
   const float *tok_l2, *tok_delta;  // [lanes][npad]
-  void* dv;      // bf16 [B, N, H, Dv] contiguous, or (more than one latent group) bf16 [groups][B][N][H][Dv]
   int groups;
   // Sequence segments (grid.z = the segments from seg_first on, segment s = chunks seg_begin[s] .. seg_begin[s + 1] - 1).
   int nseg, seg_first;
@@ -191,10 +190,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   // 16 bytes, 4 096 (dS) and 2 048 (dV) a chunk at M = D = 128, and everything else that goes through the load / store unit waits
   // behind them: at M = 64, D = 128 the descending pass took 4 400 of a chunk's 15 700 cycles and the dV rows 4 200.
   // dS is laid down where E (hi) and R (lo) were: packed, in their second copies, which are free when P, X and G have been formed;
-  // else in place, when the chunk's last product has run.  dV goes through R's first copy (packed) or the unused half of U's slot
-  // (Dv = 64); at Dv = 128 without packing there is no room and its rows are stored as they are.  B200, us a training step: B=4
-  // N=4096 H=16 M=128 D=64 482 -> 450, M=64 D=128 376 -> 362, B=8 M=64 D=64 432 -> 392, B=2 N=2048 M=256 D=128 304 -> 289.
-  constexpr bool DV_TILES = PACK || DVB == 1;
+  // else in place, when the chunk's last product has run.  dV goes through U's slot, of which Dv = 64 uses half; at Dv = 128 the next
+  // chunk's U comes when the rows have left.  B200, us a training step, dS (and dV where R's copy or U's slot had room) by threads -> in
+  // tiles: B=4 N=4096 H=16 M=128 D=64 482 -> 450, M=64 D=128 376 -> 362, B=8 M=64 D=64 432 -> 392; all dV rows through U's slot: B=4
+  // N=4096 H=32 M=128 D=128 723 -> 680, B=2 N=3000 H=8 M=96 D=128 165 -> 159, M <= 64 the same.
   pdl_wait();
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -275,7 +274,14 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         mbar_arrive_expect_tx(&misc->v_full, DVB * 16384);
 #pragma unroll
         for (int vb = 0; vb < DVB; ++vb) tma_load_4d(smem + L::OFF_V + vb * 16384, &tm_v, &misc->v_full, vb * 64, h, t0, b);
-        // U_i: read by the previous chunk's P product (which has run: px_ready above)
+        // dY: read by the previous chunk's dV and G products
+        if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
+        mbar_arrive_expect_tx(&misc->dy_full, DVB * 16384);
+#pragma unroll
+        for (int vb = 0; vb < DVB; ++vb) tma_load_4d(smem + L::OFF_DY + vb * 16384, &tm_dy, &misc->dy_full, vb * 64, h, t0, b);
+        // U_i: read by the previous chunk's P product (which has run: px_ready above); at Dv = 128 the previous (full) chunk's dV rows
+        // have left its slot
+        if (DVB == 2 && j > 0 && i + 1 < full_end && !(ok = wait_or_abort(&misc->dv_out, (j - 1 - (first - full_end)) & 1, misc))) break;
         mbar_arrive_expect_tx(&misc->u_full, DVB * 16384);
 #pragma unroll
         for (int vb = 0; vb < DVB; ++vb) {
@@ -283,11 +289,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           if constexpr (PACK)  // (boxes of 64 rows)
             tma_load_4d(smem + L::OFF_UR + vb * 16384 + 8192, &tm_u, &misc->u_full, vb * 64, 0, i, lane_id);
         }
-        // dY: read by the previous chunk's dV and G products
-        if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
-        mbar_arrive_expect_tx(&misc->dy_full, DVB * 16384);
-#pragma unroll
-        for (int vb = 0; vb < DVB; ++vb) tma_load_4d(smem + L::OFF_DY + vb * 16384, &tm_dy, &misc->dy_full, vb * 64, h, t0, b);
       }
       pdl_trigger();
     }
@@ -614,7 +615,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           for (int g = 0; g < NG; ++g) invg[g] = rcp_approx(dend[g]);
         }
         // ---- phase 1b: R = g / D rows (bf16)
-        if (PACK && after_full && !(ok = wait_or_abort(&misc->dv_out, fpar ^ 1, misc))) break;  // (the dV rows have left R)
         {
           float run = base_run;
 #pragma unroll
@@ -705,7 +705,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 
         // ---- phase 2b (descending): encoder part, dS rows to global memory as a hi + lo pair
         if (i < full_end) {
-          // dS may be laid down: see DV_TILES
+          // dS may be laid down: see above
           if (!(ok = PACK ? wait_or_abort(&misc->g_ready, par, misc) : wait_or_abort(&misc->dv_ready, par, misc))) break;
           float ccg[NG];  // block-causal: Cc + sum of R p from the start of the group's block on
           float cc = cc_carry + rp_later;
@@ -833,18 +833,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const uint32_t tl = tmem + ((uint32_t)(wq * 32) << 16);
     const int tt = wq * 32 + lane;
     const int lo = BLOCK ? (tt & ~(p.block - 1)) : tt;  // first column (token) this row keeps
-    uint8_t* const dv_stage = smem + (PACK ? L::OFF_R + (wq >> 1) * 16384 + (wq & 1) * 4096 : L::OFF_UR + 16384 + wq * 4096);
-    __nv_bfloat16* dv_base;
-    int64_t dv_stride_n;
-    {
-      const int64_t group_off = p.groups > 1 ? (int64_t)group * ((int64_t)(gridDim.x / p.H) * p.N * p.H * DV) : 0;
-      dv_base = reinterpret_cast<__nv_bfloat16*>(p.dv) + group_off + ((int64_t)b * p.N * p.H + h) * DV;
-      dv_stride_n = (int64_t)p.H * DV;
-    }
+    uint8_t* const dv_stage = smem + L::OFF_UR + (DVB == 2 ? wq * 8192 : 16384 + wq * 4096);  // this warp's tiles of the dV rows
     for (int j = 0; ok && j < steps; ++j) {
       const int i = first - 1 - j, t0 = i * C;
       const uint32_t par = j & 1, fpar = (j - (first - full_end)) & 1;
-      const int nvalid = min(C, p.N - t0);
       // masked A (bf16) into the K tile's buffer
       if (!(ok = wait_or_abort(&misc->a_ready, par, misc))) break;
       tc_fence_after_sync();
@@ -919,8 +911,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       if (!(ok = wait_or_abort(&misc->dv_ready, par, misc))) break;
       tc_fence_after_sync();
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 4);
-      // (packed: the latent group has read R)
-      if (PACK && !(ok = wait_or_abort(&misc->x_done, par, misc))) break;
 #pragma unroll
       for (int half = 0; half < DV / 32; ++half) {
         uint32_t r[32];
@@ -938,32 +928,25 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                              pack_bf16(__uint_as_float(r[ch * 8 + 2]), __uint_as_float(r[ch * 8 + 3])),
                              pack_bf16(__uint_as_float(r[ch * 8 + 4]), __uint_as_float(r[ch * 8 + 5])),
                              pack_bf16(__uint_as_float(r[ch * 8 + 6]), __uint_as_float(r[ch * 8 + 7])));
-        if constexpr (DV_TILES) {
-          // two 32 x 32 tiles per warp (64-byte swizzle), stored in turn; rows beyond the sequence end are clipped
-          uint8_t* const tile = dv_stage + (half & 1) * 2048;
-          if (lane == 0) bulk_wait_group_read1();
-          __syncwarp();
+        // a 32 x 32 tile (64-byte swizzle)
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) *reinterpret_cast<uint4*>(tile + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) = v[ch];
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_4d(&tm_dv, tile, half * 32, h, t0 + wq * 32, group * (int)(gridDim.x / p.H) + b);
-            bulk_commit_group();
-          }
-        } else if (tt < nvalid) {
-          uint4* dst = reinterpret_cast<uint4*>(dv_base + (int64_t)(t0 + tt) * dv_stride_n + half * 32);
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(dv_stage + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) = v[ch];
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) dst[ch] = v[ch];
-        }
+        for (int half = 0; half < DV / 32; ++half)  // (rows beyond the sequence end are clipped)
+          tma_store_4d(&tm_dv, dv_stage + half * 2048, half * 32, h, t0 + wq * 32, group * (int)(gridDim.x / p.H) + b);
+        bulk_commit_group();
+        bulk_wait_group_read0();
       }
-      if constexpr (PACK) {
-        if (lane == 0) bulk_wait_group_read0();
-        warp_arrive(&misc->dv_out, lane);
-      }
+      if constexpr (DVB == 2) warp_arrive(&misc->dv_out, lane);
+      else __syncwarp();
       if (tid == W_TOKEN * 32) BT_TRACE(1, j, 5);
     }
-    if (DV_TILES && lane == 0) bulk_wait_group0();
+    if (lane == 0) bulk_wait_group0();
   }
   if (!ok) {
     misc->abort_flag = 1;
@@ -1670,7 +1653,6 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     p.scale = f.scale; p.power = f.power;
     p.chunk_c = keep.c; p.chunk_d = keep.d; p.tok_l2 = tok_l2; p.tok_delta = tok_delta;
     p.groups = pl.groups;
-    p.dv = pl.groups > 1 ? static_cast<void*>(ws + pl.off_dvp) : a.dv;
     p.err = err;
     p.gate = gate;
     p.trace = trace_buffer();
