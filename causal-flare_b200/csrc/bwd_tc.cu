@@ -22,9 +22,9 @@
 // Main kernel, one CTA per (lane, group of 128 latents, sequence segment), 23 warps: 0-15 latent group (thread = latent = TMEM
 // lane, the four warps of a lane quarter take 32 tokens each; packed: see PACK), 16-19 token group (thread = token = TMEM lane:
 // causal masks of A and E^T R, dV store), 20 MMA issuer, 21 TMA producer, 22 stores of dS (elected threads: with lane 0
-// of the issuer and the producer, a training step B=4 N=4096 H=16 M=128 D=64 took 496 instead of 484 us).  Ten MMAs per chunk; every
-// operand that the latent / token threads produce (E, R, masked A, G as bf16) is written once into a 128-byte-swizzled buffer and read K-major or
-// MN-major as the product needs, so there is no transposition pass.
+// of the issuer and the producer, a training step B=4 N=4096 H=16 M=128 D=64 took 496 instead of 484 us).  Ten MMAs per chunk;
+// every operand that the latent / token threads produce (E, R, masked A, G as bf16) is written once into a 128-byte-swizzled
+// buffer and read K-major or MN-major as the product needs, so there is no transposition pass.
 #include "bwd_tc.cuh"
 
 #include <cuda.h>

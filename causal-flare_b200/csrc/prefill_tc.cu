@@ -28,12 +28,12 @@
 // 128-byte-swizzled buffers, so no transposition pass exists.  E, the bf16 copy of the state and the block whose
 // column 0 is d lie behind one another in shared memory, so that they form ONE MN-major B operand and R is read once
 // for all three products (28 MMA instructions per chunk at Dk = 64 instead of 44: every instruction costs 100-190
-// cycles from issue to issue in this kernel whatever its width, 49-130 cycles alone).
+// cycles from issue to issue in this kernel whatever its width, 60-100 where an elected thread issues, 49-130 alone).
 //
 // Warp roles (14 warps): 0-7 "latent group" (two warps per lane quarter, each half of the chunk's tokens): scores ->
 // E, R, state rescale (chunk i+1);  8-11 "token group": causal mask of W, normalisation and store of Y (chunk i);
-// 12: MMA issuer (one thread);  13: TMA producer (one thread).  The three stages work on consecutive chunks
-// concurrently.  E and R have one buffer each (every product that reads them is issued when the latent group has
+// 12: MMA issuer (one thread);  13: TMA producer (one thread);  training: 14 stores the kept states.  The three stages
+// work on consecutive chunks concurrently.  E and R have one buffer each (every product that reads them is issued when the latent group has
 // finished the chunk; the latent group waits for the state update of the previous chunk before it writes E), the
 // accumulators [W | Y | Den0] are single and go back to the MMA issuer as soon as the token group has them in
 // registers, K is single-buffered (free as soon as its score MMA has run), V has two stages.
