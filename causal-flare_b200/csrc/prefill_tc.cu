@@ -245,10 +245,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   constexpr int WS = PACK ? 4 : 2;       // slots of the frame maximum's exchange
   // The elected thread issues a chunk's products in 2 700 instead of 3 700 cycles (see elect_one).  B200, us: B=1 N=777 H=16 M=64 D=64
   // 20.7 -> 19.4, fp16 B=4 N=4096 H=16 M=64 D=128 88.9 -> 83.6, wide block-causal B=2 N=65536 H=32 M=256 D=128 2 024 -> 1 949; whole
-  // groups at (64, 64), H=16 M=128: fp16 B=8 N=4096 99.6 -> 96.1, training B=4 N=4096 432 -> 429, bf16 B=8 N=8192 the same.  Not where
+  // groups at (64, 64), H=16 M=128: fp16 B=8 N=4096 99.6 -> 96.1, training B=4 N=4096 432 -> 429.  Not where
   // products that follow one another faster only get in the way of the latent warps, which take 64 tokens a thread and are the
-  // longest chain by far (B=4 N=4096 H=8 M=128 D=128, two slices: 91.7 -> 94.1; H=16 M=192 D=64: 121.2 -> 122.4; M=96: 89.8 -> 90.2).
-  constexpr bool ELECT = PACK || WIDE || (LAT == 0 && DKB == 1 && DVB == 1 && !SPLIT);
+  // longest chain by far (B=4 N=4096 H=8 M=128 D=128, two slices: 91.7 -> 94.1; H=16 M=192 D=64: 121.2 -> 122.4; M=96: 89.8 -> 90.2; B=8 N=8192 M=128 between 174.9 of 176.1 and 182.8 of 180.2).
+  constexpr bool ELECT = PACK || WIDE || (LAT == 0 && DKB == 1 && DVB == 1 && !SPLIT && (F16 || KEEP));
   constexpr int ZS = WIDE ? 1 : DVB;  // value slices on grid.z
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_E = L::OFF_E, OFF_R = L::OFF_R, OFF_U = L::OFF_U,
