@@ -392,15 +392,18 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       for (int j = 0; ok && j < steps; ++j) {
         const int i = first - 1 - j;
         if (!(ok = wait_or_abort(&misc->x_done, j & 1, misc))) break;
-        if (i >= full_end) continue;
-        constexpr int COPY = PACK ? 8192 : 0;
+        if (i < full_end) {
+          constexpr int COPY = PACK ? 8192 : 0;
 #pragma unroll
-        for (int tb = 0; tb < 2; ++tb) {  // (rows beyond M are clipped)
-          tma_store_4d(&tm_ds, smem + L::OFF_E + tb * 16384 + COPY, i * C + tb * 64, group * 128, 0, lane_id);
-          tma_store_4d(&tm_ds, smem + L::OFF_R + tb * 16384 + COPY, i * C + tb * 64, group * 128, 1, lane_id);
+          for (int tb = 0; tb < 2; ++tb) {  // (rows beyond M are clipped)
+            tma_store_4d(&tm_ds, smem + L::OFF_E + tb * 16384 + COPY, i * C + tb * 64, group * 128, 0, lane_id);
+            tma_store_4d(&tm_ds, smem + L::OFF_R + tb * 16384 + COPY, i * C + tb * 64, group * 128, 1, lane_id);
+          }
+          bulk_commit_group();
+          bulk_wait_group_read0();
         }
-        bulk_commit_group();
-        bulk_wait_group_read0();
+        // In the chunks that only move the carries too, where there is nothing to store: the latent warps wait for this phase before
+        // their next chunk, so that x_done cannot complete twice before this warp has looked at it (it would look unfinished then).
         mbar_arrive(&misc->ds_out);
       }
       bulk_wait_group0();
@@ -537,7 +540,6 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       for (int j = 0; ok && j < steps; ++j) {
         const int i = first - 1 - j, t0 = i * C;
         const uint32_t par = j & 1, pp = (j - 1) & 1;
-        const uint32_t fpar = (j - (first - full_end)) & 1;  // parity among the full chunks
         const int nvalid = min(C, p.N - t0);
         const int lim = live ? nvalid - tok0 : 0;  // tokens of this thread's part that exist (may be <= 0)
         const bool fast = __all_sync(0xffffffffu, lim >= TOK);
@@ -550,10 +552,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         const float c_pre = (live && !STABLE && i > 1) ? ld_pinned(p.chunk_c + stat0 + (int64_t)(i - 2) * p.M) : c_nxt;
         const float l2_pre = i > 0 ? ld_pinned(l2_row + (int64_t)(i - 1) * C) : 0.f;
         const float dl_pre = i > 0 ? ld_pinned(dl_row + (int64_t)(i - 1) * C) : 0.f;
-        // E / R buffers: the previous chunk's products have read them
-        if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc))) break;
-        const bool after_full = i + 1 < full_end && j > 0;  // and the previous (full) chunk's dS has left them
-        if (after_full && !(ok = wait_or_abort(&misc->ds_out, fpar ^ 1, misc))) break;
+        // E / R buffers: the previous chunk's products have read them, and its dS has left them
+        if (j > 0 && !(ok = wait_or_abort(&misc->dv_ready, pp, misc) && wait_or_abort(&misc->ds_out, pp, misc))) break;
         if (!(ok = wait_or_abort(&misc->s_ready, par, misc))) break;
         tc_fence_after_sync();
         if (tid == 0) BT_TRACE(0, j, 0);

@@ -231,3 +231,26 @@ def test_segments_of_the_sweep(B, N, H, M, Dk, Dv, variant, bs):
     again = grads(q, k, v, dy, variant=variant, block_size=bs)
     assert all(torch.equal(got[key], again[key]) for key in got), "not run-to-run deterministic"
     assert _ops.device_status() == 0
+
+
+def check_against_exact_by_chunk(B, N, H, M, Dk, Dv, what):
+    """Against the exact kernels, every 128-token chunk of dK and dV by itself (one that another chunk's tile got into would not
+    show in the whole tensor's norm), and twice for the same bits.  The bound is SWEEP and the rounding of the exact kernels' own
+    bf16 outputs, 2^-8 / sqrt(3) at most, in squares: 6.9e-3."""
+    q, k, v, dy = orc.make_inputs(B, N, H, M, Dk, Dv, seed0=8, dtype=torch.bfloat16, with_dy=True)
+    got, ref, again = (grads(q, k, v, dy, path=path) for path in (_lib.PATH_AUTO, _lib.PATH_EXACT, _lib.PATH_AUTO))
+    assert orc.rel_l2(got["dQ"], ref["dQ"]) <= 7e-3, f"{what} dQ"
+    for key in ("dK", "dV"):
+        for t0 in range(0, N, 128):
+            err = orc.rel_l2(got[key][:, t0:t0 + 128], ref[key][:, t0:t0 + 128])
+            assert err <= 7e-3, f"{what} {key}, tokens from {t0} on: {err:.2e}"
+    assert all(torch.equal(got[key], again[key]) for key in got), "not run-to-run deterministic"
+    assert _ops.device_status() == 0
+
+
+# Chunks that only move the carries: before a segment's own ones (64 lanes in two segments), and alone (20 lanes in seven segments
+# of seven chunks that exchange theirs).
+@pytest.mark.parametrize("B,N,H,M,Dk,Dv", [(4, 2600, 16, 64, 64, 64), (4, 2600, 16, 96, 128, 128), (1, 6000, 20, 64, 128, 128),
+                                           (1, 6000, 20, 128, 64, 64)])
+def test_chunks_that_only_move_the_carries(B, N, H, M, Dk, Dv):
+    check_against_exact_by_chunk(B, N, H, M, Dk, Dv, f"carries {(B, N, H, M, Dk, Dv)}")
