@@ -248,6 +248,13 @@ def check_against_exact_by_chunk(B, N, H, M, Dk, Dv, what):
     assert _ops.device_status() == 0
 
 
+# 78 lanes: one CTA of the dK / dQ kernel walks a lane's eleven chunks, so that every stage of its rings (4 K tiles and 8 dS planes
+# down to 2 and 2) is filled several times and the tiles of dK are used again; and one CTA of the sweep does, without segments.
+@pytest.mark.parametrize("M,Dk,Dv", [(64, 64, 64), (128, 64, 128), (192, 64, 64), (64, 128, 128), (128, 128, 128), (256, 128, 128)])
+def test_rings_are_used_again(M, Dk, Dv):
+    check_against_exact_by_chunk(3, 1300, 26, M, Dk, Dv, f"rings {(M, Dk, Dv)}")
+
+
 # Chunks that only move the carries: before a segment's own ones (64 lanes in two segments), and alone (20 lanes in seven segments
 # of seven chunks that exchange theirs).
 @pytest.mark.parametrize("B,N,H,M,Dk,Dv", [(4, 2600, 16, 64, 64, 64), (4, 2600, 16, 96, 128, 128), (1, 6000, 20, 64, 128, 128),
