@@ -250,6 +250,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   // longest chain by far (B=4 N=4096 H=8 M=128 D=128, two slices: 91.7 -> 94.1; H=16 M=192 D=64: 121.2 -> 122.4; M=96: 89.8 -> 90.2; B=8 N=8192 M=128 between 174.9 of 176.1 and 182.8 of 180.2).
   constexpr bool ELECT = PACK || WIDE || (LAT == 0 && DKB == 1 && DVB == 1 && !SPLIT && (F16 || KEEP));
   constexpr int ZS = WIDE ? 1 : DVB;  // value slices on grid.z
+  constexpr bool XM = WIDE && SPLIT && FL != 1;  // may merge two latent groups on chip (never in a call with lengths)
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
   constexpr int OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_E = L::OFF_E, OFF_R = L::OFF_R, OFF_U = L::OFF_U,
                 OFF_B16 = L::OFF_B16, OFF_Q = L::OFF_Q, OFF_MISC = L::OFF_MISC, VB = L::VB, D_BYTES = L::D_BYTES;
@@ -314,7 +315,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   // on-chip merge: the partner CTA arrives on this CTA's barriers, which must be initialised first
-  const bool xmerge = WIDE && SPLIT && p.cluster_merge != 0;
+  const bool xmerge = XM && p.cluster_merge != 0;
   if (xmerge) cluster_sync_all();
   const uint32_t tmem = misc->tmem_base;
   bool ok = true;
@@ -1163,7 +1164,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // Two latent groups merged on chip: a chunk's own rows wait in registers and are merged with the partner's behind the next chunk's
     // mask, while that chunk's tril(W) V runs and the rows are long there.  B200, B=2 N=65536 H=32 M=256 D=128 blocks of 64: 1 899
     // us, 1 967 with the merge at the end of its own chunk (a chunk's period 6 200 and 6 800 cycles).
-    constexpr bool XM = WIDE && SPLIT;
     uint32_t own[XM ? 2 : 1][XM ? 32 : 1];
     float lw_own = 0.f, inv_own = 0.f;
     auto receive = [&](int i) {
@@ -1243,68 +1243,39 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint64_t rs2 = f2_pack(0.f, 0.f);  // row sum of the bf16-rounded masked W (the values the read-out MMA multiplies), as a pair of partial sums
       // last column (token of the chunk) this row may see: itself, or the end of its block
       const int be = BLOCK ? (tt | (p.block - 1)) : tt;
-      if constexpr (XM) {  // (the rows of the chunk before are in registers: 16 columns at a time)
+      // (with the rows of the chunk before in registers 16 columns at a time, else 32)
+      constexpr int MW = XM ? 16 : 32;
 #pragma unroll 1
-        for (int j = 0; j < 8; ++j) {
-          uint32_t wp[8];
-          const int last = BLOCK ? be : tt;  // last column this row may see
-          if (__any_sync(0xffffffffu, j * 16 <= last)) {
-            uint32_t r[16];
-            tmem_read(tl + TM_W + j * 16, r);
-            if (__all_sync(0xffffffffu, j * 16 + 15 <= last)) {
+      for (int j = 0; j < C / MW; ++j) {
+        uint32_t wp[MW / 2];
+        // (token-causal, 32 columns: the block below the diagonal, on it or above it is the same for the whole warp)
+        const bool any = MW == 32 ? (BLOCK ? j * MW <= be : j <= wq) : __any_sync(0xffffffffu, j * MW <= be);
+        if (any) {
+          uint32_t r[MW];
+          tmem_read(tl + TM_W + j * MW, r);
+          if (MW == 32 ? (BLOCK ? j * MW + MW - 1 <= be : j < wq) : __all_sync(0xffffffffu, j * MW + MW - 1 <= be)) {
+            // all of these columns are visible to every row of this warp
 #pragma unroll
-              for (int k = 0; k < 16; k += 2) {
-                const uint32_t pk = pack_bf16(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
-                wp[k >> 1] = pk;
-                rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; k += 2) {
-                const uint32_t pk = pack_bf16(j * 16 + k <= last ? __uint_as_float(r[k]) : 0.f,
-                                              j * 16 + k + 1 <= last ? __uint_as_float(r[k + 1]) : 0.f);
-                wp[k >> 1] = pk;
-                rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
-              }
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) wp[k] = 0u;
-          }
-          tmem_st8(tl + TM_W + j * 8, wp);
-        }
-      } else {
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        uint32_t wp[16];
-        if (BLOCK ? (j * 32 <= be) : (j <= wq)) {
-          uint32_t r[32];
-          tmem_ld32(tl + TM_W + j * 32, r);
-          tmem_wait_ld();
-          if (BLOCK ? (j * 32 + 31 <= be) : (j < wq)) {
-            // the whole 32-column block is visible to every row of this warp
-#pragma unroll
-            for (int k = 0; k < 32; k += 2) {
+            for (int k = 0; k < MW; k += 2) {
               const uint32_t pk = pack_bf16(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
               wp[k >> 1] = pk;
               rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
             }
           } else {
 #pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-              const float w0 = (BLOCK ? (j * 32 + k <= be) : (k <= lane)) ? __uint_as_float(r[k]) : 0.f;
-              const float w1 = (BLOCK ? (j * 32 + k + 1 <= be) : (k + 1 <= lane)) ? __uint_as_float(r[k + 1]) : 0.f;
-              const uint32_t pk = pack_bf16(w0, w1);
+            for (int k = 0; k < MW; k += 2) {
+              const bool v0 = MW == 32 && !BLOCK ? k <= lane : j * MW + k <= be;
+              const bool v1 = MW == 32 && !BLOCK ? k + 1 <= lane : j * MW + k + 1 <= be;
+              const uint32_t pk = pack_bf16(v0 ? __uint_as_float(r[k]) : 0.f, v1 ? __uint_as_float(r[k + 1]) : 0.f);
               wp[k >> 1] = pk;
               rs2 = f2_add(rs2, f2_pack(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u)));
             }
           }
         } else {
 #pragma unroll
-          for (int k = 0; k < 16; ++k) wp[k] = 0u;
+          for (int k = 0; k < MW / 2; ++k) wp[k] = 0u;
         }
-        tmem_st16(tl + TM_W + j * 16, wp);
-      }
+        tmem_write(tl + TM_W + j * (MW / 2), wp);
       }
       tmem_wait_st();
       tc_fence_before_sync();
@@ -1343,7 +1314,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // log-sum-exp of the token's decode scores = log of the decode weights' mass in the frame kappa
       if (!SPLIT && p.lse_dec != nullptr && tt < nvalid && value_col0<ZS, SPLIT>() == 0)
         p.lse_dec[(int64_t)lane_id * p.N + t0 + tt] = (kap_i + __log2f(den)) * kLn2;
-      if constexpr (WIDE && SPLIT) {
+      if constexpr (XM) {
         if (xmerge) {
           // Two latent groups = two CTAs of a cluster.  CTA r finalises value block r: it sends its normalised
           // partial of the OTHER block (fp16) and the log2 of its weight mass into the partner's shared memory,
