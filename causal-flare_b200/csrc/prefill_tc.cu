@@ -243,12 +243,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   constexpr int ROWS = PACK ? 64 : 128;  // latent rows of the operand buffers that the products over the latents read
   constexpr int KSM = ROWS / 16;         // their 16-latent steps
   constexpr int WS = PACK ? 4 : 2;       // slots of the frame maximum's exchange
-  // The elected thread issues a chunk's products in 2 700 instead of 3 700 cycles (see elect_one).  B200, us: B=1 N=777 H=16 M=64 D=64
-  // 20.7 -> 19.4, fp16 B=4 N=4096 H=16 M=64 D=128 88.9 -> 83.6, wide block-causal B=2 N=65536 H=32 M=256 D=128 2 024 -> 1 949; whole
-  // groups at (64, 64), H=16 M=128: fp16 B=8 N=4096 99.6 -> 96.1, training B=4 N=4096 432 -> 429.  Not where
-  // products that follow one another faster only get in the way of the latent warps, which take 64 tokens a thread and are the
-  // longest chain by far (B=4 N=4096 H=8 M=128 D=128, two slices: 91.7 -> 94.1; H=16 M=192 D=64: 121.2 -> 122.4; M=96: 89.8 -> 90.2; B=8 N=8192 M=128 between 174.9 of 176.1 and 182.8 of 180.2).
-  constexpr bool ELECT = PACK || WIDE || (LAT == 0 && DKB == 1 && DVB == 1 && !SPLIT && (F16 || KEEP));
+  // The elected thread issues a chunk's products in 2 700 instead of 3 700 cycles (see elect_one).  B200, us, lane 0 -> elected, medians
+  // that move by up to 0.5 % from run to run.  Packed: B=1 N=777 H=16 M=64 D=64 20.7 -> 19.4, fp16 B=4 N=4096 H=16 M=64 D=128 88.9 ->
+  // 83.6.  Wide: block-causal B=2 N=65536 H=32 M=256 D=128 2 024 -> 1 949.  Whole groups at (64, 64), H=16 M=128: stablemax B=8 N=8192
+  // 442.9 -> 423.3, fp16 193.8 -> 187.4, bf16 175.6 -> 175.4, B=1 N=3000 36.9 -> 36.3, B=2 N=1000 H=8 27.6 -> 27.9, training B=4 N=4096
+  // 435.5 -> 428.9.  The others keep lane 0: with 64 tokens a thread the latent warps are the longest chain by far, and products that
+  // follow one another faster may get in their way as well as help them (two slices, M=128 D=128: B=4 N=4096 H=8 91.7 -> 94.4, B=1
+  // N=3000 H=16 51.1 -> 49.3; B=4 N=4096 H=16 M=192 D=64 120.8 -> 121.5, M=96 89.9 -> 90.2, M=96 D=128 96.8 -> 94.3).
+  constexpr bool ELECT = PACK || WIDE || (LAT == 0 && DKB == 1 && DVB == 1 && !SPLIT);
   constexpr int ZS = WIDE ? 1 : DVB;  // value slices on grid.z
   constexpr bool XM = WIDE && SPLIT && FL != 1;  // may merge two latent groups on chip (never in a call with lengths)
   constexpr bool BLOCK = MODE == 1, STABLE = MODE == 2;
