@@ -58,7 +58,6 @@ struct BwdTcParams {
   float scale, power;
   const float *chunk_c, *chunk_d;  // [lanes][nch][M]
   const float *tok_l2, *tok_delta;  // [lanes][npad]
-  int groups;
   // Sequence segments (grid.z = the segments from seg_first on, segment s = chunks seg_begin[s] .. seg_begin[s + 1] - 1).
   int nseg, seg_first;
   int lead;       // the CTA of a segment first walks all later chunks for their carries alone (no exchange)
@@ -71,8 +70,8 @@ struct BwdTcParams {
 };
 
 struct GradTcParams {
-  int N, H, M, B;
-  int nch, npad, groups;
+  int H, M;
+  int nch, groups;
   int nsplit, chunks_per_split;
   float scale;
   int plane, nds, nk;  // bytes of a dS plane of the ring, stages (see grad_rings)
@@ -1652,7 +1651,6 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
     p.N = f.N; p.H = f.H; p.M = f.M; p.nch = pl.nch; p.npad = pl.npad; p.block = f.block_size;
     p.scale = f.scale; p.power = f.power;
     p.chunk_c = keep.c; p.chunk_d = keep.d; p.tok_l2 = tok_l2; p.tok_delta = tok_delta;
-    p.groups = pl.groups;
     p.err = err;
     p.gate = gate;
     p.trace = trace_buffer();
@@ -1692,7 +1690,7 @@ int bwd_tc(const flare_bwd_args_t& a, cudaStream_t stream) {
   {
     GradTcParams g;
     memset(&g, 0, sizeof(g));
-    g.N = f.N; g.H = f.H; g.M = f.M; g.B = f.B; g.nch = pl.nch; g.npad = pl.npad; g.groups = pl.groups;
+    g.H = f.H; g.M = f.M; g.nch = pl.nch; g.groups = pl.groups;
     g.nsplit = pl.nsplit; g.chunks_per_split = pl.chunks_per_split; g.scale = f.scale;
     g.dq_part = reinterpret_cast<float*>(ws + pl.off_dqp);
     g.err = err;
