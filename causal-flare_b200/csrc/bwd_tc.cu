@@ -88,8 +88,12 @@ namespace {
 
 constexpr int C = 128;
 constexpr int LW = 4;                           // latent warps per lane quarter
-constexpr int NT_MAIN = (4 * LW + 4 + 3) * 32;  // latent warps, token warps, MMA issuer, TMA producer, dS stores
-constexpr int W_TOKEN = 4 * LW, W_MMA = 4 * LW + 4, W_TMA = 4 * LW + 5, W_OUT = 4 * LW + 6;  // first token warp, issuer, producer, dS stores
+// Latent warps, token warps, MMA issuer, TMA producer, dS stores: six warps on a scheduler, 80 registers a thread, and the latent warps
+// spill.  Bytes of spill stores, softmax / block-causal / stablemax, at (Dk, Dv) = (64, 64) 132 / 44 / 128, (128, 128) 212 / 132 / 232,
+// (64, 128) 200 / 144 / 220; packed 4 / 0 / 4, 56 / 48 / 64, 12 / 52 / 16.  (With dS and dV stored by their threads, at the same 80
+// registers, the packed ones spilled at most 12 and the others up to 188; the kernel with tiles is the faster one all the same.)
+constexpr int NT_MAIN = (4 * LW + 4 + 3) * 32;
+constexpr int W_TOKEN = 4 * LW, W_MMA = 4 * LW + 4, W_TMA = 4 * LW + 5, W_OUT = 4 * LW + 6;  // (W_TOKEN: the first of four)
 constexpr float kLog2e = 1.4426950408889634f;
 
 // shared memory map of the main kernel (bytes; every operand buffer 1024-aligned for the 128B swizzle)
@@ -98,8 +102,13 @@ struct BL {
   static constexpr int OFF_KA = 0;                      // K tile [DKB][128 t][64]; later the masked A [2][128 tau][64 t]
   static constexpr int OFF_V = 32768;                   // [DVB][128 t][64]
   static constexpr int OFF_DY = OFF_V + DVB * 16384;    // [DVB][128 t][64]
-  static constexpr int OFF_UR = OFF_DY + DVB * 16384;   // U_i [DVB][128 m][64] (the 32 KB slot keeps every buffer behind it 1024-aligned for both widths)
+  // U_i [DVB][128 m][64], and the chunk's dV rows on their way out, DV / 32 tiles of 32 x 32 for each of the four token warps:
+  // at Dv = 64 behind U_i, at Dv = 128 in its place
+  static constexpr int OFF_UR = OFF_DY + DVB * 16384;
+  static constexpr int DV_TILES = DVB * 2 * 2048;  // bytes of a token warp's tiles
+  static constexpr int OFF_DVT = OFF_UR + (DVB == 1 ? 16384 : 0);
   static constexpr int OFF_GC = OFF_UR + 32768;         // G as bf16 [DVB][128 m][64]
+  static_assert(OFF_DVT + 4 * DV_TILES <= OFF_GC && OFF_DVT % 1024 == 0, "tiles of dV");
   static constexpr int OFF_E = OFF_GC + DVB * 16384;    // [2 t-blocks][128 m][64 t]
   static constexpr int OFF_R = OFF_E + 32768;
   static constexpr int OFF_MISC = OFF_R + 32768;
@@ -702,9 +711,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           rp_later += t > tp ? x : 0.f;
         }
 
-        // ---- phase 2b (descending): encoder part, dS rows to global memory as a hi + lo pair
+        // ---- phase 2b (descending): encoder part, dS as a hi + lo pair into the tiles that the store warp sends off
         if (i < full_end) {
-          // dS may be laid down: see above
+          // dS may be laid down (where E and R were, see the top of the kernel)
           if (!(ok = PACK ? wait_or_abort(&misc->g_ready, par, misc) : wait_or_abort(&misc->dv_ready, par, misc))) break;
           float ccg[NG];  // block-causal: Cc + sum of R p from the start of the group's block on
           float cc = cc_carry + rp_later;
@@ -832,7 +841,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const uint32_t tl = tmem + ((uint32_t)(wq * 32) << 16);
     const int tt = wq * 32 + lane;
     const int lo = BLOCK ? (tt & ~(p.block - 1)) : tt;  // first column (token) this row keeps
-    uint8_t* const dv_stage = smem + L::OFF_UR + (DVB == 2 ? wq * 8192 : 16384 + wq * 4096);  // this warp's tiles of the dV rows
+    uint8_t* const dv_stage = smem + L::OFF_DVT + wq * L::DV_TILES;  // this warp's tiles of the dV rows
     for (int j = 0; ok && j < steps; ++j) {
       const int i = first - 1 - j, t0 = i * C;
       const uint32_t par = j & 1, fpar = (j - (first - full_end)) & 1;

@@ -1172,62 +1172,61 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if constexpr (XM) {
         const int t0 = seg_begin + i * C, nvalid = min(C, seg_end - t0);
         const uint32_t rank = cluster_ctarank();
-                  if (!(ok = tc::wait_or_abort_cluster(&misc->xfull[wq], i & 1, &misc->abort_flag))) return;
-                  const float lw_p = *reinterpret_cast<const float*>(smem + L::OFF_XCH + 16384 + tt * 4);
-                  uint4 xp[8];
-        #pragma unroll
-                  for (int ch = 0; ch < 8; ++ch)  // [warp][32-column half][32 rows x 64 bytes, 16-byte pieces swizzled as in the staging tile]
-                    xp[ch] = *reinterpret_cast<const uint4*>(smem + L::OFF_XCH + wq * 4096 + (ch >> 2) * 2048 + lane * 64 +
-                                                             (((ch & 3) ^ ((lane >> 1) & 3)) << 4));
-                  const float mx = fmaxf(lw_own, lw_p);
-                  float ca = 0.f, cb = 0.f;  // coefficients of the raw accumulator values and of the partner's normalised rows
-                  if (mx == -INFINITY) {
-                    // every group's weights underflowed: outside the numeric domain of this path
-                    if (rank == 0 && tt < nvalid) {
-                      atomicOr(p.err, 2);
-                      misc->out_of_domain = 1;
-                    }
-                  } else {
-                    const float wa = ex2_approx(lw_own - mx), wb = ex2_approx(lw_p - mx);
-                    const float iw = rcp_approx(wa + wb);
-                    ca = wa * iw * inv_own;
-                    cb = wb * iw;
-                    if (rank == 0 && p.lse_dec != nullptr && tt < nvalid)
-                      p.lse_dec[(int64_t)lane_id * p.N + t0 + tt] = (mx + __log2f(wa + wb)) * kLn2;
-                  }
-                  // The merged rows go out from the exchange tile itself (its layout is the bulk store's 64-byte swizzle and
-                  // the partner's rows are in registers by now): both 32-column tiles are stored without waiting on each other.
-                  uint8_t* const xt = smem + L::OFF_XCH + wq * 4096;
-        #pragma unroll
-                  for (int half = 0; half < 2; ++half) {
-                    const uint32_t(&r)[32] = own[half];
-        #pragma unroll
-                    for (int ch = 0; ch < 4; ++ch) {
-                      const uint4 x = xp[half * 4 + ch];
-                      const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
-                      uint32_t o[4];
-                      float y[8];
-        #pragma unroll
-                      for (int j = 0; j < 4; ++j) {
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[j]));
-                        // own raw values * ca + partner's normalised values * cb, two columns per instruction
-                        f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
-                                         f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
-                      }
-                      pack_out(y, F16, o);
-                      *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
-                          make_uint4(o[0], o[1], o[2], o[3]);
-                    }
-                  }
-                  fence_proxy_async_smem();
-                  __syncwarp();
-                  if (lane == 0) {
-                    tma_store_4d(&tm_y, xt, (int)rank * 64, h, t0 + wq * 32, b);
-                    tma_store_4d(&tm_y, xt + 2048, (int)rank * 64 + 32, h, t0 + wq * 32, b);
-                    bulk_commit_group();
-                  }
-                  // (the partner learns that the tile is free when the next chunk's epilogue begins, see above: by then the
-                  // stores have long read it; it does not send before its own next epilogue anyway)
+        if (!(ok = tc::wait_or_abort_cluster(&misc->xfull[wq], i & 1, &misc->abort_flag))) return;
+        const float lw_p = *reinterpret_cast<const float*>(smem + L::OFF_XCH + 16384 + tt * 4);
+        uint4 xp[8];
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch)  // [warp][32-column half][32 rows x 64 bytes, 16-byte pieces swizzled as in the staging tile]
+          xp[ch] = *reinterpret_cast<const uint4*>(smem + L::OFF_XCH + wq * 4096 + (ch >> 2) * 2048 + lane * 64 +
+                                                   (((ch & 3) ^ ((lane >> 1) & 3)) << 4));
+        const float mx = fmaxf(lw_own, lw_p);
+        float ca = 0.f, cb = 0.f;  // coefficients of the raw accumulator values and of the partner's normalised rows
+        if (mx == -INFINITY) {
+          // every group's weights underflowed: outside the numeric domain of this path
+          if (rank == 0 && tt < nvalid) {
+            atomicOr(p.err, 2);
+            misc->out_of_domain = 1;
+          }
+        } else {
+          const float wa = ex2_approx(lw_own - mx), wb = ex2_approx(lw_p - mx);
+          const float iw = rcp_approx(wa + wb);
+          ca = wa * iw * inv_own;
+          cb = wb * iw;
+          if (rank == 0 && p.lse_dec != nullptr && tt < nvalid)
+            p.lse_dec[(int64_t)lane_id * p.N + t0 + tt] = (mx + __log2f(wa + wb)) * kLn2;
+        }
+        // The merged rows go out from the exchange tile itself (its layout is the bulk store's 64-byte swizzle and
+        // the partner's rows are in registers by now): both 32-column tiles are stored without waiting on each other.
+        uint8_t* const xt = smem + L::OFF_XCH + wq * 4096;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t(&r)[32] = own[half];
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            const uint4 x = xp[half * 4 + ch];
+            const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+            uint32_t o[4];
+            float y[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[j]));
+              // own raw values * ca + partner's normalised values * cb, two columns per instruction
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(r[ch * 8 + 2 * j]), __uint_as_float(r[ch * 8 + 2 * j + 1])),
+                               f2_pack(ca, ca), f2_mul(f2_pack(f.x, f.y), f2_pack(cb, cb))), y[2 * j], y[2 * j + 1]);
+            }
+            pack_out(y, F16, o);
+            *reinterpret_cast<uint4*>(xt + half * 2048 + lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4)) =
+                make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_4d(&tm_y, xt, (int)rank * 64, h, t0 + wq * 32, b);
+          tma_store_4d(&tm_y, xt + 2048, (int)rank * 64 + 32, h, t0 + wq * 32, b);
+          bulk_commit_group();
+        }
+        // (the partner learns that the tile is free in the epilogue of the chunk in flight, which waits for these stores to have read it)
       }
     };
     for (int i = 0; !state_only && ok && i < nchunks; ++i) {
